@@ -1,26 +1,33 @@
 // Packed variable-length causal GQA attention, backward, for sm_100a.
 //
-// Two tcgen05 kernels, neither of which needs atomics:
+// Two tcgen05 kernels, neither of which needs atomics, so every gradient is the same each time:
 //
 //   dQ kernel   one CTA per (128-query tile, query head); streams K/V tiles.
 //               S = Q K^T and dP = dO V^T land in TMEM, the softmax warps form
-//               dS = P o (dP - delta) * scale as a swizzled smem operand, and
-//               dQ += dS K accumulates in TMEM.
-//   dKV kernel  one CTA per (128-key tile, KV head); streams the 64-query tiles
+//               dS = P o (dP - delta) and dQ += dS K accumulates in TMEM.
+//   dKV kernel  one CTA per (128-key tile, KV head); streams the query tiles
 //               of every query head of the group. S^T = K Q^T and dP^T = V dO^T
-//               (keys on TMEM lanes), P^T and dS^T go to shared memory, and
-//               dV += P^T dO, dK += dS^T Q accumulate in TMEM across tiles and
-//               across the heads of the GQA group.
+//               (keys on TMEM lanes); dV += P^T dO and dK += dS^T Q accumulate in
+//               TMEM across tiles and across the heads of the GQA group.
+//
+// P^T, dS^T and dS go back to TMEM and are the A operand of their products there. A 128-row product
+// reads A and B from shared memory at the full rate of that memory when both are there, and the 64-row
+// tiles of K, V, Q or dO that an operand in shared memory left room for need 1.5 times that rate; with
+// these operands in TMEM the tiles have 128 rows (64 for head width 256) and half of the products read
+// only B.
 //
 // For head width 256 the dK and dV accumulators do not fit TMEM together with
 // the score buffers, so the dKV kernel runs twice (dV only, then dK only).
 // delta[h,t] = sum_d dO*O comes from a small preprocess kernel into caller
 // scratch (fp32 [Hq, T]).
 //
-// warps 0..7 softmax: warp w owns TMEM lanes 32*(w%4)..+31 and the 32-column half w/4 of
-// every score tile, so two warps per scheduler hide each other's TMEM-load and exp latency;
-// warp 8 TMA producer, warp 9 MMA.
+// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: dQ 2.42 -> 1.25 ms, dKV 3.15 -> 1.69 ms
+// against P^T and dS through shared memory in 64-row tiles.
+//
+// warps 0..7 softmax: warp w owns TMEM lanes 32*(w%4)..+31 and the left or right half (w/4) of
+// every score tile; warp 8 TMA producer, warp 9 MMA, warp 10 row statistics (dKV kernel).
 #include "sm100_ptx.cuh"
+#include "attention_tiles.cuh"
 
 #include <cudaTypedefs.h>
 #include <math.h>
@@ -30,8 +37,8 @@ namespace ss {
 int make_tmap_bf16(CUtensorMap* map, const void* base, long long rows, long long cols,
                    long long ld, int box_rows);
 
-constexpr int BW_THREADS = 320;
-constexpr int BW_TMA_WARP = 8, BW_MMA_WARP = 9;
+constexpr int BW_THREADS = 352;
+constexpr int BW_TMA_WARP = 8, BW_MMA_WARP = 9, BW_STAT_WARP = 10;
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct AttnBwdParams {
@@ -44,38 +51,6 @@ struct AttnBwdParams {
   float scale;
   int* status;
 };
-
-__device__ __forceinline__ bool find_tile128(const int* cu, int nseq, int tile, int& seq_start,
-                                             int& seq_end, int& r0) {
-  int acc = 0;
-  for (int s = 0; s < nseq; ++s) {
-    const int b = cu[s], e = cu[s + 1];
-    const int nt = (e - b + 127) / 128;
-    if (tile < acc + nt) {
-      seq_start = b; seq_end = e; r0 = b + (tile - acc) * 128;
-      return true;
-    }
-    acc += nt;
-  }
-  return false;
-}
-
-// Writes 32 consecutive bf16 columns [kcol, kcol+32) of row `row` into a
-// K-major 128B-swizzled tile whose 64-column boxes are `box_bytes` apart.
-__device__ __forceinline__ void store_swizzled_32(uint8_t* tile, int box_bytes, int row, int kcol,
-                                                  const uint32_t (&pk)[16]) {
-  uint8_t* box = tile + (kcol >> 6) * box_bytes + row * 128;
-#pragma unroll
-  for (int q8 = 0; q8 < 4; ++q8) {
-    const int chunk = ((kcol & 63) >> 3) + q8;
-    uint4 v = make_uint4(pk[q8 * 4], pk[q8 * 4 + 1], pk[q8 * 4 + 2], pk[q8 * 4 + 3]);
-    *reinterpret_cast<uint4*>(box + ((chunk ^ (row & 7)) << 4)) = v;
-  }
-}
-
-__device__ __forceinline__ void named_barrier_softmax() {
-  asm volatile("bar.sync 1, 256;" ::: "memory");
-}
 
 // ============================================================================ preprocess
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out,
@@ -98,66 +73,111 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out,
   if (lane == 0) delta[static_cast<long long>(h) * T + t] = acc;
 }
 
+// ============================================================================ TMEM operands
+// P^T, dS^T and dS go back into the TMEM columns of the scores they come from: the two warps of a
+// lane quarter own the left and the right half of a score tile, and each packs its half into the
+// first half of its own columns, so neither overwrites columns that the other still has to read.
+// Column offset of the 16-element step kk of such an operand whose score tile has BN columns:
+template <int BN>
+__device__ __forceinline__ constexpr uint32_t packed_col(int kk) {
+  return (kk * 16) / (BN / 2) * (BN / 2) + ((kk * 16) % (BN / 2)) / 2;
+}
+
+// An explicit shared-memory load: through the aligned-up window pointer the compiler only sees a
+// generic address, whose loads take the global path (they were most of the dKV kernel's stalls).
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+
+__device__ __forceinline__ void st_shared_f32(uint32_t addr, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+
+template <int HN>   // HN score columns per warp: 64 or 32
+__device__ __forceinline__ void tmem_ld_half(uint32_t addr, uint32_t (&r)[HN]) {
+#pragma unroll
+  for (int c = 0; c < HN; c += 32) tmem_ld_32x32(addr + c, reinterpret_cast<uint32_t (&)[32]>(r[c]));
+  tmem_ld_wait();
+}
+template <int HN>
+__device__ __forceinline__ void tmem_st_half(uint32_t addr, const uint32_t (&pk)[HN / 2]) {
+  if constexpr (HN == 64) tmem_st_32x32(addr, pk);
+  else tmem_st_32x16(addr, pk);
+  tmem_st_wait();
+}
+
 // ============================================================================ dQ kernel
-template <int DH, int BKV, int KVS>
+// S is double-buffered and dP single: S of the next tile is formed under this tile's
+// exponentials, dP of the next tile under this tile's dS. K is released by the dQ product and has
+// KS stages, V already by the dP product and has VS.
+template <int DH, int BKV, int KS, int VS>
 struct DqCfg {
   static constexpr int Q_BYTES = 128 * DH * 2;
   static constexpr int KV_BYTES = BKV * DH * 2;
-  static constexpr int DS_BYTES = 128 * BKV * 2;
   static constexpr int OFF_DO = Q_BYTES;
   static constexpr int OFF_K = 2 * Q_BYTES;
-  static constexpr int OFF_V = OFF_K + KVS * KV_BYTES;
-  static constexpr int OFF_DS = OFF_V + KVS * KV_BYTES;
-  static constexpr int OFF_BAR = OFF_DS + 2 * DS_BYTES;   // dS is double-buffered
+  static constexpr int OFF_V = OFF_K + KS * KV_BYTES;
+  static constexpr int OFF_BAR = OFF_V + VS * KV_BYTES;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
-  static constexpr int TM_S = 0, TM_DP = 2 * BKV, TM_DQ = 4 * BKV;
+  static constexpr int TM_S = 0, TM_DP = 2 * BKV, TM_DQ = 3 * BKV;
   static_assert(TM_DQ + DH <= 512, "TMEM budget");
+  static_assert(SMEM <= 232448, "shared memory budget");
 };
 
-template <int DH, int BKV, int KVS>
+template <int DH, int BKV, int KS, int VS>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const AttnBwdParams p) {
-  using Cfg = DqCfg<DH, BKV, KVS>;
+  using Cfg = DqCfg<DH, BKV, KS, VS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* qdo_full = bars;            // 1
-  uint64_t* kv_full = bars + 1;         // 2
-  uint64_t* kv_empty = bars + 3;        // 2
-  uint64_t* sdp_full = bars + 5;        // 2
-  uint64_t* sdp_free = bars + 7;        // 2
-  uint64_t* ds_full = bars + 9;         // 2
-  uint64_t* dq_done = bars + 11;        // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* k_full = bars + 1;          // 3
+  uint64_t* k_empty = bars + 4;         // 3
+  uint64_t* v_full = bars + 7;          // 2
+  uint64_t* v_empty = bars + 9;         // 2
+  uint64_t* s_full = bars + 11;         // 2
+  uint64_t* dp_full = bars + 13;        // 1
+  uint64_t* dp_free = bars + 14;        // 1
+  uint64_t* ds_full = bars + 15;        // 1
+  uint64_t* dq_done = bars + 16;        // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 19);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.y;
+  const int head = blockIdx.x;
   const int kv_head = head / (p.Hq / p.Hkv);
-  int seq_start, seq_end, q0;
-  if (!find_tile128(p.cu_seqlens, p.nseq, blockIdx.x, seq_start, seq_end, q0)) return;
-  const int q_hi = min(q0 + 128, seq_end);
-  const int n_kv = (q_hi - seq_start + BKV - 1) / BKV;
 
   if (threadIdx.x == 0) {
     mbar_init(qdo_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1);
-      mbar_init(&sdp_full[i], 1); mbar_init(&sdp_free[i], 8);
-      mbar_init(&ds_full[i], 8); mbar_init(&dq_done[i], 1);
-    }
+    for (int i = 0; i < KS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
+    for (int i = 0; i < VS; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) mbar_init(&s_full[i], 1);
+    mbar_init(dp_full, 1);
+    mbar_init(dp_free, 8);
+    mbar_init(ds_full, 8);
+    mbar_init(dq_done, 1);
     mbar_fence_init();
   }
+  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
   if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const int seq_start = slot->seq_start, seq_end = slot->seq_end;
+  const int q0 = seq_start + (slot->work - 1) * 128;
+  const int q_hi = min(q0 + 128, seq_end);
+  const int n_kv = slot->work > 0 ? (q_hi - seq_start + BKV - 1) / BKV : 0;
 
   if (warp == BW_TMA_WARP) {
-    if (elect_one()) {
+    if (n_kv > 0 && elect_one()) {
       mbar_expect_tx(qdo_full, 2 * Cfg::Q_BYTES);
 #pragma unroll
       for (int c = 0; c < DH / 64; ++c) {
@@ -165,137 +185,118 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tma_load_2d(smem + Cfg::OFF_DO + c * (128 * 128), &tmDO, qdo_full, head * DH + c * 64, q0);
       }
       for (int j = 0; j < n_kv; ++j) {
-        const int st = j % KVS;
-        if (j >= KVS && !mbar_wait(&kv_empty[st], ((j / KVS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY))
-          break;
-        uint8_t* sk = smem + Cfg::OFF_K + st * Cfg::KV_BYTES;
-        uint8_t* sv = smem + Cfg::OFF_V + st * Cfg::KV_BYTES;
-        mbar_expect_tx(&kv_full[st], 2 * Cfg::KV_BYTES);
+        const int ks = j % KS, vs = j % VS;
         const int k0 = seq_start + j * BKV;
+        if (j >= KS && !mbar_wait(&k_empty[ks], ((j / KS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* sk = smem + Cfg::OFF_K + ks * Cfg::KV_BYTES;
+        mbar_expect_tx(&k_full[ks], Cfg::KV_BYTES);
 #pragma unroll
-        for (int c = 0; c < DH / 64; ++c) {
-          tma_load_2d(sk + c * (BKV * 128), &tmK, &kv_full[st], kv_head * DH + c * 64, k0);
-          tma_load_2d(sv + c * (BKV * 128), &tmV, &kv_full[st], kv_head * DH + c * 64, k0);
-        }
+        for (int c = 0; c < DH / 64; ++c)
+          tma_load_2d(sk + c * (BKV * 128), &tmK, &k_full[ks], kv_head * DH + c * 64, k0);
+        if (j >= VS && !mbar_wait(&v_empty[vs], ((j / VS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* sv = smem + Cfg::OFF_V + vs * Cfg::KV_BYTES;
+        mbar_expect_tx(&v_full[vs], Cfg::KV_BYTES);
+#pragma unroll
+        for (int c = 0; c < DH / 64; ++c)
+          tma_load_2d(sv + c * (BKV * 128), &tmV, &v_full[vs], kv_head * DH + c * 64, k0);
       }
     }
   } else if (warp == BW_MMA_WARP) {
-    if (elect_one()) {
+    if (n_kv > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, DH, false, true);
       const uint32_t sq = smem_u32(smem), sdo = smem_u32(smem + Cfg::OFF_DO);
-      const uint32_t sds = smem_u32(smem + Cfg::OFF_DS);
-      bool ok = mbar_wait(qdo_full, 0, p.status, KS_TIMEOUT_FULL);
-      auto issue_sdp = [&](int j) {
-        const int b = j & 1, st = j % KVS;
-        const uint32_t sk = smem_u32(smem + Cfg::OFF_K + st * Cfg::KV_BYTES);
-        const uint32_t sv = smem_u32(smem + Cfg::OFF_V + st * Cfg::KV_BYTES);
+      const uint32_t sk0 = smem_u32(smem + Cfg::OFF_K), sv0 = smem_u32(smem + Cfg::OFF_V);
+      auto scores = [&](uint32_t d, uint32_t a, uint32_t b) {
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint32_t ao = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
-          const uint32_t bo = (kk >> 2) * (BKV * 128) + (kk & 3) * 32;
-          umma_bf16(tmem_base + Cfg::TM_S + b * BKV, umma_smem_desc(sq + ao, 16, 1024),
-                    umma_smem_desc(sk + bo, 16, 1024), idesc_s, kk != 0);
-        }
-#pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint32_t ao = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
-          const uint32_t bo = (kk >> 2) * (BKV * 128) + (kk & 3) * 32;
-          umma_bf16(tmem_base + Cfg::TM_DP + b * BKV, umma_smem_desc(sdo + ao, 16, 1024),
-                    umma_smem_desc(sv + bo, 16, 1024), idesc_s, kk != 0);
-        }
-        umma_commit(&sdp_full[b]);
+        for (int kk = 0; kk < DH / 16; ++kk)
+          umma_bf16(d, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
+                    umma_smem_desc(b + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
       };
-      auto prefetch_next = [&](int j) -> bool {   // issue S/dP of tile j+1
-        const int jn = j + 1, b = jn & 1;
-        if (!mbar_wait(&kv_full[jn % KVS], (jn / KVS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
-        if (jn >= 2 && !mbar_wait(&sdp_free[b], ((jn >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY))
-          return false;
+      auto issue_s = [&](int j) -> bool {
+        if (!mbar_wait(&k_full[j % KS], (j / KS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        issue_sdp(jn);
+        scores(tmem_base + Cfg::TM_S + (j & 1) * BKV, sq, sk0 + (j % KS) * Cfg::KV_BYTES);
+        umma_commit(&s_full[j & 1]);
         return true;
       };
-      if (ok) ok = mbar_wait(&kv_full[0], 0, p.status, KS_TIMEOUT_FULL);
-      if (ok) { tc_fence_after(); issue_sdp(0); }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        if (KVS >= 2 && j + 1 < n_kv) { ok = prefetch_next(j); if (!ok) break; }
-        ok = mbar_wait(&ds_full[j & 1], (j >> 1) & 1, p.status, KS_TIMEOUT_FULL);
-        if (!ok) break;
+      auto issue_dp = [&](int j) -> bool {
+        if (!mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
+        if (j > 0 && !mbar_wait(dp_free, (j - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) return false;
         tc_fence_after();
-        const uint32_t sk = smem_u32(smem + Cfg::OFF_K + (j % KVS) * Cfg::KV_BYTES);
-        const uint32_t sdsj = sds + (j & 1) * Cfg::DS_BYTES;
+        scores(tmem_base + Cfg::TM_DP, sdo, sv0 + (j % VS) * Cfg::KV_BYTES);
+        umma_commit(dp_full);
+        umma_commit(&v_empty[j % VS]);
+        return true;
+      };
+      bool ok = mbar_wait(qdo_full, 0, p.status, KS_TIMEOUT_FULL) && issue_s(0) && issue_dp(0);
+      for (int j = 0; j < n_kv && ok; ++j) {
+        // S of the next tile goes to the buffer whose dS the dQ product before this point reads:
+        // products of one issuing thread run in order
+        if (j + 1 < n_kv) ok = issue_s(j + 1) && issue_dp(j + 1);
+        if (!ok || !mbar_wait(ds_full, j & 1, p.status, KS_TIMEOUT_FULL)) break;
+        tc_fence_after();
+        const uint32_t sk = sk0 + (j % KS) * Cfg::KV_BYTES;
+        const uint32_t ds = tmem_base + Cfg::TM_S + (j & 1) * BKV;
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint64_t ad = umma_smem_desc(sdsj + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = umma_smem_desc(sk + kk * (16 * 128), BKV * 128, 1024);
-          umma_bf16(tmem_base + Cfg::TM_DQ, ad, bd, idesc_dq, (j | kk) != 0);
-        }
-        umma_commit(&kv_empty[j % KVS]);
-        umma_commit(&dq_done[j & 1]);
-        if (KVS < 2 && j + 1 < n_kv) { ok = prefetch_next(j); }
+        for (int kk = 0; kk < BKV / 16; ++kk)
+          umma_bf16_ts(tmem_base + Cfg::TM_DQ, ds + packed_col<BKV>(kk),
+                       umma_smem_desc(sk + kk * (16 * 128), BKV * 128, 1024), idesc_dq, (j | kk) != 0);
+        umma_commit(&k_empty[j % KS]);
+        if (j + 1 == n_kv) umma_commit(dq_done);
       }
     }
-  } else {
-    const int quarter = warp & 3, hsel = warp >> 2;
+  } else if (warp < 8) {
+    constexpr int HN = BKV / 2;
+    const int quarter = warp & 3, half = warp >> 2;
     const int row = quarter * 32 + lane;
     const int gq = q0 + row;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const long long li = static_cast<long long>(head) * p.T + min(gq, p.T - 1);
-    const float lse2 = p.lse[li] * LOG2E;
+    const uint32_t dp_addr = lane_addr + Cfg::TM_DP + half * HN;
+    const long long li = static_cast<long long>(head) * p.T + max(0, min(gq, p.T - 1));
+    const float nlse = -p.lse[li] * LOG2E;
     const float dl = p.delta[li];
     const float c2 = p.scale * LOG2E;
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
       const int b = j & 1;
-      uint8_t* sds = smem + Cfg::OFF_DS + b * Cfg::DS_BYTES;
-      if (!mbar_wait(&sdp_full[b], (j >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-      // this dS buffer was last read by the dQ MMAs of tile j-2
-      if (j > 1 && !mbar_wait(&dq_done[b], ((j >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      const uint32_t s_addr = lane_addr + Cfg::TM_S + b * BKV + half * HN;
+      if (!mbar_wait(&s_full[b], (j >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const int k0 = seq_start + j * BKV;
-      const bool below_diagonal = k0 + BKV - 1 <= q0;   // every key of the tile is visible to every row
-#pragma unroll 1
-      for (int c = hsel; c < BKV / 32; c += 2) {
-        uint32_t s[32], d[32];
-        tmem_ld_32x32(lane_addr + Cfg::TM_S + b * BKV + c * 32, s);
-        tmem_ld_32x32(lane_addr + Cfg::TM_DP + b * BKV + c * 32, d);
-        tmem_ld_wait();
-        uint32_t pk[16];
-        if (below_diagonal) {
+      uint32_t s[HN];
+      tmem_ld_half<HN>(s_addr, s);
+      const int k0 = seq_start + j * BKV + half * HN;
+      if (k0 + HN - 1 <= q0) {                     // every key of this half is visible to every row
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float p0 = fast_exp2(fmaf(__uint_as_float(s[e]), c2, -lse2));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(s[e + 1]), c2, -lse2));
-            pk[e >> 1] = pack_bf16(p0 * (__uint_as_float(d[e]) - dl),
-                                   p1 * (__uint_as_float(d[e + 1]) - dl));
-          }
-        } else {
+        for (int e = 0; e < HN; ++e) s[e] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, nlse)));
+      } else {
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            float v[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int gk = k0 + c * 32 + e + u;
-              const float pr = (gk > gq) ? 0.f : fast_exp2(fmaf(__uint_as_float(s[e + u]), c2, -lse2));
-              v[u] = pr * (__uint_as_float(d[e + u]) - dl);   // the softmax scale is applied to dQ once
-            }
-            pk[e >> 1] = pack_bf16(v[0], v[1]);
-          }
-        }
-        store_swizzled_32(sds, 128 * 128, row, c * 32, pk);
+        for (int e = 0; e < HN; ++e)
+          s[e] = k0 + e > gq ? 0u : __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, nlse)));
       }
+      if (!mbar_wait(dp_full, j & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t d[HN];
+      tmem_ld_half<HN>(dp_addr, d);
       tc_fence_before();
-      fence_async_proxy();
       __syncwarp();
-      if (lane == 0) { mbar_arrive(&sdp_free[b]); mbar_arrive(&ds_full[b]); }
+      if (lane == 0) mbar_arrive(dp_free);
+      uint32_t pk[HN / 2];
+#pragma unroll
+      for (int e = 0; e < HN; e += 2)             // the softmax scale is applied to dQ once, at the end
+        pk[e >> 1] = pack_bf16(__uint_as_float(s[e]) * (__uint_as_float(d[e]) - dl),
+                               __uint_as_float(s[e + 1]) * (__uint_as_float(d[e + 1]) - dl));
+      tmem_st_half<HN>(s_addr, pk);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
     }
-    if (ok && n_kv > 0 && mbar_wait(&dq_done[(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, p.status,
-                                    KS_TIMEOUT_TMEM_FULL)) {
+    if (ok && n_kv > 0 && mbar_wait(dq_done, 0, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.dq) +
                             static_cast<long long>(gq) * p.ldq + head * DH;
 #pragma unroll 1
-      for (int c = hsel; c < DH / 32; c += 2) {
+      for (int c = half; c < DH / 32; c += 2) {
         uint32_t r[32];
         tmem_ld_32x32(lane_addr + Cfg::TM_DQ + c * 32, r);
         tmem_ld_wait();
@@ -320,38 +321,42 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 }
 
 // ============================================================================ dKV kernel
+// dV and dK together: one buffer each for S^T and dP^T; the products of a tile are ordered so that the tensor pipe
+// always has work while the softmax warps do theirs:
+//   softmax warps   P^T of tile i                 dS^T of tile i
+//   tensor pipe     dK of tile i-1, dP^T of i     dV of tile i, S^T of tile i+1
+// dK alone follows the same order without P^T; dV alone has no second phase to hide S^T under and
+// keeps two buffers of it instead.
 enum { MODE_BOTH = 0, MODE_DV = 1, MODE_DK = 2 };
 
-template <int DH, int QS, int MODE>
+template <int DH, int BQ, int QS, int DOS, int MODE>
 struct DkvCfg {
-  static constexpr int BQ = 64;
-  static constexpr bool NEED_DP = MODE != MODE_DV;
   static constexpr bool DO_DV = MODE != MODE_DK;
   static constexpr bool DO_DK = MODE != MODE_DV;
+  static constexpr int SB = MODE == MODE_DV ? 2 : 1;       // buffers of S^T
+  static constexpr int STS = DH == 256 ? 2 : 4;           // stages of the row statistics
   static constexpr int K_BYTES = 128 * DH * 2;
   static constexpr int QT_BYTES = BQ * DH * 2;
-  static constexpr int PT_BYTES = 128 * BQ * 2;
   static constexpr int OFF_V = K_BYTES;
-  static constexpr int OFF_Q = OFF_V + (NEED_DP ? K_BYTES : 0);
+  static constexpr int OFF_Q = OFF_V + (DO_DK ? K_BYTES : 0);
   static constexpr int OFF_DO = OFF_Q + QS * QT_BYTES;
-  static constexpr int OFF_PT = OFF_DO + QS * QT_BYTES;
-  static constexpr int OFF_DST = OFF_PT + (DO_DV ? 2 * PT_BYTES : 0);   // P^T, dS^T double-buffered
-  static constexpr int OFF_LSE = OFF_DST + (DO_DK ? 2 * PT_BYTES : 0);
-  static constexpr int OFF_BAR = OFF_LSE + 2 * 2 * BQ * 4;
+  static constexpr int OFF_STAT = OFF_DO + DOS * QT_BYTES;
+  static constexpr int OFF_BAR = OFF_STAT + STS * 2 * BQ * 4;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
-  static constexpr int TM_ST = 0, TM_DPT = 2 * BQ;
-  static constexpr int TM_ACC0 = NEED_DP ? 4 * BQ : 2 * BQ;   // dK (or dV in MODE_DV)
-  static constexpr int TM_ACC1 = TM_ACC0 + DH;                // dV in MODE_BOTH
-  static_assert((MODE == MODE_BOTH ? TM_ACC1 + DH : TM_ACC0 + DH) <= 512, "TMEM budget");
+  static constexpr int TM_ST = 0, TM_DPT = SB * BQ;
+  static constexpr int TM_DV = 2 * BQ;
+  static constexpr int TM_DK = TM_DV + (DO_DV ? DH : 0);
+  static_assert(TM_DK + (DO_DK ? DH : 0) <= 512, "TMEM budget");
+  static_assert(SMEM <= 232448, "shared memory budget");
 };
 
-template <int DH, int QS, int MODE>
+template <int DH, int BQ, int QS, int DOS, int MODE>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const AttnBwdParams p) {
-  using Cfg = DkvCfg<DH, QS, MODE>;
-  constexpr int BQ = Cfg::BQ;
+  using Cfg = DkvCfg<DH, BQ, QS, DOS, MODE>;
+  constexpr int STS = Cfg::STS, SB = Cfg::SB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -359,212 +364,244 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* kv_full = bars;             // 1
   uint64_t* q_full = bars + 1;          // 2
   uint64_t* q_empty = bars + 3;         // 2
-  uint64_t* sp_full = bars + 5;         // 2
-  uint64_t* sp_free = bars + 7;         // 2
-  uint64_t* pds_full = bars + 9;        // 2
-  uint64_t* acc_done = bars + 11;       // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
-  float* s_lse = reinterpret_cast<float*>(smem + Cfg::OFF_LSE);   // [2][2][BQ]: lse2, delta
+  uint64_t* do_full = bars + 5;         // 2
+  uint64_t* do_empty = bars + 7;        // 2
+  uint64_t* stat_full = bars + 9;       // 4
+  uint64_t* stat_empty = bars + 13;     // 4
+  uint64_t* s_full = bars + 17;         // 2
+  uint64_t* p_full = bars + 19;         // 1
+  uint64_t* dp_full = bars + 20;        // 1
+  uint64_t* ds_full = bars + 21;        // 1
+  uint64_t* s_free = bars + 22;         // 1 (only without a P^T to wait for)
+  uint64_t* acc_done = bars + 23;       // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 25);
+  float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), delta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv_head = blockIdx.y;
+  const int kv_head = blockIdx.x;
   const int rep = p.Hq / p.Hkv;
-  int seq_start, seq_end, k0;
-  if (!find_tile128(p.cu_seqlens, p.nseq, blockIdx.x, seq_start, seq_end, k0)) return;
-  const int n_q = (seq_end - k0 + BQ - 1) / BQ;     // query tiles at or after the key tile
-  const int n_it = rep * n_q;
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1);
-      mbar_init(&sp_full[i], 1); mbar_init(&sp_free[i], 8);
-      mbar_init(&pds_full[i], 8); mbar_init(&acc_done[i], 1);
-    }
+    for (int i = 0; i < QS; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
+    for (int i = 0; i < DOS; ++i) { mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); }
+    for (int i = 0; i < STS; ++i) { mbar_init(&stat_full[i], 1); mbar_init(&stat_empty[i], 8); }
+    for (int i = 0; i < SB; ++i) mbar_init(&s_full[i], 1);
+    mbar_init(p_full, 8);
+    mbar_init(dp_full, 1);
+    mbar_init(ds_full, 8);
+    mbar_init(s_free, 8);
+    mbar_init(acc_done, 1);
     mbar_fence_init();
   }
+  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
   if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const int seq_start = slot->seq_start, seq_end = slot->seq_end;
+  const int k0 = seq_start + ((seq_end - seq_start + 127) / 128 - slot->work) * 128;
+  const int n_q = slot->work > 0 ? (seq_end - k0 + BQ - 1) / BQ : 0;   // query tiles at or after the key tile
+  const int n_it = rep * n_q;
 
   if (warp == BW_TMA_WARP) {
-    if (elect_one()) {
-      mbar_expect_tx(kv_full, Cfg::NEED_DP ? 2 * Cfg::K_BYTES : Cfg::K_BYTES);
+    if (n_it > 0 && elect_one()) {
+      mbar_expect_tx(kv_full, Cfg::DO_DK ? 2 * Cfg::K_BYTES : Cfg::K_BYTES);
 #pragma unroll
       for (int c = 0; c < DH / 64; ++c) {
         tma_load_2d(smem + c * (128 * 128), &tmK, kv_full, kv_head * DH + c * 64, k0);
-        if (Cfg::NEED_DP)
+        if (Cfg::DO_DK)
           tma_load_2d(smem + Cfg::OFF_V + c * (128 * 128), &tmV, kv_full, kv_head * DH + c * 64, k0);
       }
       for (int it = 0; it < n_it; ++it) {
-        const int st = it % QS;
-        if (it >= QS && !mbar_wait(&q_empty[st], ((it / QS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY))
-          break;
+        const int qs = it % QS, ds = it % DOS;
         const int head = kv_head * rep + it / n_q;
         const int qt0 = k0 + (it % n_q) * BQ;
-        uint8_t* sq = smem + Cfg::OFF_Q + st * Cfg::QT_BYTES;
-        uint8_t* sdo = smem + Cfg::OFF_DO + st * Cfg::QT_BYTES;
-        mbar_expect_tx(&q_full[st], 2 * Cfg::QT_BYTES);
+        if (it >= QS && !mbar_wait(&q_empty[qs], ((it / QS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* sq = smem + Cfg::OFF_Q + qs * Cfg::QT_BYTES;
+        mbar_expect_tx(&q_full[qs], Cfg::QT_BYTES);
 #pragma unroll
-        for (int c = 0; c < DH / 64; ++c) {
-          tma_load_2d(sq + c * (BQ * 128), &tmQ, &q_full[st], head * DH + c * 64, qt0);
-          tma_load_2d(sdo + c * (BQ * 128), &tmDO, &q_full[st], head * DH + c * 64, qt0);
-        }
+        for (int c = 0; c < DH / 64; ++c)
+          tma_load_2d(sq + c * (BQ * 128), &tmQ, &q_full[qs], head * DH + c * 64, qt0);
+        if (it >= DOS && !mbar_wait(&do_empty[ds], ((it / DOS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* sdo = smem + Cfg::OFF_DO + ds * Cfg::QT_BYTES;
+        mbar_expect_tx(&do_full[ds], Cfg::QT_BYTES);
+#pragma unroll
+        for (int c = 0; c < DH / 64; ++c)
+          tma_load_2d(sdo + c * (BQ * 128), &tmDO, &do_full[ds], head * DH + c * 64, qt0);
       }
     }
   } else if (warp == BW_MMA_WARP) {
-    if (elect_one()) {
+    if (n_it > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, DH, false, true);
       const uint32_t sk = smem_u32(smem), sv = smem_u32(smem + Cfg::OFF_V);
-      const uint32_t spt = smem_u32(smem + Cfg::OFF_PT), sdst = smem_u32(smem + Cfg::OFF_DST);
-      bool ok = mbar_wait(kv_full, 0, p.status, KS_TIMEOUT_FULL);
-      auto issue_sp = [&](int it) {
-        const int b = it & 1, st = it % QS;
-        const uint32_t sq = smem_u32(smem + Cfg::OFF_Q + st * Cfg::QT_BYTES);
-        const uint32_t sdo = smem_u32(smem + Cfg::OFF_DO + st * Cfg::QT_BYTES);
+      const uint32_t sq0 = smem_u32(smem + Cfg::OFF_Q), sdo0 = smem_u32(smem + Cfg::OFF_DO);
+      auto scores = [&](uint32_t d, uint32_t a, uint32_t b) {
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint32_t ao = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
-          const uint32_t bo = (kk >> 2) * (BQ * 128) + (kk & 3) * 32;
-          umma_bf16(tmem_base + Cfg::TM_ST + b * BQ, umma_smem_desc(sk + ao, 16, 1024),
-                    umma_smem_desc(sq + bo, 16, 1024), idesc_s, kk != 0);
-        }
-        if (Cfg::NEED_DP) {
-#pragma unroll
-          for (int kk = 0; kk < DH / 16; ++kk) {
-            const uint32_t ao = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
-            const uint32_t bo = (kk >> 2) * (BQ * 128) + (kk & 3) * 32;
-            umma_bf16(tmem_base + Cfg::TM_DPT + b * BQ, umma_smem_desc(sv + ao, 16, 1024),
-                      umma_smem_desc(sdo + bo, 16, 1024), idesc_s, kk != 0);
-          }
-        }
-        umma_commit(&sp_full[b]);
+        for (int kk = 0; kk < DH / 16; ++kk)
+          umma_bf16(d, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
+                    umma_smem_desc(b + (kk >> 2) * (BQ * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
       };
-      auto prefetch_next = [&](int it) -> bool {
-        const int n = it + 1, b = n & 1;
-        if (!mbar_wait(&q_full[n % QS], (n / QS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
-        if (n >= 2 && !mbar_wait(&sp_free[b], ((n >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY))
-          return false;
+      auto accumulate = [&](uint32_t d, uint32_t a, uint32_t b, bool fresh) {
+#pragma unroll
+        for (int kk = 0; kk < BQ / 16; ++kk)
+          umma_bf16_ts(d, a + packed_col<BQ>(kk), umma_smem_desc(b + kk * (16 * 128), BQ * 128, 1024),
+                       idesc_acc, !(fresh && kk == 0));
+      };
+      auto issue_s = [&](int it) -> bool {
+        if (!mbar_wait(&q_full[it % QS], (it / QS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        issue_sp(n);
+        scores(tmem_base + Cfg::TM_ST + (it % SB) * BQ, sk, sq0 + (it % QS) * Cfg::QT_BYTES);
+        umma_commit(&s_full[it % SB]);
         return true;
       };
-      if (ok) ok = mbar_wait(&q_full[0], 0, p.status, KS_TIMEOUT_FULL);
-      if (ok) { tc_fence_after(); issue_sp(0); }
+      bool ok = mbar_wait(kv_full, 0, p.status, KS_TIMEOUT_FULL) && issue_s(0);
       for (int it = 0; it < n_it && ok; ++it) {
-        if (QS >= 2 && it + 1 < n_it) { ok = prefetch_next(it); if (!ok) break; }
-        ok = mbar_wait(&pds_full[it & 1], (it >> 1) & 1, p.status, KS_TIMEOUT_FULL);
+        const uint32_t sq = sq0 + (it % QS) * Cfg::QT_BYTES, sdo = sdo0 + (it % DOS) * Cfg::QT_BYTES;
+        ok = mbar_wait(&do_full[it % DOS], (it / DOS) & 1, p.status, KS_TIMEOUT_FULL);
         if (!ok) break;
         tc_fence_after();
-        const int st = it % QS;
-        const uint32_t spt_i = spt + (it & 1) * Cfg::PT_BYTES, sdst_i = sdst + (it & 1) * Cfg::PT_BYTES;
-        const uint32_t sq = smem_u32(smem + Cfg::OFF_Q + st * Cfg::QT_BYTES);
-        const uint32_t sdo = smem_u32(smem + Cfg::OFF_DO + st * Cfg::QT_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < BQ / 16; ++kk) {
-          if (Cfg::DO_DV) {
-            const uint32_t acc = tmem_base + (MODE == MODE_BOTH ? Cfg::TM_ACC1 : Cfg::TM_ACC0);
-            umma_bf16(acc, umma_smem_desc(spt_i + kk * 32, 16, 1024),
-                      umma_smem_desc(sdo + kk * (16 * 128), BQ * 128, 1024), idesc_acc,
-                      (it | kk) != 0);
-          }
-          if (Cfg::DO_DK) {
-            umma_bf16(tmem_base + Cfg::TM_ACC0, umma_smem_desc(sdst_i + kk * 32, 16, 1024),
-                      umma_smem_desc(sq + kk * (16 * 128), BQ * 128, 1024), idesc_acc,
-                      (it | kk) != 0);
-          }
+        if (Cfg::DO_DK) {
+          // dP^T overwrites the dS^T that the dK product before it reads: products of one issuing
+          // thread run in order (the same holds for S^T and P^T below)
+          scores(tmem_base + Cfg::TM_DPT, sv, sdo);
+          umma_commit(dp_full);
         }
-        umma_commit(&q_empty[st]);
-        umma_commit(&acc_done[it & 1]);
-        if (QS < 2 && it + 1 < n_it) { ok = prefetch_next(it); }
+        if (SB == 2 && it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
+        if (Cfg::DO_DV) {
+          ok = mbar_wait(p_full, it & 1, p.status, KS_TIMEOUT_FULL);
+          if (!ok) break;
+          tc_fence_after();
+          accumulate(tmem_base + Cfg::TM_DV, tmem_base + Cfg::TM_ST + (it % SB) * BQ, sdo, it == 0);
+          if (!Cfg::DO_DK) umma_commit(&q_empty[it % QS]);
+        } else {
+          ok = mbar_wait(s_free, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        umma_commit(&do_empty[it % DOS]);
+        if (SB == 1 && it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
+        if (Cfg::DO_DK) {
+          ok = mbar_wait(ds_full, it & 1, p.status, KS_TIMEOUT_FULL);
+          if (!ok) break;
+          tc_fence_after();
+          accumulate(tmem_base + Cfg::TM_DK, tmem_base + Cfg::TM_DPT, sq, it == 0);
+          umma_commit(&q_empty[it % QS]);
+        }
+        if (it + 1 == n_it) umma_commit(acc_done);
       }
     }
+  } else if (warp == BW_STAT_WARP) {
+    // log-sum-exp and delta of each tile's queries, fetched ahead of the softmax warps. A query past
+    // the end of the sequence gets a probability of zero. All loads of a tile are issued before its
+    // first store: with a store between them, each waits for the one before it (a full memory
+    // latency per load, which held the whole kernel back).
+    constexpr int NU = BQ / 32;
+    for (int it = 0; it < n_it; ++it) {
+      const int st = it % STS;
+      const int qt0 = k0 + (it % n_q) * BQ;
+      const long long base = static_cast<long long>(kv_head * rep + it / n_q) * p.T;
+      float nl[NU], dl[NU];
+#pragma unroll
+      for (int u = 0; u < NU; ++u) {
+        const int gq = qt0 + lane + u * 32;
+        const bool in = gq < seq_end;
+        nl[u] = in ? -__ldg(p.lse + base + gq) * LOG2E : -INFINITY;
+        dl[u] = in ? __ldg(p.delta + base + gq) : 0.f;
+      }
+      if (it >= STS && !mbar_wait(&stat_empty[st], ((it / STS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+      const uint32_t dst = smem_u32(s_stat + st * (2 * BQ) + lane);
+#pragma unroll
+      for (int u = 0; u < NU; ++u) {
+        st_shared_f32(dst + u * 128, nl[u]);
+        st_shared_f32(dst + BQ * 4 + u * 128, dl[u]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&stat_full[st]);
+    }
   } else {
-    const int quarter = warp & 3, hsel = warp >> 2;
+    constexpr int HN = BQ / 2;
+    const int quarter = warp & 3, half = warp >> 2;
     const int row = quarter * 32 + lane;     // key row within the tile
     const int gk = k0 + row;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t dp_addr = lane_addr + Cfg::TM_DPT + half * HN;
     const float c2 = p.scale * LOG2E;
+    const uint32_t stat = smem_u32(s_stat);
     bool ok = true;
-    // log-sum-exp and delta of the tile's queries: threads 0..2*BQ-1 fetch one value each, one
-    // iteration ahead, so that the global-memory latency is not on the path of every tile
-    auto fetch_row_stat = [&](int it) -> float {
-      if (threadIdx.x >= 2 * BQ || it >= n_it) return 0.f;
-      const int head_i = kv_head * rep + it / n_q;
-      const int col = threadIdx.x & (BQ - 1);
-      const long long li = static_cast<long long>(head_i) * p.T + min(k0 + (it % n_q) * BQ + col, p.T - 1);
-      return threadIdx.x < BQ ? p.lse[li] * LOG2E : p.delta[li];
-    };
-    float row_stat = fetch_row_stat(0);
     for (int it = 0; it < n_it; ++it) {
-      const int b = it & 1;
-      const int head = kv_head * rep + it / n_q;
+      const int st = it % STS;
       const int qt0 = k0 + (it % n_q) * BQ;
-      float* sl = s_lse + b * (2 * BQ);
-      if (threadIdx.x < 2 * BQ) sl[threadIdx.x] = row_stat;     // [0,BQ): lse, [BQ,2BQ): delta
-      row_stat = fetch_row_stat(it + 1);
-      named_barrier_softmax();
-      if (!mbar_wait(&sp_full[b], (it >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
-      // the P^T / dS^T buffers of this parity were last read by the MMAs of iteration it-2
-      if (it > 1 && !mbar_wait(&acc_done[b], ((it >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      const uint32_t nlse = stat + (st * (2 * BQ) + half * HN) * 4, delta = nlse + BQ * 4;
+      if (!mbar_wait(&stat_full[st], (it / STS) & 1, p.status, KS_TIMEOUT_FULL)) { ok = false; break; }
+      const uint32_t s_addr = lane_addr + Cfg::TM_ST + (it % SB) * BQ + half * HN;
+      if (!mbar_wait(&s_full[it % SB], (it / SB) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-#pragma unroll 1
-      for (int c = hsel; c < BQ / 32; c += 2) {
-        uint32_t s[32], d[32];
-        tmem_ld_32x32(lane_addr + Cfg::TM_ST + b * BQ + c * 32, s);
-        if (Cfg::NEED_DP) tmem_ld_32x32(lane_addr + Cfg::TM_DPT + b * BQ + c * 32, d);
-        tmem_ld_wait();
-        uint32_t pkp[16], pkd[16];
-        // whole tile visible: every query of the tile is at or after every key, none past the end
-        const bool all_valid = (qt0 >= k0 + 127) && (qt0 + BQ <= seq_end);
-        if (all_valid) {
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const int col = c * 32 + e;
-            const float p0 = fast_exp2(fmaf(__uint_as_float(s[e]), c2, -sl[col]));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(s[e + 1]), c2, -sl[col + 1]));
-            pkp[e >> 1] = pack_bf16(p0, p1);
-            pkd[e >> 1] = Cfg::NEED_DP
-                ? pack_bf16(p0 * (__uint_as_float(d[e]) - sl[BQ + col]),
-                            p1 * (__uint_as_float(d[e + 1]) - sl[BQ + col + 1]))
-                : 0u;
-          }
-        } else
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          float pv[2], dv[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int col = c * 32 + e + u;
-            const int gqc = qt0 + col;
-            const bool valid = (gqc < seq_end) && (gk <= gqc);
-            const float pr = valid ? fast_exp2(fmaf(__uint_as_float(s[e + u]), c2, -sl[col])) : 0.f;
-            pv[u] = pr;
-            dv[u] = Cfg::NEED_DP ? pr * (__uint_as_float(d[e + u]) - sl[BQ + col]) : 0.f;   // dK scaled once at the end
-          }
-          pkp[e >> 1] = pack_bf16(pv[0], pv[1]);
-          pkd[e >> 1] = pack_bf16(dv[0], dv[1]);
-        }
-        if (Cfg::DO_DV) store_swizzled_32(smem + Cfg::OFF_PT + b * Cfg::PT_BYTES, 128 * 128, row, c * 32, pkp);
-        if (Cfg::DO_DK) store_swizzled_32(smem + Cfg::OFF_DST + b * Cfg::PT_BYTES, 128 * 128, row, c * 32, pkd);
+      uint32_t s[HN];
+      tmem_ld_half<HN>(s_addr, s);
+      if (!Cfg::DO_DV) {                      // nothing goes back into these columns
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_free);
       }
-      tc_fence_before();
-      fence_async_proxy();
+      // whole tile visible: every query of the tile is at or after every key, none past the end
+      const bool all_valid = qt0 >= k0 + 127 && qt0 + BQ <= seq_end;
+#pragma unroll
+      for (int e = 0; e < HN; e += 4) {
+        const float4 l = ld_shared_f4(nlse + e * 4);
+        s[e] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, l.x)));
+        s[e + 1] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 1]), c2, l.y)));
+        s[e + 2] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 2]), c2, l.z)));
+        s[e + 3] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 3]), c2, l.w)));
+      }
+      if (!all_valid) {
+        const int first = gk - (qt0 + half * HN), last = seq_end - (qt0 + half * HN);   // columns in [first, last)
+#pragma unroll
+        for (int e = 0; e < HN; ++e)
+          if (e < first || e >= last) s[e] = 0u;
+      }
+      if (Cfg::DO_DV) {
+        uint32_t pk[HN / 2];
+#pragma unroll
+        for (int e = 0; e < HN; e += 2) pk[e >> 1] = pack_bf16(__uint_as_float(s[e]), __uint_as_float(s[e + 1]));
+        tmem_st_half<HN>(s_addr, pk);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (Cfg::DO_DK) {
+        if (!mbar_wait(dp_full, it & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t d[HN], pk[HN / 2];
+        tmem_ld_half<HN>(dp_addr, d);
+#pragma unroll
+        for (int e = 0; e < HN; e += 4) {     // the softmax scale is applied to dK once, at the end
+          const float4 dl = ld_shared_f4(delta + e * 4);
+          pk[e >> 1] = pack_bf16(__uint_as_float(s[e]) * (__uint_as_float(d[e]) - dl.x),
+                                 __uint_as_float(s[e + 1]) * (__uint_as_float(d[e + 1]) - dl.y));
+          pk[(e >> 1) + 1] = pack_bf16(__uint_as_float(s[e + 2]) * (__uint_as_float(d[e + 2]) - dl.z),
+                                       __uint_as_float(s[e + 3]) * (__uint_as_float(d[e + 3]) - dl.w));
+        }
+        tmem_st_half<HN>(dp_addr, pk);
+        tc_fence_before();
+      }
       __syncwarp();
-      if (lane == 0) { mbar_arrive(&sp_free[b]); mbar_arrive(&pds_full[b]); }
+      if (lane == 0) {
+        if (Cfg::DO_DK) mbar_arrive(ds_full);
+        mbar_arrive(&stat_empty[st]);
+      }
     }
-    if (ok && n_it > 0 && mbar_wait(&acc_done[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, p.status,
-                                    KS_TIMEOUT_TMEM_FULL)) {
+    if (ok && n_it > 0 && mbar_wait(acc_done, 0, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const bool valid = gk < seq_end;
       auto store_acc = [&](uint32_t tm_col, void* base, long long ld, float sc) {
         __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(base) +
                               static_cast<long long>(gk) * ld + kv_head * DH;
 #pragma unroll 1
-        for (int c = hsel; c < DH / 32; c += 2) {
+        for (int c = half; c < DH / 32; c += 2) {
           uint32_t r[32];
           tmem_ld_32x32(lane_addr + tm_col + c * 32, r);
           tmem_ld_wait();
@@ -581,8 +618,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           }
         }
       };
-      if (Cfg::DO_DK) store_acc(Cfg::TM_ACC0, p.dk, p.ldk, p.scale);
-      if (Cfg::DO_DV) store_acc(MODE == MODE_BOTH ? Cfg::TM_ACC1 : Cfg::TM_ACC0, p.dv, p.ldv, 1.f);
+      if (Cfg::DO_DK) store_acc(Cfg::TM_DK, p.dk, p.ldk, p.scale);
+      if (Cfg::DO_DV) store_acc(Cfg::TM_DV, p.dv, p.ldv, 1.f);
     }
   }
   tc_fence_before();
@@ -590,25 +627,25 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (warp == BW_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
-template <int DH, int BKV, int KVS>
+template <int DH, int BKV, int KS, int VS>
 static int launch_dq(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk,
                      const CUtensorMap& tv, const AttnBwdParams& p, int tiles, cudaStream_t s) {
-  using Cfg = DqCfg<DH, BKV, KVS>;
-  auto kern = attn_bwd_dq_kernel<DH, BKV, KVS>;
+  using Cfg = DqCfg<DH, BKV, KS, VS>;
+  auto kern = attn_bwd_dq_kernel<DH, BKV, KS, VS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
-  kern<<<dim3(tiles, p.Hq), BW_THREADS, Cfg::SMEM, s>>>(tq, tdo, tk, tv, p);
+  kern<<<dim3(p.Hq, tiles), BW_THREADS, Cfg::SMEM, s>>>(tq, tdo, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
 
-template <int DH, int QS, int MODE>
+template <int DH, int BQ, int QS, int DOS, int MODE>
 static int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk,
                       const CUtensorMap& tv, const AttnBwdParams& p, int tiles, cudaStream_t s) {
-  using Cfg = DkvCfg<DH, QS, MODE>;
-  auto kern = attn_bwd_dkv_kernel<DH, QS, MODE>;
+  using Cfg = DkvCfg<DH, BQ, QS, DOS, MODE>;
+  auto kern = attn_bwd_dkv_kernel<DH, BQ, QS, DOS, MODE>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
-  kern<<<dim3(tiles, p.Hkv), BW_THREADS, Cfg::SMEM, s>>>(tq, tdo, tk, tv, p);
+  kern<<<dim3(p.Hkv, tiles), BW_THREADS, Cfg::SMEM, s>>>(tq, tdo, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -642,28 +679,29 @@ extern "C" int ss_attn_bwd_g(const void* q, const void* k, const void* v, const 
   p.scale = scale; p.status = status;
   const int tiles = (T + 127) / 128 + nseq;
   const long long qc = static_cast<long long>(Hq) * dh, kc = static_cast<long long>(Hkv) * dh;
-  CUtensorMap tq128, tdo128, tk64, tv64, tq64, tdo64, tk128, tv128;
+  const int stream_rows = dh == 256 ? 64 : 128;     // rows of the streamed tiles
+  CUtensorMap tq128, tdo128, tk128, tv128, tqs, tdos, tks, tvs;
   int r;
   if ((r = make_tmap_bf16(&tq128, q, T, qc, ldq, 128))) return r;
   if ((r = make_tmap_bf16(&tdo128, dout, T, qc, ldo, 128))) return r;
-  if ((r = make_tmap_bf16(&tk64, k, T, kc, ldk, 64))) return r;
-  if ((r = make_tmap_bf16(&tv64, v, T, kc, ldv, 64))) return r;
-  if ((r = make_tmap_bf16(&tq64, q, T, qc, ldq, 64))) return r;
-  if ((r = make_tmap_bf16(&tdo64, dout, T, qc, ldo, 64))) return r;
   if ((r = make_tmap_bf16(&tk128, k, T, kc, ldk, 128))) return r;
   if ((r = make_tmap_bf16(&tv128, v, T, kc, ldv, 128))) return r;
+  if ((r = make_tmap_bf16(&tqs, q, T, qc, ldq, stream_rows))) return r;
+  if ((r = make_tmap_bf16(&tdos, dout, T, qc, ldo, stream_rows))) return r;
+  if ((r = make_tmap_bf16(&tks, k, T, kc, ldk, stream_rows))) return r;
+  if ((r = make_tmap_bf16(&tvs, v, T, kc, ldv, stream_rows))) return r;
   if (dh == 128) {
-    if ((r = launch_dq<128, 64, 2>(tq128, tdo128, tk64, tv64, p, tiles, s))) return r;
-    return launch_dkv<128, 2, MODE_BOTH>(tq64, tdo64, tk128, tv128, p, tiles, s);
+    if ((r = launch_dq<128, 128, 3, 2>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
+    return launch_dkv<128, 128, 2, 2, MODE_BOTH>(tqs, tdos, tk128, tv128, p, tiles, s);
   }
   if (dh == 64) {
-    if ((r = launch_dq<64, 64, 2>(tq128, tdo128, tk64, tv64, p, tiles, s))) return r;
-    return launch_dkv<64, 2, MODE_BOTH>(tq64, tdo64, tk128, tv128, p, tiles, s);
+    if ((r = launch_dq<64, 128, 3, 2>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
+    return launch_dkv<64, 128, 2, 2, MODE_BOTH>(tqs, tdos, tk128, tv128, p, tiles, s);
   }
   if (dh == 256) {
-    if ((r = launch_dq<256, 64, 1>(tq128, tdo128, tk64, tv64, p, tiles, s))) return r;
-    if ((r = launch_dkv<256, 2, MODE_DV>(tq64, tdo64, tk128, tv128, p, tiles, s))) return r;
-    return launch_dkv<256, 1, MODE_DK>(tq64, tdo64, tk128, tv128, p, tiles, s);
+    if ((r = launch_dq<256, 64, 2, 1>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
+    if ((r = launch_dkv<256, 64, 2, 2, MODE_DV>(tqs, tdos, tk128, tv128, p, tiles, s))) return r;
+    return launch_dkv<256, 64, 2, 1, MODE_DK>(tqs, tdos, tk128, tv128, p, tiles, s);
   }
   return -2;
 }

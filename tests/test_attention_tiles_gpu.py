@@ -1,0 +1,57 @@
+"""The attention kernels at the edges of their tiles: sequences one row short of, at and past 128 and
+256 rows, more sequences than a warp has lanes, strided operands and a negative scale."""
+import pytest
+import torch
+
+from shadowspill_b200.ops import _lib, attention, reference as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _inputs(lens, Hq, Hkv, dh, seed):
+    """Views of one fused projection, as a decoder layer passes them."""
+    g = torch.Generator(device="cpu").manual_seed(seed)
+    T = sum(lens)
+    qkv = (torch.randn(T, (Hq + 2 * Hkv) * dh, generator=g) * 0.8).to(torch.bfloat16).to(DEV)
+    q = qkv[:, :Hq * dh].view(T, Hq, dh)
+    k = qkv[:, Hq * dh:(Hq + Hkv) * dh].view(T, Hkv, dh)
+    v = qkv[:, (Hq + Hkv) * dh:].view(T, Hkv, dh)
+    dout = (torch.randn(T, Hq, dh, generator=g) * 0.5).to(torch.bfloat16).to(DEV)
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device=DEV)
+    return q, k, v, dout, cu
+
+
+def _rel(a, b):
+    return float((a.float() - b.float()).norm() / (b.float().norm() + 1e-12))
+
+
+EDGES = [[1], [127, 128, 129], [255, 256, 257], [64, 63, 65, 384, 1], [640]]
+
+
+@pytest.mark.parametrize("dh", [64, 128, 256])
+@pytest.mark.parametrize("lens", EDGES + [[3 + 17 * i for i in range(40)]], ids=lambda x: f"{len(x)}seq{sum(x)}")
+@pytest.mark.parametrize("scale", [None, -0.05])
+def test_against_the_definition(lens, dh, scale):
+    q, k, v, dout, cu = _inputs(lens, 4, 2, dh, seed=sum(lens))
+    out, lse = attention.forward(q, k, v, cu, max(lens), scale)
+    dq, dk, dv = attention.backward(q, k, v, out, lse, dout, cu, max(lens), scale)
+    _lib.check_status()
+    out_r, lse_r = R.attention_varlen(q, k, v, cu, scale)
+    dq_r, dk_r, dv_r = R.attention_varlen_bwd(q, k, v, out_r, lse_r, dout, cu, scale)
+    # bf16 probabilities and results: 2^-9 relative rounding each, a few such roundings per output
+    assert _rel(out, out_r) < 1e-2
+    assert float((lse - lse_r).abs().max()) < 1e-3
+    # the gradients of a one-token sequence are zero up to cancellation in dP - delta
+    if max(lens) > 1:
+        assert _rel(dq, dq_r) < 2e-2
+        assert _rel(dk, dk_r) < 2e-2
+    assert _rel(dv, dv_r) < 2e-2
+
+
+def test_gradients_repeat_bit_for_bit():
+    q, k, v, dout, cu = _inputs([300, 700, 129], 8, 2, 128, seed=5)
+    out, lse = attention.forward(q, k, v, cu, 700)
+    runs = [attention.backward(q, k, v, out, lse, dout, cu, 700) for _ in range(3)]
+    for other in runs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(runs[0], other))
