@@ -1,20 +1,24 @@
 // Packed variable-length causal GQA attention, forward, for sm_100a.
 //
-// One CTA per (128-query tile of one sequence, query head). K/V tiles stream
-// through a two-stage TMA ring; S = Q K^T and O += P V run on tcgen05 with S
-// double-buffered and O resident in TMEM; four softmax warps own one query row
-// per thread (online softmax in the exp2 domain, lazy rescaling of O), write P
-// as a 128B-swizzled K-major operand into shared memory, and at the end
-// normalise O and store it with the log-sum-exp.
+// Head widths 64 and 128: one CTA per (two adjacent 128-query tiles of one sequence, query head).
+// Each tile has its own softmax warpgroup, its own score columns and its own O accumulator in TMEM
+// (2 x 128 + 2 x DH columns), and the products alternate between the tiles, so one tile's O += P V
+// and next S = Q K^T run under the other tile's exponentials.
+// Head width 256: O takes half of TMEM, so a CTA has one tile and two score buffers instead; S of
+// the next 64 keys is formed under the exponentials of these.
+// P goes back to TMEM over the scores it comes from and is the A operand of P V from there: it never
+// passes through shared memory, whose bandwidth the two products need for K, V and Q.
+// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: 1.41 -> 1.09 ms; 6,001 tokens, 16/4 heads
+// of 256: 0.285 -> 0.159 ms, against one tile per CTA and P through shared memory.
 //
-//   warps 0..3  softmax / correction / epilogue  (TMEM lanes 32w..32w+31)
-//   warp  4     TMA producer
-//   warp  5     MMA issuer + TMEM allocator
+//   warps 0..4*NT-1  softmax, rescaling of O, epilogue: one query row per thread
+//   then one TMA producer warp and one MMA warp
 //
 // Semantics: the reference's packed attention contract
 // (packages/workloads/src/shadowspill_workloads/models/shared/decoder.py:251):
 // each [cu_seqlens[i], cu_seqlens[i+1]) is an independent causal sequence.
 #include "sm100_ptx.cuh"
+#include "attention_tiles.cuh"
 
 #include <cudaTypedefs.h>
 #include <math.h>
@@ -24,28 +28,22 @@ namespace ss {
 int make_tmap_bf16(CUtensorMap* map, const void* base, long long rows, long long cols,
                    long long ld, int box_rows);  // gemm_tcgen05.cu
 
-constexpr int ATT_BM = 128;
-constexpr int ATT_THREADS = 192;
-
-template <int DH, int BKV>
+// NT query tiles per CTA, BKV keys per step, KS / VS stages of K and V (K is released by its score
+// products, V one step later by P V).
+template <int DH, int NT, int BKV, int KS, int VS>
 struct AttnCfg {
-  static constexpr int Q_BYTES = ATT_BM * DH * 2;
+  static constexpr int THREADS = NT * 128 + 64;
+  static constexpr int TMA_WARP = NT * 4, MMA_WARP = NT * 4 + 1;
+  static constexpr int SB = 3 - NT;                    // score buffers of one tile
+  static constexpr int QT_BYTES = 128 * DH * 2;
   static constexpr int KV_BYTES = BKV * DH * 2;        // one of K or V
-  static constexpr int P_BYTES = ATT_BM * BKV * 2;
-  static constexpr int OFF_K = Q_BYTES;
-  static constexpr int OFF_V = OFF_K + 2 * KV_BYTES;
-  static constexpr int OFF_P = OFF_V + 2 * KV_BYTES;
-  static constexpr int OFF_BAR = OFF_P + P_BYTES;
-  // Two CTAs share an SM when they fit (dh <= 128 with 64-key tiles): while one CTA's softmax
-  // warps work, the other CTA's MMAs keep the tensor pipe busy. Shared memory has no room for a
-  // blanket alignment slack then; the kernel checks the aligned layout against what it was given.
-  static constexpr int USED = OFF_BAR + 128;
-  // an SM has 228 KiB of shared memory and keeps 1 KiB per resident CTA for itself
-  static constexpr bool PAIR = 2 * (USED + 1024) <= 233472;
-  static constexpr int SMEM = PAIR ? USED : USED + 1024;
-  static constexpr int TMEM_S0 = 0;
-  static constexpr int TMEM_O = 2 * BKV;
-  static constexpr int TMEM_COLS = (2 * BKV + DH) <= 256 ? 256 : 512;
+  static constexpr int OFF_K = NT * QT_BYTES;
+  static constexpr int OFF_V = OFF_K + KS * KV_BYTES;
+  static constexpr int OFF_BAR = OFF_V + VS * KV_BYTES;
+  static constexpr int SMEM = OFF_BAR + 256 + 1024;
+  static constexpr int TM_O = 2 * BKV;                 // behind the two score buffers
+  static_assert(TM_O + NT * DH <= 512, "TMEM budget");
+  static_assert(SMEM <= 232448, "shared memory budget");
 };
 
 struct AttnParams {
@@ -58,258 +56,248 @@ struct AttnParams {
   int* status;
 };
 
-// Maps a linear tile index to (sequence, tile within sequence); false if out of range.
-__device__ __forceinline__ bool find_tile(const int* cu, int nseq, int tile, int& seq_start,
-                                          int& seq_end, int& q0) {
-  int acc = 0;
-  for (int s = 0; s < nseq; ++s) {
-    const int b = cu[s], e = cu[s + 1];
-    const int nt = (e - b + ATT_BM - 1) / ATT_BM;
-    if (tile < acc + nt) {
-      seq_start = b;
-      seq_end = e;
-      q0 = b + (tile - acc) * ATT_BM;
-      return true;
-    }
-    acc += nt;
-  }
-  return false;
-}
-
-template <int DH, int BKV>
-__global__ void __launch_bounds__(ATT_THREADS, (AttnCfg<DH, BKV>::TMEM_COLS <= 256 &&
-                                                AttnCfg<DH, BKV>::PAIR) ? 2 : 1)
+template <int DH, int NT, int BKV, int KS, int VS>
+__global__ void __launch_bounds__(NT * 128 + 64, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
-  using Cfg = AttnCfg<DH, BKV>;
+  using Cfg = AttnCfg<DH, NT, BKV, KS, VS>;
+  constexpr int SB = Cfg::SB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  if (smem + Cfg::USED > smem_raw + Cfg::SMEM) {      // the launch gave an unaligned window
-    if (threadIdx.x == 0) report(p.status, KS_BAD_ARGUMENT);
-    return;
-  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* q_full = bars;          // 1
-  uint64_t* kv_full = bars + 1;     // 2
-  uint64_t* kv_empty = bars + 3;    // 2
-  uint64_t* s_full = bars + 5;      // 2
-  uint64_t* s_free = bars + 7;      // 2
-  uint64_t* p_full = bars + 9;      // 1
-  uint64_t* o_done = bars + 10;     // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t* k_full = bars + 1;      // 3
+  uint64_t* k_empty = bars + 4;     // 3
+  uint64_t* v_full = bars + 7;      // 3
+  uint64_t* v_empty = bars + 10;    // 3
+  uint64_t* s_full = bars + 13;     // 2: by tile, or by buffer of the one tile
+  uint64_t* p_full = bars + 15;     // 2: by tile
+  uint64_t* o_done = bars + 17;     // 2: by tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 21);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int head = blockIdx.y;
+  const int head = blockIdx.x;
   const int kv_head = head / (p.Hq / p.Hkv);
-
-  int seq_start, seq_end, q0;
-  if (!find_tile(p.cu_seqlens, p.nseq, blockIdx.x, seq_start, seq_end, q0)) return;
-  const int q_hi = min(q0 + ATT_BM, seq_end);           // exclusive
-  const int n_kv = (q_hi - seq_start + BKV - 1) / BKV;  // tiles up to the diagonal
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
+    for (int i = 0; i < KS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
+    for (int i = 0; i < VS; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], 4);
+      mbar_init(&p_full[i], 4);
+      mbar_init(&o_done[i], 1);
     }
-    mbar_init(p_full, 4);
-    mbar_init(o_done, 1);
     mbar_fence_init();
   }
-  if (warp == 5) {
-    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+  if (warp == Cfg::TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, NT * 128, blockIdx.y, slot);
+  if (warp == Cfg::MMA_WARP) {
+    tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const int seq_start = slot->seq_start, seq_end = slot->seq_end;
+  const int q0 = seq_start + (slot->work - 1) * (NT * 128);
+  // key steps of each tile, up to its diagonal; none for a tile past the end of the sequence
+  int n_kv[NT];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    const int lo = q0 + i * 128, hi = min(lo + 128, seq_end);
+    n_kv[i] = (slot->work > 0 && hi > lo) ? (hi - seq_start + BKV - 1) / BKV : 0;
+  }
+  const int n_max = max(n_kv[0], n_kv[NT - 1]);
 
-  if (warp == 4) {
+  if (warp == Cfg::TMA_WARP) {
     // ---------------------------------------------------------------- producer
-    if (elect_one()) {
+    if (n_max > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
-      mbar_expect_tx(q_full, Cfg::Q_BYTES);
+      mbar_expect_tx(q_full, NT * Cfg::QT_BYTES);
 #pragma unroll
-      for (int c = 0; c < DH / 64; ++c)
-        tma_load_2d(smem + c * (ATT_BM * 128), &tmQ, q_full, head * DH + c * 64, q0);
-      for (int j = 0; j < n_kv; ++j) {
-        const int st = j & 1;
-        if (j >= 2 &&
-            !mbar_wait(&kv_empty[st], ((j >> 1) - 1) & 1, p.status, KS_TIMEOUT_EMPTY))
-          break;
-        uint8_t* sk = smem + Cfg::OFF_K + st * Cfg::KV_BYTES;
-        uint8_t* sv = smem + Cfg::OFF_V + st * Cfg::KV_BYTES;
-        mbar_expect_tx(&kv_full[st], 2 * Cfg::KV_BYTES);
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int c = 0; c < DH / 64; ++c)
+          tma_load_2d(smem + i * Cfg::QT_BYTES + c * (128 * 128), &tmQ, q_full, head * DH + c * 64, q0 + i * 128);
+      for (int j = 0; j < n_max; ++j) {
+        const int ks = j % KS, vs = j % VS;
         const int k0 = seq_start + j * BKV;
+        if (j >= KS && !mbar_wait(&k_empty[ks], ((j / KS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* sk = smem + Cfg::OFF_K + ks * Cfg::KV_BYTES;
+        mbar_expect_tx(&k_full[ks], Cfg::KV_BYTES);
 #pragma unroll
-        for (int c = 0; c < DH / 64; ++c) {
-          tma_load_2d(sk + c * (BKV * 128), &tmK, &kv_full[st], kv_head * DH + c * 64, k0);
-          tma_load_2d(sv + c * (BKV * 128), &tmV, &kv_full[st], kv_head * DH + c * 64, k0);
-        }
+        for (int c = 0; c < DH / 64; ++c)
+          tma_load_2d(sk + c * (BKV * 128), &tmK, &k_full[ks], kv_head * DH + c * 64, k0);
+        if (j >= VS && !mbar_wait(&v_empty[vs], ((j / VS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* sv = smem + Cfg::OFF_V + vs * Cfg::KV_BYTES;
+        mbar_expect_tx(&v_full[vs], Cfg::KV_BYTES);
+#pragma unroll
+        for (int c = 0; c < DH / 64; ++c)
+          tma_load_2d(sv + c * (BKV * 128), &tmV, &v_full[vs], kv_head * DH + c * 64, k0);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == Cfg::MMA_WARP) {
     // ---------------------------------------------------------------- MMA issuer
-    if (elect_one()) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(ATT_BM, BKV, false, false);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(ATT_BM, DH, false, true);
+    if (n_max > 0 && elect_one()) {
+      constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
+      constexpr uint32_t idesc_o = umma_idesc_bf16(128, DH, false, true);
       const uint32_t sq = smem_u32(smem);
-      const uint32_t sp = smem_u32(smem + Cfg::OFF_P);
-      bool ok = mbar_wait(q_full, 0, p.status, KS_TIMEOUT_FULL);
-      auto issue_s = [&](int j) {
-        const int b = j & 1;
-        const uint32_t sk = smem_u32(smem + Cfg::OFF_K + b * Cfg::KV_BYTES);
-        const uint32_t d = tmem_base + Cfg::TMEM_S0 + b * BKV;
+      const uint32_t sk0 = smem_u32(smem + Cfg::OFF_K), sv0 = smem_u32(smem + Cfg::OFF_V);
+      // products of one issuing thread run in order: S may be issued over the P that the P V product
+      // before it reads
+      auto issue_s = [&](int i, int j) {
+        const int b = NT == 2 ? i : (j & 1);
+        const uint32_t a = sq + i * Cfg::QT_BYTES, k = sk0 + (j % KS) * Cfg::KV_BYTES;
 #pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk) {
-          const uint64_t ad = umma_smem_desc(sq + (kk >> 2) * (ATT_BM * 128) + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = umma_smem_desc(sk + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024);
-          umma_bf16(d, ad, bd, idesc_s, kk != 0);
-        }
+        for (int kk = 0; kk < DH / 16; ++kk)
+          umma_bf16(tmem_base + b * BKV, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
+                    umma_smem_desc(k + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
         umma_commit(&s_full[b]);
       };
-      if (ok) ok = mbar_wait(&kv_full[0], 0, p.status, KS_TIMEOUT_FULL);
-      if (ok) {
+      auto wait_k = [&](int j) -> bool {
+        if (!mbar_wait(&k_full[j % KS], (j / KS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        issue_s(0);
+        return true;
+      };
+      bool ok = mbar_wait(q_full, 0, p.status, KS_TIMEOUT_FULL) && wait_k(0);
+      if (ok) {
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+          if (n_kv[i] > 0) issue_s(i, 0);
+        umma_commit(&k_empty[0]);
       }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        if (j + 1 < n_kv) {
-          const int b = (j + 1) & 1;
-          ok = mbar_wait(&kv_full[b], ((j + 1) >> 1) & 1, p.status, KS_TIMEOUT_FULL);
-          if (ok && j + 1 >= 2)
-            ok = mbar_wait(&s_free[b], (((j + 1) >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY);
+      for (int j = 0; j < n_max && ok; ++j) {
+        const bool more = j + 1 < n_max;
+        if (more) ok = wait_k(j + 1);
+        if (ok && SB == 2 && more) { issue_s(0, j + 1); umma_commit(&k_empty[(j + 1) % KS]); }
+        if (ok) ok = mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL);
+        if (!ok) break;
+        const uint32_t v = sv0 + (j % VS) * Cfg::KV_BYTES;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+          if (j >= n_kv[i]) continue;
+          ok = mbar_wait(&p_full[i], j & 1, p.status, KS_TIMEOUT_FULL);
           if (!ok) break;
           tc_fence_after();
-          issue_s(j + 1);
-        }
-        ok = mbar_wait(p_full, j & 1, p.status, KS_TIMEOUT_FULL);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t sv = smem_u32(smem + Cfg::OFF_V + (j & 1) * Cfg::KV_BYTES);
-        const uint32_t d = tmem_base + Cfg::TMEM_O;
+          const uint32_t pa = tmem_base + (NT == 2 ? i : (j & 1)) * BKV;
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint64_t ad = umma_smem_desc(sp + (kk >> 2) * (ATT_BM * 128) + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = umma_smem_desc(sv + kk * (16 * 128), BKV * 128, 1024);
-          umma_bf16(d, ad, bd, idesc_o, (j | kk) != 0);
+          for (int kk = 0; kk < BKV / 16; ++kk)
+            umma_bf16_ts(tmem_base + Cfg::TM_O + i * DH, pa + kk * 8,
+                         umma_smem_desc(v + kk * (16 * 128), BKV * 128, 1024), idesc_o, (j | kk) != 0);
+          if (NT == 1 || j + 1 == n_kv[i]) umma_commit(&o_done[i]);
+          if (SB == 1 && j + 1 < n_kv[i]) issue_s(i, j + 1);
         }
-        umma_commit(&kv_empty[j & 1]);
-        umma_commit(o_done);
+        if (!ok) break;
+        umma_commit(&v_empty[j % VS]);
+        if (SB == 1 && more) umma_commit(&k_empty[(j + 1) % KS]);
       }
     }
   } else {
     // ---------------------------------------------------------------- softmax warps
-    const int row = warp * 32 + lane;            // row within the tile == TMEM lane
-    const int gq = q0 + row;                     // global query index
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    const int tile = warp >> 2, quarter = warp & 3;
+    const int n = NT == 2 && tile ? n_kv[NT - 1] : n_kv[0];
+    const int tq0 = q0 + tile * 128;
+    const int gq = tq0 + quarter * 32 + lane;    // global query index; its row is the TMEM lane
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t o_addr = lane_addr + Cfg::TM_O + tile * DH;
+    const bool negative = p.scale_log2 < 0.f;    // the row maximum is taken before the scale
+    const float c = fabsf(p.scale_log2);
     float m_used = -INFINITY;                    // reference max (log2 domain, scaled)
     float l = 0.f;
     bool ok = true;
-    uint8_t* sp = smem + Cfg::OFF_P;
-    for (int j = 0; j < n_kv; ++j) {
-      const int b = j & 1;
-      if (!mbar_wait(&s_full[b], (j >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+    for (int j = 0; j < n; ++j) {
+      const int b = NT == 2 ? tile : (j & 1);
+      const uint32_t s_addr = lane_addr + b * BKV;
+      if (!mbar_wait(&s_full[b], (NT == 2 ? j : (j >> 1)) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      const int k0 = seq_start + j * BKV;
-      const bool diag = (k0 + BKV - 1) > q0;     // some key of this tile may exceed some query
-      const uint32_t s_addr = lane_addr + Cfg::TMEM_S0 + b * BKV;
-      // one read of S: the row stays in registers for the maximum and for the exponentials
-      float sv[BKV];
+      float s[BKV];
 #pragma unroll
-      for (int c = 0; c < BKV / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(s_addr + c * 32, r);
-        tmem_ld_wait();
+      for (int x = 0; x < BKV; x += 32)
+        tmem_ld_32x32(s_addr + x, reinterpret_cast<uint32_t (&)[32]>(s[x]));
+      tmem_ld_wait();
+      if (negative) {
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          float s = __uint_as_float(r[e]) * p.scale_log2;
-          if (diag && (k0 + c * 32 + e) > gq) s = -INFINITY;
-          sv[c * 32 + e] = s;
-        }
+        for (int e = 0; e < BKV; ++e) s[e] = -s[e];
       }
-      // S is in registers: the MMA warp may overwrite this buffer with the tile after next
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_free[b]);
-      float m_t = -INFINITY;
+      const int k0 = seq_start + j * BKV;
+      const bool diag = k0 + BKV - 1 > tq0;      // some key of this step may exceed some query
+      if (diag) {
 #pragma unroll
-      for (int e = 0; e < BKV; ++e) m_t = fmaxf(m_t, sv[e]);
+        for (int e = 0; e < BKV; ++e)
+          if (k0 + e > gq) s[e] = -INFINITY;
+      }
+      float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+      for (int e = 4; e < BKV; e += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], s[e + u]);
+      }
+      const float m_t = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;
       // lazy rescale: move the reference max only when it would grow by > 8 (2^8 headroom)
       const bool want = m_t > m_used + 8.f;
-      const bool first = (j == 0);
-      const bool warp_rescale = first || (__ballot_sync(0xffffffffu, want) != 0u);
-      float alpha = 1.f;
-      if (warp_rescale) {
+      if (j == 0) {
+        m_used = fmaxf(m_used, m_t);
+      } else if (__ballot_sync(0xffffffffu, want) != 0u) {
         const float m_new = fmaxf(m_used, m_t);
-        alpha = (m_used == -INFINITY) ? 0.f : fast_exp2(m_used - m_new);
+        const float alpha = m_used == -INFINITY ? 0.f : fast_exp2(m_used - m_new);
         m_used = m_new;
         l *= alpha;
-      }
-      // probabilities -> swizzled K-major P tile in shared memory. The previous P·V has to be
-      // done with the tile first (o_done also covers the rescale of O below).
-      if (j > 0) {
-        if (!mbar_wait(o_done, (j - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        // O of the steps before this one is complete: with two tiles S of this step was issued after
+        // the last P V of its tile, with one tile that product has a barrier of its own
+        if (NT == 1 && !mbar_wait(&o_done[0], (j - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
-        if (warp_rescale) {
 #pragma unroll 1
-          for (int c = 0; c < DH / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32(lane_addr + Cfg::TMEM_O + c * 32, r);
-            tmem_ld_wait();
+        for (int x = 0; x < DH; x += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(o_addr + x, r);
+          tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
-            tmem_st_32x32(lane_addr + Cfg::TMEM_O + c * 32, r);
-          }
-          tmem_st_wait();
+          for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) * alpha);
+          tmem_st_32x32(o_addr + x, r);
         }
       }
-      float lsum = 0.f;
+      const float nm = -m_used;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int c = 0; c < BKV / 32; ++c) {
+      for (int x = 0; x < BKV; x += 32) {
         uint32_t pk[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
-          const float p0 = fast_exp2(sv[c * 32 + e] - m_used);
-          const float p1 = fast_exp2(sv[c * 32 + e + 1] - m_used);
-          lsum += p0 + p1;
+          float p0 = fast_exp2(fmaf(s[x + e], c, nm));
+          float p1 = fast_exp2(fmaf(s[x + e + 1], c, nm));
+          if (diag) {
+            if (k0 + x + e > gq) p0 = 0.f;
+            if (k0 + x + e + 1 > gq) p1 = 0.f;
+          }
+          sum[e & 2] += p0;
+          sum[(e & 2) + 1] += p1;
           pk[e >> 1] = pack_bf16(p0, p1);
         }
-        // columns [c*32, c*32+32) of row `row`: 64 bytes = four 16-byte chunks
-        const int kcol = c * 32;
-        uint8_t* box = sp + (kcol >> 6) * (ATT_BM * 128) + row * 128;
-#pragma unroll
-        for (int q8 = 0; q8 < 4; ++q8) {
-          const int chunk = ((kcol & 63) >> 3) + q8;
-          uint4 v = make_uint4(pk[q8 * 4], pk[q8 * 4 + 1], pk[q8 * 4 + 2], pk[q8 * 4 + 3]);
-          *reinterpret_cast<uint4*>(box + ((chunk ^ (row & 7)) << 4)) = v;
-        }
+        tmem_st_32x16(s_addr + (x >> 1), pk);
       }
-      l += lsum;
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      tmem_st_wait();
       tc_fence_before();
-      fence_async_proxy();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&p_full[tile]);
     }
     // ---------------------------------------------------------------- epilogue
-    if (ok && n_kv > 0 && mbar_wait(o_done, (n_kv - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
+    if (ok && n > 0 && mbar_wait(&o_done[tile], NT == 1 ? (n - 1) & 1 : 0, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
-      const bool valid = gq < q_hi;
+      const bool valid = gq < seq_end;
       __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) +
                             static_cast<long long>(gq) * p.ldo + head * DH;
 #pragma unroll 1
-      for (int c = 0; c < DH / 32; ++c) {
+      for (int x = 0; x < DH; x += 32) {
         uint32_t r[32];
-        tmem_ld_32x32(lane_addr + Cfg::TMEM_O + c * 32, r);
+        tmem_ld_32x32(o_addr + x, r);
         tmem_ld_wait();
         if (valid) {
 #pragma unroll
@@ -319,7 +307,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             v.y = pack_bf16(__uint_as_float(r[e + 2]) * inv, __uint_as_float(r[e + 3]) * inv);
             v.z = pack_bf16(__uint_as_float(r[e + 4]) * inv, __uint_as_float(r[e + 5]) * inv);
             v.w = pack_bf16(__uint_as_float(r[e + 6]) * inv, __uint_as_float(r[e + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + c * 32 + e) = v;
+            *reinterpret_cast<uint4*>(orow + x + e) = v;
           }
         }
       }
@@ -331,26 +319,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) {
+  if (warp == Cfg::MMA_WARP) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    tmem_dealloc(tmem_base, 512);
   }
 }
 
-template <int DH, int BKV>
+template <int DH, int NT, int BKV, int KS, int VS>
 static int launch_fwd(const void* q, const void* k, const void* v, AttnParams p, long long ldq,
-                      long long ldk, long long ldv, int max_tiles, cudaStream_t stream) {
-  using Cfg = AttnCfg<DH, BKV>;
+                      long long ldk, long long ldv, cudaStream_t stream) {
+  using Cfg = AttnCfg<DH, NT, BKV, KS, VS>;
   CUtensorMap tq, tk, tv;
   int r;
-  if ((r = make_tmap_bf16(&tq, q, p.T, static_cast<long long>(p.Hq) * DH, ldq, ATT_BM))) return r;
+  if ((r = make_tmap_bf16(&tq, q, p.T, static_cast<long long>(p.Hq) * DH, ldq, 128))) return r;
   if ((r = make_tmap_bf16(&tk, k, p.T, static_cast<long long>(p.Hkv) * DH, ldk, BKV))) return r;
   if ((r = make_tmap_bf16(&tv, v, p.T, static_cast<long long>(p.Hkv) * DH, ldv, BKV))) return r;
-  auto kern = attn_fwd_kernel<DH, BKV>;
+  auto kern = attn_fwd_kernel<DH, NT, BKV, KS, VS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
-  dim3 grid(max_tiles, p.Hq);
-  kern<<<grid, ATT_THREADS, Cfg::SMEM, stream>>>(tq, tk, tv, p);
+  // every sequence adds at most one partial tile
+  const dim3 grid(p.Hq, (p.T + NT * 128 - 1) / (NT * 128) + p.nseq);
+  kern<<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(tq, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -366,11 +355,9 @@ extern "C" int ss_attn_fwd(const void* q, const void* k, const void* v, void* ou
   AttnParams p;
   p.out = out; p.lse = lse; p.cu_seqlens = cu_seqlens; p.nseq = nseq; p.T = T; p.Hq = Hq;
   p.Hkv = Hkv; p.ldo = ldo; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-  // every sequence adds at most one partial tile
-  const int max_tiles = (T + ATT_BM - 1) / ATT_BM + nseq;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (dh == 128) return launch_fwd<128, 64>(q, k, v, p, ldq, ldk, ldv, max_tiles, s);
-  if (dh == 64) return launch_fwd<64, 64>(q, k, v, p, ldq, ldk, ldv, max_tiles, s);
-  if (dh == 256) return launch_fwd<256, 64>(q, k, v, p, ldq, ldk, ldv, max_tiles, s);
+  if (dh == 128) return launch_fwd<128, 2, 128, 3, 2>(q, k, v, p, ldq, ldk, ldv, s);
+  if (dh == 64) return launch_fwd<64, 2, 128, 3, 3>(q, k, v, p, ldq, ldk, ldv, s);
+  if (dh == 256) return launch_fwd<256, 1, 64, 3, 2>(q, k, v, p, ldq, ldk, ldv, s);
   return -2;
 }
