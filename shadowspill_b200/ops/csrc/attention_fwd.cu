@@ -1,15 +1,18 @@
 // Packed variable-length causal GQA attention, forward, for sm_100a.
 //
 // Head widths 64 and 128: one CTA per (two adjacent 128-query tiles of one sequence, query head).
-// Each tile has its own softmax warpgroup, its own score columns and its own O accumulator in TMEM
-// (2 x 128 + 2 x DH columns), and the products alternate between the tiles, so one tile's O += P V
-// and next S = Q K^T run under the other tile's exponentials.
-// Head width 256: O takes half of TMEM, so a CTA has one tile and two score buffers instead; S of
-// the next 64 keys is formed under the exponentials of these.
+// Each tile has its own softmax warpgroup, its own two score buffers and its own O accumulator in
+// TMEM (4 x 64 + 2 x DH columns). Head width 256: O takes half of TMEM, so a CTA has one tile.
+// S = Q K^T of the next 64 keys is always issued before O += P V of these, so the softmax warps never
+// wait for a product; the 64-key score products read shared memory at 1.5 times its rate, but one
+// 128-key buffer per tile instead left each tile waiting for P V and S in turn (1.09 against 1.02 ms
+// in the long case below).
 // P goes back to TMEM over the scores it comes from and is the A operand of P V from there: it never
 // passes through shared memory, whose bandwidth the two products need for K, V and Q.
-// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: 1.41 -> 1.09 ms; 6,001 tokens, 16/4 heads
-// of 256: 0.285 -> 0.159 ms, against one tile per CTA and P through shared memory.
+// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: 1.41 -> 1.02 ms; 8,192 packed tokens:
+// 0.317 -> 0.225 ms; 6,001 tokens, 16/4 heads of 256: 0.285 -> 0.160 ms, against one tile per CTA and
+// P through shared memory. The softmax warps bound it: of 1980 cycles per 128 x 128 scores, 1024 are
+// exponentials and 1280 products.
 //
 //   warps 0..4*NT-1  softmax, rescaling of O, epilogue: one query row per thread
 //   then one TMA producer warp and one MMA warp
@@ -34,14 +37,13 @@ template <int DH, int NT, int BKV, int KS, int VS>
 struct AttnCfg {
   static constexpr int THREADS = NT * 128 + 64;
   static constexpr int TMA_WARP = NT * 4, MMA_WARP = NT * 4 + 1;
-  static constexpr int SB = 3 - NT;                    // score buffers of one tile
   static constexpr int QT_BYTES = 128 * DH * 2;
   static constexpr int KV_BYTES = BKV * DH * 2;        // one of K or V
   static constexpr int OFF_K = NT * QT_BYTES;
   static constexpr int OFF_V = OFF_K + KS * KV_BYTES;
   static constexpr int OFF_BAR = OFF_V + VS * KV_BYTES;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
-  static constexpr int TM_O = 2 * BKV;                 // behind the two score buffers
+  static constexpr int TM_O = NT * 2 * BKV;            // behind the two score buffers of each tile
   static_assert(TM_O + NT * DH <= 512, "TMEM budget");
   static_assert(SMEM <= 232448, "shared memory budget");
 };
@@ -61,21 +63,21 @@ __global__ void __launch_bounds__(NT * 128 + 64, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
   using Cfg = AttnCfg<DH, NT, BKV, KS, VS>;
-  constexpr int SB = Cfg::SB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
-  uint64_t* q_full = bars;          // 1
-  uint64_t* k_full = bars + 1;      // 3
-  uint64_t* k_empty = bars + 4;     // 3
-  uint64_t* v_full = bars + 7;      // 3
-  uint64_t* v_empty = bars + 10;    // 3
-  uint64_t* s_full = bars + 13;     // 2: by tile, or by buffer of the one tile
-  uint64_t* p_full = bars + 15;     // 2: by tile
-  uint64_t* o_done = bars + 17;     // 2: by tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
-  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 21);
+  uint64_t* q_full = bars;                // 1
+  uint64_t* k_full = bars + 1;            // KS
+  uint64_t* k_empty = k_full + KS;        // KS
+  uint64_t* v_full = k_empty + KS;        // VS
+  uint64_t* v_empty = v_full + VS;        // VS
+  uint64_t* s_full = v_empty + VS;        // [tile][buffer]
+  uint64_t* p_full = s_full + 2 * NT;     // by tile
+  uint64_t* o_done = p_full + NT;         // by tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + NT);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(o_done + NT + 1);
+  static_assert((1 + 2 * KS + 2 * VS + 4 * NT + 3) * 8 <= 256, "barrier space");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -86,8 +88,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(q_full, 1);
     for (int i = 0; i < KS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < VS; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&s_full[i], 1);
+    for (int i = 0; i < NT; ++i) {
+      mbar_init(&s_full[2 * i], 1);
+      mbar_init(&s_full[2 * i + 1], 1);
       mbar_init(&p_full[i], 4);
       mbar_init(&o_done[i], 1);
     }
@@ -152,7 +155,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // products of one issuing thread run in order: S may be issued over the P that the P V product
       // before it reads
       auto issue_s = [&](int i, int j) {
-        const int b = NT == 2 ? i : (j & 1);
+        const int b = 2 * i + (j & 1);
         const uint32_t a = sq + i * Cfg::QT_BYTES, k = sk0 + (j % KS) * Cfg::KV_BYTES;
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk)
@@ -175,27 +178,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int j = 0; j < n_max && ok; ++j) {
         const bool more = j + 1 < n_max;
         if (more) ok = wait_k(j + 1);
-        if (ok && SB == 2 && more) { issue_s(0, j + 1); umma_commit(&k_empty[(j + 1) % KS]); }
         if (ok) ok = mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL);
         if (!ok) break;
         const uint32_t v = sv0 + (j % VS) * Cfg::KV_BYTES;
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
+          if (j + 1 < n_kv[i]) issue_s(i, j + 1);
+          if (more && i == NT - 1) umma_commit(&k_empty[(j + 1) % KS]);
           if (j >= n_kv[i]) continue;
           ok = mbar_wait(&p_full[i], j & 1, p.status, KS_TIMEOUT_FULL);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t pa = tmem_base + (NT == 2 ? i : (j & 1)) * BKV;
+          const uint32_t pa = tmem_base + (2 * i + (j & 1)) * BKV;
 #pragma unroll
           for (int kk = 0; kk < BKV / 16; ++kk)
             umma_bf16_ts(tmem_base + Cfg::TM_O + i * DH, pa + kk * 8,
                          umma_smem_desc(v + kk * (16 * 128), BKV * 128, 1024), idesc_o, (j | kk) != 0);
-          if (NT == 1 || j + 1 == n_kv[i]) umma_commit(&o_done[i]);
-          if (SB == 1 && j + 1 < n_kv[i]) issue_s(i, j + 1);
+          umma_commit(&o_done[i]);
         }
         if (!ok) break;
         umma_commit(&v_empty[j % VS]);
-        if (SB == 1 && more) umma_commit(&k_empty[(j + 1) % KS]);
       }
     }
   } else {
@@ -212,9 +214,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float l = 0.f;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      const int b = NT == 2 ? tile : (j & 1);
+      const int b = 2 * tile + (j & 1);
       const uint32_t s_addr = lane_addr + b * BKV;
-      if (!mbar_wait(&s_full[b], (NT == 2 ? j : (j >> 1)) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait(&s_full[b], (j >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       float s[BKV];
 #pragma unroll
@@ -248,9 +250,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const float alpha = m_used == -INFINITY ? 0.f : fast_exp2(m_used - m_new);
         m_used = m_new;
         l *= alpha;
-        // O of the steps before this one is complete: with two tiles S of this step was issued after
-        // the last P V of its tile, with one tile that product has a barrier of its own
-        if (NT == 1 && !mbar_wait(&o_done[0], (j - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        if (!mbar_wait(&o_done[tile], (j - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int x = 0; x < DH; x += 32) {
@@ -288,7 +288,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (lane == 0) mbar_arrive(&p_full[tile]);
     }
     // ---------------------------------------------------------------- epilogue
-    if (ok && n > 0 && mbar_wait(&o_done[tile], NT == 1 ? (n - 1) & 1 : 0, p.status, KS_TIMEOUT_TMEM_FULL)) {
+    if (ok && n > 0 && mbar_wait(&o_done[tile], (n - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const bool valid = gq < seq_end;
@@ -356,8 +356,8 @@ extern "C" int ss_attn_fwd(const void* q, const void* k, const void* v, void* ou
   p.out = out; p.lse = lse; p.cu_seqlens = cu_seqlens; p.nseq = nseq; p.T = T; p.Hq = Hq;
   p.Hkv = Hkv; p.ldo = ldo; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (dh == 128) return launch_fwd<128, 2, 128, 3, 2>(q, k, v, p, ldq, ldk, ldv, s);
-  if (dh == 64) return launch_fwd<64, 2, 128, 3, 3>(q, k, v, p, ldq, ldk, ldv, s);
+  if (dh == 128) return launch_fwd<128, 2, 64, 4, 4>(q, k, v, p, ldq, ldk, ldv, s);
+  if (dh == 64) return launch_fwd<64, 2, 64, 4, 4>(q, k, v, p, ldq, ldk, ldv, s);
   if (dh == 256) return launch_fwd<256, 1, 64, 3, 2>(q, k, v, p, ldq, ldk, ldv, s);
   return -2;
 }
