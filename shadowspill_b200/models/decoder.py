@@ -347,13 +347,10 @@ class DenseLayerStage(Stage):
         T = qkv.shape[0]
         dh, Hq, Hkv = c.head_dim, c.n_heads, c.n_kv_heads
         # keep the pre-norm q/k for the backward pass
-        I["qk_raw"] = qkv[:, :(Hq + Hkv) * dh].clone()
-        qv = qkv[:, :Hq * dh].reshape(T * Hq, dh)
-        kv = qkv[:, Hq * dh:(Hq + Hkv) * dh].reshape(T * Hkv, dh)
-        qn, I["q_rstd"] = F.rmsnorm_fwd(qv, P["q_norm"], c.norm_epsilon, c.zero_centered_norm)
-        kn, I["k_rstd"] = F.rmsnorm_fwd(kv, P["k_norm"], c.norm_epsilon, c.zero_centered_norm)
-        qkv[:, :Hq * dh] = qn.view(T, Hq * dh)
-        qkv[:, Hq * dh:(Hq + Hkv) * dh] = kn.view(T, Hkv * dh)
+        nq, n = Hq * dh, (Hq + Hkv) * dh
+        raw = I["qk_raw"] = torch.empty((T, n), dtype=qkv.dtype, device=qkv.device)
+        I["q_rstd"] = F.head_norm_(qkv[:, :nq], P["q_norm"], Hq, c.norm_epsilon, c.zero_centered_norm, raw=raw[:, :nq])
+        I["k_rstd"] = F.head_norm_(qkv[:, nq:n], P["k_norm"], Hkv, c.norm_epsilon, c.zero_centered_norm, raw=raw[:, nq:])
 
     def forward(self, P, x, meta: BatchMeta, keep: tuple[str, ...] = (), out=None, saved_out=None):
         """Returns ``(y, saved)`` where ``saved`` holds the intermediates named in ``keep``.
@@ -430,14 +427,9 @@ class DenseLayerStage(Stage):
         T = dqkv.shape[0]
         dh, Hq, Hkv = c.head_dim, c.n_heads, c.n_kv_heads
         raw = I["qk_raw"]
-        dqn = dqkv[:, :Hq * dh].reshape(T * Hq, dh)
-        dkn = dqkv[:, Hq * dh:(Hq + Hkv) * dh].reshape(T * Hkv, dh)
-        dq = F.rmsnorm_bwd(raw[:, :Hq * dh].reshape(T * Hq, dh), P["q_norm"], dqn, I["q_rstd"],
-                           G["q_norm"], c.zero_centered_norm)
-        dk = F.rmsnorm_bwd(raw[:, Hq * dh:].reshape(T * Hkv, dh), P["k_norm"], dkn, I["k_rstd"],
-                           G["k_norm"], c.zero_centered_norm)
-        dqkv[:, :Hq * dh] = dq.view(T, Hq * dh)
-        dqkv[:, Hq * dh:(Hq + Hkv) * dh] = dk.view(T, Hkv * dh)
+        nq, n = Hq * dh, (Hq + Hkv) * dh
+        F.head_norm_bwd_(raw[:, :nq], P["q_norm"], dqkv[:, :nq], I["q_rstd"], G["q_norm"], Hq, c.zero_centered_norm)
+        F.head_norm_bwd_(raw[:, nq:], P["k_norm"], dqkv[:, nq:n], I["k_rstd"], G["k_norm"], Hkv, c.zero_centered_norm)
 
 
 def _heads(t: torch.Tensor) -> torch.Tensor:

@@ -1,11 +1,10 @@
-// Bandwidth-bound model ops for sm_100a: RMSNorm (+ fused residual add), rotary
-// embedding, SwiGLU, embedding gather / scatter-add, masked weighted cross-entropy
+// Bandwidth-bound model ops for sm_100a: rotary embedding, SwiGLU, embedding gather / scatter-add, masked weighted cross-entropy
 // over a logits block, AdamW with bf16 stochastic rounding, sum-of-squares.
 //
 // All kernels move 16-byte vectors, keep reductions in fp32 and take explicit
 // extents. The math follows the reference's pure-PyTorch definitions in
 // packages/workloads/src/shadowspill_workloads/models/shared/decoder.py
-// (RMSNorm :18, apply_rotary :232, swiglu :292, language_model_loss :320).
+// (apply_rotary :232, swiglu :292, language_model_loss :320).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -70,227 +69,6 @@ __device__ __forceinline__ float block_max(float v, float* red) {
   }
   __syncthreads();
   return red[32];
-}
-
-// =============================================================== RMSNorm forward
-// Optionally first folds `delta` into the residual stream: x <- x + delta (x is
-// rewritten), then y = x * rstd * w  (zero_centered: * (1 + w)). rstd[T] is saved.
-constexpr int NORM_THREADS = 256;
-constexpr int NORM_MAXV = 4;  // vectors of 8 per thread held in registers: D <= 8192
-
-__global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_fwd_kernel(bf16* __restrict__ x, const bf16* __restrict__ delta,
-                   const bf16* __restrict__ w, bf16* __restrict__ y, float* __restrict__ rstd,
-                   int T, int D, float eps, int zero_centered) {
-  __shared__ float red[33];
-  const int nv = D >> 3;
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    uint4* xr = reinterpret_cast<uint4*>(x + static_cast<size_t>(row) * D);
-    const uint4* dr = delta ? reinterpret_cast<const uint4*>(delta + static_cast<size_t>(row) * D)
-                            : nullptr;
-    float v[NORM_MAXV][8];
-    float ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < NORM_MAXV; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nv) {
-        unpack8(xr[c], v[i]);
-        if (dr) {
-          float d[8];
-          unpack8(dr[c], d);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[i][e] += d[e];
-          // The residual stream is kept in bf16: round once here so that the
-          // normalised value and the stored stream agree.
-          const uint4 rounded = pack8(v[i]);
-          xr[c] = rounded;
-          unpack8(rounded, v[i]);
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) ss += v[i][e] * v[i][e];
-      }
-    }
-    const float tot = block_sum(ss, red);
-    const float r = rsqrtf(tot / static_cast<float>(D) + eps);
-    if (threadIdx.x == 0 && rstd) rstd[row] = r;
-    uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * D);
-    const uint4* wr = reinterpret_cast<const uint4*>(w);
-#pragma unroll
-    for (int i = 0; i < NORM_MAXV; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nv) {
-        float ww[8], o[8];
-        unpack8(wr[c], ww);
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          o[e] = v[i][e] * r * (zero_centered ? 1.f + ww[e] : ww[e]);
-        yr[c] = pack8(o);
-      }
-    }
-  }
-}
-
-// =============================================================== RMSNorm backward
-// dx = rstd * (g*w - xhat * mean(g*w*xhat)),  dw += sum_t g * xhat   (fp32 atomics)
-// dx is ADDED into dx_acc when accumulate != 0 (residual-stream gradient).
-//
-// One warp per row, two passes over the row (the second hits L1/L2): no block barrier
-// per row and few live registers, so many rows are in flight per SM. The weight
-// gradient is accumulated with shared-memory atomics (one fp32 per column per block)
-// and flushed to global memory once per block.
-constexpr int NORM_BWD_WARPS = 8;
-__global__ void __launch_bounds__(NORM_BWD_WARPS * 32)
-rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                   const bf16* __restrict__ gy, const float* __restrict__ rstd,
-                   bf16* __restrict__ dx, float* __restrict__ dw, int T, int D, int zero_centered,
-                   int accumulate) {
-  extern __shared__ float s_dw[];          // [8][D/8]: element e of vector c at e*nv + c (conflict-free lanes)
-  const int nv = D >> 3;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (dw) {
-    for (int c = threadIdx.x; c < D; c += blockDim.x) s_dw[c] = 0.f;
-    __syncthreads();
-  }
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
-  for (int row = blockIdx.x * NORM_BWD_WARPS + warp; row < T; row += gridDim.x * NORM_BWD_WARPS) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * D);
-    const uint4* gr = reinterpret_cast<const uint4*>(gy + static_cast<size_t>(row) * D);
-    const float r = rstd[row];
-    float dot = 0.f;
-#pragma unroll 4
-    for (int c = lane; c < nv; c += 32) {
-      float xv[8], gv[8], ww[8];
-      unpack8(xr[c], xv);
-      unpack8(gr[c], gv);
-      unpack8(wr[c], ww);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float xh = xv[e] * r;
-        dot += gv[e] * (zero_centered ? 1.f + ww[e] : ww[e]) * xh;
-        if (dw) atomicAdd(&s_dw[e * nv + c], gv[e] * xh);
-      }
-    }
-    const float mean = warp_sum(dot) / static_cast<float>(D);
-    uint4* dr = reinterpret_cast<uint4*>(dx + static_cast<size_t>(row) * D);
-#pragma unroll 4
-    for (int c = lane; c < nv; c += 32) {
-      float xv[8], gv[8], ww[8], o[8];
-      unpack8(xr[c], xv);
-      unpack8(gr[c], gv);
-      unpack8(wr[c], ww);
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        o[e] = r * (gv[e] * (zero_centered ? 1.f + ww[e] : ww[e]) - xv[e] * r * mean);
-      if (accumulate) {
-        float prev[8];
-        unpack8(dr[c], prev);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] += prev[e];
-      }
-      dr[c] = pack8(o);
-    }
-  }
-  if (dw) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-      const float v = s_dw[i];
-      const int e = i / nv, c = i - e * nv;
-      if (v != 0.f) atomicAdd(dw + c * 8 + e, v);
-    }
-  }
-}
-
-// Block-per-row form for D <= 8192: a thread owns up to NORM_MAXV fixed vectors of eight columns,
-// so the row is read once (x and gy stay in registers across the row reduction) and the weight
-// gradient accumulates in registers over every row the block handles; one global atomic per
-// column per block at the end. Same arithmetic as the warp-per-row kernel above.
-template <int VPT>
-__global__ void __launch_bounds__(NORM_THREADS, VPT <= 2 ? 3 : 1)
-rmsnorm_bwd_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                        const bf16* __restrict__ gy, const float* __restrict__ rstd,
-                        bf16* __restrict__ dx, float* __restrict__ dw, int T, int D, int zero_centered,
-                        int accumulate) {
-  __shared__ float red[33];
-  const int nv = D >> 3;
-  const float wofs = zero_centered ? 1.f : 0.f;
-  uint4 wq[VPT];
-  float acc[VPT][8];
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int c = threadIdx.x + i * NORM_THREADS;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[i][e] = 0.f;
-    wq[i] = c < nv ? reinterpret_cast<const uint4*>(w)[c] : make_uint4(0, 0, 0, 0);
-  }
-  // rows are software-pipelined: the next row's x and gy are in flight while this one reduces
-  uint4 xq[VPT], gq[VPT], xn[VPT], gn[VPT];
-  auto fetch = [&](int row, uint4 (&xo)[VPT], uint4 (&go)[VPT]) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * D);
-    const uint4* gr = reinterpret_cast<const uint4*>(gy + static_cast<size_t>(row) * D);
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nv) { xo[i] = xr[c]; go[i] = gr[c]; }
-    }
-  };
-  int row = blockIdx.x;
-  if (row < T) fetch(row, xq, gq);
-  for (; row < T; row += gridDim.x) {
-    const int next = row + gridDim.x;
-    if (next < T) fetch(next, xn, gn);
-    const float r = rstd[row];
-    float dot = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nv) {
-        float xv[8], gv[8], ww[8];
-        unpack8(xq[i], xv);
-        unpack8(gq[i], gv);
-        unpack8(wq[i], ww);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float xh = xv[e] * r;
-          acc[i][e] += gv[e] * xh;
-          dot += gv[e] * (ww[e] + wofs) * xh;
-        }
-      }
-    }
-    const float mean = block_sum(dot, red) / static_cast<float>(D);
-    uint4* dr = reinterpret_cast<uint4*>(dx + static_cast<size_t>(row) * D);
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nv) {
-        float xv[8], gv[8], ww[8], o[8];
-        unpack8(xq[i], xv);
-        unpack8(gq[i], gv);
-        unpack8(wq[i], ww);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = r * (gv[e] * (ww[e] + wofs) - xv[e] * r * mean);
-        if (accumulate) {
-          float prev[8];
-          unpack8(dr[c], prev);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] += prev[e];
-        }
-        dr[c] = pack8(o);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) { xq[i] = xn[i]; gq[i] = gn[i]; }
-  }
-  if (dw) {
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nv) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          if (acc[i][e] != 0.f) atomicAdd(dw + c * 8 + e, acc[i][e]);
-      }
-    }
-  }
 }
 
 // =============================================================== rotary embedding
@@ -764,37 +542,6 @@ static inline int grid_for(long long work, int threads, int cap = 148 * 8) {
 extern "C" {
 using namespace ss;
 
-int ss_rmsnorm_fwd(void* x, const void* delta, const void* w, void* y, float* rstd, int T, int D,
-                   float eps, int zero_centered, void* stream) {
-  if (D % 8 || D > NORM_THREADS * NORM_MAXV * 8) return -2;
-  if (T <= 0) return 0;
-  rmsnorm_fwd_kernel<<<T < 148 * 8 ? T : 148 * 8, NORM_THREADS, 0, (cudaStream_t)stream>>>(
-      (bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)y, rstd, T, D, eps, zero_centered);
-  return (int)cudaGetLastError();
-}
-int ss_rmsnorm_bwd(const void* x, const void* w, const void* gy, const float* rstd, void* dx,
-                   float* dw, int T, int D, int zero_centered, int accumulate, void* stream) {
-  if (D % 8 || D > 12288) return -2;       // the block's fp32 column sums live in 48 KB of shared memory
-  if (T <= 0) return 0;
-  if (D <= NORM_THREADS * NORM_MAXV * 8 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-    const int vpt = (D / 8 + NORM_THREADS - 1) / NORM_THREADS;
-    const int grid = T < 148 * 3 ? T : 148 * 3;
-    auto launch = [&](auto kern) {
-      kern<<<grid, NORM_THREADS, 0, (cudaStream_t)stream>>>(
-          (const bf16*)x, (const bf16*)w, (const bf16*)gy, rstd, (bf16*)dx, dw, T, D, zero_centered, accumulate);
-    };
-    if (vpt <= 1) launch(rmsnorm_bwd_rows_kernel<1>);
-    else if (vpt == 2) launch(rmsnorm_bwd_rows_kernel<2>);
-    else launch(rmsnorm_bwd_rows_kernel<4>);
-    return (int)cudaGetLastError();
-  }
-  const int row_blocks = (T + NORM_BWD_WARPS - 1) / NORM_BWD_WARPS;
-  rmsnorm_bwd_kernel<<<row_blocks < 148 * 4 ? row_blocks : 148 * 4, NORM_BWD_WARPS * 32,
-                       sizeof(float) * D, (cudaStream_t)stream>>>(
-      (const bf16*)x, (const bf16*)w, (const bf16*)gy, rstd, (bf16*)dx, dw, T, D, zero_centered,
-      accumulate);
-  return (int)cudaGetLastError();
-}
 int ss_rope(void* buf, const int* positions, int T, long long row_stride, int col0, int heads,
             int dh, int rot, float theta, int inverse, void* stream) {
   if (rot % 4 || rot > dh || row_stride % 2 || col0 % 2) return -2;

@@ -224,6 +224,49 @@ def rmsnorm_bwd(x, w, gy, rstd, dw, zero_centered=False, dx=None, accumulate=Fal
     return dx
 
 
+def _heads_in_place(dh, *tensors) -> bool:
+    """Can the strided head kernels read and write these views? They move 16-byte pieces and keep a head
+    in at most two of them per lane; other views are copied to contiguous rows."""
+    return dh % 8 == 0 and dh <= 512 and all(
+        t is None or (_cuda(t) and t.dtype == _BF16 and t.stride(1) == 1 and t.stride(0) % 8 == 0
+                      and t.data_ptr() % 16 == 0) for t in tensors)
+
+
+def head_norm_(buf, w, heads, eps=1e-5, zero_centered=False, raw=None):
+    """RMSNorm of each of the ``heads`` adjacent heads in the rows of ``buf`` (``[T, heads * dh]``, a view
+    with unit inner stride), in place; ``raw`` (same shape) receives the input. Returns ``rstd``
+    ``[T * heads]``."""
+    T, dh = buf.shape[0], buf.shape[1] // heads
+    if not _heads_in_place(dh, buf, raw):
+        if raw is not None:
+            raw.copy_(buf)
+        y, rs = rmsnorm_fwd(buf.reshape(T * heads, dh), w, eps, zero_centered)
+        buf.copy_(y.view(T, heads * dh))
+        return rs
+    rs = torch.empty(T * heads, dtype=torch.float32, device=buf.device)
+    _lib.check(_lib.lib().ss_headnorm_fwd(
+        buf.data_ptr(), buf.stride(0), w.data_ptr(), buf.data_ptr(), buf.stride(0), _ptr(raw),
+        0 if raw is None else raw.stride(0), rs.data_ptr(), T, heads, dh, float(eps), int(zero_centered),
+        _lib.stream_ptr()), "ss_headnorm_fwd")
+    return rs
+
+
+def head_norm_bwd_(raw, w, dbuf, rstd, dw, heads, zero_centered=False):
+    """Rewrites ``dbuf`` (``[T, heads * dh]``, a view) with the gradient of :func:`head_norm_`'s input
+    ``raw``; ``dw`` (fp32) is accumulated in place."""
+    T, dh = dbuf.shape[0], dbuf.shape[1] // heads
+    if not _heads_in_place(dh, dbuf, raw):
+        dx = rmsnorm_bwd(raw.reshape(T * heads, dh), w, dbuf.reshape(T * heads, dh), rstd, dw, zero_centered)
+        return dbuf.copy_(dx.view(T, heads * dh))
+    if dw is not None and dw.dtype != torch.float32:
+        raise TypeError("rmsnorm dw accumulator must be fp32")
+    _lib.check(_lib.lib().ss_headnorm_bwd(
+        raw.data_ptr(), raw.stride(0), w.data_ptr(), dbuf.data_ptr(), dbuf.stride(0), rstd.data_ptr(),
+        dbuf.data_ptr(), dbuf.stride(0), _ptr(dw), T, heads, dh, int(zero_centered), _lib.stream_ptr()),
+        "ss_headnorm_bwd")
+    return dbuf
+
+
 # ------------------------------------------------------------------------ rotary
 def rope_(buf, positions, *, col0, heads, dh, rot=None, theta=10000.0, inverse=False):
     """In-place rotary on ``heads`` heads of width ``dh`` starting at column ``col0``
