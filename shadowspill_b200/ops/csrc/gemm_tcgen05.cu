@@ -17,10 +17,11 @@
 // One CTA per SM, 192 threads:
 //   warp 0      TMA producer (one elected lane)
 //   warp 1      TMEM allocator + MMA issuer (one elected lane)
-//   warps 2..5  epilogue; warp w owns TMEM lanes 32*(w%4)..+31
+//   warps 2..9  epilogue; warp w owns TMEM lanes 32*(w%4)..+31
 // Two 128x256 fp32 accumulators (2 x 256 TMEM columns) let the epilogue of tile
 // i overlap the main loop of tile i+1.
 #include "sm100_ptx.cuh"
+#include "gemm_epilogue.cuh"
 
 #include <cudaTypedefs.h>
 #include <stdio.h>
@@ -30,7 +31,7 @@ namespace ss {
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int GEMM_THREADS = 192;
+constexpr int GEMM_THREADS = 64 + EPI_WARPS * 32;
 
 template <int BN>
 struct GemmCfg {
@@ -148,7 +149,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 4);  // one arrival per epilogue warp
+      mbar_init(&tempty[a], EPI_WARPS);  // one arrival per epilogue warp
     }
     mbar_fence_init();
   }
@@ -251,6 +252,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may touch
+    const int part = (warp - 2) >> 2;    // the left or the right half of the tile's columns
+    const uint32_t stage_out = smem_u32(smem + Cfg::STAGES * Cfg::STAGE_BYTES + 256) + (warp - 2) * EPI_WARP_STAGE;
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
@@ -261,7 +264,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // an expert without rows: its gradient tile is zero (nothing to add when accumulating)
         if (!p.accumulate) {
           const int zr = mb * BM + q * 32 + lane;
-          for (int c = nb * BN; zr < p.M && c < min(p.N, (nb + 1) * BN); c += 8) {
+          for (int c = nb * BN + part * (BN / 2); zr < p.M && c < min(p.N, nb * BN + (part + 1) * (BN / 2)); c += 8) {
             if (p.c_f32) {
               float* d = reinterpret_cast<float*>(p.C) + w.c_off + static_cast<long long>(zr) * p.ldc + c;
               *reinterpret_cast<float4*>(d) = make_float4(0, 0, 0, 0);
@@ -286,7 +289,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         uint8_t* stg = smem + Cfg::STAGES * Cfg::STAGE_BYTES + 256 + q * (32 * 256);
         const long long my_dst = (row < p.M) ? p.g.row_dst[row] : 0;
 #pragma unroll 1
-        for (int half = 0; half < BN / 128; ++half) {
+        for (int half = 0; half < (part == 0 ? BN / 128 : 0); ++half) {   // one staging tile per lane quarter
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             uint32_t r[32];
@@ -319,49 +322,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       } else
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = part * (BN / 64); c < (part + 1) * (BN / 64); ++c) {
+        const int col0 = nb * BN + c * 32;
+        if (col0 >= p.N) break;
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
         tmem_ld_wait();
-        const int col0 = nb * BN + c * 32;
-        if (row < p.M && col0 < p.N) {
-          const int ncols = min(32, p.N - col0);
-          if (p.c_f32) {
-            float* dst = reinterpret_cast<float*>(p.C) + w.c_off + static_cast<long long>(row) * p.ldc + col0;
-            for (int j = 0; j < ncols; j += 4) {
-              float4 v = make_float4(__uint_as_float(r[j]) * p.alpha,
-                                     __uint_as_float(r[j + 1]) * p.alpha,
-                                     __uint_as_float(r[j + 2]) * p.alpha,
-                                     __uint_as_float(r[j + 3]) * p.alpha);
-              if (p.accumulate) {
-                const float4 o = *reinterpret_cast<const float4*>(dst + j);
-                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-              }
-              *reinterpret_cast<float4*>(dst + j) = v;
-            }
-          } else {
-            __nv_bfloat16* dst =
-                reinterpret_cast<__nv_bfloat16*>(p.C) + w.c_off + static_cast<long long>(row) * p.ldc + col0;
-            for (int j = 0; j < ncols; j += 8) {
-              float f[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[j + e]) * p.alpha;
-              if (p.accumulate) {
-                const uint4 o = *reinterpret_cast<const uint4*>(dst + j);
-                const float2 o0 = unpack_bf16(o.x), o1 = unpack_bf16(o.y), o2 = unpack_bf16(o.z),
-                             o3 = unpack_bf16(o.w);
-                f[0] += o0.x; f[1] += o0.y; f[2] += o1.x; f[3] += o1.y;
-                f[4] += o2.x; f[5] += o2.y; f[6] += o3.x; f[7] += o3.y;
-              }
-              uint4 v;
-              v.x = pack_bf16(f[0], f[1]);
-              v.y = pack_bf16(f[2], f[3]);
-              v.z = pack_bf16(f[4], f[5]);
-              v.w = pack_bf16(f[6], f[7]);
-              *reinterpret_cast<uint4*>(dst + j) = v;
-            }
-          }
-        }
+        const int row0 = mb * BM + q * 32;
+        if (p.c_f32)
+          epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C) + w.c_off, p.accumulate, p.alpha, p.ldc,
+                               row0, p.M, col0, p.N);
+        else
+          epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C) + w.c_off, p.accumulate, p.alpha,
+                               p.ldc, row0, p.M, col0, p.N);
       }
       tc_fence_before();
       __syncwarp();
@@ -447,7 +420,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
   static SmemOptIn opt_in;
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN>;
   if (int e = opt_in.ensure(kern, Cfg::SMEM + Cfg::SCATTER_STAGE)) return e;
-  const int smem_bytes = Cfg::SMEM + (p.g.row_dst != nullptr ? Cfg::SCATTER_STAGE : 0);
+  const int smem_bytes = Cfg::SMEM + (p.g.row_dst != nullptr ? Cfg::SCATTER_STAGE : EPI_WARPS * EPI_WARP_STAGE);
   const long long tiles = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) *
                           (p.g.mode == 2 ? p.g.n_experts : 1);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;

@@ -13,7 +13,7 @@
 //   warp 0      TMA producer of this CTA's operands; the byte counts of BOTH CTAs
 //               complete on the LEADER's (rank 0) full barrier
 //   warp 1      TMEM allocator; in the leader also the MMA issuer for the pair
-//   warps 2..5  epilogue of this CTA's 128 rows
+//   warps 2..9  epilogue of this CTA's 128 rows
 // The leader's tcgen05.commit multicasts "stage free" and "accumulator ready" to the
 // same barrier in both CTAs; the peer's epilogue warps arrive remotely on the leader's
 // "accumulator drained" barrier. Every wait is bounded (status word); both CTAs always
@@ -34,6 +34,7 @@
 // fp32 output); reference: shadowspill::accumulate_matmul_
 // (packages/engine/src/shadowspill/pytorch/operations.py:15).
 #include "sm100_ptx.cuh"
+#include "gemm_epilogue.cuh"
 
 #include <cudaTypedefs.h>
 
@@ -50,12 +51,12 @@ constexpr int BM = 128;          // rows per CTA (256 per pair)
 constexpr int BN = 256;          // columns per pair tile; each CTA stages BN/2 rows of B
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int THREADS = 192;
+constexpr int THREADS = 64 + EPI_WARPS * 32;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int B_BYTES = (BN / 2) * BK * 2;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;       // 32 KB per CTA per stage
-constexpr int STAGES = 7;
-constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+constexpr int STAGES = 6;
+constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + EPI_WARPS * EPI_WARP_STAGE;
 constexpr int TMEM_COLS = 2 * BN;
 
 struct Params {
@@ -67,7 +68,7 @@ struct Params {
   int* status;
 };
 
-constexpr int GATHER_THREADS = 128;                  // warps 6..9 of the GATHER form
+constexpr int GATHER_THREADS = 128;                  // warps 10..13 of the GATHER form
 constexpr int PIECE_BYTES = 32768;
 constexpr int MAX_RANKS = 16;
 
@@ -181,7 +182,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* full = bars;                    // used in the leader only
   uint64_t* empty = bars + STAGES;          // per CTA, signalled by the leader's commit
   uint64_t* tfull = bars + 2 * STAGES;      // per CTA, signalled by the leader's commit
-  uint64_t* tempty = tfull + 2;             // leader only: 8 arrivals (4 warps x 2 CTAs)
+  uint64_t* tempty = tfull + 2;             // leader only: the epilogue warps of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
   const int warp = threadIdx.x >> 5;
@@ -204,7 +205,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 8);
+      mbar_init(&tempty[a], 2 * EPI_WARPS);
     }
     mbar_fence_init();
   }
@@ -303,9 +304,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
-  } else if (warp < 6) {
+  } else if (warp < 2 + EPI_WARPS) {
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
+    const uint32_t stage_out = smem_u32(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * EPI_WARP_STAGE;
+    const int part = (warp - 2) >> 2;    // the left or the right half of the tile's columns
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = pair_id; t < num_tiles; t += num_pairs) {
@@ -313,51 +316,22 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tile_coords<GATHER>(t, num_m, num_n, mb, nb);
       if (!mbar_wait(&tfull[acc], acc_phase, p.status, KS_TIMEOUT_TMEM_FULL)) break;
       tc_fence_after();
-      const int row = mb * (2 * BM) + static_cast<int>(rank) * BM + q * 32 + lane;
+      const int row0 = mb * (2 * BM) + static_cast<int>(rank) * BM + q * 32;
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = part * (BN / 64); c < (part + 1) * (BN / 64); ++c) {
+        const int col0 = nb * BN + c * 32;
+        if (col0 >= p.N) break;
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
         tmem_ld_wait();
-        const int col0 = nb * BN + c * 32;
-        if (row < p.M && col0 < p.N) {
-          const int ncols = min(32, p.N - col0);
-          if (p.c_f32) {
-            float* dst = reinterpret_cast<float*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
-            for (int j = 0; j < ncols; j += 4) {
-              float4 v = make_float4(__uint_as_float(r[j]) * p.alpha, __uint_as_float(r[j + 1]) * p.alpha,
-                                     __uint_as_float(r[j + 2]) * p.alpha, __uint_as_float(r[j + 3]) * p.alpha);
-              if (p.accumulate) {
-                const float4 o = *reinterpret_cast<const float4*>(dst + j);
-                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-              }
-              *reinterpret_cast<float4*>(dst + j) = v;
-            }
-          } else {
-            __nv_bfloat16* dst =
-                reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
-            for (int j = 0; j < ncols; j += 8) {
-              float f[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[j + e]) * p.alpha;
-              if (p.accumulate) {
-                const uint4 o = *reinterpret_cast<const uint4*>(dst + j);
-                const float2 o0 = unpack_bf16(o.x), o1 = unpack_bf16(o.y), o2 = unpack_bf16(o.z),
-                             o3 = unpack_bf16(o.w);
-                f[0] += o0.x; f[1] += o0.y; f[2] += o1.x; f[3] += o1.y;
-                f[4] += o2.x; f[5] += o2.y; f[6] += o3.x; f[7] += o3.y;
-              }
-              uint4 v;
-              v.x = pack_bf16(f[0], f[1]);
-              v.y = pack_bf16(f[2], f[3]);
-              v.z = pack_bf16(f[4], f[5]);
-              v.w = pack_bf16(f[6], f[7]);
-              *reinterpret_cast<uint4*>(dst + j) = v;
-            }
-          }
-        }
+        if (p.c_f32)
+          epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C), p.accumulate, p.alpha, p.ldc, row0, p.M,
+                               col0, p.N);
+        else
+          epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C), p.accumulate, p.alpha, p.ldc, row0,
+                               p.M, col0, p.N);
       }
       tc_fence_before();
       __syncwarp();

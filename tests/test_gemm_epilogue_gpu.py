@@ -1,0 +1,32 @@
+"""GEMM outputs at the edges of the epilogue's 32 x 16 blocks, written and accumulated, bf16 and fp32,
+into a wider buffer whose other columns must not change; both GEMM kernels."""
+import pytest
+import torch
+
+from shadowspill_b200.ops import _lib, functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 31, 128, 161, 255, 257, 400])
+@pytest.mark.parametrize("N", [8, 24, 128, 136, 264, 520])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_edges(M, N, dtype):
+    g = torch.Generator().manual_seed(M * 1000 + N)
+    K = 72
+    a = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
+    b = torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
+    wide = torch.randn(M, N + 16, generator=g).to(dtype).cuda()
+    before = wide.clone()
+    out = wide[:, 8:8 + N]
+    ref = a.double() @ b.double().t()
+    # one rounding to the output type (2^-9 for bf16) on top of fp32 sums of 72 products
+    tol = 4e-3 if dtype == torch.bfloat16 else 1e-5
+    scale = float(ref.abs().max())
+    F.gemm(a, b, out=out, alpha=0.5)
+    assert float((out.double() - 0.5 * ref).abs().max()) <= tol * scale
+    first = out.clone()
+    F.gemm(a, b, out=out, accumulate=True)
+    assert float((out.double() - (first.double() + ref)).abs().max()) <= 2 * tol * scale
+    assert torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, 8 + N:], before[:, 8 + N:])
+    _lib.check_status()
