@@ -185,8 +185,11 @@ __device__ __forceinline__ void split_index(long long idx, int nv, long long& t,
 // =============================================================== SwiGLU
 // gu is [T, 2F] with gate in columns [0,F) and up in [F,2F) (one fused GEMM
 // output). h = bf16(silu(float(gate))) * up.
-__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ h, int T, int F) {
+// `used` (optional, device memory): rows at and past *used are left alone.
+__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ h, int T, int F,
+                                  const int* __restrict__ used) {
   const int nv = F >> 3;
+  if (used) T = min(T, *used);
   const long long total = static_cast<long long>(T) * nv;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
        idx += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -564,7 +567,15 @@ int ss_swiglu_fwd(const void* gu, void* h, int T, int F, void* stream) {
   if (F % 8) return -2;
   if (T <= 0) return 0;
   swiglu_fwd_kernel<<<grid_for((long long)T * (F >> 3), 256, 148 * 16), 256, 0,
-                      (cudaStream_t)stream>>>((const bf16*)gu, (bf16*)h, T, F);
+                      (cudaStream_t)stream>>>((const bf16*)gu, (bf16*)h, T, F, nullptr);
+  return (int)cudaGetLastError();
+}
+// The first *used rows only (`used` in device memory): sorted expert rows, whose count the host does not know.
+int ss_swiglu_fwd_used(const void* gu, void* h, int T, int F, const int* used, void* stream) {
+  if (F % 8) return -2;
+  if (T <= 0) return 0;
+  swiglu_fwd_kernel<<<grid_for((long long)T * (F >> 3), 256, 148 * 16), 256, 0, (cudaStream_t)stream>>>(
+      (const bf16*)gu, (bf16*)h, T, F, used);
   return (int)cudaGetLastError();
 }
 int ss_swiglu_bwd(const void* gu, const void* dh, void* dgu, int T, int F, void* stream) {

@@ -13,15 +13,19 @@ from __future__ import annotations
 import torch
 
 from . import _lib
-from . import functional as F
 
 _c = _lib
 _lib.register("ss_moe_route", [_c.c_p, _c.c_ll, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_p,
                                _c.c_p, _c.c_p, _c.c_p])
 _lib.register("ss_moe_layout", [_c.c_p, _c.c_p, _c.c_int, _c.c_int, _c.c_int, _c.c_p, _c.c_p,
-                                _c.c_int, _c.c_p, _c.c_p, _c.c_p])
-_lib.register("ss_moe_gather", [_c.c_p, _c.c_ll, _c.c_p, _c.c_p, _c.c_p, _c.c_ll, _c.c_int,
+                                _c.c_int, _c.c_p, _c.c_p, _c.c_p, _c.c_int, _c.c_p])
+_lib.register("ss_moe_route_bwd", [_c.c_p, _c.c_ll, _c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_int, _c.c_int, _c.c_int,
+                                   _c.c_int, _c.c_p])
+_lib.register("ss_moe_gather", [_c.c_p, _c.c_ll, _c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_ll, _c.c_int,
                                 _c.c_int, _c.c_int, _c.c_p])
+_lib.register("ss_moe_act_bwd", [_c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_int, _c.c_int,
+                                 _c.c_p])
+_lib.register("ss_swiglu_fwd_used", [_c.c_p, _c.c_p, _c.c_int, _c.c_int, _c.c_p, _c.c_p])
 _lib.register("ss_moe_combine", [_c.c_p, _c.c_ll, _c.c_p, _c.c_p, _c.c_p, _c.c_ll, _c.c_int,
                                  _c.c_int, _c.c_int, _c.c_int, _c.c_p, _c.c_ll, _c.c_p, _c.c_p])
 _lib.register("ss_gemm_grouped_bf16", [_c.c_p, _c.c_p, _c.c_p, _c.c_int, _c.c_int, _c.c_int,
@@ -42,6 +46,17 @@ def route(logits: torch.Tensor, k: int, renormalize: bool):
     return ids, wts, counts
 
 
+def route_bwd(logits: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, dwts: torch.Tensor,
+              renormalize: bool) -> torch.Tensor:
+    """Gradient of ``route``'s weights, fp32 [T,k], as a gradient of its logits, fp32 [T,E]."""
+    T, E = logits.shape
+    dlogits = torch.empty((T, E), dtype=torch.float32, device=logits.device)
+    _lib.check(_lib.lib().ss_moe_route_bwd(logits.data_ptr(), logits.stride(0), ids.data_ptr(), wts.data_ptr(),
+                                           dwts.data_ptr(), dlogits.data_ptr(), T, E, ids.shape[1],
+                                           int(renormalize), _lib.stream_ptr()), "ss_moe_route_bwd")
+    return dlogits
+
+
 class Layout:
     """Expert-sorted row layout of one routing decision."""
 
@@ -55,20 +70,41 @@ class Layout:
         self.offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
         self.tile_expert = torch.empty(self.tiles, dtype=torch.int32, device=dev)
         self.dest = torch.empty(T * k, dtype=torch.int32, device=dev)
+        self.src = torch.empty(self.rows, dtype=torch.int32, device=dev)     # inverse of dest, -1 = padding
+        self.used = self.offsets[E:]                         # rows in use; the rest are never read
         cursor = torch.empty(E, dtype=torch.int32, device=dev)
         _lib.check(_lib.lib().ss_moe_layout(counts.data_ptr(), ids.data_ptr(), T, E, k,
                                             self.offsets.data_ptr(), self.tile_expert.data_ptr(),
                                             self.tiles, cursor.data_ptr(), self.dest.data_ptr(),
-                                            _lib.stream_ptr()), "ss_moe_layout")
+                                            self.src.data_ptr(), self.rows, _lib.stream_ptr()), "ss_moe_layout")
 
     def gather(self, x: torch.Tensor, weights: torch.Tensor | None = None) -> torch.Tensor:
-        """Token rows -> zero-padded expert-sorted rows (scaled by ``weights`` when given)."""
-        out = torch.zeros((self.rows, x.shape[1]), dtype=x.dtype, device=x.device)
-        _lib.check(_lib.lib().ss_moe_gather(x.data_ptr(), x.stride(0), self.dest.data_ptr(),
+        """Token rows -> zero-padded expert-sorted rows (scaled by ``weights`` when given); rows past
+        the last expert's segment are not written."""
+        out = torch.empty((self.rows, x.shape[1]), dtype=x.dtype, device=x.device)
+        _lib.check(_lib.lib().ss_moe_gather(x.data_ptr(), x.stride(0), self.src.data_ptr(), self.used.data_ptr(),
                                             None if weights is None else weights.data_ptr(),
-                                            out.data_ptr(), out.stride(0), self.T, self.k,
+                                            out.data_ptr(), out.stride(0), self.rows, self.k,
                                             x.shape[1], _lib.stream_ptr()), "ss_moe_gather")
         return out
+
+    def swiglu(self, gu: torch.Tensor) -> torch.Tensor:
+        """``silu(gate) * up`` of the rows in use."""
+        F2 = gu.shape[1]
+        h = torch.empty((self.rows, F2 // 2), dtype=gu.dtype, device=gu.device)
+        _lib.check(_lib.lib().ss_swiglu_fwd_used(gu.data_ptr(), h.data_ptr(), self.rows, F2 // 2,
+                                                 self.used.data_ptr(), _lib.stream_ptr()), "ss_swiglu_fwd_used")
+        return h
+
+    def act_bwd(self, gu: torch.Tensor, d: torch.Tensor, weights: torch.Tensor):
+        """Backward of ``weight * swiglu(gu)`` for the unweighted gradient ``d`` of the activation rows:
+        ``(dgu, weight * h, <d, h>)``, the last per assignment."""
+        dgu, hw = torch.empty_like(gu), torch.empty_like(d)
+        dots = torch.empty((self.T, self.k), dtype=torch.float32, device=gu.device)
+        _lib.check(_lib.lib().ss_moe_act_bwd(gu.data_ptr(), d.data_ptr(), self.src.data_ptr(), self.used.data_ptr(),
+                                             weights.data_ptr(), dgu.data_ptr(), hw.data_ptr(), dots.data_ptr(),
+                                             self.rows, d.shape[1], _lib.stream_ptr()), "ss_moe_act_bwd")
+        return dgu, hw, dots
 
     def combine(self, y: torch.Tensor, weights: torch.Tensor | None, out: torch.Tensor | None = None,
                 accumulate: bool = False, dots_with: torch.Tensor | None = None,
@@ -133,7 +169,7 @@ class _Experts(torch.autograd.Function):
         lay = Layout(ids, counts)
         xs = lay.gather(h)
         gu = grouped_linear(xs, w13, lay)
-        ys = grouped_linear(F.swiglu_fwd(gu), w2, lay)
+        ys = grouped_linear(lay.swiglu(gu), w2, lay)
         out = lay.combine(ys, wts)
         ctx.save_for_backward(logits, ids, wts, xs, gu, w13, w2)
         ctx.lay, ctx.sink, ctx.renormalize = lay, sink, renormalize
@@ -144,25 +180,20 @@ class _Experts(torch.autograd.Function):
         logits, ids, wts, xs, gu, w13, w2 = ctx.saved_tensors
         lay, sink = ctx.lay, ctx.sink
         dout = dout.contiguous()
-        hm = F.swiglu_fwd(gu)
-        ys = grouped_linear(hm, w2, lay)
-        _, dwts = lay.combine(ys, None, dots_with=dout, only_dots=True)
-        del ys
-        dys = lay.gather(dout, wts)                      # w * dout at every assignment
+        # the expert outputs are not formed again: <dout, h w2^T> = <dout w2, h>, and the routing weight
+        # of a row goes with h, not with dout, into w2's gradient
+        dos = lay.gather(dout)
+        d = grouped_linear(dos, w2, lay, transpose=True)
+        dgu, hw, dwts = lay.act_bwd(gu, d, wts)
+        del d
         if sink is not None and sink.wants("w2"):            # a frozen bank has no gradient buffer
-            grouped_wgrad(dys, hm, lay, sink.G["w2"], sink.accumulate("w2"))
-        dhm = grouped_linear(dys, w2, lay, transpose=True)
-        del dys, hm
-        dgu = F.swiglu_bwd(gu, dhm)
-        del dhm
+            grouped_wgrad(dos, hw, lay, sink.G["w2"], sink.accumulate("w2"))
+        del dos, hw
         if sink is not None and sink.wants("w13"):
             grouped_wgrad(dgu, xs, lay, sink.G["w13"], sink.accumulate("w13"))
         dxs = grouped_linear(dgu, w13, lay, transpose=True)
         dh = lay.combine(dxs, None)
-        with torch.enable_grad():
-            l = logits.detach().requires_grad_(True)
-            _weights_from_logits(l, ids.long(), ctx.renormalize).backward(dwts)
-        return dh, l.grad, None, None, None, None, None
+        return dh, route_bwd(logits, ids, wts, dwts, ctx.renormalize), None, None, None, None, None
 
 
 def experts(h, logits, w13, w2, k: int, renormalize: bool, sink):

@@ -1,0 +1,68 @@
+"""Sorted expert rows: layout and its inverse, padding, the activation's backward and the router's
+gradient, from one token to many blocks, with idle and crowded experts."""
+import pytest
+import torch
+import torch.nn.functional as TF
+
+from shadowspill_b200.ops import _lib, moe
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+SHAPES = [(1, 1, 1), (1, 8, 2), (33, 8, 8), (700, 64, 8), (513, 65, 3), (300, 128, 8), (90, 512, 32), (5000, 16, 4)]
+
+
+def _route(T, E, k, renorm, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed + T)
+    logits = torch.randn(T, E, generator=g, device=DEV) + 3.0 * torch.randn(1, E, generator=g, device=DEV)
+    return g, logits, *moe.route(logits, k, renorm)
+
+
+@pytest.mark.parametrize("T,E,k", SHAPES)
+def test_layout_gather_and_activation(T, E, k):
+    g, logits, ids, wts, counts = _route(T, E, k, False)
+    assert torch.equal(counts.long(), torch.bincount(ids.reshape(-1).long(), minlength=E))
+    lay = moe.Layout(ids, counts)
+    off, dest, src = lay.offsets.tolist(), lay.dest.long(), lay.src.long()
+    used = off[-1]
+    assert off[0] == 0 and [b - a for a, b in zip(off, off[1:])] == [-(-n // 128) * 128 for n in counts.tolist()]
+    assert torch.equal(src[dest], torch.arange(T * k, device=DEV)) and int((src >= 0).sum()) == T * k
+    start = lay.offsets.long()[ids.reshape(-1).long()]
+    assert bool(((dest >= start) & (dest < start + counts.long()[ids.reshape(-1).long()])).all())
+    x = torch.randn(T, 72, generator=g, device=DEV).to(torch.bfloat16)
+    xs = lay.gather(x)[:used]
+    real = src[:used] >= 0
+    assert torch.equal(xs[real], x[src[:used][real] // k]) and not bool(xs[~real].any())
+    # activation backward against autograd in fp64 on the same bf16 inputs
+    Fw = 136
+    gu = torch.zeros(lay.rows, 2 * Fw, dtype=torch.bfloat16, device=DEV)
+    d = torch.zeros(lay.rows, Fw, dtype=torch.bfloat16, device=DEV)
+    rows = dest
+    gu[rows] = torch.randn(T * k, 2 * Fw, generator=g, device=DEV).to(torch.bfloat16)
+    d[rows] = torch.randn(T * k, Fw, generator=g, device=DEV).to(torch.bfloat16)
+    h = lay.swiglu(gu)
+    dgu, hw, dots = lay.act_bwd(gu, d, wts)
+    _lib.check_status()
+    leaf = gu[rows].double().requires_grad_(True)
+    href = TF.silu(leaf[:, :Fw]) * leaf[:, Fw:]
+    w = wts.double().reshape(-1, 1)
+    (want,) = torch.autograd.grad(href, leaf, w * d[rows].double())
+    rel = lambda a, b: float((a.double() - b).norm() / (b.norm() + 1e-30))
+    # silu and h are rounded to bf16 (2^-9 each), the results once more
+    assert rel(h[rows], href.detach()) < 8e-3 and rel(dgu[rows], want) < 8e-3
+    assert rel(hw[rows], w * href.detach()) < 8e-3
+    assert rel(dots.reshape(-1), (d[rows].double() * h[rows].double()).sum(1)) < 1e-5
+    pad = torch.nonzero(~real).reshape(-1)
+    assert not bool(dgu[pad].any()) and not bool(hw[pad].any())
+
+
+@pytest.mark.parametrize("T,E,k", SHAPES)
+@pytest.mark.parametrize("renorm", [True, False])
+def test_router_gradient(T, E, k, renorm):
+    g, logits, ids, wts, _ = _route(T, E, k, renorm, seed=3)
+    dwts = torch.randn(T, k, generator=g, device=DEV)
+    got = moe.route_bwd(logits, ids, wts, dwts, renorm)
+    leaf = logits.double().requires_grad_(True)
+    moe._weights_from_logits(leaf, ids.long(), renorm).backward(dwts.double())
+    # fp32 weights and sums; for one expert or one pick the exact gradient may be zero
+    assert float((got.double() - leaf.grad).abs().max()) < 1e-5 * (1.0 + float(leaf.grad.abs().max()))
