@@ -145,13 +145,17 @@ struct PrepParams {
   Geo geo; float scale; int* status;
 };
 namespace prep {
-constexpr int OFF_KQ = 0, OFF_V = 32768, OFF_XW = 65536, OFF_XU = 81920, OFF_AF = 98304;
-constexpr int OFF_MISC = OFF_AF + 2 * 64 * 65 * 4;      // 131584
+// A (fp32) and, once the inverse has been formed from it, the two operands share one region: two CTAs
+// fit an SM, and one's substitution runs under the other's loads and stores.
+constexpr int AP = 68;                                  // pitch of A: rows 16-byte aligned for float4 reads
+constexpr int OFF_KQ = 0, OFF_V = 32768, OFF_XW = 65536, OFF_XU = 81920, OFF_AF = 65536;
+constexpr int OFF_MISC = OFF_AF + 2 * 64 * AP * 4;      // 100352
 constexpr int OFF_BAR = OFF_MISC + 2048;
 constexpr int SMEM = OFF_BAR + 64 + 1024;
+static_assert(2 * (SMEM + 1024) <= 233472, "two CTAs per SM");
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(THREADS, 2)
 dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const PrepParams p) {
   using namespace prep;
@@ -175,7 +179,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   const int t0 = c * CH;
 
   if (tid == 0) { mbar_init(tma_bar, 1); mbar_init(mma_bar, 1); mbar_fence_init(); }
-  if (warp == 4) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 4) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -237,7 +241,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     if (tid < 64) {
       for (int hh = 0; hh < nh; ++hh) {
         const float gt = gam_s[hh * 64 + t], bt = beta_s[hh * 64 + t];
-        float* a = Af + hh * 64 * 65 + t * 65;
+        float* a = Af + (hh * 64 + t) * AP;
 #pragma unroll
         for (int i = 0; i < 64; ++i)
           a[i] = (i < t && sid_s[i] == my) ? bt * __expf(gt - gam_s[hh * 64 + i]) * row[i] : 0.f;
@@ -258,21 +262,27 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   // ---- Tm = (I + A)^-1: thread (hh, j) owns column j
   if (tid < 128) {
     const int hh = tid >> 6, j = tid & 63;
+    float col[64];
     if (hh < nh) {
-      float col[64];
-      const float* A = Af + hh * 64 * 65;
+      const float* A = Af + hh * 64 * AP;
 #pragma unroll
       for (int t = 0; t < 64; ++t) {
         float a0 = (t == j) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-        const float* ar = A + t * 65;
+        const float4* ar = reinterpret_cast<const float4*>(A + t * AP);
+        // row t is zero from column t on, so whole groups of four may be read past t - 1
 #pragma unroll
-        for (int i = 0; i < t; ++i) {
-          const float v = ar[i] * col[i];
-          if ((i & 3) == 0) a0 -= v; else if ((i & 3) == 1) a1 -= v;
-          else if ((i & 3) == 2) a2 -= v; else a3 -= v;
+        for (int i = 0; i < t; i += 4) {
+          const float4 v = ar[i >> 2];
+          a0 -= v.x * col[i];
+          if (i + 1 < t) a1 -= v.y * col[i + 1];
+          if (i + 2 < t) a2 -= v.z * col[i + 2];
+          if (i + 3 < t) a3 -= v.w * col[i + 3];
         }
         col[t] = (a0 + a1) + (a2 + a3);
       }
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");      // A has been read: its region takes the operands
+    if (hh < nh) {
       const float bj = beta_s[tid];
       const float gtj = (sid_s[j] == sid_s[64]) ? __expf(gam_s[tid]) : 0.f;
       const int row = hh * 64 + j;
@@ -303,11 +313,11 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     for (int hh = 0; hh < nh; ++hh) {
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem_base + 64 + hh * 64, umma_smem_desc(sk + kk * 2048, 16384, 1024),
+        umma_bf16(tmem_base + hh * 64, umma_smem_desc(sk + kk * 2048, 16384, 1024),
                   umma_smem_desc(sxw + hh * 8192 + kk * 2048, 8192, 1024), idesc, kk != 0);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem_base + 192 + hh * 64, umma_smem_desc(sv + hh * 16384 + kk * 2048, 8192, 1024),
+        umma_bf16(tmem_base + 128 + hh * 64, umma_smem_desc(sv + hh * 16384 + kk * 2048, 8192, 1024),
                   umma_smem_desc(sxu + hh * 8192 + kk * 2048, 8192, 1024), idesc, kk != 0);
     }
     umma_commit(mma_bar);
@@ -319,9 +329,9 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const long long prow = ((static_cast<long long>(c) * G.NP + pr) * 128 + tid) * 128;
     for (int hh = 0; hh < nh; ++hh) {
       float r[64];
-      tmem_row64(lane_addr + 64 + hh * 64, r);
+      tmem_row64(lane_addr + hh * 64, r);
       store_row64(p.WTp + prow + hh * 64, r);
-      tmem_row64(lane_addr + 192 + hh * 64, r);
+      tmem_row64(lane_addr + 128 + hh * 64, r);
       store_row64(p.U0Tp + prow + hh * 64, r);
     }
     // Kd (threads 0..63, K rows) and Qg (threads 64..127, Q rows)
@@ -349,7 +359,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
 
 // ============================================================================ state walks
