@@ -160,8 +160,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmV, const PrepParams p) {
   using namespace prep;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* smem = align_smem_1024(smem_raw);
   float* Af = reinterpret_cast<float*>(smem + OFF_AF);
   float* gam_s = reinterpret_cast<float*>(smem + OFF_MISC);        // [2][64]
   float* beta_s = gam_s + 128;
@@ -427,8 +426,7 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
               const __grid_constant__ CUtensorMap tmUT, const __grid_constant__ CUtensorMap tmO, const WalkParams p) {
   using namespace walk;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* smem = align_smem_1024(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* full = bars;               // [2] a stage has arrived
   uint64_t* stage_free = bars + 2;     // [2] its products are done
@@ -620,8 +618,7 @@ dn_bwd_state_kernel(const __grid_constant__ CUtensorMap tmDO, const __grid_const
                     const __grid_constant__ CUtensorMap tmDUT, const WalkParams p) {
   using namespace walk;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* smem = align_smem_1024(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* full = bars;               // [2]
   uint64_t* stage_free = bars + 2;     // [2]
@@ -775,8 +772,7 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
                     const __grid_constant__ CUtensorMap tmDO, const ChunkParams p) {
   using namespace chunkk;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* smem = align_smem_1024(smem_raw);
   float* red = reinterpret_cast<float*>(smem + OFF_RED);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
@@ -899,8 +895,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const BwdPrepParams p) {
   using namespace bprep;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* smem = align_smem_1024(smem_raw);
   float* KKf = reinterpret_cast<float*>(smem + OFF_KKF);
   float* QKf = reinterpret_cast<float*>(smem + OFF_QKF);
   float* KKa = reinterpret_cast<float*>(smem + OFF_KKA);

@@ -176,8 +176,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + G
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const Params p, const GatherArgs ga) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* smem = align_smem_1024(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* full = bars;                    // used in the leader only
   uint64_t* empty = bars + STAGES;          // per CTA, signalled by the leader's commit

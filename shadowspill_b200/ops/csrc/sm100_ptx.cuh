@@ -53,6 +53,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The next 1024-byte boundary at or after `p` (dynamic shared memory). Rounding up through an integer
+// would lose the address space: every access through the result would be a generic one, which takes the
+// global path and several times the latency.
+__device__ __forceinline__ uint8_t* align_smem_1024(uint8_t* p) {
+  return p + ((0u - smem_u32(p)) & 1023u);
+}
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
