@@ -102,25 +102,44 @@ __device__ __forceinline__ void load_row64(const __nv_bfloat16* src, float* f) {
 #pragma unroll
   for (int q = 0; q < 8; ++q) unpack8(reinterpret_cast<const uint4*>(src)[q], f + q * 8);
 }
-// Column sums over the row threads. Each row thread first writes its 64 values into its row of
-// `red` ([128][65] fp32); red_sums then adds them up: per group of 64 threads into out[g*64+i]
-// (per_group), or over all 128 into out[i]. red_sums must be called by every thread of the block.
-__device__ __forceinline__ void red_sums(float* red, float* out, bool per_group) {
-  const int tid = threadIdx.x;
-  __syncthreads();
-  if (tid < 128) {
-    const int g = tid >> 6, i = tid & 63;
-    if (per_group) {
-      float s = 0.f;
-      for (int t = 0; t < 64; ++t) s += red[(g * 64 + t) * 65 + i];
-      out[g * 64 + i] = s;
-    } else if (g == 0) {
-      float s = 0.f;
-      for (int t = 0; t < 128; ++t) s += red[t * 65 + i];
-      out[i] = s;
+// Sums of 64 values per lane over the warp's lanes: lane l returns those of columns 2l and 2l + 1. Each
+// step hands half of the remaining columns to the partner lane (62 shuffles; through shared memory it
+// was 64 stores and a chain of 64 dependent loads per sum). The values are consumed.
+__device__ __forceinline__ float2 warp_col_sums(float (&v)[64]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16, n = 32; o > 0; o >>= 1, n >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  __syncthreads();
+  return make_float2(v[0], v[1]);
+}
+__device__ __forceinline__ void row_threads_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// The first chunk position of each token's sequence: `starts` has a bit where a sequence begins.
+__device__ __forceinline__ int seq_begin(const unsigned* starts, int t) {
+  const unsigned long long m = (static_cast<unsigned long long>(starts[1]) << 32) | starts[0];
+  return 63 - __clzll(static_cast<long long>(m & (~0ull >> (63 - t))));
+}
+// 64 tokens of one feature per row thread -> token rows of 128 features, through a 16 KiB tile: two-byte
+// stores of 64 bytes per warp took several times longer. Called by the 128 row threads; `tile` is free
+// to be written, and again after the call's end only behind another row_threads_sync.
+__device__ __forceinline__ void store_tokens(const float (&v)[64], uint8_t* tile, __nv_bfloat16* dst, long long ld,
+                                             int lim) {
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int t = 0; t < 64; ++t)
+    *reinterpret_cast<__nv_bfloat16*>(tile + t * 256 + tid * 2) = __float2bfloat16_rn(v[t]);
+  row_threads_sync();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int t = q * 8 + (tid >> 4), c = tid & 15;
+    if (t < lim)
+      *reinterpret_cast<uint4*>(dst + t * ld + c * 8) = *reinterpret_cast<const uint4*>(tile + t * 256 + c * 16);
+  }
 }
 
 // ============================================================================ sequence ids
@@ -166,6 +185,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   float* beta_s = gam_s + 128;
   float* g_s = beta_s + 128;
   int* sid_s = reinterpret_cast<int*>(g_s + 128);                  // [65]; [64] = previous chunk's last
+  unsigned* starts_s = reinterpret_cast<unsigned*>(sid_s + 68);    // [2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
@@ -205,6 +225,10 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
   if (tid < 65) sid_s[tid] = tid < 64 ? p.sid[t0 + tid] : (c > 0 ? p.sid[t0 - 1] : -1);
   __syncthreads();
+  if (tid < 64) {
+    const unsigned m = __ballot_sync(0xffffffffu, tid == 0 || sid_s[tid] != sid_s[tid - 1]);
+    if ((tid & 31) == 0) starts_s[warp] = m;
+  }
   if (tid < 128) {
     const int hh = tid >> 6, j = tid & 63;
     float s = 0.f;
@@ -231,28 +255,34 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   mbar_wait(mma_bar, 0, p.status, KS_TIMEOUT_TMEM_FULL);
   tc_fence_after();
 
-  // ---- A (fp32, shared memory) and Mq (global)
+  // ---- A (fp32, shared memory) and Mq (global): a row's decays are read into registers first, so that no
+  // store stands between the loads
   if (tid < 128) {
     const int t = tid & 63;
     float row[64];
     tmem_row64(lane_addr, row);
-    const int my = sid_s[t];
-    if (tid < 64) {
-      for (int hh = 0; hh < nh; ++hh) {
-        const float gt = gam_s[hh * 64 + t], bt = beta_s[hh * 64 + t];
-        float* a = Af + (hh * 64 + t) * AP;
+    const int lo = seq_begin(starts_s, t);
+    const bool is_q = tid >= 64;
+#pragma unroll 1
+    for (int hh = 0; hh < nh; ++hh) {
+      const float gt = gam_s[hh * 64 + t], f = is_q ? p.scale : beta_s[hh * 64 + t];
+      const int hi = is_q ? t : t - 1;                   // Mq includes the diagonal, A does not
+      float* a = Af + (hh * 64 + t) * AP;
+      __nv_bfloat16* mq = p.MQ + ((static_cast<long long>(c) * G.NP + pr) * 128 + hh * 64 + t) * 64;
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          a[i] = (i < t && sid_s[i] == my) ? bt * __expf(gt - gam_s[hh * 64 + i]) * row[i] : 0.f;
-      }
-    } else {
-      for (int hh = 0; hh < nh; ++hh) {
-        const float gt = gam_s[hh * 64 + t];
-        float m[64];
+      for (int i0 = 0; i0 < 64; i0 += 8) {
+        float m[8];
+        *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0);
+        *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0 + 4);
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          m[i] = (i <= t && sid_s[i] == my) ? p.scale * __expf(gt - gam_s[hh * 64 + i]) * row[i] : 0.f;
-        store_row64(p.MQ + ((static_cast<long long>(c) * G.NP + pr) * 128 + hh * 64 + t) * 64, m);
+        for (int e = 0; e < 8; ++e)
+          m[e] = i0 + e >= lo && i0 + e <= hi ? f * __expf(gt - m[e]) * row[i0 + e] : 0.f;
+        if (is_q) {
+          *reinterpret_cast<uint4*>(mq + i0) = pack8(m);
+        } else {
+          *reinterpret_cast<float4*>(a + i0) = *reinterpret_cast<const float4*>(m);
+          *reinterpret_cast<float4*>(a + i0 + 4) = *reinterpret_cast<const float4*>(m + 4);
+        }
       }
     }
   }
@@ -879,9 +909,10 @@ constexpr int OFF_KKF = 49152, OFF_QKF = OFF_KKF + 16640;          // fp32 [64][
 constexpr int OFF_DTM = 82944, OFF_XOP = OFF_DTM + 16384;          // operands
 constexpr int OFF_SYM = OFF_XOP + 16384, OFF_DQK = OFF_SYM + 8192;
 constexpr int OFF_KKA = OFF_DQK + 8192, OFF_QKA = OFF_KKA + 16640;  // fp32 accumulators over heads
-constexpr int OFF_RED = OFF_QKA + 16640;                           // 165376, [128][65] fp32
-constexpr int OFF_MISC = OFF_RED + 33280;                          // 198656
-constexpr int OFF_BAR = OFF_MISC + 8192;
+constexpr int OFF_OUT = OFF_DTM;                                   // 16 KiB tile of the output transposes
+constexpr int OFF_MISC = OFF_XU + 16384;                           // 180224
+constexpr int OFF_BAR = OFF_MISC + 10240;
+static_assert(OFF_QKA + 16640 <= OFF_MISC, "scratch overlaps the per-token values");
 constexpr int SMEM = OFF_BAR + 64 + 1024;
 static_assert(OFF_KKF >= OFF_TMT + 16384, "scratch overlaps a tile that stays live");
 static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
@@ -900,19 +931,20 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   float* QKf = reinterpret_cast<float*>(smem + OFF_QKF);
   float* KKa = reinterpret_cast<float*>(smem + OFF_KKA);
   float* QKa = reinterpret_cast<float*>(smem + OFF_QKA);
-  float* red = reinterpret_cast<float*>(smem + OFF_RED);
   float* misc = reinterpret_cast<float*>(smem + OFF_MISC);
   float* gam_s = misc;            // [2][64] each from here on
   float* beta_s = misc + 128;
   float* gt_s = misc + 256;       // exp(gam) [continues the previous chunk's sequence]
   float* d_s = misc + 384;        // exp(gam_63 - gam) [same sequence as the chunk's end]
+  // column sums, one part per row warp: [4][64]; of the two heads' dot products: [2][4][64]
   float* cs1 = misc + 512;
-  float* cs2 = misc + 640;
-  float* colG = misc + 768;
-  float* dotq = misc + 896;
-  float* dotk = misc + 1024;
-  float* dgam_s = misc + 1152;
-  int* sid_s = reinterpret_cast<int*>(misc + 1280);     // [65]
+  float* cs2 = misc + 768;
+  float* colG = misc + 1024;
+  float* dotq = misc + 1280;
+  float* dotk = misc + 1792;
+  float* dgam_s = misc + 2304;
+  int* sid_s = reinterpret_cast<int*>(misc + 2432);     // [65]
+  unsigned* starts_s = reinterpret_cast<unsigned*>(misc + 2500);   // [2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
@@ -959,6 +991,10 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     beta_s[tid] = live ? p.beta[static_cast<long long>(tok) * G.H + h0 + hh] : 0.f;
   }
   __syncthreads();
+  if (tid < 64) {
+    const unsigned m = __ballot_sync(0xffffffffu, tid == 0 || sid_s[tid] != sid_s[tid - 1]);
+    if ((tid & 31) == 0) starts_s[warp] = m;
+  }
   if (tid < 128) {
     const int hh = tid >> 6, j = tid & 63;
     gt_s[tid] = (sid_s[j] == sid_s[64]) ? __expf(gam_s[tid]) : 0.f;
@@ -1013,34 +1049,28 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int hh_me = tid >> 6, t_me = tid & 63;
   const bool live = tid < 128 && hh_me < nh;
   // ---- dTm = (P1, P2) scaled per column; column sums of Tm o P1 and Tm o P2
-  {
-    float z2[64];
-    if (tid < 128) {
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        float p1[32], p2[32], dtm[32];
-        tmem_row32(lane_addr + 64 + half * 32, p1);
-        tmem_row32(lane_addr + 128 + (hh_me < nh ? hh_me : 0) * 64 + half * 32, p2);
+  if (tid < 128) {
+    float z1[64], z2[64];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const int i = half * 32 + e;
-          const float tm = bf16_at(smem + OFF_TMT + (hh_me * 64 + i) * 128 +
-                                   (((t_me >> 3) ^ (i & 7)) << 4) + (t_me & 7) * 2);
-          dtm[e] = live ? beta_s[hh_me * 64 + i] * (gt_s[hh_me * 64 + i] * p1[e] + p2[e]) : 0.f;
-          red[tid * 65 + i] = live ? tm * p1[e] : 0.f;
-          z2[i] = live ? tm * p2[e] : 0.f;
-        }
+    for (int half = 0; half < 2; ++half) {
+      float p1[32], p2[32], dtm[32];
+      tmem_row32(lane_addr + 64 + half * 32, p1);
+      tmem_row32(lane_addr + 128 + (hh_me < nh ? hh_me : 0) * 64 + half * 32, p2);
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(smem + OFF_DTM + sw_off(128, tid, half * 4 + q)) = pack8(dtm + q * 8);
+      for (int e = 0; e < 32; ++e) {
+        const int i = half * 32 + e;
+        const float tm = bf16_at(smem + OFF_TMT + (hh_me * 64 + i) * 128 +
+                                 (((t_me >> 3) ^ (i & 7)) << 4) + (t_me & 7) * 2);
+        dtm[e] = live ? beta_s[hh_me * 64 + i] * (gt_s[hh_me * 64 + i] * p1[e] + p2[e]) : 0.f;
+        z1[i] = live ? tm * p1[e] : 0.f;
+        z2[i] = live ? tm * p2[e] : 0.f;
       }
-    }
-    red_sums(red, cs1, true);
-    if (tid < 128) {
 #pragma unroll
-      for (int i = 0; i < 64; ++i) red[tid * 65 + i] = z2[i];
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(smem + OFF_DTM + sw_off(128, tid, half * 4 + q)) = pack8(dtm + q * 8);
     }
-    red_sums(red, cs2, true);
+    reinterpret_cast<float2*>(cs1 + warp * 64)[tid & 31] = warp_col_sums(z1);
+    reinterpret_cast<float2*>(cs2 + warp * 64)[tid & 31] = warp_col_sums(z2);
   }
   publish();
 
@@ -1082,49 +1112,60 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   mma_phase ^= 1;
   tc_fence_after();
 
-  // ---- gradients through A and Mq. The two heads of the pair take turns so that dKK and dQK
-  // accumulate in one pair of shared-memory matrices.
+  // ---- gradients through A and Mq, 16 columns at a time: everything a step reads is in registers before
+  // it writes, head 0 writes its dKK and dQK to KKa / QKa and head 1 over the scores both have just read
   float rowG = 0.f, rowdb = 0.f;
-  for (int pass = 0; pass < 2; ++pass) {
-    if (tid < 128 && hh_me == pass) {
-      float acc[64], dmq[64];
-      tmem_row64(lane_addr + (hh_me == 0 ? 192 : 0), acc);
-      if (live) load_row64(p.dMQ + (prow0 + tid) * 64, dmq);
-      const int my = sid_s[t_me];
-      const float gt = gam_s[tid], bt = beta_s[tid];
+  if (tid < 128) {
+    uint4 mq[8];
 #pragma unroll
-      for (int i = 0; i < 64; ++i) {
-        float dkk = 0.f, dqk = 0.f, w = 0.f;
-        if (live) {
-          const bool same = sid_s[i] == my;
-          const float R = (i <= t_me && same) ? __expf(gt - gam_s[hh_me * 64 + i]) : 0.f;
-          const float da = (i < t_me && same) ? -acc[i] : 0.f;
-          const float kkv = KKf[t_me * 65 + i], qkv = QKf[t_me * 65 + i];
-          rowdb += da * R * kkv;
-          dkk = da * bt * R;
-          dqk = dmq[i] * p.scale * R;
-          w = dkk * kkv + dqk * qkv;               // dR o R
-          rowG += w;
-        }
-        red[tid * 65 + i] = w;
-        if (pass == 0) { KKa[t_me * 65 + i] = dkk; QKa[t_me * 65 + i] = dqk; }
-        else if (live) { KKa[t_me * 65 + i] += dkk; QKa[t_me * 65 + i] += dqk; }
+    for (int x = 0; x < 8; ++x)
+      mq[x] = live ? reinterpret_cast<const uint4*>(p.dMQ + (prow0 + tid) * 64)[x] : make_uint4(0, 0, 0, 0);
+    const int lo = seq_begin(starts_s, t_me);
+    const float gt = gam_s[tid], bt = beta_s[tid];
+    float w[64];
+#pragma unroll
+    for (int i0 = 0; i0 < 64; i0 += 16) {
+      uint32_t acc[16];
+      tmem_ld_32x16(lane_addr + (hh_me == 0 ? 192 : 0) + i0, acc);
+      float gi[16], kk[16], qk[16], dmq[16];
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        *reinterpret_cast<float4*>(gi + 4 * x) = *reinterpret_cast<const float4*>(gam_s + hh_me * 64 + i0 + 4 * x);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) { kk[e] = KKf[t_me * 65 + i0 + e]; qk[e] = QKf[t_me * 65 + i0 + e]; }
+      unpack8(mq[i0 / 8], dmq);
+      unpack8(mq[i0 / 8 + 1], dmq + 8);
+      tmem_ld_wait();
+      row_threads_sync();
+      float* ko = (hh_me == 0 ? KKa : KKf) + t_me * 65 + i0;
+      float* qo = (hh_me == 0 ? QKa : QKf) + t_me * 65 + i0;
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const int i = i0 + e;
+        const bool seen = live && i >= lo && i <= t_me;
+        const float R = seen ? __expf(gt - gi[e]) : 0.f;
+        const float da = seen && i < t_me ? -__uint_as_float(acc[e]) : 0.f;
+        rowdb += da * R * kk[e];
+        const float dkk = da * bt * R, dqk = dmq[e] * p.scale * R;
+        w[i] = seen ? dkk * kk[e] + dqk * qk[e] : 0.f;           // dR o R
+        rowG += w[i];
+        ko[e] = dkk;
+        qo[e] = seen ? dqk : 0.f;
       }
     }
-    __syncthreads();
-  }
-  red_sums(red, colG, true);
-  if (tid < 128) {
+    reinterpret_cast<float2*>(colG + warp * 64)[tid & 31] = warp_col_sums(w);
+    row_threads_sync();
     float o[64];
     if (tid < 64) {
 #pragma unroll
-      for (int i = 0; i < 64; ++i) o[i] = KKa[t_me * 65 + i] + KKa[i * 65 + t_me];
+      for (int i = 0; i < 64; ++i)
+        o[i] = (KKa[t_me * 65 + i] + KKa[i * 65 + t_me]) + (KKf[t_me * 65 + i] + KKf[i * 65 + t_me]);
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *reinterpret_cast<uint4*>(smem + OFF_SYM + sw_off(64, t_me, q)) = pack8(o + q * 8);
     } else {
 #pragma unroll
-      for (int i = 0; i < 64; ++i) o[i] = QKa[t_me * 65 + i];
+      for (int i = 0; i < 64; ++i) o[i] = QKa[t_me * 65 + i] + QKf[t_me * 65 + i];
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *reinterpret_cast<uint4*>(smem + OFF_DQK + sw_off(64, t_me, q)) = pack8(o + q * 8);
@@ -1159,52 +1200,60 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     return bf16_at(smem + OFF_KQ + (tid >> 6) * 16384 + (which * 64 + i) * 128 +
                    (((((tid & 63) >> 3)) ^ (i & 7)) << 4) + (tid & 7) * 2);
   };
+  if (tid < 128) {
 #pragma unroll 1
-  for (int which = 0; which < 2; ++which) {          // 0: dk (with Kd), 1: dq (with Qg)
-    float acc[64];
-    if (tid < 128) tmem_row64(lane_addr + (which == 0 ? 256 : 448), acc);
-    for (int hh = 0; hh < nh; ++hh) {
-      if (tid < 128) {
+    for (int which = 0; which < 2; ++which) {          // 0: dk (with Kd), 1: dq (with Qg)
+      float acc[64];
+      tmem_row64(lane_addr + (which == 0 ? 256 : 448), acc);
+      const float* fs = which == 0 ? d_s : gt_s;
+      const float fmul = which == 0 ? 1.f : p.scale;
+#pragma unroll 1
+      for (int hh = 0; hh < nh; ++hh) {
         float a[64];
         load_row64((which == 0 ? p.dKdTp : p.dQgTp) + (prow0 + tid) * 128 + hh * 64, a);
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          const float f = which == 0 ? d_s[hh * 64 + i] : p.scale * gt_s[hh * 64 + i];
-          acc[i] += f * a[i];
-          red[tid * 65 + i] = a[i] * kq_at(which, i);     // dKd o K  /  dQg o Q
-        }
-      }
-      red_sums(red, (which == 0 ? dotk : dotq) + hh * 64, false);
-    }
-    if (tid < 128) {
-      __nv_bfloat16* dst = (which == 0 ? p.dk : p.dq) + (static_cast<long long>(t0) * G.NP + pr) * D + tid;
+        for (int i0 = 0; i0 < 64; i0 += 4) {
+          const float4 f = *reinterpret_cast<const float4*>(fs + hh * 64 + i0);
+          acc[i0] += f.x * fmul * a[i0];
+          acc[i0 + 1] += f.y * fmul * a[i0 + 1];
+          acc[i0 + 2] += f.z * fmul * a[i0 + 2];
+          acc[i0 + 3] += f.w * fmul * a[i0 + 3];
 #pragma unroll
-      for (int i = 0; i < 64; ++i)
-        if (i < lim) dst[static_cast<long long>(i) * G.NP * D] = __float2bfloat16_rn(acc[i]);
+          for (int e = 0; e < 4; ++e) a[i0 + e] *= kq_at(which, i0 + e);     // dKd o K  /  dQg o Q
+        }
+        reinterpret_cast<float2*>((which == 0 ? dotk : dotq) + (hh * 4 + warp) * 64)[tid & 31] = warp_col_sums(a);
+      }
+      row_threads_sync();                               // the tile's last reader is done
+      store_tokens(acc, smem + OFF_OUT, (which == 0 ? p.dk : p.dq) + (static_cast<long long>(t0) * G.NP + pr) * D,
+                   static_cast<long long>(G.NP) * D, lim);
     }
-  }
-  if (tid < 128) {
+#pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
       float r[64];
       tmem_row64(lane_addr + 320 + hh * 64, r);
-      __nv_bfloat16* dvp = p.dv + (static_cast<long long>(t0) * G.H + h0 + hh) * D + tid;
-#pragma unroll
-      for (int i = 0; i < 64; ++i)
-        if (i < lim) dvp[static_cast<long long>(i) * G.H * D] = __float2bfloat16_rn(r[i]);
+      row_threads_sync();
+      store_tokens(r, smem + OFF_OUT, p.dv + (static_cast<long long>(t0) * G.H + h0 + hh) * D,
+                   static_cast<long long>(G.H) * D, lim);
     }
   }
   __syncthreads();
 
   // ---- per-token scalars: dgam -> dg (suffix sum), dbeta
+  // sums of a column's parts: over one head's two row warps, or over all four
+  auto two = [&](const float* part, int i) { return part[(hh_me * 2) * 64 + i] + part[(hh_me * 2 + 1) * 64 + i]; };
+  auto four = [&](const float* part, int i) {
+    const float* x = part + hh_me * 256 + i;
+    return (x[0] + x[64]) + (x[128] + x[192]);
+  };
   if (tid < 128) {
     float dgam = 0.f;
     if (live) {
       const int o = hh_me * 64;
-      dgam = rowG - colG[tid] + beta_s[tid] * gt_s[tid] * cs1[tid] + p.scale * gt_s[tid] * dotq[tid] -
-             d_s[tid] * dotk[tid];
+      dgam = rowG - two(colG, t_me) + beta_s[tid] * gt_s[tid] * two(cs1, t_me) +
+             p.scale * gt_s[tid] * four(dotq, t_me) - d_s[tid] * four(dotk, t_me);
       if (t_me == 63) {
         float tail = 0.f;
-        for (int i = 0; i < 64; ++i) tail += d_s[o + i] * dotk[o + i];
+        for (int i = 0; i < 64; ++i) tail += d_s[o + i] * four(dotk, i);
         const long long hi = static_cast<long long>(c) * G.H + h0 + hh_me;
         dgam += tail + p.dgc[hi] * p.gc[hi];
       }
@@ -1217,7 +1266,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     for (int i = t_me; i < 64; ++i) s += dgam_s[hh_me * 64 + i];
     const long long o = static_cast<long long>(t0 + t_me) * G.H + h0 + hh_me;
     p.dg[o] = s;
-    p.dbeta[o] = rowdb + gt_s[tid] * cs1[tid] + cs2[tid];
+    p.dbeta[o] = rowdb + gt_s[tid] * two(cs1, t_me) + two(cs2, t_me);
   }
   tc_fence_before();
   __syncthreads();
