@@ -102,13 +102,18 @@ __device__ __forceinline__ void load_row64(const __nv_bfloat16* src, float* f) {
 #pragma unroll
   for (int q = 0; q < 8; ++q) unpack8(reinterpret_cast<const uint4*>(src)[q], f + q * 8);
 }
-// Sums of 64 values per lane over the warp's lanes: lane l returns those of columns 2l and 2l + 1. Each
-// step hands half of the remaining columns to the partner lane (62 shuffles; through shared memory it
-// was 64 stores and a chain of 64 dependent loads per sum). The values are consumed.
-__device__ __forceinline__ float2 warp_col_sums(float (&v)[64]) {
+// Sums of N values per lane over the warp's lanes (each step hands half of the remaining columns to the
+// partner lane; through shared memory it was N stores and a chain of dependent loads per sum), written to
+// out[0..N). The values are consumed.
+template <int N>
+__device__ __forceinline__ void warp_col_sums(float (&v)[N], float* out) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int o = 16, n = 32; o > 0; o >>= 1, n >>= 1) {
+  for (int o = 16, n = N / 2; o > 0; o >>= 1, n >>= 1) {
+    if (n == 0) {                               // one column left, in both partners
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+      continue;
+    }
     const bool up = lane & o;
 #pragma unroll
     for (int i = 0; i < n; ++i) {
@@ -116,7 +121,9 @@ __device__ __forceinline__ float2 warp_col_sums(float (&v)[64]) {
       v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  return make_float2(v[0], v[1]);
+  if constexpr (N == 64) reinterpret_cast<float2*>(out)[lane] = make_float2(v[0], v[1]);
+  else if constexpr (N == 32) out[lane] = v[0];
+  else if ((lane & 1) == 0) out[lane >> 1] = v[0];
 }
 __device__ __forceinline__ void row_threads_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 // The first chunk position of each token's sequence: `starts` has a bit where a sequence begins.
@@ -159,7 +166,8 @@ __global__ void dn_seq_ids_kernel(const int* __restrict__ cu, int nseq, int T, i
 // ============================================================================ prep (forward)
 struct PrepParams {
   const float* beta; const float* g; const int* sid;
-  __nv_bfloat16 *WTp, *U0Tp, *QG, *KD, *MQ, *TMT, *XW, *XU;   // TMT/XW/XU: null unless a backward follows
+  __nv_bfloat16 *MQ, *TMT;         // TMT: null unless a backward follows
+  int save;                        // a backward follows: keep the inverse and its two scaled forms
   float *gam, *gc;
   Geo geo; float scale; int* status;
 };
@@ -176,7 +184,10 @@ static_assert(2 * (SMEM + 1024) <= 233472, "two CTAs per SM");
 
 __global__ void __launch_bounds__(THREADS, 2)
 dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-               const __grid_constant__ CUtensorMap tmV, const PrepParams p) {
+               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmWT,
+               const __grid_constant__ CUtensorMap tmU0T, const __grid_constant__ CUtensorMap tmQG,
+               const __grid_constant__ CUtensorMap tmKD, const __grid_constant__ CUtensorMap tmXW,
+               const __grid_constant__ CUtensorMap tmXU, const PrepParams p) {
   using namespace prep;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
@@ -322,13 +333,11 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *reinterpret_cast<uint4*>(smem + OFF_XW + sw_off(128, row, q)) = pack8(w + q * 8);
-      if (p.XW) store_row64(p.XW + grow, w);
 #pragma unroll
       for (int t = 0; t < 64; ++t) w[t] = col[t] * bj;
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *reinterpret_cast<uint4*>(smem + OFF_XU + sw_off(128, row, q)) = pack8(w + q * 8);
-      if (p.XU) store_row64(p.XU + grow, w);
       if (p.TMT) store_row64(p.TMT + grow, col);
     }
   }
@@ -350,42 +359,91 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                   umma_smem_desc(sxu + hh * 8192 + kk * 2048, 8192, 1024), idesc, kk != 0);
     }
     umma_commit(mma_bar);
+    if (p.save) {                                // the operands are saved from the tiles the products read
+      for (int hh = 0; hh < nh; ++hh) {
+        tma_store_2d(&tmXW, smem + OFF_XW + hh * 8192, 0, (c * G.NP + pr) * 128 + hh * 64);
+        tma_store_2d(&tmXU, smem + OFF_XU + hh * 8192, 0, (c * G.NP + pr) * 128 + hh * 64);
+      }
+      tma_store_commit();
+      tma_store_wait_read<0>();
+    }
   }
   mbar_wait(mma_bar, 1, p.status, KS_TIMEOUT_TMEM_FULL);
   tc_fence_after();
+  __syncthreads();                               // V and the operands have been read: their tiles are free
 
-  if (tid < 128) {
-    const long long prow = ((static_cast<long long>(c) * G.NP + pr) * 128 + tid) * 128;
-    for (int hh = 0; hh < nh; ++hh) {
-      float r[64];
-      tmem_row64(lane_addr + hh * 64, r);
-      store_row64(p.WTp + prow + hh * 64, r);
-      tmem_row64(lane_addr + 128 + hh * 64, r);
-      store_row64(p.U0Tp + prow + hh * 64, r);
+  // ---- every result leaves by TMA from a tile laid out like its operands (a row per thread straight to
+  // memory is 16 bytes to each of 32 lines per store, half of this kernel's time): W^T over V, U0^T over
+  // the operands, then the scaled K and Q rows of the last head in place and those of the first over W^T.
+  uint4 kq[16];
+  const int t = tid & 63;
+  const bool is_q = tid >= 64;
+  auto factor = [&](int hh) {                    // Kd (threads 0..63, K rows) and Qg (threads 64..127, Q rows)
+    const float gt = gam_s[hh * 64 + t];
+    if (is_q) return (sid_s[t] == sid_s[64]) ? p.scale * __expf(gt) : 0.f;
+    return (sid_s[t] == sid_s[63]) ? __expf(gam_s[hh * 64 + 63] - gt) : 0.f;
+  };
+  auto write_kq = [&](uint8_t* tile, int hh) {
+    const float f = factor(hh);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      float v[8];
+      unpack8(kq[q], v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] *= f;
+      *reinterpret_cast<uint4*>(tile + sw_off(128, tid, q)) = pack8(v);
     }
-    // Kd (threads 0..63, K rows) and Qg (threads 64..127, Q rows)
-    const int t = tid & 63;
-    const bool is_q = tid >= 64;
+  };
+  auto store_kq = [&](const uint8_t* tile, int hh) {
+    const int hrow = (c * G.H + h0 + hh) * 64;
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      tma_store_2d(&tmKD, tile + b * 16384, b * 64, hrow);
+      tma_store_2d(&tmQG, tile + b * 16384 + 8192, b * 64, hrow);
+    }
+    tma_store_commit();
+  };
+  if (tid < 128) {
+#pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
-      const float gt = gam_s[hh * 64 + t];
-      float f;
-      if (is_q) f = (sid_s[t] == sid_s[64]) ? p.scale * __expf(gt) : 0.f;
-      else f = (sid_s[t] == sid_s[63]) ? __expf(gam_s[hh * 64 + 63] - gt) : 0.f;
-      __nv_bfloat16* dst = (is_q ? p.QG : p.KD) +
-                           ((static_cast<long long>(c) * G.H + h0 + hh) * 64 + t) * 128;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        float w[32], u[32];
+        tmem_row32(lane_addr + hh * 64 + half * 32, w);
+        tmem_row32(lane_addr + 128 + hh * 64 + half * 32, u);
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        float v[8];
-        unpack8(*reinterpret_cast<const uint4*>(smem + OFF_KQ + sw_off(128, tid, q)), v);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] *= f;
-        reinterpret_cast<uint4*>(dst)[q] = pack8(v);
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t at = hh * 16384 + sw_off(128, tid, half * 4 + q);
+          *reinterpret_cast<uint4*>(smem + OFF_V + at) = pack8(w + q * 8);
+          *reinterpret_cast<uint4*>(smem + OFF_XW + at) = pack8(u + q * 8);
+        }
       }
-      if (tid == 63)
-        p.gc[static_cast<long long>(c) * G.H + h0 + hh] =
-            (sid_s[63] == sid_s[64]) ? __expf(gam_s[hh * 64 + 63]) : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) kq[q] = *reinterpret_cast<const uint4*>(smem + OFF_KQ + sw_off(128, tid, q));
+    write_kq(smem + OFF_KQ, nh - 1);
+    if (tid < nh) {
+      const float g63 = gam_s[tid * 64 + 63];
+      p.gc[static_cast<long long>(c) * G.H + h0 + tid] = (sid_s[63] == sid_s[64]) ? __expf(g63) : 0.f;
     }
   }
+  publish();
+  if (tid == CTRL) {
+    for (int hh = 0; hh < nh; ++hh) {
+      tma_store_2d(&tmWT, smem + OFF_V + hh * 16384, hh * 64, (c * G.NP + pr) * 128);
+      tma_store_2d(&tmU0T, smem + OFF_XW + hh * 16384, hh * 64, (c * G.NP + pr) * 128);
+    }
+    tma_store_commit();
+    store_kq(smem + OFF_KQ, nh - 1);
+    if (nh == 2) tma_store_wait_read<1>();       // W^T has left its tile
+  }
+  if (nh == 2) {
+    __syncthreads();
+    if (tid < 128) write_kq(smem + OFF_V, 0);
+    publish();
+    if (tid == CTRL) store_kq(smem + OFF_V, 0);
+  }
+  if (tid == CTRL) tma_store_wait<0>();
   tc_fence_before();
   __syncthreads();
   if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
@@ -1050,8 +1108,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const bool live = tid < 128 && hh_me < nh;
   // ---- dTm = (P1, P2) scaled per column; column sums of Tm o P1 and Tm o P2
   if (tid < 128) {
-    float z1[64], z2[64];
-#pragma unroll
+#pragma unroll 1
     for (int half = 0; half < 2; ++half) {
       float p1[32], p2[32], dtm[32];
       tmem_row32(lane_addr + 64 + half * 32, p1);
@@ -1062,15 +1119,15 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const float tm = bf16_at(smem + OFF_TMT + (hh_me * 64 + i) * 128 +
                                  (((t_me >> 3) ^ (i & 7)) << 4) + (t_me & 7) * 2);
         dtm[e] = live ? beta_s[hh_me * 64 + i] * (gt_s[hh_me * 64 + i] * p1[e] + p2[e]) : 0.f;
-        z1[i] = live ? tm * p1[e] : 0.f;
-        z2[i] = live ? tm * p2[e] : 0.f;
+        p1[e] = live ? tm * p1[e] : 0.f;
+        p2[e] = live ? tm * p2[e] : 0.f;
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         *reinterpret_cast<uint4*>(smem + OFF_DTM + sw_off(128, tid, half * 4 + q)) = pack8(dtm + q * 8);
+      warp_col_sums(p1, cs1 + warp * 64 + half * 32);
+      warp_col_sums(p2, cs2 + warp * 64 + half * 32);
     }
-    reinterpret_cast<float2*>(cs1 + warp * 64)[tid & 31] = warp_col_sums(z1);
-    reinterpret_cast<float2*>(cs2 + warp * 64)[tid & 31] = warp_col_sums(z2);
   }
   publish();
 
@@ -1113,18 +1170,19 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_after();
 
   // ---- gradients through A and Mq, 16 columns at a time: everything a step reads is in registers before
-  // it writes, head 0 writes its dKK and dQK to KKa / QKa and head 1 over the scores both have just read
+  // it writes, head 0 writes its dKK and dQK to KKa / QKa and head 1 over the scores both have just read.
+  // The loops of this kernel stay rolled where registers allow: it runs each line once per block with one
+  // warp per scheduler, and fetching straight-line code was its largest stall.
   float rowG = 0.f, rowdb = 0.f;
   if (tid < 128) {
-    uint4 mq[8];
-#pragma unroll
-    for (int x = 0; x < 8; ++x)
-      mq[x] = live ? reinterpret_cast<const uint4*>(p.dMQ + (prow0 + tid) * 64)[x] : make_uint4(0, 0, 0, 0);
+    const uint4* mq = reinterpret_cast<const uint4*>(p.dMQ + (prow0 + tid) * 64);
+    uint4 m0 = make_uint4(0, 0, 0, 0), m1 = m0;
+    if (live) { m0 = mq[0]; m1 = mq[1]; }
     const int lo = seq_begin(starts_s, t_me);
     const float gt = gam_s[tid], bt = beta_s[tid];
-    float w[64];
-#pragma unroll
+#pragma unroll 1
     for (int i0 = 0; i0 < 64; i0 += 16) {
+      float w[16];
       uint32_t acc[16];
       tmem_ld_32x16(lane_addr + (hh_me == 0 ? 192 : 0) + i0, acc);
       float gi[16], kk[16], qk[16], dmq[16];
@@ -1133,8 +1191,9 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         *reinterpret_cast<float4*>(gi + 4 * x) = *reinterpret_cast<const float4*>(gam_s + hh_me * 64 + i0 + 4 * x);
 #pragma unroll
       for (int e = 0; e < 16; ++e) { kk[e] = KKf[t_me * 65 + i0 + e]; qk[e] = QKf[t_me * 65 + i0 + e]; }
-      unpack8(mq[i0 / 8], dmq);
-      unpack8(mq[i0 / 8 + 1], dmq + 8);
+      unpack8(m0, dmq);
+      unpack8(m1, dmq + 8);
+      if (live && i0 < 48) { m0 = mq[i0 / 8 + 2]; m1 = mq[i0 / 8 + 3]; }
       tmem_ld_wait();
       row_threads_sync();
       float* ko = (hh_me == 0 ? KKa : KKf) + t_me * 65 + i0;
@@ -1147,28 +1206,28 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const float da = seen && i < t_me ? -__uint_as_float(acc[e]) : 0.f;
         rowdb += da * R * kk[e];
         const float dkk = da * bt * R, dqk = dmq[e] * p.scale * R;
-        w[i] = seen ? dkk * kk[e] + dqk * qk[e] : 0.f;           // dR o R
-        rowG += w[i];
+        w[e] = seen ? dkk * kk[e] + dqk * qk[e] : 0.f;           // dR o R
+        rowG += w[e];
         ko[e] = dkk;
         qo[e] = seen ? dqk : 0.f;
       }
+      warp_col_sums(w, colG + warp * 64 + i0);
     }
-    reinterpret_cast<float2*>(colG + warp * 64)[tid & 31] = warp_col_sums(w);
     row_threads_sync();
-    float o[64];
-    if (tid < 64) {
+#pragma unroll 1
+    for (int q = 0; q < 8; ++q) {
+      float o[8];
+      if (tid < 64) {
 #pragma unroll
-      for (int i = 0; i < 64; ++i)
-        o[i] = (KKa[t_me * 65 + i] + KKa[i * 65 + t_me]) + (KKf[t_me * 65 + i] + KKf[i * 65 + t_me]);
+        for (int e = 0; e < 8; ++e) {
+          const int i = q * 8 + e;
+          o[e] = (KKa[t_me * 65 + i] + KKa[i * 65 + t_me]) + (KKf[t_me * 65 + i] + KKf[i * 65 + t_me]);
+        }
+      } else {
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<uint4*>(smem + OFF_SYM + sw_off(64, t_me, q)) = pack8(o + q * 8);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 64; ++i) o[i] = QKa[t_me * 65 + i] + QKf[t_me * 65 + i];
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<uint4*>(smem + OFF_DQK + sw_off(64, t_me, q)) = pack8(o + q * 8);
+        for (int e = 0; e < 8; ++e) o[e] = QKa[t_me * 65 + q * 8 + e] + QKf[t_me * 65 + q * 8 + e];
+      }
+      *reinterpret_cast<uint4*>(smem + (tid < 64 ? OFF_SYM : OFF_DQK) + sw_off(64, t_me, q)) = pack8(o);
     }
   }
   publish();
@@ -1221,7 +1280,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
           for (int e = 0; e < 4; ++e) a[i0 + e] *= kq_at(which, i0 + e);     // dKd o K  /  dQg o Q
         }
-        reinterpret_cast<float2*>((which == 0 ? dotk : dotq) + (hh * 4 + warp) * 64)[tid & 31] = warp_col_sums(a);
+        warp_col_sums(a, (which == 0 ? dotk : dotq) + (hh * 4 + warp) * 64);
       }
       row_threads_sync();                               // the tile's last reader is done
       store_tokens(acc, smem + OFF_OUT, (which == 0 ? p.dk : p.dq) + (static_cast<long long>(t0) * G.NP + pr) * D,
@@ -1305,20 +1364,28 @@ int ss_dn_prep(const void* q, const void* k, const void* v, const float* beta, c
   if (T <= 0) return 0;
   if (H <= 0 || Hk <= 0 || H % Hk) return -2;
   const Geo geo = make_geo(T, H, Hk);
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tq, tk, tv, twt, tu0, tqg, tkd, txw, txu;
   int r;
+  const bool save = TMT != nullptr;
+  if ((XW != nullptr) != save || (XU != nullptr) != save) return -2;
+  const long long prow = (long long)geo.n * geo.NP * 128, hrow = (long long)geo.n * H * 64;
   if ((r = ss::make_tmap_bf16(&tq, q, T, (long long)Hk * D, (long long)Hk * D, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tk, k, T, (long long)Hk * D, (long long)Hk * D, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tv, v, T, (long long)H * D, (long long)H * D, 64))) return r;
+  if ((r = ss::make_tmap_bf16(&twt, WTp, prow, 128, 128, 128))) return r;
+  if ((r = ss::make_tmap_bf16(&tu0, U0Tp, prow, 128, 128, 128))) return r;
+  if ((r = ss::make_tmap_bf16(&tqg, QG, hrow, 128, 128, 64))) return r;
+  if ((r = ss::make_tmap_bf16(&tkd, KD, hrow, 128, 128, 64))) return r;
+  if ((r = ss::make_tmap_bf16(&txw, save ? XW : MQ, prow, 64, 64, 64))) return r;
+  if ((r = ss::make_tmap_bf16(&txu, save ? XU : MQ, prow, 64, 64, 64))) return r;
   PrepParams p;
   p.beta = beta; p.g = g; p.sid = sid;
-  p.WTp = (__nv_bfloat16*)WTp; p.U0Tp = (__nv_bfloat16*)U0Tp; p.QG = (__nv_bfloat16*)QG;
-  p.KD = (__nv_bfloat16*)KD; p.MQ = (__nv_bfloat16*)MQ; p.TMT = (__nv_bfloat16*)TMT;
-  p.XW = (__nv_bfloat16*)XW; p.XU = (__nv_bfloat16*)XU; p.gam = gam; p.gc = gc;
+  p.MQ = (__nv_bfloat16*)MQ; p.TMT = (__nv_bfloat16*)TMT; p.save = save; p.gam = gam; p.gc = gc;
   p.geo = geo; p.scale = scale; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_prep_kernel, prep::SMEM)) return e;
-  dn_prep_kernel<<<dim3(geo.n, geo.NP), THREADS, prep::SMEM, (cudaStream_t)stream>>>(tq, tk, tv, p);
+  dn_prep_kernel<<<dim3(geo.n, geo.NP), THREADS, prep::SMEM, (cudaStream_t)stream>>>(tq, tk, tv, twt, tu0, tqg, tkd,
+                                                                                     txw, txu, p);
   return (int)cudaGetLastError();
 }
 
