@@ -80,7 +80,7 @@ def forward(q, k, v, cu_seqlens, max_seqlen, scale=None, out=None, lse=None):
     rc = _lib.lib().ss_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                                 lse.data_ptr(), cu_seqlens.data_ptr(), nseq, T, Hq, Hkv, dh,
                                 _row_stride(q), _row_stride(k), _row_stride(v), _row_stride(o),
-                                float(scale), _lib.status_word(q.device).data_ptr(),
+                                float(scale), _lib.status_ptr(q),
                                 _lib.stream_ptr())
     _lib.check(rc, "ss_attn_fwd")
     return o, lse
@@ -116,7 +116,7 @@ def backward(q, k, v, out, lse, dout, cu_seqlens, max_seqlen, scale=None, dq=Non
                                   Hq, Hkv, dh,
                                   _row_stride(q), _row_stride(k), _row_stride(v), _row_stride(dout),
                                   _row_stride(dq), _row_stride(dk), _row_stride(dv),
-                                  float(scale), _lib.status_word(q.device).data_ptr(),
+                                  float(scale), _lib.status_ptr(q),
                                   _lib.stream_ptr())
     _lib.check(rc, "ss_attn_bwd")
     return dq, dk, dv

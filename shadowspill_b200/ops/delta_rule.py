@@ -97,7 +97,7 @@ def _forward(q, k, v, beta, g, cu_seqlens, backward: bool):
     H = v.shape[1]
     geo = _Geometry(T, H, Hk)
     B = _Buffers(geo, q.device, backward)
-    L, st, status = _lib.lib(), _lib.stream_ptr(), _lib.status_word(q.device).data_ptr()
+    L, st, status = _lib.lib(), _lib.stream_ptr(), _lib.status_ptr(q)
     _lib.check(L.ss_dn_seq_ids(cu_seqlens.data_ptr(), cu_seqlens.numel() - 1, T, B.sid.data_ptr(), st),
                "ss_dn_seq_ids")
     scale = WIDTH ** -0.5
@@ -191,7 +191,7 @@ def _backward_all(q, k, v, beta, g, cu_seqlens, dout):
         q, k, v, beta, g = _operands(q, k, v, beta, g)
         _, B, geo = _forward(q, k, v, beta, g, cu_seqlens, backward=True)
     T, H, Hk = geo.T, geo.H, geo.Hk
-    L, st, status = _lib.lib(), _lib.stream_ptr(), _lib.status_word(q.device).data_ptr()
+    L, st, status = _lib.lib(), _lib.stream_ptr(), _lib.status_ptr(q)
     _lib.check(L.ss_dn_bwd_state(dout.data_ptr(), B.MQ.data_ptr(), B.KD.data_ptr(), B.QG.data_ptr(),
                                  B.WTp.data_ptr(), B.gc.data_ptr(), B.dSpT.data_ptr(), B.dUTp.data_ptr(),
                                  T, H, Hk, status, st), "ss_dn_bwd_state")

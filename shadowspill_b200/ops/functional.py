@@ -80,29 +80,31 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                               alpha=alpha, out_dtype=out_dtype or a.dtype)
     if a.dtype != _BF16 or b.dtype != _BF16:
         raise TypeError("gemm operands must be bfloat16 on CUDA")
-    if a.stride(-1) != 1 or b.stride(-1) != 1:
+    lda, sa = a.stride()
+    ldb, sb = b.stride()
+    if sa != 1 or sb != 1:
         raise ValueError("gemm operands must have unit inner stride")
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    if out.stride(-1) != 1 or out.dtype not in (_BF16, torch.float32):
+    ldc, sc = out.stride()
+    f32 = out.dtype == torch.float32
+    if sc != 1 or not (f32 or out.dtype == _BF16):
         raise ValueError("gemm output must be bf16/fp32 with unit inner stride")
-    if N % 8 or a.stride(0) % 8 or b.stride(0) % 8 or out.stride(0) % (4 if out.dtype == torch.float32 else 8):
+    if N % 8 or lda % 8 or ldb % 8 or ldc % (4 if f32 else 8):
         # TMA moves 16-byte pieces: say which size breaks that instead of returning the kernel's code
         raise ValueError(f"gemm on the GPU needs N and the row strides in multiples of 8 elements "
-                         f"(N={N}, strides {a.stride(0)}, {b.stride(0)}, {out.stride(0)}); pad the operand")
+                         f"(N={N}, strides {lda}, {ldb}, {ldc}); pad the operand")
     if _PAIR_GEMM and bn == 0 and M >= 256 and N >= 128:
         # CTA-pair kernel (tcgen05 cta_group::2): 256x256 tiles, half the shared-memory
         # traffic per FLOP of the single-CTA kernel
         rc = _lib.lib().ss_gemm2_bf16(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-            out.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate),
-            float(alpha), 0, _lib.status_word(a.device).data_ptr(), _lib.stream_ptr())
+            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), int(f32),
+            int(accumulate), float(alpha), 0, _lib.status_ptr(a), _lib.stream_ptr())
         _lib.check(rc, "ss_gemm2_bf16")
         return out
     rc = _lib.lib().ss_gemm_bf16(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-        out.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate),
-        float(alpha), int(bn), 0, _lib.status_word(a.device).data_ptr(), _lib.stream_ptr())
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), int(f32), int(accumulate),
+        float(alpha), int(bn), 0, _lib.status_ptr(a), _lib.stream_ptr())
     _lib.check(rc, "ss_gemm_bf16")
     return out
 
@@ -147,7 +149,7 @@ def _gemm_gather(x: torch.Tensor, info: PendingGather, out, accumulate: bool):
     rc = _lib.lib().ss_gemm2_gather_bf16(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), out.stride(0),
         int(out.dtype == torch.float32), int(accumulate), 1.0, ptrs, info.per, info.world, info.rank,
-        counters.data_ptr(), 0, 0, _lib.status_word(x.device).data_ptr(), _lib.stream_ptr())
+        counters.data_ptr(), 0, 0, _lib.status_ptr(x), _lib.stream_ptr())
     _lib.check(rc, "ss_gemm2_gather_bf16")
     fused_gather_launches += 1
     return out

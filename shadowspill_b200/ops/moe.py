@@ -140,7 +140,7 @@ def grouped_linear(x_sorted: torch.Tensor, bank: torch.Tensor, lay: Layout, tran
     _lib.check(_lib.lib().ss_gemm_grouped_bf16(
         x_sorted.data_ptr(), bank.data_ptr(), out.data_ptr(), 1, lay.rows, 0, N, K, E,
         x_sorted.stride(0), bank.stride(1), out.stride(0), int(transpose), 0, 0,
-        lay.tile_expert.data_ptr(), None, 0, _lib.status_word(x_sorted.device).data_ptr(),
+        lay.tile_expert.data_ptr(), None, 0, _lib.status_ptr(x_sorted),
         _lib.stream_ptr()), "ss_gemm_grouped_bf16")
     return out
 
@@ -153,7 +153,7 @@ def grouped_wgrad(dy_sorted: torch.Tensor, x_sorted: torch.Tensor, lay: Layout, 
         dy_sorted.data_ptr(), x_sorted.data_ptr(), out.data_ptr(), 2, lay.rows, M, N, 0, E,
         dy_sorted.stride(0), x_sorted.stride(0), out.stride(1), 1, int(out.dtype == torch.float32),
         int(accumulate), None, lay.offsets.data_ptr(), 0,
-        _lib.status_word(out.device).data_ptr(), _lib.stream_ptr()), "ss_gemm_grouped_bf16")
+        _lib.status_ptr(out), _lib.stream_ptr()), "ss_gemm_grouped_bf16")
 
 
 def _weights_from_logits(logits, ids, renormalize):
