@@ -442,6 +442,14 @@ static int dispatch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPara
 #undef SS_DISPATCH
 }
 
+// Do the 128x128 tiles of an output fit one wave? Such a tile takes about half the time of a 128x256 one
+// or of a CTA pair's 256x256 one (512 x 2048 over 2048: 9.9 us against 15.2 and 16.0; 1024 x 2048 over
+// 6144: 21.4 against 33.3 and 34.1; 768 x 256 over 256: 5.1 against 7.0 and 7.7), so wider tiles only pay
+// once there is more than one wave of them (1999 x 4096 over 2048: 30.3 against 26.8 and 26.3).
+bool gemm_fits_one_wave(int M, int N, int num_sms) {
+  return N <= 128 || static_cast<long long>((M + 127) / 128) * ((N + 127) / 128) <= num_sms;
+}
+
 static int sm_count() {
   int dev = 0, n = 0;
   cudaGetDevice(&dev);
@@ -465,8 +473,8 @@ int ss_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
       (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
       (reinterpret_cast<uintptr_t>(C) & 15))
     return -2;
-  if (bn != 128 && bn != 256) bn = (N <= 128) ? 128 : 256;
   if (num_sms <= 0) num_sms = sm_count();
+  if (bn != 128 && bn != 256) bn = gemm_fits_one_wave(M, N, num_sms) ? 128 : 256;
   CUtensorMap ta, tb;
   int r;
   if (!a_mn) r = make_tmap_bf16(&ta, A, M, K, lda, BM);

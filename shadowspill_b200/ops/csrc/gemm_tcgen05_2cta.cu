@@ -45,6 +45,8 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, long long rows, long long
 int make_tmap3_bf16(CUtensorMap* map, const void* base, long long experts, long long rows,
                     long long cols, long long ld, long long expert_pitch_elems, int box_rows);
 
+bool gemm_fits_one_wave(int M, int N, int num_sms);   // gemm_tcgen05.cu
+
 namespace pair {
 
 constexpr int BM = 128;          // rows per CTA (256 per pair)
@@ -405,7 +407,12 @@ static int launch_gather(const CUtensorMap& ta, const CUtensorMap& tb, const Par
 
 extern "C" {
 
-// Same arguments and return codes as ss_gemm_bf16 (without the tile-width hint).
+int ss_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                 long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn, int num_sms,
+                 int* status, void* stream);
+
+// Same arguments and return codes as ss_gemm_bf16 (without the tile-width hint), which takes the outputs
+// whose 128x128 tiles fit one wave.
 int ss_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                   long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate,
                   float alpha, int num_sms, int* status, void* stream) {
@@ -421,6 +428,9 @@ int ss_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
+  if (gemm_fits_one_wave(M, N, num_sms))
+    return ss_gemm_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, c_f32, accumulate, alpha, 128, num_sms, status,
+                        stream);
   CUtensorMap ta, tb;
   int r;
   if (!a_mn) r = make_tmap_bf16(&ta, A, M, K, lda, BM);

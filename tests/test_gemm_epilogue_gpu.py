@@ -29,4 +29,13 @@ def test_edges(M, N, dtype):
     F.gemm(a, b, out=out, accumulate=True)
     assert float((out.double() - (first.double() + ref)).abs().max()) <= 2 * tol * scale
     assert torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, 8 + N:], before[:, 8 + N:])
+    if M >= 256 and N >= 128:                         # the pair kernel, which one SM pair's grid selects
+        ldc = wide.stride(0)
+        wide.copy_(before)
+        _lib.check(_lib.lib().ss_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, K, K, ldc, 0, 0,
+                                            int(dtype == torch.float32), 1, 2.0, 2, _lib.status_ptr(a),
+                                            _lib.stream_ptr()), "ss_gemm2_bf16")
+        want = before[:, 8:8 + N].double() + 2.0 * ref
+        assert float((out.double() - want).abs().max()) <= 2 * tol * scale
+        assert torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, 8 + N:], before[:, 8 + N:])
     _lib.check_status()
