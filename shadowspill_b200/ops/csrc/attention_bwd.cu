@@ -47,6 +47,7 @@ struct AttnBwdParams {
   const float* delta;    // [Hq, T]
   const int* cu_seqlens;
   int nseq, T, Hq, Hkv;
+  int split;                 // CTAs that share a key tile of the dKV kernel: a divisor of Hq / Hkv
   long long ldq, ldk, ldv;   // row pitches of dq / dk / dv (elements)
   float scale;
   int* status;
@@ -334,6 +335,26 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // keeps two buffers of it instead.
 enum { MODE_BOTH = 0, MODE_DV = 1, MODE_DK = 2 };
 
+// Short batches: a key tile's queries are those of every head of its group, one CTA after another, and a
+// few long tiles outlast the rest of the grid. With `split` > 1 a cluster of that many CTAs shares the
+// tile, each with its part of the group's heads; their fp32 sums are added through distributed shared
+// memory in the order of the CTAs, each CTA finishing its share of the rows.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local, uint32_t rank) {
+  float4 v;
+  asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\t"
+               "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(local), "r"(rank) : "memory");
+  return v;
+}
+// Byte offset of four consecutive sums of a row; rows are a multiple of 128 bytes, so without the swizzle
+// the lanes of a warp (a row each) would share banks.
+__device__ __forceinline__ uint32_t sum_offset(int row, int cols, int c4) {
+  return row * cols * 4 + (((c4 & ~7) | ((c4 ^ row) & 7)) << 4);
+}
+
 template <int DH, int BQ, int QS, int DOS, int MODE>
 struct DkvCfg {
   static constexpr bool DO_DV = MODE != MODE_DK;
@@ -351,7 +372,9 @@ struct DkvCfg {
   static constexpr int TM_ST = 0, TM_DPT = SB * BQ;
   static constexpr int TM_DV = 2 * BQ;
   static constexpr int TM_DK = TM_DV + (DO_DV ? DH : 0);
+  static constexpr int SUMS = (DO_DV ? DH : 0) + (DO_DK ? DH : 0);
   static_assert(TM_DK + (DO_DK ? DH : 0) <= 512, "TMEM budget");
+  static_assert(128 * SUMS * 4 <= OFF_STAT, "the sums of a tile reuse the operands' space");
   static_assert(SMEM <= 232448, "shared memory budget");
 };
 
@@ -383,8 +406,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), delta
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kv_head = blockIdx.x;
-  const int rep = p.Hq / p.Hkv;
+  const int kv_head = blockIdx.x / p.split, part = blockIdx.x % p.split;
+  const int rep = p.Hq / p.Hkv / p.split;                  // query heads of this CTA
+  const int head0 = kv_head * (p.Hq / p.Hkv) + part * rep;
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -421,7 +445,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       for (int it = 0; it < n_it; ++it) {
         const int qs = it % QS, ds = it % DOS;
-        const int head = kv_head * rep + it / n_q;
+        const int head = head0 + it / n_q;
         const int qt0 = k0 + (it % n_q) * BQ;
         if (it >= QS && !mbar_wait(&q_empty[qs], ((it / QS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
         uint8_t* sq = smem + Cfg::OFF_Q + qs * Cfg::QT_BYTES;
@@ -507,7 +531,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int it = 0; it < n_it; ++it) {
       const int st = it % STS;
       const int qt0 = k0 + (it % n_q) * BQ;
-      const long long base = static_cast<long long>(kv_head * rep + it / n_q) * p.T;
+      const long long base = static_cast<long long>(head0 + it / n_q) * p.T;
       float nl[NU], dl[NU];
 #pragma unroll
       for (int u = 0; u < NU; ++u) {
@@ -601,6 +625,18 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (ok && n_it > 0 && mbar_wait(acc_done, 0, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const bool valid = gk < seq_end;
+      auto leave_sums = [&](uint32_t tm_col, int col0) {
+#pragma unroll 1
+        for (int c = half; c < DH / 32; c += 2) {
+          uint32_t r[32];
+          tmem_ld_32x32(lane_addr + tm_col + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; e += 4)
+            *reinterpret_cast<uint4*>(smem + sum_offset(row, Cfg::SUMS, (col0 + c * 32 + e) >> 2)) =
+                make_uint4(r[e], r[e + 1], r[e + 2], r[e + 3]);
+        }
+      };
       auto store_acc = [&](uint32_t tm_col, void* base, long long ld, float sc) {
         __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(base) +
                               static_cast<long long>(gk) * ld + kv_head * DH;
@@ -622,9 +658,38 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           }
         }
       };
-      if (Cfg::DO_DK) store_acc(Cfg::TM_DK, p.dk, p.ldk, p.scale);
-      if (Cfg::DO_DV) store_acc(Cfg::TM_DV, p.dv, p.ldv, 1.f);
+      if (p.split > 1) {
+        if (Cfg::DO_DV) leave_sums(Cfg::TM_DV, 0);
+        if (Cfg::DO_DK) leave_sums(Cfg::TM_DK, Cfg::DO_DV ? DH : 0);
+      } else {
+        if (Cfg::DO_DK) store_acc(Cfg::TM_DK, p.dk, p.ldk, p.scale);
+        if (Cfg::DO_DV) store_acc(Cfg::TM_DV, p.dv, p.ldv, 1.f);
+      }
     }
+  }
+  if (p.split > 1) {
+    __syncwarp();
+    cluster_sync();                                        // every CTA's sums are in its shared memory
+    if (warp < 8 && n_it > 0) {
+      const int rows = 128 / p.split, per_row = Cfg::SUMS / 4;
+      for (int x = threadIdx.x; x < rows * per_row; x += 256) {
+        const int row = part * rows + x / per_row, c4 = x % per_row, gk = k0 + row;
+        const uint32_t at = smem_u32(smem) + sum_offset(row, Cfg::SUMS, c4);
+        float4 v = ld_cluster_f4(at, 0);
+        for (int r = 1; r < p.split; ++r) {
+          const float4 o = ld_cluster_f4(at, r);
+          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+        }
+        if (gk >= seq_end) continue;
+        const bool is_dk = !Cfg::DO_DV || (Cfg::DO_DK && c4 * 4 >= DH);
+        const int col = c4 * 4 - (is_dk && Cfg::DO_DV ? DH : 0);
+        const float sc = is_dk ? p.scale : 1.f;
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(is_dk ? p.dk : p.dv) +
+                             static_cast<long long>(gk) * (is_dk ? p.ldk : p.ldv) + kv_head * DH + col;
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v.x * sc, v.y * sc), pack_bf16(v.z * sc, v.w * sc));
+      }
+    }
+    cluster_sync();                                        // no CTA leaves while another reads its sums
   }
   tc_fence_before();
   __syncthreads();
@@ -649,8 +714,32 @@ static int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tdo, const CUten
   auto kern = attn_bwd_dkv_kernel<DH, BQ, QS, DOS, MODE>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
-  kern<<<dim3(p.Hkv, tiles), BW_THREADS, Cfg::SMEM, s>>>(tq, tdo, tk, tv, p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.Hkv * p.split, tiles);
+  cfg.blockDim = dim3(BW_THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute cluster[1];
+  cluster[0].id = cudaLaunchAttributeClusterDimension;
+  cluster[0].val.clusterDim.x = p.split;
+  cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+  cfg.attrs = cluster;
+  cfg.numAttrs = p.split > 1 ? 1 : 0;
+  if (cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tq, tdo, tk, tv, p)) return static_cast<int>(e);
   return static_cast<int>(cudaGetLastError());
+}
+
+// CTAs per key tile of the dKV kernel, from the number of key tiles (all KV heads) and the heads of a group.
+// A split halves the longest tile and costs each CTA its own K, V and the exchange of its sums. Measured
+// (dKV kernels, us at split 1 / 2 / 4):
+//   16 tiles   256 x 32/8 heads of 128      23.5 / 18.7 / 15.2      48   3000 x 8/2 of 256    539 / 293 / 159
+//   64         1000 x 32/8 of 128             48 / 32 / 47         128   2048 x 32/8 of 64     66 / 51 / 80
+//  188         6001 x 16/4 of 256            723 / 444 / 603       256   4096 x 32/8 of 128   166 / 180 / 234
+//  256         8192 x 16/4 of 256            564 / 580 / 743       512   8192 x 32/8 of 128   326 / 378 / 498
+static int key_tile_split(long long tiles, int group) {
+  if (group % 4 == 0 && tiles * 8 <= 3 * 148) return 4;
+  if (group % 2 == 0 && tiles * 3 <= 4 * 148) return 2;
+  return 1;
 }
 
 }  // namespace ss
@@ -688,6 +777,7 @@ extern "C" int ss_attn_bwd_g(const void* q, const void* k, const void* v, const 
   p.nseq = nseq; p.T = T; p.Hq = Hq; p.Hkv = Hkv; p.ldq = lddq; p.ldk = lddk; p.ldv = lddv;
   p.scale = scale; p.status = status;
   const int tiles = (T + 127) / 128 + nseq;
+  p.split = key_tile_split(static_cast<long long>((T + 127) / 128) * Hkv, Hq / Hkv);
   const long long qc = static_cast<long long>(Hq) * dh, kc = static_cast<long long>(Hkv) * dh;
   const int stream_rows = dh == 256 ? 64 : 128;     // rows of the streamed tiles
   CUtensorMap tq128, tdo128, tk128, tv128, tqs, tdos, tks, tvs;

@@ -55,3 +55,19 @@ def test_gradients_repeat_bit_for_bit():
     runs = [attention.backward(q, k, v, out, lse, dout, cu, 700) for _ in range(3)]
     for other in runs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(runs[0], other))
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(8, 2), (6, 1), (4, 4), (16, 1)])
+@pytest.mark.parametrize("dh", [64, 128, 256])
+@pytest.mark.parametrize("lens", [[200], [130, 700, 70], [4000, 2700]], ids=lambda x: f"sum{sum(x)}")
+def test_groups_shared_by_clusters(lens, dh, Hq, Hkv):
+    """Group sizes that are and are not divisible by the cluster sizes, few and many key tiles."""
+    q, k, v, dout, cu = _inputs(lens, Hq, Hkv, dh, seed=Hq + dh)
+    out, lse = attention.forward(q, k, v, cu, max(lens))
+    dq, dk, dv = attention.backward(q, k, v, out, lse, dout, cu, max(lens))
+    again = attention.backward(q, k, v, out, lse, dout, cu, max(lens))
+    _lib.check_status()
+    assert all(torch.equal(a, b) for a, b in zip((dq, dk, dv), again))
+    out_r, lse_r = R.attention_varlen(q, k, v, cu)
+    dq_r, dk_r, dv_r = R.attention_varlen_bwd(q, k, v, out_r, lse_r, dout, cu)
+    assert _rel(dq, dq_r) < 2e-2 and _rel(dk, dk_r) < 2e-2 and _rel(dv, dv_r) < 2e-2
