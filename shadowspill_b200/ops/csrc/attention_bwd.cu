@@ -156,7 +156,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 19);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int head = blockIdx.x;
   const int kv_head = head / (p.Hq / p.Hkv);
 
@@ -176,7 +176,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int seq_start = slot->seq_start, seq_end = slot->seq_end;
   const int q0 = seq_start + (slot->work - 1) * 128;
   const int q_hi = min(q0 + 128, seq_end);
@@ -208,7 +208,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == BW_MMA_WARP) {
-    if (n_kv > 0 && elect_one()) {
+    if (n_kv > 0) {
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, DH, false, true);
       const uint32_t sq = smem_u32(smem), sdo = smem_u32(smem + Cfg::OFF_DO);
@@ -216,14 +217,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       auto scores = [&](uint32_t d, uint32_t a, uint32_t b) {
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk)
-          umma_bf16(d, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
+          umma_bf16_if(leader, d, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
                     umma_smem_desc(b + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
       };
       auto issue_s = [&](int j) -> bool {
         if (!mbar_wait(&k_full[j % KS], (j / KS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
         tc_fence_after();
         scores(tmem_base + Cfg::TM_S + (j & 1) * BKV, sq, sk0 + (j % KS) * Cfg::KV_BYTES);
-        umma_commit(&s_full[j & 1]);
+        umma_commit_if(leader, &s_full[j & 1]);
         return true;
       };
       auto issue_dp = [&](int j) -> bool {
@@ -231,8 +232,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (j > 0 && !mbar_wait(dp_free, (j - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) return false;
         tc_fence_after();
         scores(tmem_base + Cfg::TM_DP, sdo, sv0 + (j % VS) * Cfg::KV_BYTES);
-        umma_commit(dp_full);
-        umma_commit(&v_empty[j % VS]);
+        umma_commit_if(leader, dp_full);
+        umma_commit_if(leader, &v_empty[j % VS]);
         return true;
       };
       bool ok = mbar_wait(qdo_full, 0, p.status, KS_TIMEOUT_FULL) && issue_s(0) && issue_dp(0);
@@ -246,10 +247,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t ds = tmem_base + Cfg::TM_S + (j & 1) * BKV;
 #pragma unroll
         for (int kk = 0; kk < BKV / 16; ++kk)
-          umma_bf16_ts(tmem_base + Cfg::TM_DQ, ds + packed_col<BKV>(kk),
+          umma_bf16_ts_if(leader, tmem_base + Cfg::TM_DQ, ds + packed_col<BKV>(kk),
                        umma_smem_desc(sk + kk * (16 * 128), BKV * 128, 1024), idesc_dq, (j | kk) != 0);
-        umma_commit(&k_empty[j % KS]);
-        if (j + 1 == n_kv) umma_commit(dq_done);
+        umma_commit_if(leader, &k_empty[j % KS]);
+        if (j + 1 == n_kv) umma_commit_if(leader, dq_done);
       }
     }
   } else if (warp < 8) {
@@ -405,7 +406,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 25);
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), delta
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int kv_head = blockIdx.x / p.split, part = blockIdx.x % p.split;
   const int rep = p.Hq / p.Hkv / p.split;                  // query heads of this CTA
   const int head0 = kv_head * (p.Hq / p.Hkv) + part * rep;
@@ -428,7 +429,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int seq_start = slot->seq_start, seq_end = slot->seq_end;
   const int k0 = seq_start + ((seq_end - seq_start + 127) / 128 - slot->work) * 128;
   const int n_q = slot->work > 0 ? (seq_end - k0 + BQ - 1) / BQ : 0;   // query tiles at or after the key tile
@@ -462,7 +463,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
   } else if (warp == BW_MMA_WARP) {
-    if (n_it > 0 && elect_one()) {
+    if (n_it > 0) {
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BQ, false, false);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, DH, false, true);
       const uint32_t sk = smem_u32(smem), sv = smem_u32(smem + Cfg::OFF_V);
@@ -470,20 +472,20 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       auto scores = [&](uint32_t d, uint32_t a, uint32_t b) {
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk)
-          umma_bf16(d, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
+          umma_bf16_if(leader, d, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
                     umma_smem_desc(b + (kk >> 2) * (BQ * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
       };
       auto accumulate = [&](uint32_t d, uint32_t a, uint32_t b, bool fresh) {
 #pragma unroll
         for (int kk = 0; kk < BQ / 16; ++kk)
-          umma_bf16_ts(d, a + packed_col<BQ>(kk), umma_smem_desc(b + kk * (16 * 128), BQ * 128, 1024),
+          umma_bf16_ts_if(leader, d, a + packed_col<BQ>(kk), umma_smem_desc(b + kk * (16 * 128), BQ * 128, 1024),
                        idesc_acc, !(fresh && kk == 0));
       };
       auto issue_s = [&](int it) -> bool {
         if (!mbar_wait(&q_full[it % QS], (it / QS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
         tc_fence_after();
         scores(tmem_base + Cfg::TM_ST + (it % SB) * BQ, sk, sq0 + (it % QS) * Cfg::QT_BYTES);
-        umma_commit(&s_full[it % SB]);
+        umma_commit_if(leader, &s_full[it % SB]);
         return true;
       };
       bool ok = mbar_wait(kv_full, 0, p.status, KS_TIMEOUT_FULL) && issue_s(0);
@@ -496,7 +498,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           // dP^T overwrites the dS^T that the dK product before it reads: products of one issuing
           // thread run in order (the same holds for S^T and P^T below)
           scores(tmem_base + Cfg::TM_DPT, sv, sdo);
-          umma_commit(dp_full);
+          umma_commit_if(leader, dp_full);
         }
         if (SB == 2 && it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
         if (Cfg::DO_DV) {
@@ -504,22 +506,22 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (!ok) break;
           tc_fence_after();
           accumulate(tmem_base + Cfg::TM_DV, tmem_base + Cfg::TM_ST + (it % SB) * BQ, sdo, it == 0);
-          if (!Cfg::DO_DK) umma_commit(&q_empty[it % QS]);
+          if (!Cfg::DO_DK) umma_commit_if(leader, &q_empty[it % QS]);
         } else {
           ok = mbar_wait(s_free, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY);
           if (!ok) break;
           tc_fence_after();
         }
-        umma_commit(&do_empty[it % DOS]);
+        umma_commit_if(leader, &do_empty[it % DOS]);
         if (SB == 1 && it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
         if (Cfg::DO_DK) {
           ok = mbar_wait(ds_full, it & 1, p.status, KS_TIMEOUT_FULL);
           if (!ok) break;
           tc_fence_after();
           accumulate(tmem_base + Cfg::TM_DK, tmem_base + Cfg::TM_DPT, sq, it == 0);
-          umma_commit(&q_empty[it % QS]);
+          umma_commit_if(leader, &q_empty[it % QS]);
         }
-        if (it + 1 == n_it) umma_commit(acc_done);
+        if (it + 1 == n_it) umma_commit_if(leader, acc_done);
       }
     }
   } else if (warp == BW_STAT_WARP) {

@@ -78,7 +78,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   TileSlot* slot = reinterpret_cast<TileSlot*>(o_done + NT + 1);
   static_assert((1 + 2 * KS + 2 * VS + 4 * NT + 3) * 8 <= 256, "barrier space");
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const int head = blockIdx.x;
   const int kv_head = head / (p.Hq / p.Hkv);
@@ -103,7 +103,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int seq_start = slot->seq_start, seq_end = slot->seq_end;
   const int q0 = seq_start + (slot->work - 1) * (NT * 128);
   // key steps of each tile, up to its diagonal; none for a tile past the end of the sequence
@@ -146,7 +146,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == Cfg::MMA_WARP) {
     // ---------------------------------------------------------------- MMA issuer
-    if (n_max > 0 && elect_one()) {
+    if (n_max > 0) {
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, DH, false, true);
       const uint32_t sq = smem_u32(smem);
@@ -158,9 +159,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t a = sq + i * Cfg::QT_BYTES, k = sk0 + (j % KS) * Cfg::KV_BYTES;
 #pragma unroll
         for (int kk = 0; kk < DH / 16; ++kk)
-          umma_bf16(tmem_base + b * BKV, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
+          umma_bf16_if(leader, tmem_base + b * BKV, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
                     umma_smem_desc(k + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
-        umma_commit(&s_full[b]);
+        umma_commit_if(leader, &s_full[b]);
       };
       auto wait_k = [&](int j) -> bool {
         if (!mbar_wait(&k_full[j % KS], (j / KS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
@@ -172,7 +173,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int i = 0; i < NT; ++i)
           if (n_kv[i] > 0) issue_s(i, 0);
-        umma_commit(&k_empty[0]);
+        umma_commit_if(leader, &k_empty[0]);
       }
       for (int j = 0; j < n_max && ok; ++j) {
         const bool more = j + 1 < n_max;
@@ -183,7 +184,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
           if (j + 1 < n_kv[i]) issue_s(i, j + 1);
-          if (more && i == NT - 1) umma_commit(&k_empty[(j + 1) % KS]);
+          if (more && i == NT - 1) umma_commit_if(leader, &k_empty[(j + 1) % KS]);
           if (j >= n_kv[i]) continue;
           ok = mbar_wait(&p_full[i], j & 1, p.status, KS_TIMEOUT_FULL);
           if (!ok) break;
@@ -191,12 +192,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const uint32_t pa = tmem_base + (2 * i + (j & 1)) * BKV;
 #pragma unroll
           for (int kk = 0; kk < BKV / 16; ++kk)
-            umma_bf16_ts(tmem_base + Cfg::TM_O + i * DH, pa + kk * 8,
+            umma_bf16_ts_if(leader, tmem_base + Cfg::TM_O + i * DH, pa + kk * 8,
                          umma_smem_desc(v + kk * (16 * 128), BKV * 128, 1024), idesc_o, (j | kk) != 0);
-          umma_commit(&o_done[i]);
+          umma_commit_if(leader, &o_done[i]);
         }
         if (!ok) break;
-        umma_commit(&v_empty[j % VS]);
+        umma_commit_if(leader, &v_empty[j % VS]);
       }
     }
   } else {
