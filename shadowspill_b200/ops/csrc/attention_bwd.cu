@@ -116,6 +116,13 @@ __device__ __forceinline__ void tmem_st_half(uint32_t addr, const uint32_t (&pk)
   tmem_st_wait();
 }
 
+template <int PN>   // PN packed pairs' columns: 32 or 16 score columns
+__device__ __forceinline__ void tmem_st_quarter(uint32_t addr, const uint32_t (&pk)[PN / 2]) {
+  if constexpr (PN == 32) tmem_st_32x16(addr, pk);
+  else tmem_st_32x8(addr, pk);
+  tmem_st_wait();
+}
+
 // ============================================================================ dQ kernel
 // S is double-buffered and dP single: S of the next tile is formed under this tile's
 // exponentials, dP of the next tile under this tile's dS. K is released by the dQ product and has
@@ -397,13 +404,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* stat_full = bars + 9;       // 4
   uint64_t* stat_empty = bars + 13;     // 4
   uint64_t* s_full = bars + 17;         // 2
-  uint64_t* p_full = bars + 19;         // 1
-  uint64_t* dp_full = bars + 20;        // 1
-  uint64_t* ds_full = bars + 21;        // 1
-  uint64_t* s_free = bars + 22;         // 1 (only without a P^T to wait for)
-  uint64_t* acc_done = bars + 23;       // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
-  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 25);
+  uint64_t* p_full = bars + 19;         // 2: first and second half of every warp's columns
+  uint64_t* dp_full = bars + 21;        // 1
+  uint64_t* ds_full = bars + 22;        // 1
+  uint64_t* s_free = bars + 23;         // 1 (only without a P^T to wait for)
+  uint64_t* acc_done = bars + 24;       // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 26);
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), delta
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
@@ -417,7 +424,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int i = 0; i < DOS; ++i) { mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); }
     for (int i = 0; i < STS; ++i) { mbar_init(&stat_full[i], 1); mbar_init(&stat_empty[i], 8); }
     for (int i = 0; i < SB; ++i) mbar_init(&s_full[i], 1);
-    mbar_init(p_full, 8);
+    mbar_init(&p_full[0], 8);
+    mbar_init(&p_full[1], 8);
     mbar_init(dp_full, 1);
     mbar_init(ds_full, 8);
     mbar_init(s_free, 8);
@@ -475,10 +483,12 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           umma_bf16_if(leader, d, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
                     umma_smem_desc(b + (kk >> 2) * (BQ * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
       };
-      auto accumulate = [&](uint32_t d, uint32_t a, uint32_t b, bool fresh) {
+      // part 0 / 1: the steps over the first / second half of each warp's columns; -1: all
+      auto accumulate = [&](uint32_t d, uint32_t a, uint32_t b, bool fresh, int part) {
 #pragma unroll
         for (int kk = 0; kk < BQ / 16; ++kk)
-          umma_bf16_ts_if(leader, d, a + packed_col<BQ>(kk), umma_smem_desc(b + kk * (16 * 128), BQ * 128, 1024),
+          if (part < 0 || (kk * 16) % (BQ / 2) / (BQ / 4) == part)
+            umma_bf16_ts_if(leader, d, a + packed_col<BQ>(kk), umma_smem_desc(b + kk * (16 * 128), BQ * 128, 1024),
                        idesc_acc, !(fresh && kk == 0));
       };
       auto issue_s = [&](int it) -> bool {
@@ -502,10 +512,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         if (SB == 2 && it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
         if (Cfg::DO_DV) {
-          ok = mbar_wait(p_full, it & 1, p.status, KS_TIMEOUT_FULL);
+          // S^T of the next tile waits behind this product, and P^T of the next tile for that: its first half
+          // starts under the exponentials of the second
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            ok = mbar_wait(&p_full[x], it & 1, p.status, KS_TIMEOUT_FULL);
+            if (!ok) break;
+            tc_fence_after();
+            accumulate(tmem_base + Cfg::TM_DV, tmem_base + Cfg::TM_ST + (it % SB) * BQ, sdo, it == 0, x);
+          }
           if (!ok) break;
-          tc_fence_after();
-          accumulate(tmem_base + Cfg::TM_DV, tmem_base + Cfg::TM_ST + (it % SB) * BQ, sdo, it == 0);
           if (!Cfg::DO_DK) umma_commit_if(leader, &q_empty[it % QS]);
         } else {
           ok = mbar_wait(s_free, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY);
@@ -518,7 +534,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           ok = mbar_wait(ds_full, it & 1, p.status, KS_TIMEOUT_FULL);
           if (!ok) break;
           tc_fence_after();
-          accumulate(tmem_base + Cfg::TM_DK, tmem_base + Cfg::TM_DPT, sq, it == 0);
+          accumulate(tmem_base + Cfg::TM_DK, tmem_base + Cfg::TM_DPT, sq, it == 0, -1);
           umma_commit_if(leader, &q_empty[it % QS]);
         }
         if (it + 1 == n_it) umma_commit_if(leader, acc_done);
@@ -579,28 +595,33 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       // whole tile visible: every query of the tile is at or after every key, none past the end
       const bool all_valid = qt0 >= k0 + 127 && qt0 + BQ <= seq_end;
+      const int first = gk - (qt0 + half * HN), last = seq_end - (qt0 + half * HN);   // visible: [first, last)
 #pragma unroll
-      for (int e = 0; e < HN; e += 4) {
-        const float4 l = ld_shared_f4(nlse + e * 4);
-        s[e] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, l.x)));
-        s[e + 1] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 1]), c2, l.y)));
-        s[e + 2] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 2]), c2, l.z)));
-        s[e + 3] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 3]), c2, l.w)));
-      }
-      if (!all_valid) {
-        const int first = gk - (qt0 + half * HN), last = seq_end - (qt0 + half * HN);   // columns in [first, last)
+      for (int x = 0; x < 2; ++x) {
+        constexpr int PN = HN / 2;
+        uint32_t pk[PN / 2];
 #pragma unroll
-        for (int e = 0; e < HN; ++e)
-          if (e < first || e >= last) s[e] = 0u;
-      }
-      if (Cfg::DO_DV) {
-        uint32_t pk[HN / 2];
+        for (int e = x * PN; e < (x + 1) * PN; e += 4) {
+          const float4 l = ld_shared_f4(nlse + e * 4);
+          s[e] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, l.x)));
+          s[e + 1] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 1]), c2, l.y)));
+          s[e + 2] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 2]), c2, l.z)));
+          s[e + 3] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 3]), c2, l.w)));
+        }
+        if (!all_valid) {
 #pragma unroll
-        for (int e = 0; e < HN; e += 2) pk[e >> 1] = pack_bf16(__uint_as_float(s[e]), __uint_as_float(s[e + 1]));
-        tmem_st_half<HN>(s_addr, pk);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(p_full);
+          for (int e = x * PN; e < (x + 1) * PN; ++e)
+            if (e < first || e >= last) s[e] = 0u;
+        }
+        if (Cfg::DO_DV) {
+#pragma unroll
+          for (int e = 0; e < PN; e += 2)
+            pk[e >> 1] = pack_bf16(__uint_as_float(s[x * PN + e]), __uint_as_float(s[x * PN + e + 1]));
+          tmem_st_quarter<PN>(s_addr + x * (PN / 2), pk);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_full[x]);
+        }
       }
       if (Cfg::DO_DK) {
         if (!mbar_wait(dp_full, it & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
