@@ -21,7 +21,7 @@
 // delta[h,t] = sum_d dO*O comes from a small preprocess kernel into caller
 // scratch (fp32 [Hq, T]).
 //
-// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: dQ 2.42 -> 1.25 ms, dKV 3.15 -> 1.69 ms
+// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: dQ 2.42 -> 1.19 ms, dKV 3.15 -> 1.58 ms
 // against P^T and dS through shared memory in 64-row tiles.
 //
 // warps 0..7 softmax: warp w owns TMEM lanes 32*(w%4)..+31 and the left or right half (w/4) of
@@ -92,11 +92,8 @@ __device__ __forceinline__ constexpr uint32_t packed_col(int kk) {
 
 // An explicit shared-memory load: through the aligned-up window pointer the compiler only sees a
 // generic address, whose loads take the global path (they were most of the dKV kernel's stalls).
-__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-  return v;
+__device__ __forceinline__ void ld_shared_2x2(uint32_t addr, f32x2& a, f32x2& b) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }
 
 __device__ __forceinline__ void st_shared_f32(uint32_t addr, float v) {
@@ -268,9 +265,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t dp_addr = lane_addr + Cfg::TM_DP + half * HN;
     const long long li = static_cast<long long>(head) * p.T + max(0, min(gq, p.T - 1));
-    const float nlse = -p.lse[li] * LOG2E;
-    const float dl = p.delta[li];
-    const float c2 = p.scale * LOG2E;
+    const float nlse1 = -p.lse[li] * LOG2E, ndl1 = -p.delta[li], c21 = p.scale * LOG2E;
+    const f32x2 nlse = pack_x2(nlse1, nlse1), ndl = pack_x2(ndl1, ndl1), c2 = pack_x2(c21, c21);
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
       const int b = j & 1;
@@ -280,13 +276,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       uint32_t s[HN];
       tmem_ld_half<HN>(s_addr, s);
       const int k0 = seq_start + j * BKV + half * HN;
-      if (k0 + HN - 1 <= q0) {                     // every key of this half is visible to every row
 #pragma unroll
-        for (int e = 0; e < HN; ++e) s[e] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, nlse)));
-      } else {
+      for (int e = 0; e < HN; e += 2) {
+        const float2 t = unpack_x2(fma_x2(pack_x2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), c2, nlse));
+        s[e] = __float_as_uint(fast_exp2(t.x));
+        s[e + 1] = __float_as_uint(fast_exp2(t.y));
+      }
+      if (k0 + HN - 1 > q0) {                      // some key of this half is hidden from some row
 #pragma unroll
         for (int e = 0; e < HN; ++e)
-          s[e] = k0 + e > gq ? 0u : __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, nlse)));
+          if (k0 + e > gq) s[e] = 0u;
       }
       if (!mbar_wait(dp_full, j & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
@@ -297,9 +296,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (lane == 0) mbar_arrive(dp_free);
       uint32_t pk[HN / 2];
 #pragma unroll
-      for (int e = 0; e < HN; e += 2)             // the softmax scale is applied to dQ once, at the end
-        pk[e >> 1] = pack_bf16(__uint_as_float(s[e]) * (__uint_as_float(d[e]) - dl),
-                               __uint_as_float(s[e + 1]) * (__uint_as_float(d[e + 1]) - dl));
+      for (int e = 0; e < HN; e += 2) {           // the softmax scale is applied to dQ once, at the end
+        const float2 ds = unpack_x2(mul_x2(pack_x2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])),
+                                           add_x2(pack_x2(__uint_as_float(d[e]), __uint_as_float(d[e + 1])), ndl)));
+        pk[e >> 1] = pack_bf16(ds.x, ds.y);
+      }
       tmem_st_half<HN>(s_addr, pk);
       tc_fence_before();
       __syncwarp();
@@ -411,7 +412,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* acc_done = bars + 24;       // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
   TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 26);
-  float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), delta
+  float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), -delta
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int kv_head = blockIdx.x / p.split, part = blockIdx.x % p.split;
@@ -556,7 +557,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const int gq = qt0 + lane + u * 32;
         const bool in = gq < seq_end;
         nl[u] = in ? -__ldg(p.lse + base + gq) * LOG2E : -INFINITY;
-        dl[u] = in ? __ldg(p.delta + base + gq) : 0.f;
+        dl[u] = in ? -__ldg(p.delta + base + gq) : 0.f;
       }
       if (it >= STS && !mbar_wait(&stat_empty[st], ((it / STS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
       const uint32_t dst = smem_u32(s_stat + st * (2 * BQ) + lane);
@@ -575,13 +576,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int gk = k0 + row;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t dp_addr = lane_addr + Cfg::TM_DPT + half * HN;
-    const float c2 = p.scale * LOG2E;
+    const f32x2 c2 = pack_x2(p.scale * LOG2E, p.scale * LOG2E);
     const uint32_t stat = smem_u32(s_stat);
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
       const int st = it % STS;
       const int qt0 = k0 + (it % n_q) * BQ;
-      const uint32_t nlse = stat + (st * (2 * BQ) + half * HN) * 4, delta = nlse + BQ * 4;
+      const uint32_t nlse = stat + (st * (2 * BQ) + half * HN) * 4, ndelta = nlse + BQ * 4;
       if (!mbar_wait(&stat_full[st], (it / STS) & 1, p.status, KS_TIMEOUT_FULL)) { ok = false; break; }
       const uint32_t s_addr = lane_addr + Cfg::TM_ST + (it % SB) * BQ + half * HN;
       if (!mbar_wait(&s_full[it % SB], (it / SB) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
@@ -602,11 +603,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         uint32_t pk[PN / 2];
 #pragma unroll
         for (int e = x * PN; e < (x + 1) * PN; e += 4) {
-          const float4 l = ld_shared_f4(nlse + e * 4);
-          s[e] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e]), c2, l.x)));
-          s[e + 1] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 1]), c2, l.y)));
-          s[e + 2] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 2]), c2, l.z)));
-          s[e + 3] = __float_as_uint(fast_exp2(fmaf(__uint_as_float(s[e + 3]), c2, l.w)));
+          f32x2 l[2];
+          ld_shared_2x2(nlse + e * 4, l[0], l[1]);
+#pragma unroll
+          for (int u = 0; u < 4; u += 2) {
+            const float2 t = unpack_x2(fma_x2(pack_x2(__uint_as_float(s[e + u]), __uint_as_float(s[e + u + 1])), c2,
+                                              l[u >> 1]));
+            s[e + u] = __float_as_uint(fast_exp2(t.x));
+            s[e + u + 1] = __float_as_uint(fast_exp2(t.y));
+          }
         }
         if (!all_valid) {
 #pragma unroll
@@ -630,11 +635,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tmem_ld_half<HN>(dp_addr, d);
 #pragma unroll
         for (int e = 0; e < HN; e += 4) {     // the softmax scale is applied to dK once, at the end
-          const float4 dl = ld_shared_f4(delta + e * 4);
-          pk[e >> 1] = pack_bf16(__uint_as_float(s[e]) * (__uint_as_float(d[e]) - dl.x),
-                                 __uint_as_float(s[e + 1]) * (__uint_as_float(d[e + 1]) - dl.y));
-          pk[(e >> 1) + 1] = pack_bf16(__uint_as_float(s[e + 2]) * (__uint_as_float(d[e + 2]) - dl.z),
-                                       __uint_as_float(s[e + 3]) * (__uint_as_float(d[e + 3]) - dl.w));
+          f32x2 ndl[2];
+          ld_shared_2x2(ndelta + e * 4, ndl[0], ndl[1]);
+#pragma unroll
+          for (int u = 0; u < 4; u += 2) {
+            const float2 ds =
+                unpack_x2(mul_x2(pack_x2(__uint_as_float(s[e + u]), __uint_as_float(s[e + u + 1])),
+                                 add_x2(pack_x2(__uint_as_float(d[e + u]), __uint_as_float(d[e + u + 1])), ndl[u >> 1])));
+            pk[(e + u) >> 1] = pack_bf16(ds.x, ds.y);
+          }
         }
         tmem_st_half<HN>(dp_addr, pk);
         tc_fence_before();

@@ -9,10 +9,11 @@
 // in the long case below).
 // P goes back to TMEM over the scores it comes from and is the A operand of P V from there: it never
 // passes through shared memory, whose bandwidth the two products need for K, V and Q.
-// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: 1.41 -> 1.02 ms; 8,192 packed tokens:
-// 0.317 -> 0.225 ms; 6,001 tokens, 16/4 heads of 256: 0.285 -> 0.160 ms, against one tile per CTA and
-// P through shared memory. The softmax warps bound it: of 1980 cycles per 128 x 128 scores, 1024 are
-// exponentials and 1280 products.
+// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: 1.41 -> 0.95 ms; 8,192 packed tokens:
+// 0.317 -> 0.209 ms; 6,001 tokens, 16/4 heads of 256: 0.285 -> 0.150 ms, against one tile per CTA and
+// P through shared memory. The softmax warps' instruction stream bounds it: of 1850 cycles per 128 x 128
+// scores, 1024 are exponentials and 1280 products, and replacing a quarter of the exponentials by
+// polynomials of ten instructions made it slower (1.08 against 0.97 ms).
 //
 //   warps 0..4*NT-1  softmax, rescaling of O, epilogue: one query row per thread
 //   then one TMA producer warp and one MMA warp
@@ -236,10 +237,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-      for (int e = 4; e < BKV; e += 4) {
+      for (int e = 4; e + 8 <= BKV; e += 8) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], s[e + u]);
+        for (int u = 0; u < 4; ++u) mx[u] = max3(mx[u], s[e + u], s[e + 4 + u]);
       }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], s[BKV - 4 + u]);
       const float m_t = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;
       // lazy rescale: move the reference max only when it would grow by > 8 (2^8 headroom)
       const bool want = m_t > m_used + 8.f;
@@ -262,26 +265,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_st_32x32(o_addr + x, r);
         }
       }
-      const float nm = -m_used;
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      const f32x2 nm = pack_x2(-m_used, -m_used), cc = pack_x2(c, c);
+      f32x2 sum[2] = {0ull, 0ull};
 #pragma unroll
       for (int x = 0; x < BKV; x += 32) {
         uint32_t pk[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
-          float p0 = fast_exp2(fmaf(s[x + e], c, nm));
-          float p1 = fast_exp2(fmaf(s[x + e + 1], c, nm));
+          const float2 t = unpack_x2(fma_x2(pack_x2(s[x + e], s[x + e + 1]), cc, nm));
+          float p0 = fast_exp2(t.x);
+          float p1 = fast_exp2(t.y);
           if (diag) {
             if (k0 + x + e > gq) p0 = 0.f;
             if (k0 + x + e + 1 > gq) p1 = 0.f;
           }
-          sum[e & 2] += p0;
-          sum[(e & 2) + 1] += p1;
+          sum[(e & 2) >> 1] = add_x2(sum[(e & 2) >> 1], pack_x2(p0, p1));
           pk[e >> 1] = pack_bf16(p0, p1);
         }
         tmem_st_32x16(s_addr + (x >> 1), pk);
       }
-      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      const float2 sa = unpack_x2(sum[0]), sb = unpack_x2(sum[1]);
+      l += (sa.x + sa.y) + (sb.x + sb.y);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
