@@ -64,10 +64,11 @@ __host__ __device__ constexpr int norm_ring(int vpt) { return vpt > 4 ? 3 : 4; }
 // ============================================================================ rows of <= 512 channels
 // Row r of a tensor is head r % heads of token r / heads: `ld` elements between tokens, D between heads.
 struct NormRows {
-  const bf16* x; long long ldx;
+  bf16* x; long long ldx;
   bf16* y; long long ldy;               // normalised rows, or dx
   const bf16* z; long long ldz;         // backward: gy
   bf16* raw; long long ldraw;           // forward: a copy of the input rows, optional
+  const bf16* delta;                    // forward: folded into x first; x is rewritten (rows of one head)
   const bf16* w;
   float* rstd;                          // [rows]
   float* dw;                            // [D] fp32, accumulated; optional
@@ -81,7 +82,9 @@ struct NormRows {
   }
 };
 
-template <int LANES, int VPT>
+// The row's sum is formed the same way with and without DELTA, so a residual add that one caller fuses and
+// another does not gives both the same bits.
+template <int LANES, int VPT, bool DELTA>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_short_kernel(const NormRows p) {
   const int lane = threadIdx.x & (LANES - 1), nv = p.D >> 3;
@@ -93,26 +96,42 @@ rmsnorm_fwd_short_kernel(const NormRows p) {
     wq[i] = c < nv ? reinterpret_cast<const uint4*>(p.w)[c] : make_uint4(0, 0, 0, 0);
   }
   const long long step = static_cast<long long>(gridDim.x) * (NORM_THREADS / LANES);
-  auto fetch = [&](long long r, uint4 (&o)[VPT]) {
+  uint4 xq[VPT], xn[VPT], dq[VPT], dn[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) xq[i] = xn[i] = dq[i] = dn[i] = make_uint4(0, 0, 0, 0);
+  auto fetch = [&](long long r, uint4 (&o)[VPT], uint4 (&d)[VPT]) {
     const uint4* xr = reinterpret_cast<const uint4*>(p.x + p.at(r, p.ldx));
+    const uint4* er = DELTA ? reinterpret_cast<const uint4*>(p.delta + r * p.D) : nullptr;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i)
-      if (lane + i * LANES < nv) o[i] = xr[lane + i * LANES];
+    for (int i = 0; i < VPT; ++i) {
+      if (lane + i * LANES >= nv) continue;
+      o[i] = xr[lane + i * LANES];
+      if (DELTA) d[i] = er[lane + i * LANES];
+    }
   };
-  uint4 xq[VPT], xn[VPT];
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) xq[i] = xn[i] = make_uint4(0, 0, 0, 0);
   const long long r0 = blockIdx.x * static_cast<long long>(NORM_THREADS / LANES) + threadIdx.x / LANES;
-  if (r0 < p.rows) fetch(r0, xq);
+  if (r0 < p.rows) fetch(r0, xq, dq);
   // a warp's lanes stay together through the shuffles: rows past the end are computed and not stored
   for (long long r = r0, base = blockIdx.x * static_cast<long long>(NORM_THREADS / LANES); base < p.rows;
        r += step, base += step) {
-    if (r + step < p.rows) fetch(r + step, xn);
+    if (r + step < p.rows) fetch(r + step, xn, dn);
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       float v[8];
       norm_unpack8(xq[i], v);
+      if (DELTA) {
+        float d[8];
+        norm_unpack8(dq[i], d);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] += d[e];
+        // The residual stream is kept in bf16: round once here so that the
+        // normalised value and the stored stream agree.
+        xq[i] = norm_pack8(v);
+        norm_unpack8(xq[i], v);
+        if (r < p.rows && lane + i * LANES < nv)
+          reinterpret_cast<uint4*>(p.x + p.at(r, p.ldx))[lane + i * LANES] = xq[i];
+      }
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
     }
@@ -135,7 +154,7 @@ rmsnorm_fwd_short_kernel(const NormRows p) {
       }
     }
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) xq[i] = xn[i];
+    for (int i = 0; i < VPT; ++i) { xq[i] = xn[i]; dq[i] = dn[i]; }
   }
 }
 
@@ -438,20 +457,22 @@ struct LongShape {
   }
 };
 
-template <bool FWD>
+enum { FWD, FWD_DELTA, BWD };
+template <int KIND, int LANES, int VPT>
+static int launch_short_as(const NormRows& p, cudaStream_t s) {
+  const long long per = NORM_THREADS / LANES, blocks = (p.rows + per - 1) / per;
+  const long long cap = 148 * (KIND == BWD ? 4 : 8);
+  const int grid = static_cast<int>(blocks < cap ? blocks : cap);
+  if constexpr (KIND == BWD) rmsnorm_bwd_short_kernel<LANES, VPT><<<grid, NORM_THREADS, 0, s>>>(p);
+  else rmsnorm_fwd_short_kernel<LANES, VPT, KIND == FWD_DELTA><<<grid, NORM_THREADS, 0, s>>>(p);
+  return static_cast<int>(cudaGetLastError());
+}
+template <int KIND>
 static int launch_short(const NormRows& p, cudaStream_t s) {
-  auto go = [&](auto fwd, auto bwd, int lanes) -> int {
-    const long long per = NORM_THREADS / lanes, blocks = (p.rows + per - 1) / per;
-    const long long cap = 148 * (FWD ? 8 : 4);
-    const int grid = static_cast<int>(blocks < cap ? blocks : cap);
-    if (FWD) fwd<<<grid, NORM_THREADS, 0, s>>>(p);
-    else bwd<<<grid, NORM_THREADS, 0, s>>>(p);
-    return static_cast<int>(cudaGetLastError());
-  };
-  if (p.D <= 64) return go(rmsnorm_fwd_short_kernel<8, 1>, rmsnorm_bwd_short_kernel<8, 1>, 8);
-  if (p.D <= 128) return go(rmsnorm_fwd_short_kernel<16, 1>, rmsnorm_bwd_short_kernel<16, 1>, 16);
-  if (p.D <= 256) return go(rmsnorm_fwd_short_kernel<32, 1>, rmsnorm_bwd_short_kernel<32, 1>, 32);
-  return go(rmsnorm_fwd_short_kernel<32, 2>, rmsnorm_bwd_short_kernel<32, 2>, 32);
+  if (p.D <= 64) return launch_short_as<KIND, 8, 1>(p, s);
+  if (p.D <= 128) return launch_short_as<KIND, 16, 1>(p, s);
+  if (p.D <= 256) return launch_short_as<KIND, 32, 1>(p, s);
+  return launch_short_as<KIND, 32, 2>(p, s);
 }
 
 }  // namespace ss
@@ -465,11 +486,11 @@ int ss_rmsnorm_fwd(void* x, const void* delta, const void* w, void* y, float* rs
   if (!aligned16(x) || !aligned16(delta) || !aligned16(w) || !aligned16(y)) return -2;
   if (T <= 0) return 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (D <= 512 && delta == nullptr) {
+  if (D <= 512) {
     NormRows p{};
-    p.x = (const bf16*)x; p.y = (bf16*)y; p.w = (const bf16*)w; p.rstd = rstd;
+    p.x = (bf16*)x; p.delta = (const bf16*)delta; p.y = (bf16*)y; p.w = (const bf16*)w; p.rstd = rstd;
     p.ldx = p.ldy = D; p.rows = T; p.heads = 1; p.D = D; p.zero_centered = zero_centered; p.eps = eps;
-    return launch_short<true>(p, s);
+    return delta ? launch_short<FWD_DELTA>(p, s) : launch_short<FWD>(p, s);
   }
   auto go = [&](auto kern, SmemOptIn& opt_in, int vpt) -> int {
     const LongShape shape(T, D, delta ? 2 : 1, norm_ring(vpt), 4, 1);
@@ -492,11 +513,11 @@ int ss_rmsnorm_bwd(const void* x, const void* w, const void* gy, const float* rs
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (D <= 512) {
     NormRows p{};
-    p.x = (const bf16*)x; p.z = (const bf16*)gy; p.y = (bf16*)dx; p.w = (const bf16*)w;
+    p.x = (bf16*)x; p.z = (const bf16*)gy; p.y = (bf16*)dx; p.w = (const bf16*)w;
     p.rstd = const_cast<float*>(rstd); p.dw = dw;
     p.ldx = p.ldy = p.ldz = D; p.rows = T; p.heads = 1; p.D = D; p.zero_centered = zero_centered;
     p.accumulate = accumulate;
-    return launch_short<false>(p, s);
+    return launch_short<BWD>(p, s);
   }
   auto go = [&](auto kern, SmemOptIn& opt_in, int vpt) -> int {
     const LongShape shape(T, D, accumulate ? 3 : 2, norm_ring(vpt), 4, 8);   // eight rows to a weight-gradient flush
@@ -522,10 +543,10 @@ int ss_headnorm_fwd(const void* x, long long ldx, const void* w, void* y, long l
   if (static_cast<long long>(T) * heads > 0x7fffffffLL) return -2;
   if (T <= 0) return 0;
   NormRows p{};
-  p.x = (const bf16*)x; p.ldx = ldx; p.y = (bf16*)y; p.ldy = ldy; p.raw = (bf16*)raw; p.ldraw = ldraw;
+  p.x = (bf16*)x; p.ldx = ldx; p.y = (bf16*)y; p.ldy = ldy; p.raw = (bf16*)raw; p.ldraw = ldraw;
   p.w = (const bf16*)w; p.rstd = rstd; p.rows = static_cast<long long>(T) * heads; p.heads = heads; p.D = D;
   p.zero_centered = zero_centered; p.eps = eps;
-  return launch_short<true>(p, reinterpret_cast<cudaStream_t>(stream));
+  return launch_short<FWD>(p, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // Backward of ss_headnorm_fwd; dx may be gy. dw (fp32 [D]) is accumulated.
@@ -536,10 +557,10 @@ int ss_headnorm_bwd(const void* x, long long ldx, const void* w, const void* gy,
   if (static_cast<long long>(T) * heads > 0x7fffffffLL) return -2;
   if (T <= 0) return 0;
   NormRows p{};
-  p.x = (const bf16*)x; p.ldx = ldx; p.z = (const bf16*)gy; p.ldz = ldg; p.y = (bf16*)dx; p.ldy = lddx;
+  p.x = (bf16*)x; p.ldx = ldx; p.z = (const bf16*)gy; p.ldz = ldg; p.y = (bf16*)dx; p.ldy = lddx;
   p.w = (const bf16*)w; p.rstd = const_cast<float*>(rstd); p.dw = dw;
   p.rows = static_cast<long long>(T) * heads; p.heads = heads; p.D = D; p.zero_centered = zero_centered;
-  return launch_short<false>(p, reinterpret_cast<cudaStream_t>(stream));
+  return launch_short<BWD>(p, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -73,3 +73,15 @@ def test_heads_in_place(dh, T, heads, rest):
     assert _rel(d[:, :n], dx_r.view(T, n)) < TOL and _rel(dw, dw_r) < 1e-4
     assert torch.equal(d[:, n:], dtail)
     _lib.check_status()
+
+
+@pytest.mark.parametrize("D", [64, 128, 256, 512, 1024, 2048, 4096, 8192])
+def test_fused_residual_add_gives_the_same_bits(D):
+    """One frontend folds the residual add into the norm and another adds first: same results."""
+    g = torch.Generator().manual_seed(D)
+    x, w, delta = _rand(g, 300, D), _rand(g, D), _rand(g, 300, D)
+    added = x + delta
+    y, rstd = F.rmsnorm_fwd(added.clone(), w, EPS)
+    folded = x.clone()
+    y2, rstd2 = F.rmsnorm_fwd(folded, w, EPS, delta=delta)
+    assert torch.equal(folded, added) and torch.equal(y, y2) and torch.equal(rstd, rstd2)
