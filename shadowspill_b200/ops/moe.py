@@ -30,7 +30,7 @@ _lib.register("ss_moe_combine", [_c.c_p, _c.c_ll, _c.c_p, _c.c_p, _c.c_p, _c.c_l
                                  _c.c_int, _c.c_int, _c.c_int, _c.c_p, _c.c_ll, _c.c_p, _c.c_p])
 _lib.register("ss_gemm_grouped_bf16", [_c.c_p, _c.c_p, _c.c_p, _c.c_int, _c.c_int, _c.c_int,
                                        _c.c_int, _c.c_int, _c.c_int, _c.c_ll, _c.c_ll, _c.c_ll,
-                                       _c.c_int, _c.c_int, _c.c_int, _c.c_p, _c.c_p, _c.c_int,
+                                       _c.c_int, _c.c_int, _c.c_int, _c.c_p, _c.c_p, _c.c_p, _c.c_int,
                                        _c.c_p, _c.c_p])
 
 
@@ -65,6 +65,7 @@ class Layout:
         E = counts.numel()
         dev = ids.device
         self.T, self.k, self.E = T, k, E
+        self.counts = counts
         self.rows = -(-(T * k + E * 127) // 128) * 128      # worst-case padded rows
         self.tiles = self.rows // 128
         self.offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
@@ -140,7 +141,7 @@ def grouped_linear(x_sorted: torch.Tensor, bank: torch.Tensor, lay: Layout, tran
     _lib.check(_lib.lib().ss_gemm_grouped_bf16(
         x_sorted.data_ptr(), bank.data_ptr(), out.data_ptr(), 1, lay.rows, 0, N, K, E,
         x_sorted.stride(0), bank.stride(1), out.stride(0), int(transpose), 0, 0,
-        lay.tile_expert.data_ptr(), None, 0, _lib.status_ptr(x_sorted),
+        lay.tile_expert.data_ptr(), None, None, 0, _lib.status_ptr(x_sorted),
         _lib.stream_ptr()), "ss_gemm_grouped_bf16")
     return out
 
@@ -149,10 +150,11 @@ def grouped_wgrad(dy_sorted: torch.Tensor, x_sorted: torch.Tensor, lay: Layout, 
                   accumulate: bool) -> None:
     """``out[e] (+)= dy[rows_e]^T @ x[rows_e]`` for every expert of a bank gradient [E, M, N]."""
     E, M, N = out.shape
+    counts = getattr(lay, "counts", None)      # a layout without them has its padding contracted too
     _lib.check(_lib.lib().ss_gemm_grouped_bf16(
         dy_sorted.data_ptr(), x_sorted.data_ptr(), out.data_ptr(), 2, lay.rows, M, N, 0, E,
         dy_sorted.stride(0), x_sorted.stride(0), out.stride(1), 1, int(out.dtype == torch.float32),
-        int(accumulate), None, lay.offsets.data_ptr(), 0,
+        int(accumulate), None, lay.offsets.data_ptr(), None if counts is None else counts.data_ptr(), 0,
         _lib.status_ptr(out), _lib.stream_ptr()), "ss_gemm_grouped_bf16")
 
 

@@ -66,3 +66,24 @@ def test_router_gradient(T, E, k, renorm):
     moe._weights_from_logits(leaf, ids.long(), renorm).backward(dwts.double())
     # fp32 weights and sums; for one expert or one pick the exact gradient may be zero
     assert float((got.double() - leaf.grad).abs().max()) < 1e-5 * (1.0 + float(leaf.grad.abs().max()))
+
+
+@pytest.mark.parametrize("M,N", [(256, 512), (136, 72)])
+def test_bank_gradient_leaves_out_blocks_of_padding(M, N):
+    loads = [0, 1, 63, 64, 65, 127, 128, 129, 192, 300, 0]
+    ids = torch.repeat_interleave(torch.arange(len(loads), dtype=torch.int32, device=DEV),
+                                  torch.tensor(loads, device=DEV)).reshape(-1, 1)
+    lay = moe.Layout(ids, torch.tensor(loads, dtype=torch.int32, device=DEV))
+    g = torch.Generator(device=DEV).manual_seed(M)
+    dy, x = (lay.gather(torch.randn(ids.numel(), w, generator=g, device=DEV).to(torch.bfloat16)) for w in (M, N))
+    out = torch.full((len(loads), M, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    moe.grouped_wgrad(dy, x, lay, out, False)
+    whole, lay.counts = torch.full_like(out, 5.0), None            # the padding contracted as well
+    moe.grouped_wgrad(dy, x, lay, whole, False)
+    _lib.check_status()
+    assert torch.equal(out, whole)
+    off = lay.offsets.tolist()
+    for e, n in enumerate(loads):
+        want = dy[off[e]:off[e] + n].double().T @ x[off[e]:off[e] + n].double()
+        # fp32 sums of exact products, rounded to bf16 once (2^-9 of each value)
+        assert float((out[e].double() - want).abs().max()) <= 2.0 ** -8 * (1e-3 + float(want.abs().max() if n else 0))
