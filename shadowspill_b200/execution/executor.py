@@ -344,6 +344,7 @@ class TaskRunner:
 
     def _optimizer(self, stage: int, B) -> None:
         st, h = self.stages[stage], self.hyper
+        fused: dict[tuple, list] = {}         # (learning rate, weight decay) -> flat tensors
         for p in st.params:
             if not p.trainable:
                 continue
@@ -367,12 +368,13 @@ class TaskRunner:
                                        beta1=h.beta1, beta2=h.beta2, eps=h.eps, weight_decay=wd,
                                        step=self.completed_updates + 1, grad_scale=h.grad_scale)
                 continue
-            F.adamw_(B["params"][p.name].view(-1), B["grads"][p.name].view(-1),
-                     B["m"][p.name].view(-1), B["v"][p.name].view(-1), lr=lr, beta1=h.beta1,
-                     beta2=h.beta2, eps=h.eps, weight_decay=wd,
-                     step=self.completed_updates + 1, grad_scale=h.grad_scale, seed=self.seed,
-                     offset=self.param_offsets[(stage, p.name)], stochastic_param=self.sr,
-                     stochastic_state=self.sr)
+            fused.setdefault((lr, wd), []).append((
+                B["params"][p.name].view(-1), B["grads"][p.name].view(-1), B["m"][p.name].view(-1),
+                B["v"][p.name].view(-1), self.param_offsets[(stage, p.name)]))
+        for (lr, wd), tensors in fused.items():
+            F.adamw_many_(tensors, lr=lr, beta1=h.beta1, beta2=h.beta2, eps=h.eps, weight_decay=wd,
+                          step=self.completed_updates + 1, grad_scale=h.grad_scale, seed=self.seed,
+                          stochastic_param=self.sr, stochastic_state=self.sr)
 
 
 class Executor:

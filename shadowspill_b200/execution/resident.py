@@ -82,24 +82,24 @@ class ResidentTrainer:
     def optim_step(self, grad_scale: float = 1.0) -> None:
         self.step_count += 1
         offset = 0
+        fused = []
         for si, st in enumerate(self.stages):
             for p in st.params:
                 if not p.trainable:
                     offset += (p.numel + 7) // 8 * 8
                     continue
-                pt, gt = self.P[si][p.name], self.G[si][p.name]
+                flat = (self.P[si][p.name].view(-1), self.G[si][p.name].view(-1),
+                        self.M[si][p.name].view(-1), self.V[si][p.name].view(-1))
                 if self.rule != "adamw":
                     from ..ops import reference
-                    reference.update_rule_(self.rule, pt.view(-1), gt.view(-1), self.M[si][p.name].view(-1),
-                                           self.V[si][p.name].view(-1), step=self.step_count,
+                    reference.update_rule_(self.rule, *flat, step=self.step_count,
                                            grad_scale=grad_scale, **self.hyper)
-                    offset += (p.numel + 7) // 8 * 8
-                    continue
-                F.adamw_(pt.view(-1), gt.view(-1), self.M[si][p.name].view(-1),
-                         self.V[si][p.name].view(-1), step=self.step_count,
-                         grad_scale=grad_scale, seed=self.seed, offset=offset,
-                         stochastic_param=self.sr, stochastic_state=self.sr, **self.hyper)
+                else:
+                    fused.append((*flat, offset))
                 offset += (p.numel + 7) // 8 * 8
+        if fused:
+            F.adamw_many_(fused, step=self.step_count, grad_scale=grad_scale, seed=self.seed,
+                          stochastic_param=self.sr, stochastic_state=self.sr, **self.hyper)
         self._accum = 0
 
     def step(self, microbatches: list[BatchMeta]) -> float:

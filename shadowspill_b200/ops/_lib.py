@@ -40,6 +40,7 @@ _SIGNATURES = {
                            c_f, c_p, c_f, c_p],
     "ss_adamw_sr": [c_p, c_p, c_p, c_p, c_ll, c_int, c_f, c_f, c_f, c_f, c_f, c_int, c_f, c_ull,
                     c_ull, c_int, c_int, c_p],
+    "ss_adamw_sr_many": [c_p, c_int, c_f, c_f, c_f, c_f, c_f, c_int, c_f, c_ull, c_int, c_int, c_p],
     "ss_adamw_f32": [c_p, c_p, c_p, c_p, c_ll, c_f, c_f, c_f, c_f, c_f, c_int, c_f, c_p],
     "ss_sumsq": [c_p, c_ll, c_p, c_p, c_int, c_p],
     "ss_cast_f32_bf16": [c_p, c_p, c_ll, c_f, c_p],
