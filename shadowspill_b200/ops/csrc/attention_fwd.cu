@@ -292,7 +292,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (lane == 0) mbar_arrive(&p_full[tile]);
     }
     // ---------------------------------------------------------------- epilogue
-    if (ok && n > 0 && mbar_wait(&o_done[tile], (n - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
+    // The last scores only say that the product before the last two is done, and a wait by parity cannot
+    // tell the last product from the one three back: the last but one is waited for first.
+    if (ok && n > 0 && (n < 2 || mbar_wait(&o_done[tile], n & 1, p.status, KS_TIMEOUT_TMEM_FULL)) &&
+        mbar_wait(&o_done[tile], (n - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const bool valid = gq < seq_end;

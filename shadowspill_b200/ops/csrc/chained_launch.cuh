@@ -1,0 +1,31 @@
+// Launches whose blocks may start before the kernel ahead of them in the stream has ended.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace ss {
+
+// A kernel started by launch_chained may begin before the one ahead of it in the stream has ended. It sets
+// up its barriers and TMEM, waits in chain_wait() until that kernel is complete and its writes are visible,
+// and only then touches global memory; every thread of every block waits, so the end of a kernel implies the
+// end of all before it. chain_release() lets the next kernel's blocks take what this one's leave free: it
+// follows chain_wait() and, where there is TMEM, the allocation, so that no waiting block can hold columns
+// that a block of this kernel still needs.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline void launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute chained[1];
+  chained[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  chained[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = chained;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);   // the launchers return cudaGetLastError()
+}
+
+}  // namespace ss
