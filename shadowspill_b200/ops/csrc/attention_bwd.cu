@@ -60,6 +60,8 @@ template <int DH>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                   float* __restrict__ delta, int T, int Hq, long long ld_out, long long ld_dout) {
+  chain_wait();
+  chain_release();
   constexpr int LANES = DH / 8;
   const long long row = (blockIdx.x * 256ll + threadIdx.x) / LANES;
   const int lane = threadIdx.x % LANES;
@@ -175,11 +177,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(dq_done, 1);
     mbar_fence_init();
   }
-  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
   if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  chain_wait();
+  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_release();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int seq_start = slot->seq_start, seq_end = slot->seq_end;
   const int q0 = seq_start + (slot->work - 1) * 128;
@@ -433,11 +437,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(acc_done, 1);
     mbar_fence_init();
   }
-  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
   if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  chain_wait();
+  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_release();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int seq_start = slot->seq_start, seq_end = slot->seq_end;
   const int k0 = seq_start + ((seq_end - seq_start + 127) / 128 - slot->work) * 128;
@@ -735,7 +741,7 @@ static int launch_dq(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtens
   auto kern = attn_bwd_dq_kernel<DH, BKV, KS, VS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
-  kern<<<dim3(p.Hq, tiles), BW_THREADS, Cfg::SMEM, s>>>(tq, tdo, tk, tv, p);
+  launch_chained(kern, dim3(p.Hq, tiles), BW_THREADS, Cfg::SMEM, s, tq, tdo, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -751,12 +757,14 @@ static int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tdo, const CUten
   cfg.blockDim = dim3(BW_THREADS);
   cfg.dynamicSmemBytes = Cfg::SMEM;
   cfg.stream = s;
-  cudaLaunchAttribute cluster[1];
-  cluster[0].id = cudaLaunchAttributeClusterDimension;
-  cluster[0].val.clusterDim.x = p.split;
-  cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
-  cfg.attrs = cluster;
-  cfg.numAttrs = p.split > 1 ? 1 : 0;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // as launch_chained
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = p.split;
+  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = p.split > 1 ? 2 : 1;
   if (cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tq, tdo, tk, tv, p)) return static_cast<int>(e);
   return static_cast<int>(cudaGetLastError());
 }
@@ -796,7 +804,7 @@ extern "C" int ss_attn_bwd_g(const void* q, const void* k, const void* v, const 
   {
     const long long blocks = (static_cast<long long>(T) * Hq * (dh / 8) + 255) / 256;
     auto run = [&](auto kern) {
-      kern<<<static_cast<unsigned>(blocks), 256, 0, s>>>(
+      launch_chained(kern, static_cast<unsigned>(blocks), 256, 0, s,
           reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta_scratch, T,
           Hq, static_cast<long long>(Hq) * dh, ldo);
     };

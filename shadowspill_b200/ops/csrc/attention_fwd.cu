@@ -96,14 +96,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     mbar_fence_init();
   }
-  if (warp == Cfg::TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, NT * 128, blockIdx.y, slot);
   if (warp == Cfg::MMA_WARP) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  chain_wait();
+  if (warp == Cfg::TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, NT * 128, blockIdx.y, slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_release();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int seq_start = slot->seq_start, seq_end = slot->seq_end;
   const int q0 = seq_start + (slot->work - 1) * (NT * 128);
@@ -346,7 +348,7 @@ static int launch_fwd(const void* q, const void* k, const void* v, AttnParams p,
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
   // every sequence adds at most one partial tile
   const dim3 grid(p.Hq, (p.T + NT * 128 - 1) / (NT * 128) + p.nseq);
-  kern<<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(tq, tk, tv, p);
+  launch_chained(kern, grid, Cfg::THREADS, Cfg::SMEM, stream, tq, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -10,6 +10,12 @@ namespace ss {
 // end of all before it. chain_release() lets the next kernel's blocks take what this one's leave free: it
 // follows chain_wait() and, where there is TMEM, the allocation, so that no waiting block can hold columns
 // that a block of this kernel still needs.
+//
+// What it saves is the gap between two kernels, 2 to 3 us: a layer of 1,999 tokens and 2,048 channels, forward and
+// backward, 1004 -> 955 us (41 launches), attention on 2,048 tokens with heads of 64 121 -> 112 us, a layer of 8,192
+// tokens and 4,096 channels 1.4 %. Kernels that wait for other ranks are launched plainly and do not release, so
+// nothing takes room beside them early; so are the expert banks' and the delta rule's, which were 5 % and 1 %
+// slower chained.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chained_launch.cuh"
+
 namespace ss {
 
 typedef __nv_bfloat16 bf16;
@@ -80,6 +82,8 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 __global__ void rope_kernel(bf16* __restrict__ buf, const int* __restrict__ positions, int T,
                             long long row_stride, int col0, int heads, int dh, int rot,
                             float log2_theta, int inverse) {
+  chain_wait();
+  chain_release();
   const int half = rot >> 1;
   const int pairs_per_head = half >> 1;  // two pairs per thread (bf16x2)
   const long long total = static_cast<long long>(T) * heads * pairs_per_head;
@@ -117,6 +121,8 @@ __global__ void rope_kernel(bf16* __restrict__ buf, const int* __restrict__ posi
 __global__ void rope_vec_kernel(bf16* __restrict__ buf, const int* __restrict__ positions, int T,
                                 long long row_stride, int col0, int heads, int dh, int rot,
                                 float log2_theta, int inverse, int slots) {
+  chain_wait();
+  chain_release();
   const int half = rot >> 1;
   const int vph = half >> 3;
   const int per_token = vph * slots;
@@ -188,6 +194,8 @@ __device__ __forceinline__ void split_index(long long idx, int nv, long long& t,
 // `used` (optional, device memory): rows at and past *used are left alone.
 __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ h, int T, int F,
                                   const int* __restrict__ used) {
+  chain_wait();
+  chain_release();
   const int nv = F >> 3;
   if (used) T = min(T, *used);
   const long long total = static_cast<long long>(T) * nv;
@@ -210,6 +218,8 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
 // dgu[T,2F] from dh[T,F] and the saved gu.
 __global__ void swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dh,
                                   bf16* __restrict__ dgu, int T, int F) {
+  chain_wait();
+  chain_release();
   const int nv = F >> 3;
   const long long total = static_cast<long long>(T) * nv;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -665,20 +675,20 @@ int ss_rope(void* buf, const int* positions, int T, long long row_stride, int co
     const int hpt = heads >= 8 ? 4 : 1;              // heads walked by one thread
     const int slots = (heads + hpt - 1) / hpt;
     const long long threads = (long long)T * (rot >> 4) * slots;
-    rope_vec_kernel<<<grid_for(threads, 256), 256, 0, (cudaStream_t)stream>>>(
-        (bf16*)buf, positions, T, row_stride, col0, heads, dh, rot, log2f(theta), inverse, slots);
+    launch_chained(rope_vec_kernel, grid_for(threads, 256), 256, 0, (cudaStream_t)stream,
+                   (bf16*)buf, positions, T, row_stride, col0, heads, dh, rot, log2f(theta), inverse, slots);
     return (int)cudaGetLastError();
   }
   const long long total = (long long)T * heads * (rot >> 2);
-  rope_kernel<<<grid_for(total, 256), 256, 0, (cudaStream_t)stream>>>(
-      (bf16*)buf, positions, T, row_stride, col0, heads, dh, rot, log2f(theta), inverse);
+  launch_chained(rope_kernel, grid_for(total, 256), 256, 0, (cudaStream_t)stream,
+                 (bf16*)buf, positions, T, row_stride, col0, heads, dh, rot, log2f(theta), inverse);
   return (int)cudaGetLastError();
 }
 int ss_swiglu_fwd(const void* gu, void* h, int T, int F, void* stream) {
   if (F % 8) return -2;
   if (T <= 0) return 0;
-  swiglu_fwd_kernel<<<grid_for((long long)T * (F >> 3), 256, 148 * 16), 256, 0,
-                      (cudaStream_t)stream>>>((const bf16*)gu, (bf16*)h, T, F, nullptr);
+  launch_chained(swiglu_fwd_kernel, grid_for((long long)T * (F >> 3), 256, 148 * 16), 256, 0, (cudaStream_t)stream,
+                 (const bf16*)gu, (bf16*)h, T, F, nullptr);
   return (int)cudaGetLastError();
 }
 // The first *used rows only (`used` in device memory): sorted expert rows, whose count the host does not know.
@@ -692,8 +702,8 @@ int ss_swiglu_fwd_used(const void* gu, void* h, int T, int F, const int* used, v
 int ss_swiglu_bwd(const void* gu, const void* dh, void* dgu, int T, int F, void* stream) {
   if (F % 8) return -2;
   if (T <= 0) return 0;
-  swiglu_bwd_kernel<<<grid_for((long long)T * (F >> 3), 256, 148 * 16), 256, 0,
-                      (cudaStream_t)stream>>>((const bf16*)gu, (const bf16*)dh, (bf16*)dgu, T, F);
+  launch_chained(swiglu_bwd_kernel, grid_for((long long)T * (F >> 3), 256, 148 * 16), 256, 0, (cudaStream_t)stream,
+                 (const bf16*)gu, (const bf16*)dh, (bf16*)dgu, T, F);
   return (int)cudaGetLastError();
 }
 int ss_embedding_fwd(const long long* ids, const void* W, void* out, int T, int D, int V,

@@ -218,6 +218,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   cluster_sync_all();          // both CTAs' barriers exist before anything is signalled remotely
   tc_fence_after();
+  chain_wait();
+  if (!GATHER) chain_release();   // a kernel that waits for peers keeps the next one off the GPU
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -386,7 +388,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
   const long long tiles = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   long long pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  kern<<<static_cast<int>(2 * pairs), THREADS, SMEM, stream>>>(ta, tb, p, GatherArgs{});
+  launch_chained(kern, static_cast<int>(2 * pairs), THREADS, SMEM, stream, ta, tb, p, GatherArgs{});
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -87,6 +87,8 @@ struct NormRows {
 template <int LANES, int VPT, bool DELTA>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_short_kernel(const NormRows p) {
+  chain_wait();
+  chain_release();
   const int lane = threadIdx.x & (LANES - 1), nv = p.D >> 3;
   const float wofs = p.zero_centered ? 1.f : 0.f;
   uint4 wq[VPT];
@@ -163,6 +165,8 @@ rmsnorm_fwd_short_kernel(const NormRows p) {
 template <int LANES, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_short_kernel(const NormRows p) {
+  chain_wait();
+  chain_release();
   constexpr int GROUPS = NORM_THREADS / LANES;
   __shared__ __align__(16) float s_dw[GROUPS * LANES * VPT * 8];
   const int lane = threadIdx.x & (LANES - 1), nv = p.D >> 3;
@@ -285,6 +289,8 @@ template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, bf16* y, float* __restrict__ rstd,
                         long long T, int D, float eps, int zero_centered) {
+  chain_wait();
+  chain_release();
   extern __shared__ __align__(128) uint8_t ring_smem[];
   __shared__ __align__(16) float red[2][8];
   constexpr int NORM_RING = norm_ring(VPT);
@@ -358,6 +364,8 @@ template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_long_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* gy, const float* __restrict__ rstd,
                         bf16* dx, float* __restrict__ dw, long long T, int D, int zero_centered, int accumulate) {
+  chain_wait();
+  chain_release();
   extern __shared__ __align__(128) uint8_t ring_smem[];
   __shared__ __align__(16) float red[2][8];
   constexpr int NORM_RING = norm_ring(VPT);
@@ -463,8 +471,8 @@ static int launch_short_as(const NormRows& p, cudaStream_t s) {
   const long long per = NORM_THREADS / LANES, blocks = (p.rows + per - 1) / per;
   const long long cap = 148 * (KIND == BWD ? 4 : 8);
   const int grid = static_cast<int>(blocks < cap ? blocks : cap);
-  if constexpr (KIND == BWD) rmsnorm_bwd_short_kernel<LANES, VPT><<<grid, NORM_THREADS, 0, s>>>(p);
-  else rmsnorm_fwd_short_kernel<LANES, VPT, KIND == FWD_DELTA><<<grid, NORM_THREADS, 0, s>>>(p);
+  if constexpr (KIND == BWD) launch_chained(rmsnorm_bwd_short_kernel<LANES, VPT>, grid, NORM_THREADS, 0, s, p);
+  else launch_chained(rmsnorm_fwd_short_kernel<LANES, VPT, KIND == FWD_DELTA>, grid, NORM_THREADS, 0, s, p);
   return static_cast<int>(cudaGetLastError());
 }
 template <int KIND>
@@ -495,7 +503,7 @@ int ss_rmsnorm_fwd(void* x, const void* delta, const void* w, void* y, float* rs
   auto go = [&](auto kern, SmemOptIn& opt_in, int vpt) -> int {
     const LongShape shape(T, D, delta ? 2 : 1, norm_ring(vpt), 4, 1);
     if (int e = opt_in.ensure(kern, NORM_MAX_SMEM)) return e;
-    kern<<<shape.grid, NORM_THREADS, shape.smem, s>>>((bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)y, rstd, T, D, eps,
+    launch_chained(kern, shape.grid, NORM_THREADS, shape.smem, s, (bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)y, rstd, T, D, eps,
                                           zero_centered);
     return static_cast<int>(cudaGetLastError());
   };
@@ -522,7 +530,7 @@ int ss_rmsnorm_bwd(const void* x, const void* w, const void* gy, const float* rs
   auto go = [&](auto kern, SmemOptIn& opt_in, int vpt) -> int {
     const LongShape shape(T, D, accumulate ? 3 : 2, norm_ring(vpt), 4, 8);   // eight rows to a weight-gradient flush
     if (int e = opt_in.ensure(kern, NORM_MAX_SMEM)) return e;
-    kern<<<shape.grid, NORM_THREADS, shape.smem, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)gy, rstd, (bf16*)dx, dw, T, D,
+    launch_chained(kern, shape.grid, NORM_THREADS, shape.smem, s, (const bf16*)x, (const bf16*)w, (const bf16*)gy, rstd, (bf16*)dx, dw, T, D,
                                           zero_centered, accumulate);
     return static_cast<int>(cudaGetLastError());
   };

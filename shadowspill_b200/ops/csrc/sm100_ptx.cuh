@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chained_launch.cuh"
+
 namespace ss {
 
 // ------------------------------------------------------------------ status codes
@@ -399,6 +401,5 @@ __device__ __forceinline__ float fast_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-
 
 }  // namespace ss
