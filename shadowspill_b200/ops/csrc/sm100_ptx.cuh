@@ -290,19 +290,7 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// A from TMEM (used for P·V in attention): D[tmem] (+)= A[tmem] * B[smem].
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc,
-                                             uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same three for a whole warp in step, of which only the lane with `leader` set issues. With no branch
+// The same for a whole warp in step (`_ts`: A from TMEM), of which only the lane with `leader` set issues. With no branch
 // around them the addresses and descriptors are computed once per warp in uniform registers, where the
 // instruction takes them from; inside a one-lane branch each has to be moved there first, about 46 cycles
 // per product.
