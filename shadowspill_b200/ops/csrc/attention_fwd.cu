@@ -18,6 +18,13 @@
 //   warps 0..4*NT-1  softmax, rescaling of O, epilogue: one query row per thread
 //   then one TMA producer warp and one MMA warp
 //
+// The scores of step j + 1 are issued before P of step j is waited for, so two steps are in flight and the
+// warps of a tile may be a step apart. Whatever is arrived on or waited for once per step therefore has a
+// barrier for even and one for odd steps: with one for both, a warp a step ahead completes the phase that a
+// slower one has yet to arrive on, or a phase that is waited for passes twice and its parity turns back.
+// Scores of step j + 2 are only issued once P of step j has been taken, so no barrier is arrived on twice
+// before it has been waited for.
+//
 // Semantics: the reference's packed attention contract
 // (packages/workloads/src/shadowspill_workloads/models/shared/decoder.py:251):
 // each [cu_seqlens[i], cu_seqlens[i+1]) is an independent causal sequence.
@@ -73,11 +80,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* v_full = k_empty + KS;        // VS
   uint64_t* v_empty = v_full + VS;        // VS
   uint64_t* s_full = v_empty + VS;        // [tile][buffer]
-  uint64_t* p_full = s_full + 2 * NT;     // by tile
-  uint64_t* o_done = p_full + NT;         // by tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + NT);
-  TileSlot* slot = reinterpret_cast<TileSlot*>(o_done + NT + 1);
-  static_assert((1 + 2 * KS + 2 * VS + 4 * NT + 3) * 8 <= 256, "barrier space");
+  uint64_t* p_full = s_full + 2 * NT;     // [tile][step & 1]
+  uint64_t* o_done = p_full + 2 * NT;     // [tile][step & 1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2 * NT);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(o_done + 2 * NT + 1);
+  static_assert((1 + 2 * KS + 2 * VS + 6 * NT + 1) * 8 + sizeof(TileSlot) <= 256, "barrier space");
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -88,9 +95,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(q_full, 1);
     for (int i = 0; i < KS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < VS; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-    for (int i = 0; i < NT; ++i) {
-      mbar_init(&s_full[2 * i], 1);
-      mbar_init(&s_full[2 * i + 1], 1);
+    for (int i = 0; i < 2 * NT; ++i) {
+      mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 4);
       mbar_init(&o_done[i], 1);
     }
@@ -189,7 +195,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (j + 1 < n_kv[i]) issue_s(i, j + 1);
           if (more && i == NT - 1) umma_commit_if(leader, &k_empty[(j + 1) % KS]);
           if (j >= n_kv[i]) continue;
-          ok = mbar_wait(&p_full[i], j & 1, p.status, KS_TIMEOUT_FULL);
+          ok = mbar_wait(&p_full[2 * i + (j & 1)], (j >> 1) & 1, p.status, KS_TIMEOUT_FULL);
           if (!ok) break;
           tc_fence_after();
           const uint32_t pa = tmem_base + (2 * i + (j & 1)) * BKV;
@@ -197,7 +203,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           for (int kk = 0; kk < BKV / 16; ++kk)
             umma_bf16_ts_if(leader, tmem_base + Cfg::TM_O + i * DH, pa + kk * 8,
                          umma_smem_desc(v + kk * (16 * 128), BKV * 128, 1024), idesc_o, (j | kk) != 0);
-          umma_commit_if(leader, &o_done[i]);
+          umma_commit_if(leader, &o_done[2 * i + (j & 1)]);
         }
         if (!ok) break;
         umma_commit_if(leader, &v_empty[j % VS]);
@@ -255,7 +261,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const float alpha = m_used == -INFINITY ? 0.f : fast_exp2(m_used - m_new);
         m_used = m_new;
         l *= alpha;
-        if (!mbar_wait(&o_done[tile], (j - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+        if (!mbar_wait(&o_done[b ^ 1], ((j - 1) >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int x = 0; x < DH; x += 32) {
@@ -291,13 +297,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[tile]);
+      if (lane == 0) mbar_arrive(&p_full[b]);
     }
     // ---------------------------------------------------------------- epilogue
-    // The last scores only say that the product before the last two is done, and a wait by parity cannot
-    // tell the last product from the one three back: the last but one is waited for first.
-    if (ok && n > 0 && (n < 2 || mbar_wait(&o_done[tile], n & 1, p.status, KS_TIMEOUT_TMEM_FULL)) &&
-        mbar_wait(&o_done[tile], (n - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
+    if (ok && n > 0 && mbar_wait(&o_done[2 * tile + ((n - 1) & 1)], ((n - 1) >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const bool valid = gq < seq_end;

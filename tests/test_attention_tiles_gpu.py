@@ -101,3 +101,45 @@ def test_results_do_not_depend_on_other_work_on_the_gpu(width):
     for got in outs:
         for a, b in zip(got, (*alone, *grads)):
             assert torch.equal(a, b)
+
+
+def _growing_in_one_quarter(dh, quarter):
+    """Scores that grow by 2^11.5 with every 64 keys, in one 32-row quarter of each 128-row tile: its warp
+    moves its reference maximum at every step and waits for the product before, the others never do."""
+    lens = [700, 64, 513, 1000, 257]
+    q, k, v, dout, cu = _inputs(lens, 8, 2, dh, seed=dh + quarter)
+    q, k = q.contiguous(), k.contiguous()
+    at = torch.cat([torch.arange(n) for n in lens]).to(DEV)           # position in its sequence
+    q[:, :, 0] = torch.where(at % 128 // 32 == quarter, 16.0, 0.0)[:, None].to(q.dtype)
+    k[:, :, 0] = (at // 64 * 4)[:, None].to(k.dtype)
+    return q, k, v, dout, cu, max(lens), 0.125
+
+
+def _beside_other_work(run, repeats=30):
+    """Results of ``run()`` while another stream's blocks share the SMs with its warps."""
+    torch.cuda.synchronize()
+    side, noise = torch.cuda.Stream(), torch.randn(148 * 4 * 1024, device=DEV)
+    side.wait_stream(torch.cuda.current_stream())
+    outs = []
+    for _ in range(repeats):
+        with torch.cuda.stream(side):
+            for _ in range(6):
+                noise.sin_()
+        outs.append(run())
+    torch.cuda.synchronize()
+    _lib.check_status()
+    return outs
+
+
+@pytest.mark.parametrize("quarter", [0, 2])
+@pytest.mark.parametrize("dh", [64, 128, 256])
+def test_forward_with_one_warp_behind(dh, quarter):
+    # a warp that has finished a step must not count for one of the same tile that has not
+    q, k, v, _, cu, longest, scale = _growing_in_one_quarter(dh, quarter)
+    out, lse = attention.forward(q, k, v, cu, longest, scale)
+    _lib.check_status()
+    out_r, lse_r = R.attention_varlen(q, k, v, cu, scale)
+    assert _rel(out, out_r) < 1e-2                                    # bf16 probabilities and results
+    assert float((lse - lse_r).abs().max()) < 1e-3
+    for got in _beside_other_work(lambda: attention.forward(q, k, v, cu, longest, scale)):
+        assert torch.equal(got[0], out) and torch.equal(got[1], lse)
