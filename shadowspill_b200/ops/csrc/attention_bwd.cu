@@ -126,6 +126,9 @@ __device__ __forceinline__ void tmem_st_quarter(uint32_t addr, const uint32_t (&
 // S is double-buffered and dP single: S of the next tile is formed under this tile's
 // exponentials, dP of the next tile under this tile's dS. K is released by the dQ product and has
 // KS stages, V already by the dP product and has VS.
+// Both are issued before dS of this tile is waited for, so two warps may be a tile apart: dS has a barrier
+// for even and one for odd tiles, or a warp a tile ahead would count for one that has yet to write. dP of the
+// next tile waits until all warps have read this one's, so one barrier is enough there.
 template <int DH, int BKV, int KS, int VS>
 struct DqCfg {
   static constexpr int Q_BYTES = 128 * DH * 2;
@@ -157,8 +160,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* s_full = bars + 11;         // 2
   uint64_t* dp_full = bars + 13;        // 1
   uint64_t* dp_free = bars + 14;        // 1
-  uint64_t* ds_full = bars + 15;        // 1
-  uint64_t* dq_done = bars + 16;        // 1
+  uint64_t* ds_full = bars + 15;        // 2
+  uint64_t* dq_done = bars + 17;        // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 19);
 
@@ -170,10 +173,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(qdo_full, 1);
     for (int i = 0; i < KS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < VS; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) mbar_init(&s_full[i], 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&ds_full[i], 8); }
     mbar_init(dp_full, 1);
     mbar_init(dp_free, 8);
-    mbar_init(ds_full, 8);
     mbar_init(dq_done, 1);
     mbar_fence_init();
   }
@@ -249,7 +251,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         // S of the next tile goes to the buffer whose dS the dQ product before this point reads:
         // products of one issuing thread run in order
         if (j + 1 < n_kv) ok = issue_s(j + 1) && issue_dp(j + 1);
-        if (!ok || !mbar_wait(ds_full, j & 1, p.status, KS_TIMEOUT_FULL)) break;
+        if (!ok || !mbar_wait(&ds_full[j & 1], (j >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
         tc_fence_after();
         const uint32_t sk = sk0 + (j % KS) * Cfg::KV_BYTES;
         const uint32_t ds = tmem_base + Cfg::TM_S + (j & 1) * BKV;
@@ -308,7 +310,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tmem_st_half<HN>(s_addr, pk);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ds_full);
+      if (lane == 0) mbar_arrive(&ds_full[b]);
     }
     if (ok && n_kv > 0 && mbar_wait(dq_done, 0, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();

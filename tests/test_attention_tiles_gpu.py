@@ -143,3 +143,22 @@ def test_forward_with_one_warp_behind(dh, quarter):
     assert float((lse - lse_r).abs().max()) < 1e-3
     for got in _beside_other_work(lambda: attention.forward(q, k, v, cu, longest, scale)):
         assert torch.equal(got[0], out) and torch.equal(got[1], lse)
+
+
+def _gradients_beside_other_work(dh):
+    q, k, v, dout, cu, longest, scale = _growing_in_one_quarter(dh, 1)
+    out, lse = attention.forward(q, k, v, cu, longest, scale)
+    run = lambda: attention.backward(q, k, v, out, lse, dout, cu, longest, scale)  # noqa: E731
+    grads = run()
+    _lib.check_status()
+    out_r, lse_r = R.attention_varlen(q, k, v, cu, scale)
+    for a, b in zip(grads, R.attention_varlen_bwd(q, k, v, out_r, lse_r, dout, cu, scale)):
+        assert _rel(a, b) < 2e-2
+    for got in _beside_other_work(run):
+        assert all(torch.equal(a, b) for a, b in zip(got, grads))
+
+
+@pytest.mark.parametrize("dh", [64, 128])
+def test_backward_with_warps_a_tile_apart(dh):
+    # scores and dP of the next key tile are ready before the slowest warp has written dS of this one
+    _gradients_beside_other_work(dh)
