@@ -347,7 +347,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 //   softmax warps   P^T of tile i                 dS^T of tile i
 //   tensor pipe     dK of tile i-1, dP^T of i     dV of tile i, S^T of tile i+1
 // dK alone follows the same order without P^T; dV alone has no second phase to hide S^T under and
-// keeps two buffers of it instead.
+// keeps two buffers of it instead: S^T of tile i+1 is then issued before P^T of tile i is waited for, so
+// P^T has barriers for even and for odd tiles, as S^T has. With one buffer, every warp has arrived for a tile
+// before any can start on the next, and one barrier is enough; the same holds for dP^T and dS^T.
 enum { MODE_BOTH = 0, MODE_DV = 1, MODE_DK = 2 };
 
 // Short batches: a key tile's queries are those of every head of its group, one CTA after another, and a
@@ -411,13 +413,14 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* stat_full = bars + 9;       // 4
   uint64_t* stat_empty = bars + 13;     // 4
   uint64_t* s_full = bars + 17;         // 2
-  uint64_t* p_full = bars + 19;         // 2: first and second half of every warp's columns
-  uint64_t* dp_full = bars + 21;        // 1
-  uint64_t* ds_full = bars + 22;        // 1
-  uint64_t* s_free = bars + 23;         // 1 (only without a P^T to wait for)
-  uint64_t* acc_done = bars + 24;       // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
-  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 26);
+  uint64_t* p_full = bars + 19;         // [buffer of S^T][first and second half of every warp's columns]
+  uint64_t* dp_full = bars + 23;        // 1
+  uint64_t* ds_full = bars + 24;        // 1
+  uint64_t* s_free = bars + 25;         // 1 (only without a P^T to wait for)
+  uint64_t* acc_done = bars + 26;       // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 28);
+  static_assert(28 * 8 + sizeof(TileSlot) <= 256, "barrier space");
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), -delta
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
@@ -431,8 +434,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int i = 0; i < DOS; ++i) { mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); }
     for (int i = 0; i < STS; ++i) { mbar_init(&stat_full[i], 1); mbar_init(&stat_empty[i], 8); }
     for (int i = 0; i < SB; ++i) mbar_init(&s_full[i], 1);
-    mbar_init(&p_full[0], 8);
-    mbar_init(&p_full[1], 8);
+    for (int i = 0; i < 2 * SB; ++i) mbar_init(&p_full[i], 8);
     mbar_init(dp_full, 1);
     mbar_init(ds_full, 8);
     mbar_init(s_free, 8);
@@ -525,7 +527,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           // starts under the exponentials of the second
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
-            ok = mbar_wait(&p_full[x], it & 1, p.status, KS_TIMEOUT_FULL);
+            ok = mbar_wait(&p_full[it % SB * 2 + x], (it / SB) & 1, p.status, KS_TIMEOUT_FULL);
             if (!ok) break;
             tc_fence_after();
             accumulate(tmem_base + Cfg::TM_DV, tmem_base + Cfg::TM_ST + (it % SB) * BQ, sdo, it == 0, x);
@@ -633,7 +635,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tmem_st_quarter<PN>(s_addr + x * (PN / 2), pk);
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&p_full[x]);
+          if (lane == 0) mbar_arrive(&p_full[it % SB * 2 + x]);
         }
       }
       if (Cfg::DO_DK) {

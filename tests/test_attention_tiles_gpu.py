@@ -162,3 +162,8 @@ def _gradients_beside_other_work(dh):
 def test_backward_with_warps_a_tile_apart(dh):
     # scores and dP of the next key tile are ready before the slowest warp has written dS of this one
     _gradients_beside_other_work(dh)
+
+
+def test_wide_backward_with_warps_a_tile_apart():
+    # dV alone: scores of the next query tile are ready before the slowest warp has written P^T of this one
+    _gradients_beside_other_work(256)
