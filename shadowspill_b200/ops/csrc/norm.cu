@@ -260,13 +260,15 @@ rmsnorm_bwd_short_kernel(const NormRows p) {
 
 // ============================================================================ longer rows
 // Sum over the block of one value per thread; `red` has two sets of eight, used in turn, so one barrier
-// per row is enough. After it every thread has also read its part of the row from the ring.
-__device__ __forceinline__ float row_sum(float v, float (*red)[8], int turn) {
+// per row is enough. After it every thread has also read its part of the row from the ring. False for the
+// whole block where a thread's wait for the row ran out (`ok`).
+__device__ __forceinline__ bool row_sum(bool ok, float v, float (*red)[8], int turn, float& sum) {
   v = lanes_sum<32>(v);
   if ((threadIdx.x & 31) == 0) red[turn][threadIdx.x >> 5] = v;
-  __syncthreads();
+  ok = __syncthreads_and(ok);
   const float4 a = *reinterpret_cast<const float4*>(red[turn]), b = *reinterpret_cast<const float4*>(red[turn] + 4);
-  return ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+  sum = ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+  return ok;
 }
 
 // The ring of one block: `parts` tensors of D channels each per row.
@@ -275,6 +277,7 @@ struct NormRing {
   uint64_t* full;
   int D, parts;
   long long T;
+  int* status;
   __device__ __forceinline__ uint32_t part(int s, int k) const { return base + (s * parts + k) * (D * 2); }
   __device__ __forceinline__ void load(int s, long long row, const bf16* a, const bf16* b, const bf16* c) const {
     if (row >= T) return;
@@ -283,12 +286,25 @@ struct NormRing {
     if (parts > 1) bulk_load(part(s, 1), b + row * D, D * 2, &full[s]);
     if (parts > 2) bulk_load(part(s, 2), c + row * D, D * 2, &full[s]);
   }
+  // Row `it` of the block has arrived.
+  template <int STAGES>
+  __device__ __forceinline__ bool wait(int it) const {
+    return mbar_wait(&full[it % STAGES], (it / STAGES) & 1, status, KS_TIMEOUT_FULL);
+  }
+  // The copies in flight when row `it` (global row `row`) failed get one more bounded wait, so that none lands
+  // in memory that another block has been given.
+  template <int STAGES>
+  __device__ __forceinline__ void drain(int it, long long row) const {
+#pragma unroll 1
+    for (int i = 0; i < STAGES && row < T; ++i, ++it, row += gridDim.x) wait<STAGES>(it);
+    __syncthreads();
+  }
 };
 
 template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, bf16* y, float* __restrict__ rstd,
-                        long long T, int D, float eps, int zero_centered) {
+                        long long T, int D, float eps, int zero_centered, int* status) {
   chain_wait();
   chain_release();
   extern __shared__ __align__(128) uint8_t ring_smem[];
@@ -297,7 +313,7 @@ rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, 
   __shared__ __align__(8) uint64_t full[NORM_RING];
   const int nv = D >> 3;
   const float wofs = zero_centered ? 1.f : 0.f;
-  const NormRing ring{smem_u32(ring_smem), full, D, delta ? 2 : 1, T};
+  const NormRing ring{smem_u32(ring_smem), full, D, delta ? 2 : 1, T, status};
   if (threadIdx.x == 0) {
     for (int s = 0; s < NORM_RING; ++s) mbar_init(&full[s], 1);
     mbar_fence_init();
@@ -315,7 +331,7 @@ rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, 
   int it = 0;
   for (long long row = blockIdx.x; row < T; row += gridDim.x, ++it) {
     const int s = it % NORM_RING;
-    mbar_wait(&full[s], (it / NORM_RING) & 1, nullptr, KS_TIMEOUT_FULL);
+    const bool ok = ring.wait<NORM_RING>(it);
     uint4 xq[VPT];
     float ss = 0.f;
 #pragma unroll
@@ -339,7 +355,9 @@ rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, 
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
     }
-    const float rs = rsqrtf(row_sum(ss, red, it & 1) / static_cast<float>(D) + eps);
+    float sum;
+    if (!row_sum(ok, ss, red, it & 1, sum)) return ring.drain<NORM_RING>(it, row);   // reported; this row is not stored
+    const float rs = rsqrtf(sum / static_cast<float>(D) + eps);
     if (threadIdx.x == 0) {
       ring.load(s, row + static_cast<long long>(NORM_RING) * gridDim.x, x, delta, nullptr);
       if (rstd) rstd[row] = rs;
@@ -363,7 +381,8 @@ rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, 
 template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_long_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* gy, const float* __restrict__ rstd,
-                        bf16* dx, float* __restrict__ dw, long long T, int D, int zero_centered, int accumulate) {
+                        bf16* dx, float* __restrict__ dw, long long T, int D, int zero_centered, int accumulate,
+                        int* status) {
   chain_wait();
   chain_release();
   extern __shared__ __align__(128) uint8_t ring_smem[];
@@ -372,7 +391,7 @@ rmsnorm_bwd_long_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* g
   __shared__ __align__(8) uint64_t full[NORM_RING];
   const int nv = D >> 3;
   const float wofs = zero_centered ? 1.f : 0.f;
-  const NormRing ring{smem_u32(ring_smem), full, D, accumulate ? 3 : 2, T};
+  const NormRing ring{smem_u32(ring_smem), full, D, accumulate ? 3 : 2, T, status};
   if (threadIdx.x == 0) {
     for (int s = 0; s < NORM_RING; ++s) mbar_init(&full[s], 1);
     mbar_fence_init();
@@ -396,7 +415,7 @@ rmsnorm_bwd_long_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* g
     const int s = it % NORM_RING;
     const float rs = rn;
     if (row + gridDim.x < T) rn = rstd[row + gridDim.x];
-    mbar_wait(&full[s], (it / NORM_RING) & 1, nullptr, KS_TIMEOUT_FULL);
+    const bool ok = ring.wait<NORM_RING>(it);
     uint4 xq[VPT], gq[VPT], pq[VPT];
     float dot = 0.f;
 #pragma unroll
@@ -417,7 +436,9 @@ rmsnorm_bwd_long_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* g
         dot += gv[e] * (ww[e] + wofs) * xh;
       }
     }
-    const float mean = row_sum(dot, red, it & 1) / static_cast<float>(D);
+    float sum;
+    if (!row_sum(ok, dot, red, it & 1, sum)) return ring.drain<NORM_RING>(it, row);  // reported; neither row nor dw is stored
+    const float mean = sum / static_cast<float>(D);
     if (threadIdx.x == 0) ring.load(s, row + static_cast<long long>(NORM_RING) * gridDim.x, x, gy, dx);
     uint4* dr = reinterpret_cast<uint4*>(dx + row * D);
 #pragma unroll
@@ -489,7 +510,7 @@ extern "C" {
 using namespace ss;
 
 int ss_rmsnorm_fwd(void* x, const void* delta, const void* w, void* y, float* rstd, int T, int D,
-                   float eps, int zero_centered, void* stream) {
+                   float eps, int zero_centered, int* status, void* stream) {
   if (D % 8 || D <= 0 || D > 8192) return -2;
   if (!aligned16(x) || !aligned16(delta) || !aligned16(w) || !aligned16(y)) return -2;
   if (T <= 0) return 0;
@@ -503,8 +524,8 @@ int ss_rmsnorm_fwd(void* x, const void* delta, const void* w, void* y, float* rs
   auto go = [&](auto kern, SmemOptIn& opt_in, int vpt) -> int {
     const LongShape shape(T, D, delta ? 2 : 1, norm_ring(vpt), 4, 1);
     if (int e = opt_in.ensure(kern, NORM_MAX_SMEM)) return e;
-    launch_chained(kern, shape.grid, NORM_THREADS, shape.smem, s, (bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)y, rstd, T, D, eps,
-                                          zero_centered);
+    launch_chained(kern, shape.grid, NORM_THREADS, shape.smem, s, (bf16*)x, (const bf16*)delta, (const bf16*)w, (bf16*)y,
+                   rstd, T, D, eps, zero_centered, status);
     return static_cast<int>(cudaGetLastError());
   };
   static SmemOptIn o1, o2, o4;
@@ -514,7 +535,7 @@ int ss_rmsnorm_fwd(void* x, const void* delta, const void* w, void* y, float* rs
 }
 
 int ss_rmsnorm_bwd(const void* x, const void* w, const void* gy, const float* rstd, void* dx,
-                   float* dw, int T, int D, int zero_centered, int accumulate, void* stream) {
+                   float* dw, int T, int D, int zero_centered, int accumulate, int* status, void* stream) {
   if (D % 8 || D <= 0 || D > 12288) return -2;
   if (!aligned16(x) || !aligned16(w) || !aligned16(gy) || !aligned16(dx) || !aligned16(dw)) return -2;
   if (T <= 0) return 0;
@@ -530,8 +551,8 @@ int ss_rmsnorm_bwd(const void* x, const void* w, const void* gy, const float* rs
   auto go = [&](auto kern, SmemOptIn& opt_in, int vpt) -> int {
     const LongShape shape(T, D, accumulate ? 3 : 2, norm_ring(vpt), 4, 8);   // eight rows to a weight-gradient flush
     if (int e = opt_in.ensure(kern, NORM_MAX_SMEM)) return e;
-    launch_chained(kern, shape.grid, NORM_THREADS, shape.smem, s, (const bf16*)x, (const bf16*)w, (const bf16*)gy, rstd, (bf16*)dx, dw, T, D,
-                                          zero_centered, accumulate);
+    launch_chained(kern, shape.grid, NORM_THREADS, shape.smem, s, (const bf16*)x, (const bf16*)w, (const bf16*)gy, rstd,
+                   (bf16*)dx, dw, T, D, zero_centered, accumulate, status);
     return static_cast<int>(cudaGetLastError());
   };
   static SmemOptIn o1, o2, o4, o6;

@@ -197,7 +197,7 @@ def rmsnorm_fwd(x, w, eps=1e-5, zero_centered=False, delta=None, out=None, rstd=
     rs = torch.empty(T, dtype=torch.float32, device=x.device) if rstd is None else rstd
     rc = _lib.lib().ss_rmsnorm_fwd(x.data_ptr(), _ptr(delta), w.data_ptr(), y.data_ptr(),
                                    rs.data_ptr(), T, D, float(eps), int(zero_centered),
-                                   _lib.stream_ptr())
+                                   _lib.status_ptr(x), _lib.stream_ptr())
     _lib.check(rc, "ss_rmsnorm_fwd")
     return y, rs
 
@@ -222,7 +222,7 @@ def rmsnorm_bwd(x, w, gy, rstd, dw, zero_centered=False, dx=None, accumulate=Fal
         raise TypeError("rmsnorm dw accumulator must be fp32")
     rc = _lib.lib().ss_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), gy.data_ptr(), rstd.data_ptr(),
                                    dx.data_ptr(), _ptr(dw), T, D, int(zero_centered),
-                                   int(accumulate), _lib.stream_ptr())
+                                   int(accumulate), _lib.status_ptr(x), _lib.stream_ptr())
     _lib.check(rc, "ss_rmsnorm_bwd")
     return dx
 

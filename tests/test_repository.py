@@ -88,3 +88,33 @@ def test_build_verification_reports_every_native_artifact():
     report = build.verify()
     assert report["ok"] and report["kernels"]["missing"] == [] and report["core"]["abi"] >= 1
     assert all(report["files"].values())
+
+
+def _csrc():
+    return sorted([*(PKG / "ops" / "csrc").glob("*.cu"), *(PKG / "ops" / "csrc").glob("*.cuh")])
+
+
+def _call_args(text: str, name: str):
+    """The argument texts of every call of ``name`` in a source."""
+    for m in re.finditer(rf"\b{name}\(", text):
+        depth, args, at = 1, [""], m.end()
+        while depth:
+            c = text[at]
+            depth += (c in "([{") - (c in ")]}")
+            if c == "," and depth == 1:
+                args.append("")
+            elif depth:
+                args[-1] += c
+            at += 1
+        yield [a.strip() for a in args]
+
+
+def test_every_device_wait_reports_its_failure():
+    """A wait that runs out writes the status word: without one, what it waited for is read all the same
+    and nobody learns of it."""
+    calls = 0
+    for f in _csrc():
+        for args in _call_args(f.read_text(), "mbar_wait"):
+            assert args[2] not in ("nullptr", "NULL", "0"), f"{f.name}: mbar_wait({', '.join(args)})"
+            calls += 1
+    assert calls > 50
