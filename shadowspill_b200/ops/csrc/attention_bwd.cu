@@ -58,8 +58,8 @@ struct AttnBwdParams {
 // 8,192 x 32 heads of 128, 44 -> 26 us).
 template <int DH>
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
-                  float* __restrict__ delta, int T, int Hq, long long ld_out, long long ld_dout) {
+attn_delta_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout, float* delta, int T, int Hq,
+                  long long ld_out, long long ld_dout) {
   chain_wait();
   chain_release();
   constexpr int LANES = DH / 8;
@@ -566,8 +566,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       for (int u = 0; u < NU; ++u) {
         const int gq = qt0 + lane + u * 32;
         const bool in = gq < seq_end;
-        nl[u] = in ? -__ldg(p.lse + base + gq) * LOG2E : -INFINITY;
-        dl[u] = in ? -__ldg(p.delta + base + gq) : 0.f;
+        nl[u] = in ? -p.lse[base + gq] * LOG2E : -INFINITY;
+        dl[u] = in ? -p.delta[base + gq] : 0.f;
       }
       if (it >= STS && !mbar_wait(&stat_empty[st], ((it / STS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
       const uint32_t dst = smem_u32(s_stat + st * (2 * BQ) + lane);

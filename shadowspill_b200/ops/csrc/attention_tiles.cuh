@@ -16,7 +16,7 @@ struct TileSlot {
 
 // The tile of rank `rank` in descending work, `rows` rows to a tile. Executed by ONE full warp; the
 // slot is in shared memory and is read after the block's next barrier.
-__device__ __forceinline__ void find_tile_by_work(const int* __restrict__ cu, int nseq, int rows, int rank,
+__device__ __forceinline__ void find_tile_by_work(const int* cu, int nseq, int rows, int rank,
                                                   TileSlot* slot) {
   const int lane = threadIdx.x & 31;
   // tiles with at least `w` work; each sequence contributes max(0, n - w + 1)

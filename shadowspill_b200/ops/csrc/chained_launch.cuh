@@ -11,6 +11,10 @@ namespace ss {
 // follows chain_wait() and, where there is TMEM, the allocation, so that no waiting block can hold columns
 // that a block of this kernel still needs.
 //
+// Such a kernel's lifetime begins while the one ahead still writes, so nothing in global memory is read-only for
+// it: no `const __restrict__` parameters, __ldg or other non-coherent loads, which also are not ordered behind
+// the wait by the compiler.
+//
 // What it saves is the gap between two kernels, 2 to 3 us: a layer of 1,999 tokens and 2,048 channels, forward and
 // backward, 1004 -> 955 us (41 launches), attention on 2,048 tokens with heads of 64 121 -> 112 us, a layer of 8,192
 // tokens and 4,096 channels 1.4 %. Kernels that wait for other ranks are launched plainly and do not release, so

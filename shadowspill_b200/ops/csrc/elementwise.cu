@@ -79,7 +79,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // half-split convention: (a, b) = (x[i], x[i + rot/2]) ->
 // (a cos - b sin, b cos + a sin). inverse != 0 applies the transposed rotation,
 // which is the backward pass.
-__global__ void rope_kernel(bf16* __restrict__ buf, const int* __restrict__ positions, int T,
+__global__ void rope_kernel(bf16* buf, const int* positions, int T,
                             long long row_stride, int col0, int heads, int dh, int rot,
                             float log2_theta, int inverse) {
   chain_wait();
@@ -118,7 +118,7 @@ __global__ void rope_kernel(bf16* __restrict__ buf, const int* __restrict__ posi
 // cosines are computed once) and walks `heads_per_thread` heads with 16-byte loads, so
 // the transcendental work is amortised over the heads and the kernel runs at memory
 // speed. Needs rot % 16 == 0 and 16-byte aligned heads.
-__global__ void rope_vec_kernel(bf16* __restrict__ buf, const int* __restrict__ positions, int T,
+__global__ void rope_vec_kernel(bf16* buf, const int* positions, int T,
                                 long long row_stride, int col0, int heads, int dh, int rot,
                                 float log2_theta, int inverse, int slots) {
   chain_wait();
@@ -192,8 +192,7 @@ __device__ __forceinline__ void split_index(long long idx, int nv, long long& t,
 // gu is [T, 2F] with gate in columns [0,F) and up in [F,2F) (one fused GEMM
 // output). h = bf16(silu(float(gate))) * up.
 // `used` (optional, device memory): rows at and past *used are left alone.
-__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ h, int T, int F,
-                                  const int* __restrict__ used) {
+__global__ void swiglu_fwd_kernel(const bf16* gu, bf16* h, int T, int F, const int* used) {
   chain_wait();
   chain_release();
   const int nv = F >> 3;
@@ -216,8 +215,7 @@ __global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict_
   }
 }
 // dgu[T,2F] from dh[T,F] and the saved gu.
-__global__ void swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dh,
-                                  bf16* __restrict__ dgu, int T, int F) {
+__global__ void swiglu_bwd_kernel(const bf16* gu, const bf16* dh, bf16* dgu, int T, int F) {
   chain_wait();
   chain_release();
   const int nv = F >> 3;

@@ -303,7 +303,7 @@ struct NormRing {
 
 template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, bf16* y, float* __restrict__ rstd,
+rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* w, bf16* y, float* rstd,
                         long long T, int D, float eps, int zero_centered, int* status) {
   chain_wait();
   chain_release();
@@ -380,8 +380,8 @@ rmsnorm_fwd_long_kernel(bf16* x, const bf16* delta, const bf16* __restrict__ w, 
 
 template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_bwd_long_kernel(const bf16* x, const bf16* __restrict__ w, const bf16* gy, const float* __restrict__ rstd,
-                        bf16* dx, float* __restrict__ dw, long long T, int D, int zero_centered, int accumulate,
+rmsnorm_bwd_long_kernel(const bf16* x, const bf16* w, const bf16* gy, const float* rstd,
+                        bf16* dx, float* dw, long long T, int D, int zero_centered, int accumulate,
                         int* status) {
   chain_wait();
   chain_release();

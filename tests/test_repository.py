@@ -118,3 +118,19 @@ def test_every_device_wait_reports_its_failure():
             assert args[2] not in ("nullptr", "NULL", "0"), f"{f.name}: mbar_wait({', '.join(args)})"
             calls += 1
     assert calls > 50
+
+
+def test_chained_kernels_read_memory_coherently():
+    """A kernel that may start before the one ahead of it has ended must not use loads that are only defined
+    for memory nothing writes during the kernel, nor may the compiler move its loads above the wait."""
+    kernels = 0
+    for f in _csrc():
+        for part in re.split(r"__global__", f.read_text())[1:]:
+            # helpers between two kernels belong to neither: a kernel ends at the first line that is "}"
+            body = part.split("\n}\n")[0]
+            if "chain_wait();" not in body:
+                continue
+            kernels += 1
+            for word in ("__restrict__", "__ldg", "ld.global.nc", "__ldcs", "__ldlu"):
+                assert word not in body, f"{f.name}: {word} in a chained kernel:{body[:120]}"
+    assert kernels >= 12
