@@ -166,7 +166,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   TileSlot* slot = reinterpret_cast<TileSlot*>(bars + 19);
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
-  const int head = blockIdx.x;
+  const int head = blockIdx.x % p.Hq, rank = blockIdx.x / p.Hq;
   const int kv_head = head / (p.Hq / p.Hkv);
 
   if (threadIdx.x == 0) {
@@ -181,7 +181,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   chain_wait();
-  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
+  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, rank, slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -424,7 +424,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   float* s_stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);   // [STS][2][BQ]: -lse log2(e), -delta
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
-  const int kv_head = blockIdx.x / p.split, part = blockIdx.x % p.split;
+  const int shared = p.Hkv * p.split, rank = blockIdx.x / shared;      // tile; the CTAs of a cluster are neighbours
+  const int kv_head = blockIdx.x % shared / p.split, part = blockIdx.x % p.split;
   const int rep = p.Hq / p.Hkv / p.split;                  // query heads of this CTA
   const int head0 = kv_head * (p.Hq / p.Hkv) + part * rep;
 
@@ -443,7 +444,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
   if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   chain_wait();
-  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, blockIdx.y, slot);
+  if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, rank, slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -745,7 +746,9 @@ static int launch_dq(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtens
   auto kern = attn_bwd_dq_kernel<DH, BKV, KS, VS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
-  launch_chained(kern, dim3(p.Hq, tiles), BW_THREADS, Cfg::SMEM, s, tq, tdo, tk, tv, p);
+  const long long grid = static_cast<long long>(p.Hq) * tiles;       // see attention_fwd.cu
+  if (grid > 0x7fffffffLL) return -2;
+  launch_chained(kern, static_cast<unsigned>(grid), BW_THREADS, Cfg::SMEM, s, tq, tdo, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -757,7 +760,9 @@ static int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tdo, const CUten
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.Hkv * p.split, tiles);
+  const long long grid = static_cast<long long>(p.Hkv) * p.split * tiles;
+  if (grid > 0x7fffffffLL) return -2;
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(BW_THREADS);
   cfg.dynamicSmemBytes = Cfg::SMEM;
   cfg.stream = s;

@@ -88,7 +88,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
-  const int head = blockIdx.x;
+  const int head = blockIdx.x % p.Hq, rank = blockIdx.x / p.Hq;
   const int kv_head = head / (p.Hq / p.Hkv);
 
   if (threadIdx.x == 0) {
@@ -107,7 +107,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tmem_relinquish();
   }
   chain_wait();
-  if (warp == Cfg::TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, NT * 128, blockIdx.y, slot);
+  if (warp == Cfg::TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, NT * 128, rank, slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -349,9 +349,11 @@ static int launch_fwd(const void* q, const void* k, const void* v, AttnParams p,
   auto kern = attn_fwd_kernel<DH, NT, BKV, KS, VS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
-  // every sequence adds at most one partial tile
-  const dim3 grid(p.Hq, (p.T + NT * 128 - 1) / (NT * 128) + p.nseq);
-  launch_chained(kern, grid, Cfg::THREADS, Cfg::SMEM, stream, tq, tk, tv, p);
+  // every sequence adds at most one partial tile; heads and tiles share x, whose limit many short sequences
+  // do not reach (y ends at 65,535)
+  const long long grid = ((p.T + NT * 128 - 1) / (NT * 128) + static_cast<long long>(p.nseq)) * p.Hq;
+  if (grid > 0x7fffffffLL) return -2;
+  launch_chained(kern, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM, stream, tq, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
 }
 

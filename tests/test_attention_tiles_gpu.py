@@ -167,3 +167,25 @@ def test_backward_with_warps_a_tile_apart(dh):
 def test_wide_backward_with_warps_a_tile_apart():
     # dV alone: scores of the next query tile are ready before the slowest warp has written P^T of this one
     _gradients_beside_other_work(256)
+
+
+def test_more_sequences_than_a_grid_has_rows():
+    """66,000 one-token sequences, past the 65,535 of a grid's second dimension, and one of 200 tokens."""
+    n, tail, dh = 66000, 200, 64
+    g = torch.Generator().manual_seed(3)
+    q, k, v, dout = (torch.randn(n + tail, 1, dh, generator=g).to(torch.bfloat16).to(DEV) for _ in range(4))
+    cu = torch.tensor([*range(n + 1), n + tail], dtype=torch.int32, device=DEV)
+    out, lse = attention.forward(q, k, v, cu, tail)
+    dq, dk, dv = attention.backward(q, k, v, out, lse, dout, cu, tail)
+    _lib.check_status()
+    assert torch.equal(out[:n], v[:n]) and torch.equal(dv[:n], dout[:n])          # one key: probability one
+    assert torch.allclose(lse[0, :n], (q[:n].float() * k[:n].float()).sum((1, 2)) / 8, rtol=1e-5, atol=1e-4)
+    # dP and delta are the same sum in two orders: what is left of their difference is fp32 rounding
+    assert float(dq[:n].abs().max()) < 1e-4 and float(dk[:n].abs().max()) < 1e-4
+    one = torch.tensor([0, tail], dtype=torch.int32, device=DEV)
+    rest = [t[n:] for t in (q, k, v)]
+    out_r, lse_r = R.attention_varlen(*rest, one)
+    grads_r = R.attention_varlen_bwd(*rest, out_r, lse_r, dout[n:], one)
+    assert _rel(out[n:], out_r) < 1e-2
+    for a, b in zip((dq, dk, dv), grads_r):
+        assert _rel(a[n:], b) < 2e-2
