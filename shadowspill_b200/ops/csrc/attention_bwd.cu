@@ -55,8 +55,9 @@ struct AttnBwdParams {
 
 // ============================================================================ preprocess
 // A row of DH values per DH / 8 lanes, 16 bytes a lane (four-byte loads by a whole warp moved 3 TB/s:
-// 8,192 x 32 heads of 128, 44 -> 26 us).
-template <int DH>
+// 8,192 x 32 heads of 128, 44 -> 26 us). `out` may lie on any 4-byte boundary; off 16 bytes (WIDE = false) it is
+// read four bytes at a time. dout is a TMA operand of the kernels behind this one and always on 16.
+template <int DH, bool WIDE>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout, float* delta, int T, int Hq,
                   long long ld_out, long long ld_dout) {
@@ -68,7 +69,14 @@ attn_delta_kernel(const __nv_bfloat16* out, const __nv_bfloat16* dout, float* de
   const bool in = row < static_cast<long long>(T) * Hq;
   // heads fastest: neighbouring lane groups read neighbouring bytes
   const int t = in ? static_cast<int>(row / Hq) : 0, h = in ? static_cast<int>(row % Hq) : 0;
-  const uint4 o = *reinterpret_cast<const uint4*>(out + t * ld_out + h * DH + lane * 8);
+  uint4 o;
+  const __nv_bfloat16* at = out + t * ld_out + h * DH + lane * 8;
+  if constexpr (WIDE) {
+    o = *reinterpret_cast<const uint4*>(at);
+  } else {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(at);
+    o = make_uint4(w[0], w[1], w[2], w[3]);
+  }
   const uint4 d = *reinterpret_cast<const uint4*>(dout + t * ld_dout + h * DH + lane * 8);
   float acc = 0.f;
   const uint32_t ow[4] = {o.x, o.y, o.z, o.w}, dw[4] = {d.x, d.y, d.z, d.w};
@@ -809,7 +817,7 @@ extern "C" int ss_attn_bwd_g(const void* q, const void* k, const void* v, const 
   if ((lddq % 8) || (lddk % 8) || (lddv % 8)) return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (dh != 64 && dh != 128 && dh != 256) return -2;
-  if ((reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(dout) & 15)) return -2;
+  if ((reinterpret_cast<uintptr_t>(out) & 3) || (reinterpret_cast<uintptr_t>(dout) & 15)) return -2;
   {
     const long long blocks = (static_cast<long long>(T) * Hq * (dh / 8) + 255) / 256;
     auto run = [&](auto kern) {
@@ -817,9 +825,10 @@ extern "C" int ss_attn_bwd_g(const void* q, const void* k, const void* v, const 
           reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta_scratch, T,
           Hq, static_cast<long long>(Hq) * dh, ldo);
     };
-    if (dh == 64) run(attn_delta_kernel<64>);
-    else if (dh == 128) run(attn_delta_kernel<128>);
-    else run(attn_delta_kernel<256>);
+    const bool wide = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    if (dh == 64) run(wide ? attn_delta_kernel<64, true> : attn_delta_kernel<64, false>);
+    else if (dh == 128) run(wide ? attn_delta_kernel<128, true> : attn_delta_kernel<128, false>);
+    else run(wide ? attn_delta_kernel<256, true> : attn_delta_kernel<256, false>);
   }
   AttnBwdParams p;
   p.dq = dq; p.dk = dk; p.dv = dv; p.lse = lse; p.delta = delta_scratch; p.cu_seqlens = cu_seqlens;

@@ -189,3 +189,17 @@ def test_more_sequences_than_a_grid_has_rows():
     assert _rel(out[n:], out_r) < 1e-2
     for a, b in zip((dq, dk, dv), grads_r):
         assert _rel(a[n:], b) < 2e-2
+
+
+@pytest.mark.parametrize("dh", [64, 128, 256])
+@pytest.mark.parametrize("shift", [2, 4, 6])
+def test_saved_output_off_a_sixteen_byte_boundary(dh, shift):
+    q, k, v, dout, cu = _inputs([130, 77], 4, 2, dh, seed=dh + shift)
+    out, lse = attention.forward(q, k, v, cu, 130)
+    moved = torch.empty(out.numel() + 8, dtype=out.dtype, device=DEV)[shift:shift + out.numel()].view(out.shape)
+    moved.copy_(out)
+    assert moved.data_ptr() % 16 == 2 * shift
+    want = attention.backward(q, k, v, out, lse, dout, cu, 130)
+    got = attention.backward(q, k, v, moved, lse, dout, cu, 130)
+    _lib.check_status()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
