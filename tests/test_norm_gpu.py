@@ -85,3 +85,25 @@ def test_fused_residual_add_gives_the_same_bits(D):
     folded = x.clone()
     y2, rstd2 = F.rmsnorm_fwd(folded, w, EPS, delta=delta)
     assert torch.equal(folded, added) and torch.equal(y, y2) and torch.equal(rstd, rstd2)
+
+
+@pytest.mark.parametrize("D", [64, 256, 512, 2048, 4096, 8200])
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_weight_gradient_off_a_sixteen_byte_boundary(D, shift):
+    """A view into a flat fp32 buffer may start at any element."""
+    g = torch.Generator().manual_seed(D + shift)
+    x, w, gy = _rand(g, 150, D), _rand(g, D), _rand(g, 150, D)
+    rstd = torch.rsqrt(x.float().square().mean(-1) + EPS)
+    flat = torch.full((D + 8,), 3.0, device=DEV)
+    dw = flat[shift:shift + D]
+    assert dw.data_ptr() % 16 == 4 * shift
+    F.rmsnorm_bwd(x, w, gy, rstd, dw)
+    dx_r, dw_r = R.rmsnorm_bwd(x, w, gy, rstd)
+    assert _rel(dw - 3.0, dw_r) < 1e-4
+    assert bool((flat[:shift] == 3.0).all()) and bool((flat[shift + D:] == 3.0).all())
+    if D <= 512:
+        dw.fill_(0.0)
+        d = gy.repeat(1, 2).contiguous()
+        F.head_norm_bwd_(x.repeat(1, 2).contiguous(), w, d, rstd.repeat_interleave(2), dw, 2)
+        assert _rel(dw, 2.0 * dw_r.float()) < 1e-4 and _rel(d[:, :D], dx_r) < TOL
+    _lib.check_status()
