@@ -74,6 +74,7 @@ moe_route_kernel(const float* __restrict__ logits, long long ld, int T, int E, i
     }
     float my_v = -INFINITY;
     int my_e = 0;
+    unsigned taken = 0;                        // this lane's experts that have been picked, by i
     for (int j = 0; j < k; ++j) {
       float best = -INFINITY;
       int bi = 0x7fffffff;
@@ -89,9 +90,16 @@ moe_route_kernel(const float* __restrict__ logits, long long ld, int T, int E, i
         const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
       }
-      if (bi >= E) bi = j;                     // fewer than k comparable scores: any expert, with their weight
+      if (bi >= E) {                           // fewer than k comparable scores: the first experts not yet picked,
+        int left = 0x7fffffff;                 // each once, as the gradient of a pick is stored by its own lane
+#pragma unroll
+        for (int i = PER - 1; i >= 0; --i)
+          if (lane + i * 32 < E && !((taken >> i) & 1)) left = lane + i * 32;
+        bi = __reduce_min_sync(0xffffffffu, left);
+      }
       if (lane == j) { my_v = best; my_e = bi; }
       if ((bi & 31) == lane) {                 // remove the winner
+        taken |= 1u << (bi >> 5);
 #pragma unroll
         for (int i = 0; i < PER; ++i)
           if (i == (bi >> 5)) v[i] = -INFINITY;

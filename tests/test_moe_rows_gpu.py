@@ -87,3 +87,30 @@ def test_bank_gradient_leaves_out_blocks_of_padding(M, N):
         want = dy[off[e]:off[e] + n].double().T @ x[off[e]:off[e] + n].double()
         # fp32 sums of exact products, rounded to bf16 once (2^-9 of each value)
         assert float((out[e].double() - want).abs().max()) <= 2.0 ** -8 * (1e-3 + float(want.abs().max() if n else 0))
+
+
+@pytest.mark.parametrize("E,k,finite", [(4, 3, 2), (8, 8, 1), (64, 8, 3), (65, 6, 0), (512, 32, 31)])
+@pytest.mark.parametrize("renorm", [True, False])
+def test_fewer_comparable_scores_than_picks(E, k, finite, renorm):
+    """Masked experts (scores of -inf) fill up the picks: each once, with no weight and no gradient of their own."""
+    T = 300
+    g = torch.Generator(device=DEV).manual_seed(E + k)
+    logits = torch.full((T, E), -float("inf"), device=DEV)
+    open_ = torch.rand(T, E, generator=g, device=DEV).argsort(1)[:, :finite]
+    logits.scatter_(1, open_, torch.randn(T, finite, generator=g, device=DEV))
+    ids, wts, counts = moe.route(logits, k, renorm)
+    assert int(ids.min()) >= 0 and int(ids.max()) < E
+    assert bool((ids.sort(1).values.diff(dim=1) > 0).all())                # no expert twice
+    assert torch.equal(counts.long(), torch.bincount(ids.reshape(-1).long(), minlength=E))
+    if finite == 0:
+        return                                                             # no weights to speak of: 0 / 0
+    assert torch.equal(ids[:, :finite].long(), logits.topk(finite, 1).indices)
+    leaf = logits.double().requires_grad_(True)
+    want = (leaf.gather(1, ids.long()).softmax(1) if renorm else leaf.softmax(1).gather(1, ids.long()))
+    assert float((wts.double() - want).abs().max()) < 1e-6
+    dwts = torch.randn(T, k, generator=g, device=DEV)
+    want.backward(dwts.double())
+    got = moe.route_bwd(logits, ids, wts, dwts, renorm)
+    assert bool(torch.isfinite(got).all())
+    # fp32 products and sums of up to 32 terms of order one
+    assert float((got.double() - leaf.grad).abs().max()) < 1e-5
