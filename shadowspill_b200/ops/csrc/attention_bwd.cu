@@ -100,8 +100,7 @@ __device__ __forceinline__ constexpr uint32_t packed_col(int kk) {
   return (kk * 16) / (BN / 2) * (BN / 2) + ((kk * 16) % (BN / 2)) / 2;
 }
 
-// An explicit shared-memory load: through the aligned-up window pointer the compiler only sees a
-// generic address, whose loads take the global path (they were most of the dKV kernel's stalls).
+// Two pairs of fp32 in one 16-byte load, in the registers that the packed arithmetic takes.
 __device__ __forceinline__ void ld_shared_2x2(uint32_t addr, f32x2& a, f32x2& b) {
   asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }

@@ -488,7 +488,8 @@ __device__ __forceinline__ void adamw_tail(bf16* p, const void* g, bf16* m, bf16
 // template parameters, halves are packed by byte permutes and the inf / nan test is shared by eight
 // values. One vector per thread is always in flight behind the arithmetic, in two persistent blocks per SM
 // (three at 80 registers spill: 667 against 594 us for a 218 M element layer). 58.7 M elements: 647 -> 525
-// instructions per eight, 195 -> 160 us; the results keep their bits.
+// instructions per eight, 192 -> 153 us (kernel durations, L2 flushed before each launch); the results keep
+// their bits.
 constexpr int ADAMW_THREADS = 256;
 template <bool SR_PARAM, bool SR_STATE, bool G_F32>
 __global__ void __launch_bounds__(ADAMW_THREADS, 2)
@@ -656,7 +657,7 @@ static AdamWArgs adamw_args(float lr, float beta1, float beta2, float eps, float
   return a;
 }
 // One vector per thread of the persistent form's grid: a larger tensor fills the GPU by itself, and its next
-// vector's loads run under the arithmetic there.
+// vector's loads run under the arithmetic there. The caller of the shared form has the same number.
 constexpr long long ADAMW_MANY_ELEMENTS = 148ll * 2 * ADAMW_THREADS * 8;
 
 }  // namespace ss
@@ -766,8 +767,7 @@ int ss_adamw_sr(void* p, const void* g, void* m, void* v, long long n, int g_f32
                   : (g_f32 ? go(adamw_sr_kernel<false, false, true>) : go(adamw_sr_kernel<false, false, false>));
 }
 // `tensors`: seven values per tensor, {p, g, m, v, elements, offset, gradient is fp32}, in host memory, read
-// before the call returns. Distinct tensors of up to ss_adamw_many_elements() elements.
-long long ss_adamw_many_elements(void) { return ADAMW_MANY_ELEMENTS; }
+// before the call returns. Distinct tensors of up to ADAMW_MANY_ELEMENTS elements.
 int ss_adamw_sr_many(const long long* tensors, int count, float lr, float beta1, float beta2, float eps,
                      float weight_decay, int step, float grad_scale, unsigned long long seed, int sr_param,
                      int sr_state, void* stream) {

@@ -10,12 +10,14 @@
 //                                 wait for memory latency
 // The weight gradient is summed in registers over all rows of a thread, then over the block in shared
 // memory, and leaves as one 16-byte vector reduction per four columns and block: scalar atomics with a
-// 32-byte stride between lanes cost more than the rows themselves (33 us for 768 x 256).
+// 32-byte stride between lanes cost more than the rows themselves (37 us for 768 x 256).
 //
-// Measured (one B200; before: one 256-thread block per row, next row prefetched in registers):
-//   forward   8192 x 4096            33 -> 24.5 us (5.5 TB/s)    1999 x 16 heads of 128    59 -> 8 us
-//   backward  8192 x 4096, + dx     126 -> 53 us   (5.0 TB/s)    1999 x 16 heads of 128    96 -> 9 us
-//   backward  768 x 256              33 -> 2.8 us                1999 x 2048               38 -> 13-18 us
+// Measured (one B200, kernel durations with the L2 flushed before each launch; before: one 256-thread block per
+// row, next row prefetched in registers):
+//   forward   8192 x 4096           33 -> 26 us (5.1 TB/s)    + residual add     52 -> 47 us (5.7 TB/s)
+//   backward  8192 x 4096           89 -> 41 us (4.9 TB/s)    added to dx       110 -> 47 us (5.7 TB/s)
+//   backward   768 x 256            37 -> 3.3 us              1999 x 2048        43 -> 13 us
+//   1999 x 16 rows of 128, forward  68 -> 7 us                backward           92 -> 8 us
 // Heads of a projection are normalised where they lie: no copy to contiguous rows and back.
 //
 // The math follows the reference's pure-PyTorch definition

@@ -292,8 +292,8 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
 }
 // The same for a whole warp in step (`_ts`: A from TMEM), of which only the lane with `leader` set issues. With no branch
 // around them the addresses and descriptors are computed once per warp in uniform registers, where the
-// instruction takes them from; inside a one-lane branch each has to be moved there first, about 46 cycles
-// per product.
+// instruction takes them from; inside a one-lane branch each has to be moved there first (attention on 16,384
+// tokens: forward 1020 -> 968 us, dQ 1260 -> 1205, dK/dV 1710 -> 1632).
 __device__ __forceinline__ void umma_bf16_if(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -348,8 +348,8 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
   return __bfloat1622float2(v);
 }
 
-// Two fp32 operations per instruction (same rounding as the scalar forms). The softmax warps of the
-// attention kernels are bound by the instructions they issue, not by the special-function unit.
+// Two fp32 operations per instruction (same rounding as the scalar forms), for the softmax warps of the attention
+// kernels, whose chain from a score to its probability is what the products wait for.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack_x2(float lo, float hi) {
   f32x2 v;

@@ -2,7 +2,7 @@
 
 Forward is two launches after a tiny sequence-id kernel: ``ss_dn_prep`` (per chunk and pair of
 V heads: K K^T, Q K^T, the 64x64 triangular inverse, W^T, U0^T) and ``ss_dn_fwd`` (per V head, the
-state walk over chunks with S^T resident in TMEM). Backward recomputes both with their saves
+state walk over chunks with the state in the registers of eight warps). Backward recomputes both with their saves
 switched on, then runs the reverse state walk, the per-chunk products and the gradient of the
 chunk-local algebra. Nothing but the inputs is kept between forward and backward.
 

@@ -50,7 +50,8 @@ def _ptr(t: torch.Tensor | None) -> int | None:
 
 
 # ------------------------------------------------------------------------ GEMM
-# plain GEMMs run on the CTA-pair kernel; SS_GEMM_PAIR=0 selects the single-CTA kernel
+# plain GEMMs of 256 x 128 and more enter at the CTA-pair kernel, which hands outputs of one wave of 128 x 128 tiles
+# to the single-CTA kernel; SS_GEMM_PAIR=0 keeps all of them on that one
 _PAIR_GEMM = os.environ.get("SS_GEMM_PAIR", "1") == "1"
 
 
@@ -97,7 +98,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                          f"(N={N}, strides {lda}, {ldb}, {ldc}); pad the operand")
     if _PAIR_GEMM and bn == 0 and M >= 256 and N >= 128:
         # CTA-pair kernel (tcgen05 cta_group::2): 256x256 tiles, half the shared-memory
-        # traffic per FLOP of the single-CTA kernel
+        # traffic per FLOP of the single-CTA kernel, which takes the outputs of one wave from there
         rc = _lib.lib().ss_gemm2_bf16(
             a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), int(f32),
             int(accumulate), float(alpha), 0, _lib.status_ptr(a), _lib.stream_ptr())
@@ -410,7 +411,7 @@ def adamw_(p, g, m, v, *, lr, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.0,
                              int(stochastic_state), _lib.stream_ptr()), "ss_adamw_sr")
 
 
-ADAMW_MANY_ELEMENTS = 148 * 2 * 256 * 8     # as the kernel's launcher has it
+ADAMW_MANY_ELEMENTS = 148 * 2 * 256 * 8     # as the kernel's launcher has it, which refuses larger ones
 
 
 def adamw_many_(tensors, *, lr, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.0, step=1, grad_scale=1.0,

@@ -75,8 +75,8 @@ def test_groups_shared_by_clusters(lens, dh, Hq, Hkv):
 
 @pytest.mark.parametrize("width", [64, 128, 256])
 def test_results_do_not_depend_on_other_work_on_the_gpu(width):
-    # work of another stream on the same SMs slows some warps of a tile: one that is a key step ahead of
-    # the others must still wait for the last product over values before it reads the output
+    # work of another stream on the same SMs slows some warps of a tile: those that are a step ahead must
+    # neither count for the others nor be lapped by the products that wait for them
     from shadowspill_b200.ops import functional as F
     lens = [128, 200, 100, 128, 450, 128, 60, 128, 256, 120] * 6
     T, H, Hk = sum(lens), 32, 8
