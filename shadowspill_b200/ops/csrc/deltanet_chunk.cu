@@ -450,57 +450,112 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 }
 
 // ============================================================================ state walks
-// One CTA per V head walks the chunks; nothing but the chain state -> (W S) -> U -> state has to be
+// A CTA walks a run of chunks of one V head; nothing but the chain state -> (W S) -> U -> state has to be
 // serial, so that chain is all the state warps wait for:
-//   * the state lives in their registers (two warps per lane quarter, 64 of the 128 columns each),
+//   * the state lives in their registers (fp32, STATE_COLS of the 128 columns per warp),
 //     S <- Gc S + dS with dS fresh from the tensor cores, so it is never scaled in TMEM;
+//   * its bf16 form and U go back to the products as A operands in TMEM; the copies that are saved are written
+//     to shared memory behind them, off the chain, and leave by TMA;
 //   * products that do not need the chain's next value (S^T Qg^T; dO^T Mq, dO^T Qg) are issued while
-//     the state warps work, and the forward output has its own accumulators, warps and barrier;
-//   * the saved copies leave by TMA from the very operand tiles the products read.
-// Measured, 8,192 tokens, 32 V heads: forward 0.660 -> 0.254 ms, backward 0.497 -> 0.210 ms
-// (forward 5.1 -> 2.0 us per chunk: every step waited for all products, and every warp for all stores).
+//     the state warps work, and the forward output has its own accumulators, warps and barrier.
+// A chunk in which a sequence ends passes nothing on (its Gc is 0, and its rows of Kd belong to the sequence it
+// ends with, whose rows of W are 0), so the chunks behind it are a run of their own, which takes that chunk first,
+// from a zero state and without results ("warm"). The same holds in reverse, where the chunk belongs to the later
+// run. Runs are taken by position: bucket r of a head has the chunks between the first run start at or behind
+// chunk r * bucket and the next bucket's; most buckets of long sequences are empty and leave at once.
+// Measured, 8,192 tokens in four sequences (the longest 47 chunks of 128), 32 V heads: forward 0.237 -> 0.095 ms,
+// backward 0.206 -> 0.094 ms; the chain takes 1.9 us a chunk either way, 32 heads alone on 148 SMs were the loss.
 struct WalkParams {
   const float* gc;
+  const int* sid;
+  int bucket;                               // chunks
   int save;                                 // forward: keep S and U for the backward pass
   Geo geo; int* status;
 };
 namespace walk {
 constexpr int STAGE = 73728;
-constexpr int OFF_SOP = 2 * STAGE;          // [128 x 128] K-major operand
-constexpr int OFF_UOP = OFF_SOP + 32768;    // [128 x 64] K-major operand
-constexpr int OFF_UST = OFF_UOP + 16384;    // forward: O of a chunk; backward: the saved dU^T (other sign)
-constexpr int OFF_BAR = OFF_UST + 16384;
+constexpr int OFF_SOP = 2 * STAGE;          // [128 x 128] saved copy of the state
+constexpr int OFF_UOP = OFF_SOP + 32768;    // [128 x 64] saved copy of U or dU
+constexpr int OFF_O = OFF_UOP + 16384;      // forward: O of a chunk
+constexpr int OFF_BAR = OFF_O + 16384;
 constexpr int SMEM = OFF_BAR + 256 + 1024;
-constexpr int STATE_WARPS = 8;
-constexpr int TM_DS = 0, TM_WS = 128, TM_O = 192;      // TMEM columns: 128, 64, 2 x 64
+constexpr int STATE_WARPS = 8, STATE_COLS = 512 / STATE_WARPS, TOKEN_COLS = STATE_COLS / 2;
+constexpr int TM_DS = 0, TM_WS = 128, TM_O = 192, TM_SOP = 320, TM_UOP = 384;   // TMEM columns: 128, 64, 2 x 64, 64, 32
 constexpr int FWD_THREADS = (STATE_WARPS + 4 + 2) * 32, BWD_THREADS = (STATE_WARPS + 2) * 32;
 static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
 }
 
-// 32 or 64 fp32 columns of this thread's lane, one wait for all of them.
-template <int N>
-__device__ __forceinline__ void tmem_cols(uint32_t addr, float (&out)[N]) {
-#pragma unroll
-  for (int c = 0; c < N; c += 32) tmem_ld_32x32(addr + c, reinterpret_cast<uint32_t (&)[32]>(out[c]));
-  tmem_ld_wait();
+// The first chunk at or behind `c` that a run may start at: 0, the number of chunks, or one with a sequence begun
+// in it or in the chunk before behind its first token. Sequence ids rise with the tokens. Executed by a full warp.
+__device__ __forceinline__ int run_start(const int* sid, int n, int c) {
+  if (c <= 0) return 0;
+  if (c >= n) return n;
+  const int lane = threadIdx.x & 31, before = sid[(c - 1) * CH];
+  int lo = c, hi = n;
+  while (lo < hi) {
+    const int step = (hi - lo + 31) >> 5, s = lo + lane * step;
+    const unsigned past = __ballot_sync(0xffffffffu, s >= hi || sid[s * CH] != before);
+    if (past == 0) { lo += 31 * step + 1; continue; }
+    const int first = __ffs(static_cast<int>(past)) - 1;
+    hi = min(hi, lo + first * step);
+    lo = first ? lo + (first - 1) * step + 1 : hi;
+  }
+  return lo;
+}
+// Does the sequence of chunk s begin before it, so that a run that starts there needs the chunk before?
+__device__ __forceinline__ bool run_warm(const int* sid, int n, int s) {
+  return s > 0 && s < n && sid[s * CH - 1] == sid[s * CH];
 }
 
-// The state warps' half rows: S <- gc S + dS (dS in TMEM, none before the first chunk), bf16 into SOP.
-__device__ __forceinline__ void state_step(float (&S)[64], bool fresh, float gc, uint32_t ds_addr, uint8_t* sop,
-                                           int row, int half) {
-  if (!fresh) {
-    float d[64];
-    tmem_cols(ds_addr, d);
+// N fp32 columns of this thread's lane, one wait for all of them.
+template <int N>
+__device__ __forceinline__ void tmem_cols(uint32_t addr, float (&out)[N]) {
+  if constexpr (N == 16) {
+    tmem_ld_32x16(addr, reinterpret_cast<uint32_t (&)[16]>(out));
+  } else {
 #pragma unroll
-    for (int e = 0; e < 64; ++e) S[e] = fmaf(gc, S[e], d[e]);
+    for (int c = 0; c < N; c += 32) tmem_ld_32x32(addr + c, reinterpret_cast<uint32_t (&)[32]>(out[c]));
   }
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-    *reinterpret_cast<uint4*>(sop + sw_off(128, row, half * 8 + q)) = pack8(S + q * 8);
+  tmem_ld_wait();
 }
-// Operands written by this warp are visible to the MMAs and TMA stores that wait for `bar`.
+// N fp32 values -> N / 2 columns of bf16 pairs of this thread's lane: the A operand of a product.
+template <int N>
+__device__ __forceinline__ void tmem_put_bf16(uint32_t addr, const float (&v)[N], uint32_t (&pk)[N / 2]) {
+#pragma unroll
+  for (int e = 0; e < N / 2; ++e) pk[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
+  if constexpr (N == 64) tmem_st_32x32(addr, pk);
+  else if constexpr (N == 32) tmem_st_32x16(addr, pk);
+  else tmem_st_32x8(addr, pk);
+  tmem_st_wait();
+}
+// The same values as columns [N * part, N * part + N) of `row` of a swizzled tile of 128 rows.
+template <int N>
+__device__ __forceinline__ void smem_put_bf16(uint8_t* tile, int row, int part, const uint32_t (&pk)[N / 2]) {
+#pragma unroll
+  for (int q = 0; q < N / 8; ++q)
+    *reinterpret_cast<uint4*>(tile + sw_off(128, row, part * (N / 8) + q)) =
+        make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+}
+// The state warps' part of a row: S <- gc S + dS (dS in TMEM, none before the first chunk).
+template <int N>
+__device__ __forceinline__ void state_step(float (&S)[N], float gc, uint32_t ds_addr) {
+  constexpr int M = N < 32 ? N : 32;           // all of a row's dS at once does not fit the registers beside S
+#pragma unroll
+  for (int c = 0; c < N; c += M) {
+    float d[M];
+    tmem_cols(ds_addr + c, d);
+#pragma unroll
+    for (int e = 0; e < M; ++e) S[c + e] = fmaf(gc, S[c + e], d[e]);
+  }
+}
+// What this warp wrote to TMEM is visible to the products that wait for `bar`.
 __device__ __forceinline__ void warp_publish(uint64_t* bar) {
   tc_fence_before();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+// What this warp wrote to shared memory is visible to the TMA stores that wait for `bar`.
+__device__ __forceinline__ void warp_publish_copy(uint64_t* bar) {
   fence_async_proxy();
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
@@ -524,14 +579,23 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
   uint64_t* s_done = bars + 7;
   uint64_t* o_full = bars + 8;         // [2]
   uint64_t* o_free = bars + 10;        // [2]
-  uint64_t* saved = bars + 12;         // both operands have been read by their stores
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint64_t* s_copied = bars + 12;      // the copies to be saved have been written
+  uint64_t* u_copied = bars + 13;
+  uint64_t* saved = bars + 14;         // both have been read by their stores
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  int* run = reinterpret_cast<int*>(bars + 16);          // first chunk, one behind the last, warm
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const Geo G = p.geo;
   const int h = blockIdx.x;
   int pr, hh;
   head_slot(G, h, pr, hh);
 
+  if (warp == 0) {
+    const int first = run_start(p.sid, G.n, blockIdx.y * p.bucket);
+    const int end = run_start(p.sid, G.n, (blockIdx.y + 1) * p.bucket);
+    if (lane == 0) { run[0] = first; run[1] = end; run[2] = run_warm(p.sid, G.n, first); }
+  }
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&full[i], 1); mbar_init(&stage_free[i], 1);
@@ -539,57 +603,73 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
     }
     mbar_init(sop_ready, STATE_WARPS); mbar_init(ws_done, 1);
     mbar_init(u_ready, STATE_WARPS); mbar_init(s_done, 1);
-    mbar_init(saved, 1);
+    mbar_init(s_copied, STATE_WARPS); mbar_init(u_copied, STATE_WARPS); mbar_init(saved, 1);
     mbar_fence_init();
   }
+  __syncthreads();
+  if (run[0] >= run[1]) return;
+  const int skip = run[2], c0 = run[0] - skip, steps = run[1] - c0;    // the first `skip` steps leave no results
   if (warp == STATE_WARPS + 4) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   const int row = (warp & 3) * 32 + lane;      // V feature
 
   if (warp < STATE_WARPS) {
-    const int half = warp >> 2;
-    float S[64];
+    const int part = warp >> 2;
+    float S[STATE_COLS];
 #pragma unroll
-    for (int e = 0; e < 64; ++e) S[e] = 0.f;
+    for (int e = 0; e < STATE_COLS; ++e) S[e] = 0.f;
     float gc = 0.f;
-    for (int c = 0; c < G.n; ++c) {
-      const int st = c & 1;
-      const float gc_next = p.gc[static_cast<long long>(c) * G.H + h];
-      if (c > 0 && !mbar_wait(s_done, (c - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
-      if (c > 0 && p.save && !mbar_wait(saved, (c - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
-      tc_fence_after();
-      state_step(S, c == 0, gc, lane_addr + TM_DS + half * 64, smem + OFF_SOP, row, half);
+    for (int it = 0; it < steps; ++it) {
+      const int st = it & 1;
+      const bool keep = p.save && it >= skip;
+      const float gc_next = p.gc[static_cast<long long>(c0 + it) * G.H + h];
+      if (it > 0) {
+        if (!mbar_wait(s_done, (it - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
+        tc_fence_after();
+        state_step(S, gc, lane_addr + TM_DS + part * STATE_COLS);
+      }
+      uint32_t sk[STATE_COLS / 2];
+      tmem_put_bf16(lane_addr + TM_SOP + part * (STATE_COLS / 2), S, sk);
       warp_publish(sop_ready);
       gc = gc_next;
-      if (!mbar_wait(&full[st], (c >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
-      float u[32];
+      if (keep) {
+        if (it > skip && !mbar_wait(saved, (it - skip - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        smem_put_bf16<STATE_COLS>(smem + OFF_SOP, row, part, sk);
+        warp_publish_copy(s_copied);
+      }
+      if (!mbar_wait(&full[st], (it >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
+      float u[TOKEN_COLS];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        unpack8(*reinterpret_cast<const uint4*>(smem + st * STAGE + 16384 + sw_off(128, row, half * 4 + q)), u + q * 8);
-      if (!mbar_wait(ws_done, c & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
+      for (int q = 0; q < TOKEN_COLS / 8; ++q)
+        unpack8(*reinterpret_cast<const uint4*>(smem + st * STAGE + 16384 +
+                                                sw_off(128, row, part * (TOKEN_COLS / 8) + q)), u + q * 8);
+      if (!mbar_wait(ws_done, it & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
       tc_fence_after();
-      float ws[32];
-      tmem_cols(lane_addr + TM_WS + half * 32, ws);
+      float ws[TOKEN_COLS];
+      tmem_cols(lane_addr + TM_WS + part * TOKEN_COLS, ws);
 #pragma unroll
-      for (int e = 0; e < 32; ++e) u[e] -= ws[e];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<uint4*>(smem + OFF_UOP + sw_off(128, row, half * 4 + q)) = pack8(u + q * 8);
+      for (int e = 0; e < TOKEN_COLS; ++e) u[e] -= ws[e];
+      uint32_t uk[TOKEN_COLS / 2];
+      tmem_put_bf16(lane_addr + TM_UOP + part * (TOKEN_COLS / 2), u, uk);
       warp_publish(u_ready);
+      if (keep) {
+        smem_put_bf16<TOKEN_COLS>(smem + OFF_UOP, row, part, uk);
+        warp_publish_copy(u_copied);
+      }
     }
   } else if (warp < STATE_WARPS + 4) {
     // O^T is transposed through shared memory and leaves by TMA, which also clips the last chunk's
     // rows: 64 two-byte stores per thread straight to memory took longer than the rest of the chunk
-    uint8_t* so = smem + OFF_UST + (row >> 6) * 8192;
+    uint8_t* so = smem + OFF_O + (row >> 6) * 8192;
     const int col = (row & 63) * 2;
     const bool issuer = tid == STATE_WARPS * 32;
-    for (int c = 0; c < G.n; ++c) {
-      const int b = c & 1;
-      const bool ok = mbar_wait(&o_full[b], (c >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL);
+    for (int it = 0; it < steps; ++it) {
+      const int b = it & 1;
+      const bool ok = mbar_wait(&o_full[b], (it >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       float o[64];
       if (ok) tmem_cols(lane_addr + TM_O + b * 64, o);
@@ -603,6 +683,7 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
       asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\t"
                    "selp.u32 %0, 1, 0, q;\n\t}" : "=r"(all_ok) : "r"(static_cast<uint32_t>(ok)) : "memory");
       if (!all_ok) break;
+      if (it < skip) continue;
 #pragma unroll
       for (int t = 0; t < 64; ++t)
         *reinterpret_cast<__nv_bfloat16*>(so + t * 128 + (col ^ ((t & 7) << 4))) = __float2bfloat16_rn(o[t]);
@@ -610,54 +691,53 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
       asm volatile("bar.sync 2, 128;" ::: "memory");
       if (issuer) {
 #pragma unroll
-        for (int x = 0; x < 2; ++x) tma_store_2d(&tmO, smem + OFF_UST + x * 8192, h * D + x * 64, c * CH);
+        for (int x = 0; x < 2; ++x) tma_store_2d(&tmO, smem + OFF_O + x * 8192, h * D + x * 64, (c0 + it) * CH);
         tma_store_commit();
       }
     }
     if (issuer) tma_store_wait<0>();
   } else if (warp == STATE_WARPS + 4) {
-    if (elect_one()) {
-      const uint32_t sop = smem_u32(smem + OFF_SOP), uop = smem_u32(smem + OFF_UOP);
-      constexpr uint32_t idesc_w = umma_idesc_bf16(128, 64, false, true);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(128, 64, false, false);
-      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, true);
-      for (int c = 0; c < G.n; ++c) {
-        const int st = c & 1;
-        const uint32_t sst = smem_u32(smem + st * STAGE), to = tmem_base + TM_O + st * 64;
-        if (!mbar_wait(&full[st], (c >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
-        if (!mbar_wait(sop_ready, c & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
-        // (W S)^T = S^T W^T
+    const uint32_t leader = elect_one();
+    const uint32_t sop = tmem_base + TM_SOP, uop = tmem_base + TM_UOP;
+    constexpr uint32_t idesc_w = umma_idesc_bf16(128, 64, false, true);
+    constexpr uint32_t idesc_o = umma_idesc_bf16(128, 64, false, false);
+    constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, true);
+    for (int it = 0; it < steps; ++it) {
+      const int st = it & 1;
+      const uint32_t sst = smem_u32(smem + st * STAGE), to = tmem_base + TM_O + st * 64;
+      if (!mbar_wait(&full[st], (it >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
+      if (!mbar_wait(sop_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+      tc_fence_after();
+      // (W S)^T = S^T W^T
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(tmem_base + TM_WS, umma_smem_desc(sop + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                    umma_smem_desc(sst + kk * 2048, 16384, 1024), idesc_w, kk != 0);
-        umma_commit(ws_done);
-        // O^T = S^T Qg^T, while the state warps form U
-        if (c >= 2 && !mbar_wait(&o_free[st], ((c >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
+      for (int kk = 0; kk < 8; ++kk)
+        umma_bf16_ts_if(leader, tmem_base + TM_WS, sop + kk * 8, umma_smem_desc(sst + kk * 2048, 16384, 1024), idesc_w,
+                        kk != 0);
+      umma_commit_if(leader, ws_done);
+      // O^T = S^T Qg^T, while the state warps form U
+      if (it >= 2 && !mbar_wait(&o_free[st], ((it >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+      tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(to, umma_smem_desc(sop + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                    umma_smem_desc(sst + 32768 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), idesc_o, kk != 0);
-        if (!mbar_wait(u_ready, c & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
-        // dS^T = U^T Kd, then O^T += U^T Mq^T behind it
+      for (int kk = 0; kk < 8; ++kk)
+        umma_bf16_ts_if(leader, to, sop + kk * 8,
+                        umma_smem_desc(sst + 32768 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), idesc_o, kk != 0);
+      if (!mbar_wait(u_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+      tc_fence_after();
+      // dS^T = U^T Kd, then O^T += U^T Mq^T behind it
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem_base + TM_DS, umma_smem_desc(uop + kk * 32, 16, 1024),
-                    umma_smem_desc(sst + 49152 + kk * 2048, 8192, 1024), idesc_s, kk != 0);
-        umma_commit(s_done);
+      for (int kk = 0; kk < 4; ++kk)
+        umma_bf16_ts_if(leader, tmem_base + TM_DS, uop + kk * 8, umma_smem_desc(sst + 49152 + kk * 2048, 8192, 1024),
+                        idesc_s, kk != 0);
+      umma_commit_if(leader, s_done);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(to, umma_smem_desc(uop + kk * 32, 16, 1024), umma_smem_desc(sst + 65536 + kk * 32, 16, 1024),
-                    idesc_o, 1);
-        umma_commit(&o_full[st]);
-        umma_commit(&stage_free[st]);
-      }
+      for (int kk = 0; kk < 4; ++kk)
+        umma_bf16_ts_if(leader, to, uop + kk * 8, umma_smem_desc(sst + 65536 + kk * 32, 16, 1024), idesc_o, 1);
+      umma_commit_if(leader, &o_full[st]);
+      umma_commit_if(leader, &stage_free[st]);
     }
   } else if (elect_one()) {
-    auto load_stage = [&](int c, int st) {
+    auto load_stage = [&](int it) {
+      const int c = c0 + it, st = it & 1;
       uint8_t* s = smem + st * STAGE;
       const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 64;
       mbar_expect_tx(&full[st], STAGE);
@@ -670,23 +750,25 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
       }
       tma_load_2d(s + 65536, &tmMQ, &full[st], 0, prow + hh * 64);
     };
-    load_stage(0, 0);
-    if (G.n > 1) load_stage(1, 1);
-    for (int c = 0; c < G.n; ++c) {
-      if (p.save) {
-        if (!mbar_wait(sop_ready, c & 1, p.status, KS_TIMEOUT_FULL)) break;
+    load_stage(0);
+    if (steps > 1) load_stage(1);
+    for (int it = 0; it < steps; ++it) {
+      if (p.save && it >= skip) {
+        const int c = c0 + it;
+        if (!mbar_wait(s_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
 #pragma unroll
         for (int b = 0; b < 2; ++b)
           tma_store_2d(&tmST, smem + OFF_SOP + b * 16384, b * 64, (c * G.H + h) * 128);
-        if (!mbar_wait(u_ready, c & 1, p.status, KS_TIMEOUT_FULL)) break;
+        tma_store_commit();
+        if (!mbar_wait(u_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
         tma_store_2d(&tmUT, smem + OFF_UOP, hh * 64, (c * G.NP + pr) * 128);
         tma_store_commit();
         tma_store_wait_read<0>();
         mbar_arrive(saved);
       }
-      if (c + 2 < G.n) {
-        if (!mbar_wait(&stage_free[c & 1], (c >> 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
-        load_stage(c + 2, c & 1);
+      if (it + 2 < steps) {
+        if (!mbar_wait(&stage_free[it & 1], (it >> 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        load_stage(it + 2);
       }
     }
     tma_store_wait<0>();
@@ -712,99 +794,123 @@ dn_bwd_state_kernel(const __grid_constant__ CUtensorMap tmDO, const __grid_const
   uint64_t* stage_free = bars + 2;     // [2]
   uint64_t* sop_ready = bars + 4;      // dS'^T operand written
   uint64_t* du_done = bars + 5;
-  uint64_t* u_ready = bars + 6;        // -dU^T operand and the saved dU^T written
+  uint64_t* u_ready = bars + 6;        // -dU^T operand written
   uint64_t* s_done = bars + 7;
-  uint64_t* saved = bars + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint64_t* s_copied = bars + 8;       // the copies to be saved have been written
+  uint64_t* u_copied = bars + 9;
+  uint64_t* saved = bars + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  int* run = reinterpret_cast<int*>(bars + 12);          // lowest chunk with results, one behind the highest, warm
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const Geo G = p.geo;
   const int h = blockIdx.x;
   int pr, hh;
   head_slot(G, h, pr, hh);
 
+  if (warp == 0) {
+    // a chunk in which a run's sequence begins belongs to that run here; the run before takes it first, as its warm
+    const int first = run_start(p.sid, G.n, blockIdx.y * p.bucket);
+    const int end = run_start(p.sid, G.n, (blockIdx.y + 1) * p.bucket);
+    const int warm = run_warm(p.sid, G.n, end);
+    if (lane == 0) { run[0] = first - run_warm(p.sid, G.n, first); run[1] = first < end ? end - warm : 0; run[2] = warm; }
+  }
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&full[i], 1); mbar_init(&stage_free[i], 1); }
     mbar_init(sop_ready, STATE_WARPS); mbar_init(du_done, 1);
     mbar_init(u_ready, STATE_WARPS); mbar_init(s_done, 1);
-    mbar_init(saved, 1);
+    mbar_init(s_copied, STATE_WARPS); mbar_init(u_copied, STATE_WARPS); mbar_init(saved, 1);
     mbar_fence_init();
   }
-  if (warp == STATE_WARPS) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  __syncthreads();
+  if (run[0] >= run[1]) return;
+  const int skip = run[2], c_top = run[1] - 1 + skip, steps = c_top - run[0] + 1;
+  if (warp == STATE_WARPS) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 
   if (warp < STATE_WARPS) {
-    const int half = warp >> 2, row = (warp & 3) * 32 + lane;
-    float S[64];
+    const int part = warp >> 2, row = (warp & 3) * 32 + lane;
+    float S[STATE_COLS];
 #pragma unroll
-    for (int e = 0; e < 64; ++e) S[e] = 0.f;
+    for (int e = 0; e < STATE_COLS; ++e) S[e] = 0.f;
     float gc = 0.f;
-    for (int it = 0; it < G.n; ++it) {
-      const float gc_next = p.gc[static_cast<long long>(G.n - 1 - it) * G.H + h];
-      if (it > 0 && !mbar_wait(s_done, (it - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
-      if (it > 0 && !mbar_wait(saved, (it - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
-      tc_fence_after();
-      state_step(S, it == 0, gc, lane_addr + TM_DS + half * 64, smem + OFF_SOP, row, half);
+    for (int it = 0; it < steps; ++it) {
+      const bool keep = it >= skip;
+      const float gc_next = p.gc[static_cast<long long>(c_top - it) * G.H + h];
+      if (it > 0) {
+        if (!mbar_wait(s_done, (it - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
+        tc_fence_after();
+        state_step(S, gc, lane_addr + TM_DS + part * STATE_COLS);
+      }
+      uint32_t sk[STATE_COLS / 2];
+      tmem_put_bf16(lane_addr + TM_SOP + part * (STATE_COLS / 2), S, sk);
       warp_publish(sop_ready);
       gc = gc_next;
+      if (keep) {
+        if (it > skip && !mbar_wait(saved, (it - skip - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        smem_put_bf16<STATE_COLS>(smem + OFF_SOP, row, part, sk);
+        warp_publish_copy(s_copied);
+      }
       if (!mbar_wait(du_done, it & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
       tc_fence_after();
-      float du[32];
-      tmem_cols(lane_addr + TM_WS + half * 32, du);
+      float du[TOKEN_COLS];
+      tmem_cols(lane_addr + TM_WS + part * TOKEN_COLS, du);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint4 v = pack8(du + q * 8);
-        *reinterpret_cast<uint4*>(smem + OFF_UST + sw_off(128, row, half * 4 + q)) = v;
-        // the operand is -dU: flip the signs of the packed bf16 pairs
-        *reinterpret_cast<uint4*>(smem + OFF_UOP + sw_off(128, row, half * 4 + q)) =
-            make_uint4(v.x ^ 0x80008000u, v.y ^ 0x80008000u, v.z ^ 0x80008000u, v.w ^ 0x80008000u);
-      }
+      for (int e = 0; e < TOKEN_COLS; ++e) du[e] = -du[e];
+      uint32_t uk[TOKEN_COLS / 2];
+      tmem_put_bf16(lane_addr + TM_UOP + part * (TOKEN_COLS / 2), du, uk);
       warp_publish(u_ready);
+      if (keep) {
+#pragma unroll
+        for (int e = 0; e < TOKEN_COLS / 2; ++e) uk[e] ^= 0x80008000u;   // saved is dU, the operand -dU
+        smem_put_bf16<TOKEN_COLS>(smem + OFF_UOP, row, part, uk);
+        warp_publish_copy(u_copied);
+      }
     }
   } else if (warp == STATE_WARPS) {
-    if (elect_one()) {
-      const uint32_t sop = smem_u32(smem + OFF_SOP), uop = smem_u32(smem + OFF_UOP);
-      constexpr uint32_t i_mn64 = umma_idesc_bf16(128, 64, true, true), i_k64 = umma_idesc_bf16(128, 64, false, false);
-      constexpr uint32_t i_mn128 = umma_idesc_bf16(128, 128, true, true), i_k128 = umma_idesc_bf16(128, 128, false, false);
-      for (int it = 0; it < G.n; ++it) {
-        const int st = it & 1;
-        const uint32_t sst = smem_u32(smem + st * STAGE);
-        if (!mbar_wait(&full[st], (it >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
-        tc_fence_after();
-        // dU^T = dO^T Mq (the state warps have read the dU before it: they published -dU since)
+    const uint32_t leader = elect_one();
+    const uint32_t sop = tmem_base + TM_SOP, uop = tmem_base + TM_UOP;
+    constexpr uint32_t i_mn64 = umma_idesc_bf16(128, 64, true, true), i_k64 = umma_idesc_bf16(128, 64, false, false);
+    constexpr uint32_t i_mn128 = umma_idesc_bf16(128, 128, true, true), i_k128 = umma_idesc_bf16(128, 128, false, false);
+    for (int it = 0; it < steps; ++it) {
+      const int st = it & 1;
+      const uint32_t sst = smem_u32(smem + st * STAGE);
+      if (!mbar_wait(&full[st], (it >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
+      tc_fence_after();
+      // dU^T = dO^T Mq (the state warps have read the dU before it: they published -dU since)
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem_base + TM_WS, umma_smem_desc(sst + kk * 2048, 8192, 1024),
-                    umma_smem_desc(sst + 16384 + kk * 2048, 8192, 1024), i_mn64, kk != 0);
-        if (!mbar_wait(sop_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
-        //      + dS'^T Kd^T
+      for (int kk = 0; kk < 4; ++kk)
+        umma_bf16_if(leader, tmem_base + TM_WS, umma_smem_desc(sst + kk * 2048, 8192, 1024),
+                     umma_smem_desc(sst + 16384 + kk * 2048, 8192, 1024), i_mn64, kk != 0);
+      if (!mbar_wait(sop_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+      tc_fence_after();
+      //      + dS'^T Kd^T
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(tmem_base + TM_WS, umma_smem_desc(sop + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
-                    umma_smem_desc(sst + 24576 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), i_k64, 1);
-        umma_commit(du_done);
-        // dO^T Qg while the state warps form -dU
+      for (int kk = 0; kk < 8; ++kk)
+        umma_bf16_ts_if(leader, tmem_base + TM_WS, sop + kk * 8,
+                        umma_smem_desc(sst + 24576 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), i_k64, 1);
+      umma_commit_if(leader, du_done);
+      // dO^T Qg while the state warps form -dU (they have taken dS before they published dS')
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem_base + TM_DS, umma_smem_desc(sst + kk * 2048, 8192, 1024),
-                    umma_smem_desc(sst + 40960 + kk * 2048, 8192, 1024), i_mn128, kk != 0);
-        if (!mbar_wait(u_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
-        tc_fence_after();
+      for (int kk = 0; kk < 4; ++kk)
+        umma_bf16_if(leader, tmem_base + TM_DS, umma_smem_desc(sst + kk * 2048, 8192, 1024),
+                     umma_smem_desc(sst + 40960 + kk * 2048, 8192, 1024), i_mn128, kk != 0);
+      if (!mbar_wait(u_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+      tc_fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem_base + TM_DS, umma_smem_desc(uop + kk * 32, 16, 1024),
-                    umma_smem_desc(sst + 57344 + kk * 32, 16, 1024), i_k128, 1);
-        umma_commit(s_done);
-        umma_commit(&stage_free[st]);
-      }
+      for (int kk = 0; kk < 4; ++kk)
+        umma_bf16_ts_if(leader, tmem_base + TM_DS, uop + kk * 8, umma_smem_desc(sst + 57344 + kk * 32, 16, 1024), i_k128,
+                        1);
+      umma_commit_if(leader, s_done);
+      umma_commit_if(leader, &stage_free[st]);
     }
   } else if (elect_one()) {
     auto load_stage = [&](int it) {
-      const int c = G.n - 1 - it, st = it & 1;
+      const int c = c_top - it, st = it & 1;
       uint8_t* s = smem + st * STAGE;
       const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 64;
       mbar_expect_tx(&full[st], STAGE);
@@ -818,19 +924,22 @@ dn_bwd_state_kernel(const __grid_constant__ CUtensorMap tmDO, const __grid_const
       tma_load_2d(s + 57344, &tmWT, &full[st], hh * 64, prow);
     };
     load_stage(0);
-    if (G.n > 1) load_stage(1);
-    for (int it = 0; it < G.n; ++it) {
-      const int c = G.n - 1 - it;
-      if (!mbar_wait(sop_ready, it & 1, p.status, KS_TIMEOUT_FULL)) break;
+    if (steps > 1) load_stage(1);
+    for (int it = 0; it < steps; ++it) {
+      if (it >= skip) {
+        const int c = c_top - it;
+        if (!mbar_wait(s_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
-        tma_store_2d(&tmDSP, smem + OFF_SOP + b * 16384, b * 64, (c * G.H + h) * 128);
-      if (!mbar_wait(u_ready, it & 1, p.status, KS_TIMEOUT_FULL)) break;
-      tma_store_2d(&tmDUT, smem + OFF_UST, hh * 64, (c * G.NP + pr) * 128);
-      tma_store_commit();
-      tma_store_wait_read<0>();
-      mbar_arrive(saved);
-      if (it + 2 < G.n) {
+        for (int b = 0; b < 2; ++b)
+          tma_store_2d(&tmDSP, smem + OFF_SOP + b * 16384, b * 64, (c * G.H + h) * 128);
+        tma_store_commit();
+        if (!mbar_wait(u_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
+        tma_store_2d(&tmDUT, smem + OFF_UOP, hh * 64, (c * G.NP + pr) * 128);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(saved);
+      }
+      if (it + 2 < steps) {
         if (!mbar_wait(&stage_free[it & 1], (it >> 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
         load_stage(it + 2);
       }
@@ -839,7 +948,7 @@ dn_bwd_state_kernel(const __grid_constant__ CUtensorMap tmDO, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == STATE_WARPS) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
+  if (warp == STATE_WARPS) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
 // ============================================================================ backward, per chunk and head
@@ -1359,6 +1468,14 @@ static Geo make_geo(int T, int H, int Hk) {
   return g;
 }
 
+// Chunks per bucket of the walks. Four buckets per SM, so that runs of sequences as long as a head's share of the SMs
+// seldom fall into one bucket and are walked one after the other; a bucket without a run start costs about 2 us.
+static int walk_bucket(const Geo& g) {
+  const long long chunks = static_cast<long long>(g.n) * g.H, buckets = 4 * 148;
+  const long long b = (chunks + buckets - 1) / buckets;
+  return b < 1 ? 1 : static_cast<int>(b);
+}
+
 }  // namespace ss_dnc
 
 // ---------------------------------------------------------------------------- launchers
@@ -1410,7 +1527,7 @@ int ss_dn_prep(const void* q, const void* k, const void* v, const float* beta, c
 }
 
 int ss_dn_fwd(const void* WTp, const void* U0Tp, const void* QG, const void* KD, const void* MQ,
-              const float* gc, void* out, void* ST, void* UTp, int T, int H, int Hk, int* status,
+              const float* gc, const int* sid, void* out, void* ST, void* UTp, int T, int H, int Hk, int* status,
               void* stream) {
   if (T <= 0) return 0;
   if (H <= 0 || Hk <= 0 || H % Hk) return -2;
@@ -1429,17 +1546,17 @@ int ss_dn_fwd(const void* WTp, const void* U0Tp, const void* QG, const void* KD,
   if ((r = ss::make_tmap_bf16(&to, out, T, (long long)H * D, (long long)H * D, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tut, save ? UTp : WTp, prow, 128, 128, 128))) return r;
   WalkParams p;
-  p.gc = gc; p.save = save;
+  p.gc = gc; p.sid = sid; p.bucket = walk_bucket(geo); p.save = save;
   p.geo = geo; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_fwd_kernel, walk::SMEM)) return e;
-  dn_fwd_kernel<<<H, walk::FWD_THREADS, walk::SMEM, (cudaStream_t)stream>>>(twt, tu0, tqg, tkd, tmq, tst, tut, to,
-                                                                            p);
+  dn_fwd_kernel<<<dim3(H, (geo.n + p.bucket - 1) / p.bucket), walk::FWD_THREADS, walk::SMEM, (cudaStream_t)stream>>>(
+      twt, tu0, tqg, tkd, tmq, tst, tut, to, p);
   return (int)cudaGetLastError();
 }
 
 int ss_dn_bwd_state(const void* dout, const void* MQ, const void* KD, const void* QG, const void* WTp,
-                    const float* gc, void* dSpT, void* dUTp, int T, int H, int Hk, int* status,
+                    const float* gc, const int* sid, void* dSpT, void* dUTp, int T, int H, int Hk, int* status,
                     void* stream) {
   if (T <= 0) return 0;
   if (H <= 0 || Hk <= 0 || H % Hk) return -2;
@@ -1455,11 +1572,11 @@ int ss_dn_bwd_state(const void* dout, const void* MQ, const void* KD, const void
   if ((r = ss::make_tmap_bf16(&tdsp, dSpT, (long long)geo.n * H * 128, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tdut, dUTp, prow, 128, 128, 128))) return r;
   WalkParams p;
-  p.gc = gc; p.save = 1; p.geo = geo; p.status = status;
+  p.gc = gc; p.sid = sid; p.bucket = walk_bucket(geo); p.save = 1; p.geo = geo; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_bwd_state_kernel, walk::SMEM)) return e;
-  dn_bwd_state_kernel<<<H, walk::BWD_THREADS, walk::SMEM, (cudaStream_t)stream>>>(tdo, tmq, tkd, tqg, twt, tdsp, tdut,
-                                                                                  p);
+  dn_bwd_state_kernel<<<dim3(H, (geo.n + p.bucket - 1) / p.bucket), walk::BWD_THREADS, walk::SMEM,
+                        (cudaStream_t)stream>>>(tdo, tmq, tkd, tqg, twt, tdsp, tdut, p);
   return (int)cudaGetLastError();
 }
 

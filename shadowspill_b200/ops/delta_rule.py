@@ -19,8 +19,8 @@ _c = _lib
 _P = _c.c_p
 _lib.register("ss_dn_seq_ids", [_P, _c.c_int, _c.c_int, _P, _P])
 _lib.register("ss_dn_prep", [_P] * 16 + [_c.c_int] * 3 + [_c.c_f, _P, _P])
-_lib.register("ss_dn_fwd", [_P] * 9 + [_c.c_int] * 3 + [_P, _P])
-_lib.register("ss_dn_bwd_state", [_P] * 8 + [_c.c_int] * 3 + [_P, _P])
+_lib.register("ss_dn_fwd", [_P] * 10 + [_c.c_int] * 3 + [_P, _P])
+_lib.register("ss_dn_bwd_state", [_P] * 9 + [_c.c_int] * 3 + [_P, _P])
 _lib.register("ss_dn_bwd_chunk", [_P] * 10 + [_c.c_int] * 3 + [_P, _P])
 _lib.register("ss_dn_bwd_prep", [_P] * 21 + [_c.c_int] * 3 + [_c.c_f, _P, _P])
 
@@ -107,7 +107,7 @@ def _forward(q, k, v, beta, g, cu_seqlens, backward: bool):
                             B.gam.data_ptr(), B.gc.data_ptr(), T, H, Hk, scale, status, st), "ss_dn_prep")
     out = torch.empty((T, H, WIDTH), dtype=torch.bfloat16, device=q.device)
     _lib.check(L.ss_dn_fwd(B.WTp.data_ptr(), B.U0Tp.data_ptr(), B.QG.data_ptr(), B.KD.data_ptr(),
-                           B.MQ.data_ptr(), B.gc.data_ptr(), out.data_ptr(), _ptr(B.ST), _ptr(B.UTp),
+                           B.MQ.data_ptr(), B.gc.data_ptr(), B.sid.data_ptr(), out.data_ptr(), _ptr(B.ST), _ptr(B.UTp),
                            T, H, Hk, status, st), "ss_dn_fwd")
     return out, B, geo
 
@@ -193,7 +193,7 @@ def _backward_all(q, k, v, beta, g, cu_seqlens, dout):
     T, H, Hk = geo.T, geo.H, geo.Hk
     L, st, status = _lib.lib(), _lib.stream_ptr(), _lib.status_ptr(q)
     _lib.check(L.ss_dn_bwd_state(dout.data_ptr(), B.MQ.data_ptr(), B.KD.data_ptr(), B.QG.data_ptr(),
-                                 B.WTp.data_ptr(), B.gc.data_ptr(), B.dSpT.data_ptr(), B.dUTp.data_ptr(),
+                                 B.WTp.data_ptr(), B.gc.data_ptr(), B.sid.data_ptr(), B.dSpT.data_ptr(), B.dUTp.data_ptr(),
                                  T, H, Hk, status, st), "ss_dn_bwd_state")
     _lib.check(L.ss_dn_bwd_chunk(B.dSpT.data_ptr(), B.ST.data_ptr(), B.UTp.data_ptr(), B.dUTp.data_ptr(),
                                  dout.data_ptr(), B.dKdTp.data_ptr(), B.dQgTp.data_ptr(),

@@ -198,11 +198,12 @@ def bench_deltanet(a) -> list[dict]:
                                       B.XU.data_ptr(), B.gam.data_ptr(), B.gc.data_ptr(), T, H, Hk,
                                       128 ** -0.5, status, st),
         "state_walk": lambda: L_.ss_dn_fwd(B.WTp.data_ptr(), B.U0Tp.data_ptr(), B.QG.data_ptr(), B.KD.data_ptr(),
-                                           B.MQ.data_ptr(), B.gc.data_ptr(), o.data_ptr(), B.ST.data_ptr(),
-                                           B.UTp.data_ptr(), T, H, Hk, status, st),
+                                           B.MQ.data_ptr(), B.gc.data_ptr(), B.sid.data_ptr(), o.data_ptr(),
+                                           B.ST.data_ptr(), B.UTp.data_ptr(), T, H, Hk, status, st),
         "bwd_state_walk": lambda: L_.ss_dn_bwd_state(dout.data_ptr(), B.MQ.data_ptr(), B.KD.data_ptr(),
                                                      B.QG.data_ptr(), B.WTp.data_ptr(), B.gc.data_ptr(),
-                                                     B.dSpT.data_ptr(), B.dUTp.data_ptr(), T, H, Hk, status, st),
+                                                     B.sid.data_ptr(), B.dSpT.data_ptr(), B.dUTp.data_ptr(), T, H, Hk,
+                                                     status, st),
         "bwd_chunk": lambda: L_.ss_dn_bwd_chunk(B.dSpT.data_ptr(), B.ST.data_ptr(), B.UTp.data_ptr(),
                                                 B.dUTp.data_ptr(), dout.data_ptr(), B.dKdTp.data_ptr(),
                                                 B.dQgTp.data_ptr(), B.dWTp.data_ptr(), B.dMQ.data_ptr(),

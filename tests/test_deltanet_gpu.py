@@ -167,6 +167,29 @@ def test_delta_rule_kernels_at_the_model_head_counts():
         assert _rel(x.grad, y.grad) < 3e-2, name
 
 
+@pytest.mark.parametrize("T,Hk,Hv,bounds", [
+    (64 * 40, 1, 1, [0, 64 * 7, 64 * 7 + 1, 64 * 8, 64 * 9 - 1, 64 * 9, 1500, 64 * 33 + 5, 64 * 40]),   # a bucket a chunk
+    (64 * 61 + 3, 16, 32, [0, 100, 130, 64 * 20, 64 * 21 + 9, 64 * 50, 64 * 61, 64 * 61 + 3]),          # four chunks each
+    (40, 2, 4, [0, 13, 40]), (64 * 30, 2, 6, [0, 64 * 30]),
+])
+def test_walks_split_into_runs_give_the_whole_rule(T, Hk, Hv, bounds):
+    """Sequences that begin on and off chunk edges, several in a chunk, chunks without a boundary between runs and
+    batches of one sequence, against the PyTorch chunked form (bf16 operands, as above)."""
+    from shadowspill_b200.ops import _lib
+    q, k, v, beta, gl, dout, cu = _delta_case(T, Hk, Hv, bounds, seed=T)
+    a = [t.clone().cuda().requires_grad_(True) for t in (q, k, v, beta, gl)]
+    b = [t.clone().cuda().float().requires_grad_(True) for t in (q, k, v, beta, gl)]
+    got = seq.gated_delta_rule_chunked(*a, None, 64, cu_seqlens=cu.cuda())
+    want = seq._gated_delta_rule_torch(*b, None, 64, cu_seqlens=cu.cuda())
+    got.backward(dout.cuda())
+    want.backward(dout.cuda().float())
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert _rel(got, want) < 1.5e-2
+    for name, x, y in zip("q k v beta g".split(), a, b):
+        assert _rel(x.grad, y.grad) < 3e-2, name
+
+
 @pytest.mark.gpu
 def test_head_groups_compute_the_same_rule_in_pieces():
     """Running the rule in groups of key heads (less intermediate memory) gives the same output
