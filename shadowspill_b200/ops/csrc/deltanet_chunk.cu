@@ -18,8 +18,7 @@
 //
 // Kernels (dk = dv = 128; QK heads are shared by `rep` V heads, handled two V heads at a time):
 //   dn_prep_kernel   per (chunk, pair of V heads): K K^T and Q K^T on the tensor cores, the
-//                    64x64 triangular inverse by forward substitution in registers (one column
-//                    per thread), then W^T and U0^T as MMAs; writes every per-chunk operand.
+//                    64x64 triangular inverse in blocks, then W^T and U0^T as MMAs; writes every per-chunk operand.
 //   dn_fwd_kernel    per V head, sequential over chunks: the state S^T lives in registers (fp32);
 //                    U^T = U0^T - S^T W^T, O^T = S^T Qg^T + U^T Mq^T, S'^T = Gc S^T + U^T Kd.
 //   dn_bwd_state_kernel   the same walk in reverse for dS and dU.
@@ -98,10 +97,6 @@ __device__ __forceinline__ void store_row64(__nv_bfloat16* dst, const float* f) 
 #pragma unroll
   for (int q = 0; q < 8; ++q) reinterpret_cast<uint4*>(dst)[q] = pack8(f + q * 8);
 }
-__device__ __forceinline__ void load_row64(const __nv_bfloat16* src, float* f) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q) unpack8(reinterpret_cast<const uint4*>(src)[q], f + q * 8);
-}
 // Sums of N values per lane over the warp's lanes (each step hands half of the remaining columns to the
 // partner lane; through shared memory it was N stores and a chain of dependent loads per sum), written to
 // out[0..N). The values are consumed.
@@ -126,29 +121,15 @@ __device__ __forceinline__ void warp_col_sums(float (&v)[N], float* out) {
   else if ((lane & 1) == 0) out[lane >> 1] = v[0];
 }
 __device__ __forceinline__ void row_threads_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void all_rows_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// exp(x) where `on`, else 0, without a branch: a choice between an exponential and 0 became one per element, which
+// diverged in every warp that holds a diagonal.
+__device__ __forceinline__ float decay_if(bool on, float x) { return __expf(on ? x : -INFINITY); }
 // The first chunk position of each token's sequence: `starts` has a bit where a sequence begins.
 __device__ __forceinline__ int seq_begin(const unsigned* starts, int t) {
   const unsigned long long m = (static_cast<unsigned long long>(starts[1]) << 32) | starts[0];
   return 63 - __clzll(static_cast<long long>(m & (~0ull >> (63 - t))));
 }
-// 64 tokens of one feature per row thread -> token rows of 128 features, through a 16 KiB tile: two-byte
-// stores of 64 bytes per warp took several times longer. Called by the 128 row threads; `tile` is free
-// to be written, and again after the call's end only behind another row_threads_sync.
-__device__ __forceinline__ void store_tokens(const float (&v)[64], uint8_t* tile, __nv_bfloat16* dst, long long ld,
-                                             int lim) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int t = 0; t < 64; ++t)
-    *reinterpret_cast<__nv_bfloat16*>(tile + t * 256 + tid * 2) = __float2bfloat16_rn(v[t]);
-  row_threads_sync();
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int t = q * 8 + (tid >> 4), c = tid & 15;
-    if (t < lim)
-      *reinterpret_cast<uint4*>(dst + t * ld + c * 8) = *reinterpret_cast<const uint4*>(tile + t * 256 + c * 16);
-  }
-}
-
 // ============================================================================ sequence ids
 __global__ void dn_seq_ids_kernel(const int* __restrict__ cu, int nseq, int T, int Tp,
                                   int* __restrict__ sid) {
@@ -166,7 +147,7 @@ __global__ void dn_seq_ids_kernel(const int* __restrict__ cu, int nseq, int T, i
 // ============================================================================ prep (forward)
 struct PrepParams {
   const float* beta; const float* g; const int* sid;
-  __nv_bfloat16 *MQ, *TMT;         // TMT: null unless a backward follows
+  __nv_bfloat16* TMT;              // null unless a backward follows
   int save;                        // a backward follows: keep the inverse and its two scaled forms
   float *gam, *gc;
   Geo geo; float scale; int* status;
@@ -176,18 +157,113 @@ namespace prep {
 // fit an SM, and one's substitution runs under the other's loads and stores.
 constexpr int AP = 68;                                  // pitch of A: rows 16-byte aligned for float4 reads
 constexpr int OFF_KQ = 0, OFF_V = 32768, OFF_XW = 65536, OFF_XU = 81920, OFF_AF = 65536;
-constexpr int OFF_MISC = OFF_AF + 2 * 64 * AP * 4;      // 100352
+constexpr int OFF_MQ = OFF_AF + 36864;                  // 8 KiB: Mq of a head on its way out
+constexpr int OFF_MISC = OFF_MQ + 8192;
+static_assert(2 * 64 * AP * 4 <= 36864, "A runs into the next tile");
 constexpr int OFF_BAR = OFF_MISC + 2048;
 constexpr int SMEM = OFF_BAR + 64 + 1024;
 static_assert(2 * (SMEM + 1024) <= 233472, "two CTAs per SM");
 }
 
+// (I + A)^-1 over A, 64 x 64 strictly lower triangular (fp32, pitch AP), by the 64 threads of one head (two warps),
+// j = 0..63; what lies above the diagonal 16 x 16 blocks is scratch. The diagonal blocks by forward substitution, a
+// column per thread, then twice [[P, 0], [-Q B P, Q]] from the inverses P and Q of two neighbouring blocks and the block
+// B between them. Substitution in one piece was a chain of 64 steps in 2,000 straight-line multiplications, and
+// fetching those took as long as running them.
+__device__ __forceinline__ void head_sync(int tid) {
+  if (tid < 64) asm volatile("bar.sync 2, 64;" ::: "memory");
+  else asm volatile("bar.sync 3, 64;" ::: "memory");
+}
+
+__device__ __forceinline__ void fma_row(float (&acc)[4], float a, const float4& b) {
+  acc[0] += a * b.x; acc[1] += a * b.y; acc[2] += a * b.z; acc[3] += a * b.w;
+}
+// acc[R][4] = rows r0.. of L (columns k0..k1 of it) times columns c0..c0+3 of M
+template <int R>
+__device__ __forceinline__ void block_product(float (&acc)[R][4], const float* L, const float* M, int k0, int k1) {
+  using prep::AP;
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+#pragma unroll 1
+  for (int k = k0; k < k1; k += 4) {
+    float4 l[R], m[4];
+#pragma unroll
+    for (int r = 0; r < R; ++r) l[r] = *reinterpret_cast<const float4*>(L + r * AP + k);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) m[x] = *reinterpret_cast<const float4*>(M + (k + x) * AP);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      fma_row(acc[r], l[r].x, m[0]);
+      fma_row(acc[r], l[r].y, m[1]);
+      fma_row(acc[r], l[r].z, m[2]);
+      fma_row(acc[r], l[r].w, m[3]);
+    }
+  }
+}
+
+__device__ __forceinline__ void unit_lower_inverse(float* A, int j) {
+  using prep::AP;
+  {
+    float* D = A + (j & ~15) * (AP + 1);
+    const int jj = j & 15;
+    float x[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      float a[4] = {t == jj ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < t; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(D + t * AP + i);
+        a[0] -= v.x * x[i];
+        if (i + 1 < t) a[1] -= v.y * x[i + 1];
+        if (i + 2 < t) a[2] -= v.z * x[i + 2];
+        if (i + 3 < t) a[3] -= v.w * x[i + 3];
+      }
+      x[t] = (a[0] + a[1]) + (a[2] + a[3]);
+    }
+    __syncwarp();                                  // a warp holds both blocks whose columns it has read
+#pragma unroll
+    for (int t = 0; t < 16; ++t) D[t * AP + jj] = x[t];
+    __syncwarp();
+  }
+  {                                                // 16 -> 32: one pair of blocks per warp, 2 x 4 values per thread
+    float* B0 = A + (j & 32) * (AP + 1);
+    const int r0 = (j & 31) >> 2 << 1, c0 = (j & 3) * 4;
+    float v[2][4];
+    block_product<2>(v, B0 + (16 + r0) * AP, B0 + c0, 0, 16);                     // B P
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      *reinterpret_cast<float4*>(B0 + (r0 + r) * AP + 16 + c0) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+    __syncwarp();
+    block_product<2>(v, B0 + (16 + r0) * AP + 16, B0 + 16 + c0, 0, 16);           // Q (B P)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      *reinterpret_cast<float4*>(B0 + (16 + r0 + r) * AP + c0) = make_float4(-v[r][0], -v[r][1], -v[r][2], -v[r][3]);
+  }
+  head_sync(threadIdx.x);
+  {                                                // 32 -> 64: 4 x 4 values per thread, zero blocks left out
+    const int r0 = (j >> 3) * 4, c0 = (j & 7) * 4;
+    float v[4][4];
+    block_product<4>(v, A + (32 + r0) * AP, A + c0, c0 & 16, 32);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      *reinterpret_cast<float4*>(A + (r0 + r) * AP + 32 + c0) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+    head_sync(threadIdx.x);
+    block_product<4>(v, A + (32 + r0) * AP + 32, A + 32 + c0, 0, (r0 & 16) + 16);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      *reinterpret_cast<float4*>(A + (32 + r0 + r) * AP + c0) = make_float4(-v[r][0], -v[r][1], -v[r][2], -v[r][3]);
+  }
+}
+
+// Bound by latency: two CTAs an SM, each with one warp to a scheduler. 8,192 tokens, 16 / 32 heads: 0.199 -> 0.146 ms
+// (436 MB, 0.067 ms at the copy bandwidth) with the inverse in blocks, the scalars' loads ahead of the set-up, no
+// branch around an exponential and Mq through a tile.
 __global__ void __launch_bounds__(THREADS, 2)
 dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmWT,
                const __grid_constant__ CUtensorMap tmU0T, const __grid_constant__ CUtensorMap tmQG,
-               const __grid_constant__ CUtensorMap tmKD, const __grid_constant__ CUtensorMap tmXW,
-               const __grid_constant__ CUtensorMap tmXU, const PrepParams p) {
+               const __grid_constant__ CUtensorMap tmKD, const __grid_constant__ CUtensorMap tmMQ,
+               const __grid_constant__ CUtensorMap tmXW, const __grid_constant__ CUtensorMap tmXU, const PrepParams p) {
   using namespace prep;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
@@ -201,22 +277,25 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Geo G = p.geo;
   const int c = blockIdx.x, pr = blockIdx.y;
   const int kh = pr / G.P, z = pr % G.P, h0 = kh * G.rep + 2 * z;
   const int nh = (2 * z + 1 < G.rep) ? 2 : 1;
   const int t0 = c * CH;
 
-  if (tid == 0) { mbar_init(tma_bar, 1); mbar_init(mma_bar, 1); mbar_fence_init(); }
-  if (warp == 4) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  // the chunk's scalars, asked for ahead of all else: a memory latency that the set-up runs under
+  float gam = 0.f, beta = 0.f;                           // log decay of the token, later its running sum
+  int sid = -1;
+  if (tid < 128 && (tid >> 6) < nh && t0 + (tid & 63) < G.T) {
+    const long long at = static_cast<long long>(t0 + (tid & 63)) * G.H + h0 + (tid >> 6);
+    gam = p.g[at];
+    beta = p.beta[at];
+  }
+  if (tid < 64 || (tid == 64 && c > 0)) sid = p.sid[tid < 64 ? t0 + tid : t0 - 1];
 
   if (tid == CTRL) {
+    mbar_init(tma_bar, 1); mbar_init(mma_bar, 1); mbar_fence_init();
     mbar_expect_tx(tma_bar, 32768 + nh * 16384);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
@@ -228,24 +307,33 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       for (int b = 0; b < 2; ++b)
         tma_load_2d(smem + OFF_V + hh * 16384 + b * 8192, &tmV, tma_bar, (h0 + hh) * D + b * 64, t0);
   }
+  if (warp == 4) { __syncwarp(); tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+
+  if (tid < 128) beta_s[tid] = beta;
+  if (tid < 65) sid_s[tid] = sid;
   if (tid < 128) {
-    const int hh = tid >> 6, j = tid & 63, tok = t0 + j;
-    const bool live = hh < nh && tok < G.T;
-    g_s[tid] = live ? p.g[static_cast<long long>(tok) * G.H + h0 + hh] : 0.f;
-    beta_s[tid] = live ? p.beta[static_cast<long long>(tok) * G.H + h0 + hh] : 0.f;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float before = __shfl_up_sync(0xffffffffu, gam, o);
+      if (lane >= o) gam += before;
+    }
+    if (lane == 31) g_s[warp] = gam;
   }
-  if (tid < 65) sid_s[tid] = tid < 64 ? p.sid[t0 + tid] : (c > 0 ? p.sid[t0 - 1] : -1);
   __syncthreads();
   if (tid < 64) {
     const unsigned m = __ballot_sync(0xffffffffu, tid == 0 || sid_s[tid] != sid_s[tid - 1]);
-    if ((tid & 31) == 0) starts_s[warp] = m;
+    if (lane == 0) starts_s[warp] = m;
   }
   if (tid < 128) {
     const int hh = tid >> 6, j = tid & 63;
-    float s = 0.f;
-    for (int i = 0; i <= j; ++i) s += g_s[hh * 64 + i];
-    gam_s[tid] = s;
-    if (hh < nh) p.gam[(static_cast<long long>(c) * G.H + h0 + hh) * 64 + j] = s;
+    if (j >= 32) gam += g_s[warp - 1];
+    gam_s[tid] = gam;
+    if (hh < nh) p.gam[(static_cast<long long>(c) * G.H + h0 + hh) * 64 + j] = gam;
   }
   __syncthreads();
 
@@ -266,60 +354,69 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   mbar_wait(mma_bar, 0, p.status, KS_TIMEOUT_TMEM_FULL);
   tc_fence_after();
 
-  // ---- A (fp32, shared memory) and Mq (global): a row's decays are read into registers first, so that no
-  // store stands between the loads
+  // ---- A (fp32; only below the diagonal) and Mq, eight columns at a time: a body of more instructions than the
+  // first instruction cache holds ran at a tenth of the issue rate
   if (tid < 128) {
-    const int t = tid & 63;
-    float row[64];
-    tmem_row64(lane_addr, row);
+    const int t = tid & 63, last = t | 31;               // the warp's last row
     const int lo = seq_begin(starts_s, t);
     const bool is_q = tid >= 64;
+    const int hi = is_q ? t : t - 1;                     // Mq includes the diagonal, A does not
 #pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
       const float gt = gam_s[hh * 64 + t], f = is_q ? p.scale : beta_s[hh * 64 + t];
-      const int hi = is_q ? t : t - 1;                   // Mq includes the diagonal, A does not
       float* a = Af + (hh * 64 + t) * AP;
-      __nv_bfloat16* mq = p.MQ + ((static_cast<long long>(c) * G.NP + pr) * 128 + hh * 64 + t) * 64;
-#pragma unroll
+      if (is_q && hh > 0) {                              // the head before has left the tile
+        if (tid == 64) tma_store_wait_read<0>();
+        head_sync(64);
+      }
+#pragma unroll 1
       for (int i0 = 0; i0 < 64; i0 += 8) {
         float m[8];
-        *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0);
-        *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0 + 4);
+        if (i0 > last) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          m[e] = i0 + e >= lo && i0 + e <= hi ? f * __expf(gt - m[e]) * row[i0 + e] : 0.f;
+          for (int e = 0; e < 8; ++e) m[e] = 0.f;
+        } else {
+          uint32_t r[8];
+          tmem_ld_32x8(lane_addr + i0, r);
+          *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0);
+          *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0 + 4);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const bool seen = i0 + e >= lo && i0 + e <= hi;
+            const float v = f * decay_if(seen, gt - m[e]) * __uint_as_float(r[e]);
+            m[e] = seen ? v : 0.f;
+          }
+        }
         if (is_q) {
-          *reinterpret_cast<uint4*>(mq + i0) = pack8(m);
+          *reinterpret_cast<uint4*>(smem + OFF_MQ + sw_off(64, t, i0 >> 3)) = pack8(m);
         } else {
           *reinterpret_cast<float4*>(a + i0) = *reinterpret_cast<const float4*>(m);
           *reinterpret_cast<float4*>(a + i0 + 4) = *reinterpret_cast<const float4*>(m + 4);
+        }
+      }
+      if (is_q) {
+        fence_async_proxy();
+        head_sync(64);
+        if (tid == 64) {
+          tma_store_2d(&tmMQ, smem + OFF_MQ, 0, (c * G.NP + pr) * 128 + hh * 64);
+          tma_store_commit();
         }
       }
     }
   }
   __syncthreads();
 
-  // ---- Tm = (I + A)^-1: thread (hh, j) owns column j
+  // ---- Tm = (I + A)^-1; thread (hh, j) takes its column j
   if (tid < 128) {
     const int hh = tid >> 6, j = tid & 63;
     float col[64];
+    if (hh < nh) unit_lower_inverse(Af + hh * 64 * AP, j);
+    row_threads_sync();
     if (hh < nh) {
-      const float* A = Af + hh * 64 * AP;
+      const float* at = Af + hh * 64 * AP + j;
 #pragma unroll
-      for (int t = 0; t < 64; ++t) {
-        float a0 = (t == j) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-        const float4* ar = reinterpret_cast<const float4*>(A + t * AP);
-        // row t is zero from column t on, so whole groups of four may be read past t - 1
-#pragma unroll
-        for (int i = 0; i < t; i += 4) {
-          const float4 v = ar[i >> 2];
-          a0 -= v.x * col[i];
-          if (i + 1 < t) a1 -= v.y * col[i + 1];
-          if (i + 2 < t) a2 -= v.z * col[i + 2];
-          if (i + 3 < t) a3 -= v.w * col[i + 3];
-        }
-        col[t] = (a0 + a1) + (a2 + a3);
-      }
+      for (int t = 0; t < 64; ++t) col[t] = t >= j ? at[t * AP] : 0.f;
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");      // A has been read: its region takes the operands
     if (hh < nh) {
@@ -443,7 +540,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     publish();
     if (tid == CTRL) store_kq(smem + OFF_V, 0);
   }
-  if (tid == CTRL) tma_store_wait<0>();
+  if (tid == CTRL || tid == 64) tma_store_wait<0>();
   tc_fence_before();
   __syncthreads();
   if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
@@ -957,12 +1054,17 @@ struct ChunkParams {
   Geo geo; int* status;
 };
 namespace chunkk {
-constexpr int OFF_DSP = 0, OFF_ST = 32768, OFF_UT = 65536, OFF_DUT = 81920, OFF_DO = 98304;
-constexpr int OFF_RED = 131072, OFF_BAR = OFF_RED + 64;
-constexpr int SMEM = OFF_BAR + 64 + 1024;
+// dO comes first: as the A operand of dMq it has 64 of 128 rows, and the products read what lies behind it as the
+// others, whose results nothing takes. The operands fill half of an SM's shared memory to within 1 KiB, so that two
+// CTAs fit and one's products and stores run under the other's loads (alone: 10,000 cycles a CTA, 6,200 of them
+// waiting for its operands; 0.177 -> 0.114 ms at 8,192 tokens, 32 V heads: 0.70 GB, 0.107 ms at the copy bandwidth).
+constexpr int OFF_DO = 0, OFF_DSP = 16384, OFF_ST = 49152, OFF_UT = 81920, OFF_DUT = 98304;
+constexpr int OFF_RED = 114688, OFF_BAR = OFF_RED + 64, ALIGN_SLACK = 768;
+constexpr int SMEM = OFF_BAR + 64 + ALIGN_SLACK;
+static_assert(2 * (SMEM + 1024) <= 233472, "two CTAs per SM");
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(THREADS, 2)
 dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_constant__ CUtensorMap tmST,
                     const __grid_constant__ CUtensorMap tmUT, const __grid_constant__ CUtensorMap tmDUT,
                     const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmDKD,
@@ -971,6 +1073,10 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
   using namespace chunkk;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
+  if (smem - smem_raw > ALIGN_SLACK) {             // dynamic shared memory starts on 1 KiB: there is no room if it did not
+    report(p.status, KS_BAD_ARGUMENT);
+    return;
+  }
   float* red = reinterpret_cast<float*>(smem + OFF_RED);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
@@ -991,12 +1097,12 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
 
   if (tid == CTRL) {
     const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 128;
-    mbar_expect_tx(tma_bar, 131072);
+    mbar_expect_tx(tma_bar, 114688);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       tma_load_2d(smem + OFF_DSP + b * 16384, &tmDSP, tma_bar, b * 64, hrow);
       tma_load_2d(smem + OFF_ST + b * 16384, &tmST, tma_bar, b * 64, hrow);
-      tma_load_2d(smem + OFF_DO + b * 16384, &tmDO, tma_bar, h * D + b * 64, c * CH);
+      tma_load_2d(smem + OFF_DO + b * 8192, &tmDO, tma_bar, h * D + b * 64, c * CH);
     }
     tma_load_2d(smem + OFF_UT, &tmUT, tma_bar, hh * 64, prow);
     tma_load_2d(smem + OFF_DUT, &tmDUT, tma_bar, hh * 64, prow);
@@ -1014,11 +1120,11 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
       const uint64_t a_st = umma_smem_desc(sst + kk * 2048, 16384, 1024);
       const uint64_t b_ut = umma_smem_desc(sut + kk * 2048, 16384, 1024);
       const uint64_t b_dut = umma_smem_desc(sdut + kk * 2048, 16384, 1024);
-      const uint64_t k_do = umma_smem_desc(sdo + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
+      const uint64_t k_do = umma_smem_desc(sdo + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024);
       umma_bf16(tmem_base, a_dsp, b_ut, i_mm, kk != 0);          // dKd^T = dS' U^T
       umma_bf16(tmem_base + 64, a_st, k_do, i_mk, kk != 0);      // dQg^T = S dO^T
       umma_bf16(tmem_base + 128, a_st, b_dut, i_mm, kk != 0);    // (S dU^T), negated below
-      umma_bf16(tmem_base + 192, k_do, b_ut, i_km, kk != 0);     // dMq = dO U^T (rows 0..63)
+      umma_bf16(tmem_base + 192, k_do, b_ut, i_km, kk != 0);     // dMq = dO U^T (rows 0..63; the tile has no others)
     }
     umma_commit(mma_bar);
   }
@@ -1041,9 +1147,8 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
   if (tid == 0) p.dgc[static_cast<long long>(c) * G.H + h] = (red[0] + red[1]) + (red[2] + red[3]);
   mbar_wait(mma_bar, 0, p.status, KS_TIMEOUT_TMEM_FULL);
   tc_fence_after();
-  // The results leave by TMA from tiles over the operands (all of them have been read). Bound by the
-  // latency of one block per chunk and head: rows stored by their own threads touch 32 lines a
-  // store; through shared memory 192 -> 179 us at 8192 tokens, 32 V heads.
+  // The results leave by TMA from tiles over the operands (all of them have been read): rows stored by their own
+  // threads touch 32 lines a store.
   if (tid < 128) {
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
@@ -1083,12 +1188,16 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
 // ============================================================================ backward of the chunk-local algebra
 struct BwdPrepParams {
   const float* beta; const int* sid; const float* gam; const float* gc; const float* dgc;
-  const __nv_bfloat16 *dKdTp, *dQgTp, *dMQ;
+  const __nv_bfloat16* dMQ;
   __nv_bfloat16 *dq, *dk, *dv;     // dq, dk: [T, NP, D] (summed over pairs by the caller); dv [T, H, D]
   float *dbeta, *dg;               // [T, H]
   Geo geo; float scale; int* status;
 };
+// Eight row warps, two to each quarter of the TMEM lanes: a thread has half the columns of its row. One CTA an SM, so its
+// chain of loads, products and row work is all there is: 44,000 -> 34,000 cycles, 0.373 -> 0.264 ms at 8,192 tokens
+// and 16 / 32 heads, with the tokens' dot products on the tensor cores, dKd and dQg by TMA and twice the warps.
 namespace bprep {
+constexpr int ROW_THREADS = 256, BTHREADS = ROW_THREADS + 32, BCTRL = ROW_THREADS;
 constexpr int OFF_KQ = 0, OFF_TMT = 32768, OFF_V = 49152, OFF_DWT = 81920, OFF_DUT = 114688;
 constexpr int OFF_XW = 147456, OFF_XU = 163840;
 // after the first group of MMAs the range [OFF_V, OFF_XU + 16384) is reused:
@@ -1096,8 +1205,9 @@ constexpr int OFF_KKF = 49152, OFF_QKF = OFF_KKF + 16640;          // fp32 [64][
 constexpr int OFF_DTM = 82944, OFF_XOP = OFF_DTM + 16384;          // operands
 constexpr int OFF_SYM = OFF_XOP + 16384, OFF_DQK = OFF_SYM + 8192;
 constexpr int OFF_KKA = OFF_DQK + 8192, OFF_QKA = OFF_KKA + 16640;  // fp32 accumulators over heads
-constexpr int OFF_OUT = OFF_DTM;                                   // 16 KiB tile of the output transposes
-constexpr int OFF_MISC = OFF_XU + 16384;                           // 180224
+constexpr int OFF_OUT = OFF_KKF;                                   // 16 KiB tile of the output transposes
+constexpr int OFF_DKD = OFF_XU + 16384, OFF_DQG = OFF_DTM;         // dKd^T and dQg^T of both heads, 32 KiB each
+constexpr int OFF_MISC = OFF_DKD + 32768;
 constexpr int OFF_BAR = OFF_MISC + 10240;
 static_assert(OFF_QKA + 16640 <= OFF_MISC, "scratch overlaps the per-token values");
 constexpr int SMEM = OFF_BAR + 64 + 1024;
@@ -1105,11 +1215,12 @@ static_assert(OFF_KKF >= OFF_TMT + 16384, "scratch overlaps a tile that stays li
 static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(bprep::BTHREADS, 1)
 dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDWT,
                    const __grid_constant__ CUtensorMap tmDUT, const __grid_constant__ CUtensorMap tmTMT,
                    const __grid_constant__ CUtensorMap tmXW, const __grid_constant__ CUtensorMap tmXU,
+                   const __grid_constant__ CUtensorMap tmDKD, const __grid_constant__ CUtensorMap tmDQG,
                    const BwdPrepParams p) {
   using namespace bprep;
   extern __shared__ uint8_t smem_raw[];
@@ -1123,20 +1234,22 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   float* beta_s = misc + 128;
   float* gt_s = misc + 256;       // exp(gam) [continues the previous chunk's sequence]
   float* d_s = misc + 384;        // exp(gam_63 - gam) [same sequence as the chunk's end]
-  // column sums, one part per row warp: [4][64]; of the two heads' dot products: [2][4][64]
+  // column sums, one part per row warp: [4][64]
   float* cs1 = misc + 512;
   float* cs2 = misc + 768;
   float* colG = misc + 1024;
-  float* dotq = misc + 1280;
-  float* dotk = misc + 1792;
-  float* dgam_s = misc + 2304;
+  float* dotq = misc + 1280;      // [2][64] a token's <dQg, Q> and <dKd, K>
+  float* dotk = misc + 1408;
+  float* sums_s = misc + 1536;    // [2][4] warp sums of the last step
+  float* rows_s = misc + 1552;    // [2][128] the right halves' parts of two row sums
   int* sid_s = reinterpret_cast<int*>(misc + 2432);     // [65]
   unsigned* starts_s = reinterpret_cast<unsigned*>(misc + 2500);   // [2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
+  uint64_t* dkd_bar = bars + 2; uint64_t* dqg_bar = bars + 3;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Geo G = p.geo;
   const int c = blockIdx.x, pr = blockIdx.y;
   const int kh = pr / G.P, z = pr % G.P, h0 = kh * G.rep + 2 * z;
@@ -1144,16 +1257,19 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int t0 = c * CH;
   const long long prow0 = (static_cast<long long>(c) * G.NP + pr) * 128;
 
-  if (tid == 0) { mbar_init(tma_bar, 1); mbar_init(mma_bar, 1); mbar_fence_init(); }
-  if (warp == 4) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-  uint32_t mma_phase = 0;
+  // the chunk's scalars, asked for ahead of all else: a memory latency that the set-up runs under
+  float gam = 0.f, beta = 0.f;
+  int sid = -1;
+  if (tid < 128 && (tid >> 6) < nh) {
+    const int hh = tid >> 6, j = tid & 63;
+    gam = p.gam[(static_cast<long long>(c) * G.H + h0 + hh) * 64 + j];
+    if (t0 + j < G.T) beta = p.beta[static_cast<long long>(t0 + j) * G.H + h0 + hh];
+  }
+  if (tid < 64 || (tid == 64 && c > 0)) sid = p.sid[tid < 64 ? t0 + tid : t0 - 1];
 
-  if (tid == CTRL) {
+  if (tid == BCTRL) {
+    mbar_init(tma_bar, 1); mbar_init(mma_bar, 1); mbar_init(dkd_bar, 1); mbar_init(dqg_bar, 1);
+    mbar_fence_init();
     mbar_expect_tx(tma_bar, 32768 + nh * 16384 + 32768 + 32768 + 3 * 16384);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
@@ -1169,14 +1285,20 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tma_load_2d(smem + OFF_TMT, &tmTMT, tma_bar, 0, static_cast<int>(prow0));
     tma_load_2d(smem + OFF_XW, &tmXW, tma_bar, 0, static_cast<int>(prow0));
     tma_load_2d(smem + OFF_XU, &tmXU, tma_bar, 0, static_cast<int>(prow0));
+    mbar_expect_tx(dkd_bar, nh * 16384);
+    for (int hh = 0; hh < nh; ++hh)
+      tma_load_2d(smem + OFF_DKD + hh * 16384, &tmDKD, dkd_bar, hh * 64, static_cast<int>(prow0));
   }
-  if (tid < 65) sid_s[tid] = tid < 64 ? p.sid[t0 + tid] : (c > 0 ? p.sid[t0 - 1] : -1);
-  if (tid < 128) {
-    const int hh = tid >> 6, j = tid & 63, tok = t0 + j;
-    const bool live = hh < nh && tok < G.T;
-    gam_s[tid] = hh < nh ? p.gam[(static_cast<long long>(c) * G.H + h0 + hh) * 64 + j] : 0.f;
-    beta_s[tid] = live ? p.beta[static_cast<long long>(tok) * G.H + h0 + hh] : 0.f;
-  }
+  if (warp == 8) { __syncwarp(); tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  uint32_t mma_phase = 0;
+
+  if (tid < 65) sid_s[tid] = sid;
+  if (tid < 128) { gam_s[tid] = gam; beta_s[tid] = beta; }
   __syncthreads();
   if (tid < 64) {
     const unsigned m = __ballot_sync(0xffffffffu, tid == 0 || sid_s[tid] != sid_s[tid - 1]);
@@ -1189,7 +1311,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
 
   // ---- first group of products
-  if (tid == CTRL) {
+  if (tid == BCTRL) {
     mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
     tc_fence_after();
     const uint32_t skq = smem_u32(smem + OFF_KQ), sv = smem_u32(smem + OFF_V);
@@ -1224,44 +1346,42 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_after();
 
   // ---- K K^T and Q K^T to shared memory (both heads need both)
-  if (tid < 128) {
-    float row[64];
-    tmem_row64(lane_addr, row);
-    float* dst = (tid < 64 ? KKf : QKf) + (tid & 63) * 65;
+  const int row = tid & 127, part = (tid >> 7) & 1;      // of the row threads: a lane of TMEM and the half of its columns
+  if (tid < ROW_THREADS) {
+    float v[32];
+    tmem_row32(lane_addr + part * 32, v);
+    float* dst = (row < 64 ? KKf : QKf) + (row & 63) * 65 + part * 32;
 #pragma unroll
-    for (int i = 0; i < 64; ++i) dst[i] = row[i];
+    for (int i = 0; i < 32; ++i) dst[i] = v[i];
   }
   __syncthreads();
 
-  const int hh_me = tid >> 6, t_me = tid & 63;
-  const bool live = tid < 128 && hh_me < nh;
+  const int hh_me = row >> 6, t_me = row & 63;
+  const bool live = tid < ROW_THREADS && hh_me < nh;
   // ---- dTm = (P1, P2) scaled per column; column sums of Tm o P1 and Tm o P2
-  if (tid < 128) {
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      float p1[32], p2[32], dtm[32];
-      tmem_row32(lane_addr + 64 + half * 32, p1);
-      tmem_row32(lane_addr + 128 + (hh_me < nh ? hh_me : 0) * 64 + half * 32, p2);
+  if (tid < ROW_THREADS) {
+    float p1[32], p2[32], dtm[32];
+    tmem_row32(lane_addr + 64 + part * 32, p1);
+    tmem_row32(lane_addr + 128 + (hh_me < nh ? hh_me : 0) * 64 + part * 32, p2);
 #pragma unroll
-      for (int e = 0; e < 32; ++e) {
-        const int i = half * 32 + e;
-        const float tm = bf16_at(smem + OFF_TMT + (hh_me * 64 + i) * 128 +
-                                 (((t_me >> 3) ^ (i & 7)) << 4) + (t_me & 7) * 2);
-        dtm[e] = live ? beta_s[hh_me * 64 + i] * (gt_s[hh_me * 64 + i] * p1[e] + p2[e]) : 0.f;
-        p1[e] = live ? tm * p1[e] : 0.f;
-        p2[e] = live ? tm * p2[e] : 0.f;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<uint4*>(smem + OFF_DTM + sw_off(128, tid, half * 4 + q)) = pack8(dtm + q * 8);
-      warp_col_sums(p1, cs1 + warp * 64 + half * 32);
-      warp_col_sums(p2, cs2 + warp * 64 + half * 32);
+    for (int e = 0; e < 32; ++e) {
+      const int i = part * 32 + e;
+      const float tm = bf16_at(smem + OFF_TMT + (hh_me * 64 + i) * 128 +
+                               (((t_me >> 3) ^ (i & 7)) << 4) + (t_me & 7) * 2);
+      dtm[e] = live ? beta_s[hh_me * 64 + i] * (gt_s[hh_me * 64 + i] * p1[e] + p2[e]) : 0.f;
+      p1[e] = live ? tm * p1[e] : 0.f;
+      p2[e] = live ? tm * p2[e] : 0.f;
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<uint4*>(smem + OFF_DTM + sw_off(128, row, part * 4 + q)) = pack8(dtm + q * 8);
+    warp_col_sums(p1, cs1 + (warp & 3) * 64 + part * 32);
+    warp_col_sums(p2, cs2 + (warp & 3) * 64 + part * 32);
   }
   publish();
 
   // ---- X = dTm Tm^T
-  if (tid == CTRL) {
+  if (tid == BCTRL) {
     constexpr uint32_t i_km = umma_idesc_bf16(128, 64, false, true);
     const uint32_t sd = smem_u32(smem + OFF_DTM), st = smem_u32(smem + OFF_TMT);
     for (int h2 = 0; h2 < nh; ++h2)
@@ -1275,16 +1395,16 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   mma_phase ^= 1;
   tc_fence_after();
   if (live) {
-    float x[64];
-    tmem_row64(lane_addr + 64 + hh_me * 64, x);
+    float x[32];
+    tmem_row32(lane_addr + 64 + hh_me * 64 + part * 32, x);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      *reinterpret_cast<uint4*>(smem + OFF_XOP + hh_me * 8192 + sw_off(64, t_me, q)) = pack8(x + q * 8);
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<uint4*>(smem + OFF_XOP + hh_me * 8192 + sw_off(64, t_me, part * 4 + q)) = pack8(x + q * 8);
   }
   publish();
 
   // ---- dA = -Tm^T X
-  if (tid == CTRL) {
+  if (tid == BCTRL) {
     constexpr uint32_t i_km = umma_idesc_bf16(128, 64, false, true);
     const uint32_t st = smem_u32(smem + OFF_TMT), sx = smem_u32(smem + OFF_XOP);
     for (int h2 = 0; h2 < nh; ++h2)
@@ -1297,20 +1417,26 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
   mma_phase ^= 1;
   tc_fence_after();
+  if (tid == BCTRL) {                                    // dTm and X have been read: dQg^T takes their place
+    mbar_expect_tx(dqg_bar, nh * 16384);
+    for (int hh = 0; hh < nh; ++hh)
+      tma_load_2d(smem + OFF_DQG + hh * 16384, &tmDQG, dqg_bar, hh * 64, static_cast<int>(prow0));
+  }
 
   // ---- gradients through A and Mq, 16 columns at a time: everything a step reads is in registers before
   // it writes, head 0 writes its dKK and dQK to KKa / QKa and head 1 over the scores both have just read.
-  // The loops of this kernel stay rolled where registers allow: it runs each line once per block with one
-  // warp per scheduler, and fetching straight-line code was its largest stall.
+  // The loops of this kernel stay rolled where registers allow: it runs each line once per block with two
+  // warps per scheduler, and fetching straight-line code was its largest stall.
   float rowG = 0.f, rowdb = 0.f;
-  if (tid < 128) {
-    const uint4* mq = reinterpret_cast<const uint4*>(p.dMQ + (prow0 + tid) * 64);
-    uint4 m0 = make_uint4(0, 0, 0, 0), m1 = m0;
-    if (live) { m0 = mq[0]; m1 = mq[1]; }
+  if (tid < ROW_THREADS) {
+    const uint4* mq = reinterpret_cast<const uint4*>(p.dMQ + (prow0 + row) * 64 + part * 32);
+    uint4 m[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) m[x] = live ? mq[x] : make_uint4(0, 0, 0, 0);
     const int lo = seq_begin(starts_s, t_me);
-    const float gt = gam_s[tid], bt = beta_s[tid];
+    const float gt = gam_s[row], bt = beta_s[row];
 #pragma unroll 1
-    for (int i0 = 0; i0 < 64; i0 += 16) {
+    for (int i0 = part * 32; i0 < part * 32 + 32; i0 += 16) {
       float w[16];
       uint32_t acc[16];
       tmem_ld_32x16(lane_addr + (hh_me == 0 ? 192 : 0) + i0, acc);
@@ -1320,18 +1446,18 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         *reinterpret_cast<float4*>(gi + 4 * x) = *reinterpret_cast<const float4*>(gam_s + hh_me * 64 + i0 + 4 * x);
 #pragma unroll
       for (int e = 0; e < 16; ++e) { kk[e] = KKf[t_me * 65 + i0 + e]; qk[e] = QKf[t_me * 65 + i0 + e]; }
-      unpack8(m0, dmq);
-      unpack8(m1, dmq + 8);
-      if (live && i0 < 48) { m0 = mq[i0 / 8 + 2]; m1 = mq[i0 / 8 + 3]; }
+      unpack8(m[0], dmq);
+      unpack8(m[1], dmq + 8);
+      m[0] = m[2]; m[1] = m[3];
       tmem_ld_wait();
-      row_threads_sync();
+      all_rows_sync();
       float* ko = (hh_me == 0 ? KKa : KKf) + t_me * 65 + i0;
       float* qo = (hh_me == 0 ? QKa : QKf) + t_me * 65 + i0;
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         const int i = i0 + e;
         const bool seen = live && i >= lo && i <= t_me;
-        const float R = seen ? __expf(gt - gi[e]) : 0.f;
+        const float R = decay_if(seen, gt - gi[e]);
         const float da = seen && i < t_me ? -__uint_as_float(acc[e]) : 0.f;
         rowdb += da * R * kk[e];
         const float dkk = da * bt * R, dqk = dmq[e] * p.scale * R;
@@ -1340,13 +1466,14 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         ko[e] = dkk;
         qo[e] = seen ? dqk : 0.f;
       }
-      warp_col_sums(w, colG + warp * 64 + i0);
+      warp_col_sums(w, colG + (warp & 3) * 64 + i0);
     }
-    row_threads_sync();
+    if (part) { rows_s[row] = rowG; rows_s[128 + row] = rowdb; }
+    all_rows_sync();
 #pragma unroll 1
-    for (int q = 0; q < 8; ++q) {
+    for (int q = part * 4; q < part * 4 + 4; ++q) {
       float o[8];
-      if (tid < 64) {
+      if (row < 64) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const int i = q * 8 + e;
@@ -1356,15 +1483,17 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] = QKa[t_me * 65 + q * 8 + e] + QKf[t_me * 65 + q * 8 + e];
       }
-      *reinterpret_cast<uint4*>(smem + (tid < 64 ? OFF_SYM : OFF_DQK) + sw_off(64, t_me, q)) = pack8(o);
+      *reinterpret_cast<uint4*>(smem + (row < 64 ? OFF_SYM : OFF_DQK) + sw_off(64, t_me, q)) = pack8(o);
     }
   }
   publish();
 
-  // ---- dK^T += K^T (dKK + dKK^T) + Q^T dQK;  dQ^T = K^T dQK^T
-  if (tid == CTRL) {
+  // ---- dK^T += K^T (dKK + dKK^T) + Q^T dQK;  dQ^T = K^T dQK^T;  and [K; Q] dKd^T, [K; Q] dQg^T, whose diagonals are
+  // the tokens' <dKd, K> and <dQg, Q> (as sums over the row threads they were 260 shuffles and two-byte loads each)
+  if (tid == BCTRL) {
     constexpr uint32_t i_mm = umma_idesc_bf16(128, 64, true, true);
     constexpr uint32_t i_mk = umma_idesc_bf16(128, 64, true, false);
+    constexpr uint32_t i_km = umma_idesc_bf16(128, 64, false, true);
     const uint32_t skq = smem_u32(smem + OFF_KQ), ssym = smem_u32(smem + OFF_SYM);
     const uint32_t sdqk = smem_u32(smem + OFF_DQK);
 #pragma unroll
@@ -1375,90 +1504,128 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       umma_bf16(tmem_base + 256, aq, umma_smem_desc(sdqk + kk * 2048, 8192, 1024), i_mm, 1);
       umma_bf16(tmem_base + 448, ak, umma_smem_desc(sdqk + kk * 32, 16, 1024), i_mk, kk != 0);
     }
+    mbar_wait(dkd_bar, 0, p.status, KS_TIMEOUT_FULL);
+    mbar_wait(dqg_bar, 0, p.status, KS_TIMEOUT_FULL);
+    tc_fence_after();
+#pragma unroll 1
+    for (int x = 0; x < 4; ++x) {                       // columns 0, 64: dKd of the heads, 128, 192: dQg
+      if ((x & 1) >= nh) continue;
+      const uint32_t sb = smem_u32(smem + (x < 2 ? OFF_DKD : OFF_DQG) + (x & 1) * 16384);
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        umma_bf16(tmem_base + x * 64, umma_smem_desc(skq + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+                  umma_smem_desc(sb + kk * 2048, 16384, 1024), i_km, kk != 0);
+    }
     umma_commit(mma_bar);
   }
+  mbar_wait(dkd_bar, 0, p.status, KS_TIMEOUT_FULL);
+  mbar_wait(dqg_bar, 0, p.status, KS_TIMEOUT_FULL);
   mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
   mma_phase ^= 1;
   tc_fence_after();
 
-  // ---- feature-row epilogue: dk, dq, dv and the two per-token dot products
+  // ---- the diagonals (K rows on the first two warps' lanes, Q rows on the other two's), then the feature rows:
+  // dk, dq and dv, 16 tokens at a time, through the tile that turns them into token rows
   const int lim = min(CH, G.T - t0);
-  // element [i][tid] of K (which = 0) or Q (which = 1) in the stacked tile
-  auto kq_at = [&](int which, int i) {
-    return bf16_at(smem + OFF_KQ + (tid >> 6) * 16384 + (which * 64 + i) * 128 +
-                   (((((tid & 63) >> 3)) ^ (i & 7)) << 4) + (tid & 7) * 2);
-  };
-  if (tid < 128) {
-#pragma unroll 1
-    for (int which = 0; which < 2; ++which) {          // 0: dk (with Kd), 1: dq (with Qg)
-      float acc[64];
-      tmem_row64(lane_addr + (which == 0 ? 256 : 448), acc);
-      const float* fs = which == 0 ? d_s : gt_s;
-      const float fmul = which == 0 ? 1.f : p.scale;
-#pragma unroll 1
-      for (int hh = 0; hh < nh; ++hh) {
-        float a[64];
-        load_row64((which == 0 ? p.dKdTp : p.dQgTp) + (prow0 + tid) * 128 + hh * 64, a);
+  if (tid < ROW_THREADS) {
+    if (part < nh) {                                    // the left halves' threads take head 0, the right's head 1
+      uint32_t r[32];
+      tmem_ld_32x32(lane_addr + (row < 64 ? 0 : 128) + part * 64 + (warp & 1) * 32, r);
+      tmem_ld_wait();
+      float v = 0.f;
 #pragma unroll
-        for (int i0 = 0; i0 < 64; i0 += 4) {
-          const float4 f = *reinterpret_cast<const float4*>(fs + hh * 64 + i0);
-          acc[i0] += f.x * fmul * a[i0];
-          acc[i0 + 1] += f.y * fmul * a[i0 + 1];
-          acc[i0 + 2] += f.z * fmul * a[i0 + 2];
-          acc[i0 + 3] += f.w * fmul * a[i0 + 3];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) a[i0 + e] *= kq_at(which, i0 + e);     // dKd o K  /  dQg o Q
-        }
-        warp_col_sums(a, (which == 0 ? dotk : dotq) + (hh * 4 + warp) * 64);
-      }
-      row_threads_sync();                               // the tile's last reader is done
-      store_tokens(acc, smem + OFF_OUT, (which == 0 ? p.dk : p.dq) + (static_cast<long long>(t0) * G.NP + pr) * D,
-                   static_cast<long long>(G.NP) * D, lim);
+      for (int e = 0; e < 32; ++e) v = lane == e ? __uint_as_float(r[e]) : v;
+      (row < 64 ? dotk : dotq)[part * 64 + t_me] = v;
     }
 #pragma unroll 1
-    for (int hh = 0; hh < nh; ++hh) {
-      float r[64];
-      tmem_row64(lane_addr + 320 + hh * 64, r);
-      row_threads_sync();
-      store_tokens(r, smem + OFF_OUT, p.dv + (static_cast<long long>(t0) * G.H + h0 + hh) * D,
-                   static_cast<long long>(G.H) * D, lim);
+    for (int x = 0; x < 2 + nh; ++x) {                 // dk (with Kd), dq (with Qg), dv of the heads
+      const uint32_t col = x == 0 ? 256 : x == 1 ? 448 : 320 + (x - 2) * 64;
+      if (x > 0) all_rows_sync();                    // the tile's last reader is done
+#pragma unroll 1
+      for (int i0 = part * 32; i0 < part * 32 + 32; i0 += 16) {
+        uint32_t r[16];
+        tmem_ld_32x16(lane_addr + col + i0, r);
+        tmem_ld_wait();
+        float acc[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[e] = __uint_as_float(r[e]);
+        if (x < 2) {
+          const float fmul = x == 0 ? 1.f : p.scale;
+#pragma unroll 1
+          for (int hh = 0; hh < nh; ++hh) {
+            const uint8_t* tile = smem + (x == 0 ? OFF_DKD : OFF_DQG) + hh * 16384;
+            const float* fs = (x == 0 ? d_s : gt_s) + hh * 64 + i0;
+            float a[16];
+            unpack8(*reinterpret_cast<const uint4*>(tile + sw_off(128, row, i0 >> 3)), a);
+            unpack8(*reinterpret_cast<const uint4*>(tile + sw_off(128, row, (i0 >> 3) + 1)), a + 8);
+#pragma unroll
+            for (int e = 0; e < 16; e += 4) {
+              const float4 f = *reinterpret_cast<const float4*>(fs + e);
+              acc[e] += f.x * fmul * a[e];
+              acc[e + 1] += f.y * fmul * a[e + 1];
+              acc[e + 2] += f.z * fmul * a[e + 2];
+              acc[e + 3] += f.w * fmul * a[e + 3];
+            }
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+          *reinterpret_cast<__nv_bfloat16*>(smem + OFF_OUT + (i0 + e) * 256 + row * 2) = __float2bfloat16_rn(acc[e]);
+      }
+      all_rows_sync();
+      __nv_bfloat16* dst;
+      long long ld;
+      if (x < 2) {
+        ld = static_cast<long long>(G.NP) * D;
+        dst = (x == 0 ? p.dk : p.dq) + (static_cast<long long>(t0) * G.NP + pr) * D;
+      } else {
+        ld = static_cast<long long>(G.H) * D;
+        dst = p.dv + (static_cast<long long>(t0) * G.H + h0 + x - 2) * D;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = q * 16 + (tid >> 4), ch = tid & 15;
+        if (t < lim)
+          *reinterpret_cast<uint4*>(dst + t * ld + ch * 8) =
+              *reinterpret_cast<const uint4*>(smem + OFF_OUT + t * 256 + ch * 16);
+      }
     }
   }
   __syncthreads();
 
-  // ---- per-token scalars: dgam -> dg (suffix sum), dbeta
-  // sums of a column's parts: over one head's two row warps, or over all four
+  // ---- per-token scalars: dgam -> dg (suffix sum over the chunk), dbeta
+  // sums of a column's parts over one head's two row warps
   auto two = [&](const float* part, int i) { return part[(hh_me * 2) * 64 + i] + part[(hh_me * 2 + 1) * 64 + i]; };
-  auto four = [&](const float* part, int i) {
-    const float* x = part + hh_me * 256 + i;
-    return (x[0] + x[64]) + (x[128] + x[192]);
-  };
+  float s = 0.f;
   if (tid < 128) {
-    float dgam = 0.f;
+    rowG += rows_s[row];
+    rowdb += rows_s[128 + row];
+    float tail = 0.f;                                   // of the chunk's last token alone
     if (live) {
-      const int o = hh_me * 64;
-      dgam = rowG - two(colG, t_me) + beta_s[tid] * gt_s[tid] * two(cs1, t_me) +
-             p.scale * gt_s[tid] * four(dotq, t_me) - d_s[tid] * four(dotk, t_me);
-      if (t_me == 63) {
-        float tail = 0.f;
-        for (int i = 0; i < 64; ++i) tail += d_s[o + i] * four(dotk, i);
-        const long long hi = static_cast<long long>(c) * G.H + h0 + hh_me;
-        dgam += tail + p.dgc[hi] * p.gc[hi];
-      }
+      tail = d_s[tid] * dotk[tid];
+      s = rowG - two(colG, t_me) + beta_s[tid] * gt_s[tid] * two(cs1, t_me) + p.scale * gt_s[tid] * dotq[tid] - tail;
     }
-    dgam_s[tid] = dgam;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tail += __shfl_xor_sync(0xffffffffu, tail, o);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float after = __shfl_down_sync(0xffffffffu, s, o);
+      if (lane + o < 32) s += after;
+    }
+    if (lane == 0) { sums_s[warp] = tail; sums_s[4 + warp] = s; }
   }
   __syncthreads();
-  if (live && t_me < lim) {
-    float s = 0.f;
-    for (int i = t_me; i < 64; ++i) s += dgam_s[hh_me * 64 + i];
+  if (live && tid < 128 && t_me < lim) {
+    const long long hi = static_cast<long long>(c) * G.H + h0 + hh_me;
+    s += (sums_s[hh_me * 2] + sums_s[hh_me * 2 + 1]) + p.dgc[hi] * p.gc[hi];
+    if (t_me < 32) s += sums_s[4 + hh_me * 2 + 1];
     const long long o = static_cast<long long>(t0 + t_me) * G.H + h0 + hh_me;
     p.dg[o] = s;
     p.dbeta[o] = rowdb + gt_s[tid] * two(cs1, t_me) + two(cs2, t_me);
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  if (warp == 8) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
 static Geo make_geo(int T, int H, int Hk) {
@@ -1501,7 +1668,7 @@ int ss_dn_prep(const void* q, const void* k, const void* v, const float* beta, c
   if (T <= 0) return 0;
   if (H <= 0 || Hk <= 0 || H % Hk) return -2;
   const Geo geo = make_geo(T, H, Hk);
-  CUtensorMap tq, tk, tv, twt, tu0, tqg, tkd, txw, txu;
+  CUtensorMap tq, tk, tv, twt, tu0, tqg, tkd, tmq, txw, txu;
   int r;
   const bool save = TMT != nullptr;
   if ((XW != nullptr) != save || (XU != nullptr) != save) return -2;
@@ -1513,15 +1680,16 @@ int ss_dn_prep(const void* q, const void* k, const void* v, const float* beta, c
   if ((r = ss::make_tmap_bf16(&tu0, U0Tp, prow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tqg, QG, hrow, 128, 128, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tkd, KD, hrow, 128, 128, 64))) return r;
+  if ((r = ss::make_tmap_bf16(&tmq, MQ, prow, 64, 64, 64))) return r;
   if ((r = ss::make_tmap_bf16(&txw, save ? XW : MQ, prow, 64, 64, 64))) return r;
   if ((r = ss::make_tmap_bf16(&txu, save ? XU : MQ, prow, 64, 64, 64))) return r;
   PrepParams p;
   p.beta = beta; p.g = g; p.sid = sid;
-  p.MQ = (__nv_bfloat16*)MQ; p.TMT = (__nv_bfloat16*)TMT; p.save = save; p.gam = gam; p.gc = gc;
+  p.TMT = (__nv_bfloat16*)TMT; p.save = save; p.gam = gam; p.gc = gc;
   p.geo = geo; p.scale = scale; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_prep_kernel, prep::SMEM)) return e;
-  dn_prep_kernel<<<dim3(geo.n, geo.NP), THREADS, prep::SMEM, (cudaStream_t)stream>>>(tq, tk, tv, twt, tu0, tqg, tkd,
+  dn_prep_kernel<<<dim3(geo.n, geo.NP), THREADS, prep::SMEM, (cudaStream_t)stream>>>(tq, tk, tv, twt, tu0, tqg, tkd, tmq,
                                                                                      txw, txu, p);
   return (int)cudaGetLastError();
 }
@@ -1593,7 +1761,7 @@ int ss_dn_bwd_chunk(const void* dSpT, const void* ST, const void* UTp, const voi
   if ((r = ss::make_tmap_bf16(&tst, ST, srow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tut, UTp, prow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tdut, dUTp, prow, 128, 128, 128))) return r;
-  if ((r = ss::make_tmap_bf16(&tdo, dout, T, (long long)H * D, (long long)H * D, 128))) return r;
+  if ((r = ss::make_tmap_bf16(&tdo, dout, T, (long long)H * D, (long long)H * D, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tkd, dKdTp, prow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tqg, dQgTp, prow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tdw, dWTp, prow, 128, 128, 128))) return r;
@@ -1616,7 +1784,7 @@ int ss_dn_bwd_prep(const void* q, const void* k, const void* v, const float* bet
   if (H <= 0 || Hk <= 0 || H % Hk) return -2;
   const Geo geo = make_geo(T, H, Hk);
   const long long prow = (long long)geo.n * geo.NP * 128;
-  CUtensorMap tq, tk, tv, tdw, tdu, ttm, txw, txu;
+  CUtensorMap tq, tk, tv, tdw, tdu, ttm, txw, txu, tkd, tqg;
   int r;
   if ((r = ss::make_tmap_bf16(&tq, q, T, (long long)Hk * D, (long long)Hk * D, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tk, k, T, (long long)Hk * D, (long long)Hk * D, 64))) return r;
@@ -1626,15 +1794,16 @@ int ss_dn_bwd_prep(const void* q, const void* k, const void* v, const float* bet
   if ((r = ss::make_tmap_bf16(&ttm, TMT, prow, 64, 64, 128))) return r;
   if ((r = ss::make_tmap_bf16(&txw, XW, prow, 64, 64, 128))) return r;
   if ((r = ss::make_tmap_bf16(&txu, XU, prow, 64, 64, 128))) return r;
+  if ((r = ss::make_tmap_bf16(&tkd, dKdTp, prow, 128, 128, 128))) return r;
+  if ((r = ss::make_tmap_bf16(&tqg, dQgTp, prow, 128, 128, 128))) return r;
   BwdPrepParams p;
   p.beta = beta; p.sid = sid; p.gam = gam; p.gc = gc; p.dgc = dgc;
-  p.dKdTp = (const __nv_bfloat16*)dKdTp; p.dQgTp = (const __nv_bfloat16*)dQgTp;
   p.dMQ = (const __nv_bfloat16*)dMQ; p.dq = (__nv_bfloat16*)dq; p.dk = (__nv_bfloat16*)dk;
   p.dv = (__nv_bfloat16*)dv; p.dbeta = dbeta; p.dg = dg; p.geo = geo; p.scale = scale; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_bwd_prep_kernel, bprep::SMEM)) return e;
-  dn_bwd_prep_kernel<<<dim3(geo.n, geo.NP), THREADS, bprep::SMEM, (cudaStream_t)stream>>>(
-      tq, tk, tv, tdw, tdu, ttm, txw, txu, p);
+  dn_bwd_prep_kernel<<<dim3(geo.n, geo.NP), bprep::BTHREADS, bprep::SMEM, (cudaStream_t)stream>>>(
+      tq, tk, tv, tdw, tdu, ttm, txw, txu, tkd, tqg, p);
   return (int)cudaGetLastError();
 }
 }  // extern "C"
