@@ -296,10 +296,11 @@ class DenseLayerStage(Stage):
         return gemm + attn
 
     # ---- forward
-    def _compute(self, P, x, meta: BatchMeta, have: dict, upto: str = "end", out=None, bufs=None):
+    def _compute(self, P, x, meta: BatchMeta, have: dict, upto: str = "end", out=None, bufs=None, keep_gu=True):
         """Fill in every intermediate missing from ``have`` (recompute path). ``bufs``
         names preallocated destinations (the views of a saved-set object), so that a
-        saving forward writes what it keeps exactly once, in place."""
+        saving forward writes what it keeps exactly once, in place. Without ``keep_gu`` the
+        gate/up projections may be left out."""
         c = self.cfg
         T = x.shape[0]
         dh, Hq, Hkv = c.head_dim, c.n_heads, c.n_kv_heads
@@ -329,13 +330,12 @@ class DenseLayerStage(Stage):
                                            lse=b("lse"))
             I["attn"], I["lse"] = attn.view(T, Hq * dh), lse
         if "x_mid" not in I:
-            x_mid = out if out is not None else torch.empty_like(x)
-            x_mid.copy_(x)
-            F.linear_fwd(I["attn"], P["wo"], out=x_mid, accumulate=True)
-            I["x_mid"] = x_mid
+            I["x_mid"] = F.linear_residual(I["attn"], P["wo"], x, out=out)
         if "h2" not in I or "gu" not in I:
             I["h2"], I["rstd2"] = F.rmsnorm_fwd(I["x_mid"], P["mlp_norm"], c.norm_epsilon,
                                                 c.zero_centered_norm, out=b("h2"), rstd=b("rstd2"))
+        if "gu" not in I and "hmlp" not in I:
+            I["gu"], I["hmlp"] = F.swiglu_linear(I["h2"], P["w13"], gu=b("gu"), out=b("hmlp"), keep_gu=keep_gu)
         if "gu" not in I:
             I["gu"] = F.linear_fwd(I["h2"], P["w13"], out=b("gu"))
         if "hmlp" not in I:
@@ -355,16 +355,15 @@ class DenseLayerStage(Stage):
     def forward(self, P, x, meta: BatchMeta, keep: tuple[str, ...] = (), out=None, saved_out=None):
         """Returns ``(y, saved)`` where ``saved`` holds the intermediates named in ``keep``.
         With ``saved_out`` (name -> preallocated tensor) they are produced in place."""
-        I = self._compute(P, x, meta, {}, out=out, bufs=saved_out)
-        y = I["x_mid"]
+        keep_mid = "x_mid" in keep
+        mid_out = (saved_out or {}).get("x_mid") if keep_mid else out
+        I = self._compute(P, x, meta, {}, out=mid_out, bufs=saved_out, keep_gu="gu" in keep)
         saved = {}
-        if "x_mid" in keep:
-            # the output buffer is about to absorb the MLP branch; keep a copy
-            if saved_out is not None and "x_mid" in saved_out:
-                saved["x_mid"] = saved_out["x_mid"].copy_(y)
-            else:
-                saved["x_mid"] = y.clone()
-        F.linear_fwd(I["hmlp"], P["w2"], out=y, accumulate=True)
+        if keep_mid:
+            saved["x_mid"] = I["x_mid"]
+            y = F.linear_residual(I["hmlp"], P["w2"], I["x_mid"], out=out)
+        else:                            # the MLP branch is added to it in place
+            y = F.linear_fwd(I["hmlp"], P["w2"], out=I["x_mid"], accumulate=True)
         for n in keep:
             if n != "x_mid":
                 saved[n] = I[n]
@@ -388,9 +387,7 @@ class DenseLayerStage(Stage):
                 G["q_norm"].zero_(); G["k_norm"].zero_()
         # ---- MLP branch
         F.linear_wgrad(dy, I["hmlp"], out=G["w2"], accumulate=acc)
-        dhmlp = F.linear_dgrad(dy, P["w2"])
-        dgu = F.swiglu_bwd(I["gu"], dhmlp)
-        del dhmlp
+        dgu = F.swiglu_linear_dgrad(dy, P["w2"], I["gu"])
         F.linear_wgrad(dgu, I["h2"], out=G["w13"], accumulate=acc)
         dh2 = F.linear_dgrad(dgu, P["w13"])
         del dgu

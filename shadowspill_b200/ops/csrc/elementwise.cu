@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "chained_launch.cuh"
+#include "swiglu_math.cuh"
 
 namespace ss {
 
@@ -207,10 +208,7 @@ __global__ void swiglu_fwd_kernel(const bf16* gu, bf16* h, int T, int F, const i
     unpack8(row[c], g);
     unpack8(row[nv + c], u);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float s = __fdividef(g[e], 1.f + __expf(-g[e]));
-      o[e] = __bfloat162float(__float2bfloat16_rn(s)) * u[e];
-    }
+    for (int e = 0; e < 8; ++e) o[e] = swiglu_value(g[e], u[e]);
     reinterpret_cast<uint4*>(h + t * F)[c] = pack8(o);
   }
 }
@@ -230,12 +228,7 @@ __global__ void swiglu_bwd_kernel(const bf16* gu, const bf16* dh, bf16* dgu, int
     unpack8(row[nv + c], u);
     unpack8(reinterpret_cast<const uint4*>(dh + t * F)[c], d);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float sig = __fdividef(1.f, 1.f + __expf(-g[e]));
-      const float s = g[e] * sig;
-      ou[e] = d[e] * s;
-      og[e] = d[e] * u[e] * (sig * (1.f + g[e] * (1.f - sig)));
-    }
+    for (int e = 0; e < 8; ++e) swiglu_grad(g[e], u[e], d[e], og[e], ou[e]);
     uint4* orow = reinterpret_cast<uint4*>(dgu + t * 2 * F);
     orow[c] = pack8(og);
     orow[nv + c] = pack8(ou);

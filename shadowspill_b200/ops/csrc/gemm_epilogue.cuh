@@ -12,21 +12,65 @@
 // 256-wide model 707 -> 634 us. (Staging with four warps was slower than no staging: 687 us and 862 us.)
 #pragma once
 #include "sm100_ptx.cuh"
+#include "swiglu_math.cuh"
 
 namespace ss {
 
 constexpr int EPI_WARPS = 8;
 constexpr int EPI_WARP_STAGE = 32 * 64;       // bytes of staging per epilogue warp
 
-// C(row0 + [0,32), col0 + [0,32)) (+)= alpha * r; rows >= M and columns >= N are not touched (N % 8 == 0).
+// What a GEMM does with its products besides storing them.
+//   EPI_PLAIN       C (+)= alpha * product; the values added are read from `src` (C itself, or a residual of C's shape)
+//   EPI_SWIGLU      B holds the rows of a gate matrix and those of an up matrix F rows behind: a tile takes as many of
+//                   the one as of the other, and what leaves is h = silu(gate) * up [M, F] and, unless C is null, the
+//                   two themselves, [M, 2F]
+//   EPI_SWIGLU_BWD  the products are the gradient of h; with gate and up read from `src` [M, 2F], what leaves is
+//                   their gradient, C [M, 2F]
+// h and the gradients take gate, up and dh rounded to bf16, so that they have the bits of the separate kernels.
+// Those moved 6 bytes a value of h forward and 10 backward beside the GEMMs' own (8,192 tokens, 14,336 wide:
+// 135 and 202 us), and without gate and up kept the GEMM stores a third.
+enum : int { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_SWIGLU_BWD = 2 };
+
+struct EpiArgs {
+  const void* src;
+  long long ldsrc;
+  __nv_bfloat16* h;
+  long long ldh;
+};
+
+// Half h of a warp's 32 x 32 block through its staging bytes: a thread's row in, for each of four groups of eight rows
+// the four columns of chunk (lane & 3) of row (lane >> 2) out.
+__device__ __forceinline__ void stage_half(uint32_t stage, const uint32_t (&r)[32], int h, float4 (&v)[4]) {
+  const int lane = threadIdx.x & 31, sub = lane >> 2, chunk = lane & 3;
+  __syncwarp();                                           // what was staged before has been read
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)),
+                 "r"(r[h * 16 + 4 * i]), "r"(r[h * 16 + 4 * i + 1]), "r"(r[h * 16 + 4 * i + 2]),
+                 "r"(r[h * 16 + 4 * i + 3])
+                 : "memory");
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int srow = i * 8 + sub;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i].z), "=f"(v[i].w)
+                 : "r"(stage + srow * 64 + ((chunk ^ ((srow >> 1) & 3)) << 4)) : "memory");
+  }
+}
+
+// C(row0 + [0,32), col0 + [0,32)) = alpha * r (+ src); rows >= M and columns >= N are not touched (N % 8 == 0).
 // `stage`: this warp's staging bytes (shared::cta address, 128-byte aligned). All 32 lanes call it.
 template <typename OUT>
-__device__ __forceinline__ void epilogue_store_32x32(uint32_t stage, const uint32_t (&r)[32], OUT* C, int accumulate,
-                                                     float alpha, long long ldc, int row0, int M, int col0, int N) {
+__device__ __forceinline__ void epilogue_store_32x32(uint32_t stage, const uint32_t (&r)[32], OUT* C, const OUT* add,
+                                                     long long ldadd, float alpha, long long ldc, int row0, int M,
+                                                     int col0, int N) {
+  const bool accumulate = add != nullptr;
   constexpr bool F32 = sizeof(OUT) == 4;
   const int lane = threadIdx.x & 31;
   const int sub = lane >> 2, chunk = lane & 3;            // this lane's row in a group of eight, its 4 columns
   OUT* dst = C + static_cast<long long>(row0 + sub) * ldc + col0 + chunk * 4;
+  if (accumulate) add += static_cast<long long>(row0 + sub) * ldadd + col0 + chunk * 4;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const bool col_in = col0 + h * 16 + chunk * 4 < N;
@@ -36,7 +80,7 @@ __device__ __forceinline__ void epilogue_store_32x32(uint32_t stage, const uint3
       for (int i = 0; i < 4; ++i) {
         old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (!col_in || row0 + sub + i * 8 >= M) continue;
-        const OUT* src = dst + static_cast<long long>(i) * 8 * ldc + h * 16;
+        const OUT* src = add + static_cast<long long>(i) * 8 * ldadd + h * 16;
         if constexpr (F32) {
           old[i] = *reinterpret_cast<const float4*>(src);
         } else {
@@ -46,22 +90,8 @@ __device__ __forceinline__ void epilogue_store_32x32(uint32_t stage, const uint3
         }
       }
     }
-    __syncwarp();                                         // the half before this one has been read
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)),
-                   "r"(r[h * 16 + 4 * i]), "r"(r[h * 16 + 4 * i + 1]), "r"(r[h * 16 + 4 * i + 2]),
-                   "r"(r[h * 16 + 4 * i + 3])
-                   : "memory");
-    __syncwarp();
     float4 v[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int srow = i * 8 + sub;
-      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                   : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i].z), "=f"(v[i].w)
-                   : "r"(stage + srow * 64 + ((chunk ^ ((srow >> 1) & 3)) << 4)) : "memory");
-    }
+    stage_half(stage, r, h, v);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       v[i].x *= alpha; v[i].y *= alpha; v[i].z *= alpha; v[i].w *= alpha;
@@ -70,6 +100,64 @@ __device__ __forceinline__ void epilogue_store_32x32(uint32_t stage, const uint3
       OUT* to = dst + static_cast<long long>(i) * 8 * ldc + h * 16;
       if constexpr (F32) *reinterpret_cast<float4*>(to) = v[i];
       else *reinterpret_cast<uint2*>(to) = make_uint2(pack_bf16(v[i].x, v[i].y), pack_bf16(v[i].z, v[i].w));
+    }
+  }
+}
+
+// EPI_SWIGLU: gate and up of the same 32 rows and 32 columns. C is null where gate and up are not kept.
+__device__ __forceinline__ void epilogue_swiglu_32x32(uint32_t stage, const uint32_t (&g)[32], const uint32_t (&u)[32],
+                                                      __nv_bfloat16* C, long long ldc, const EpiArgs& e, int row0, int M,
+                                                      int col0, int F) {
+  uint32_t h[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const float gb = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[i])));
+    const float ub = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[i])));
+    h[i] = __float_as_uint(swiglu_value(gb, ub));
+  }
+  const __nv_bfloat16* none = nullptr;
+  if (C != nullptr) {
+    epilogue_store_32x32(stage, g, C, none, 0, 1.f, ldc, row0, M, col0, F);
+    epilogue_store_32x32(stage, u, C + F, none, 0, 1.f, ldc, row0, M, col0, F);
+  }
+  epilogue_store_32x32(stage, h, e.h, none, 0, 1.f, e.ldh, row0, M, col0, F);
+}
+
+// EPI_SWIGLU_BWD: r is the gradient of h at columns col0.. of F; C and e.src have 2F columns.
+__device__ __forceinline__ void epilogue_swiglu_bwd_32x32(uint32_t stage, const uint32_t (&r)[32], __nv_bfloat16* C,
+                                                          long long ldc, const EpiArgs& e, int row0, int M, int col0,
+                                                          int F) {
+  const int lane = threadIdx.x & 31, sub = lane >> 2, chunk = lane & 3;
+  const __nv_bfloat16* gu = reinterpret_cast<const __nv_bfloat16*>(e.src);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int col = col0 + h * 16 + chunk * 4;
+    uint2 gv[4], uv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {                           // in flight while the block is staged
+      gv[i] = uv[i] = make_uint2(0, 0);
+      const int row = row0 + sub + i * 8;
+      if (col >= F || row >= M) continue;
+      gv[i] = *reinterpret_cast<const uint2*>(gu + row * e.ldsrc + col);
+      uv[i] = *reinterpret_cast<const uint2*>(gu + row * e.ldsrc + F + col);
+    }
+    float4 v[4];
+    stage_half(stage, r, h, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = row0 + sub + i * 8;
+      if (col >= F || row >= M) continue;
+      const float2 d0 = unpack_bf16(pack_bf16(v[i].x, v[i].y)), d1 = unpack_bf16(pack_bf16(v[i].z, v[i].w));
+      const float2 g0 = unpack_bf16(gv[i].x), g1 = unpack_bf16(gv[i].y);
+      const float2 u0 = unpack_bf16(uv[i].x), u1 = unpack_bf16(uv[i].y);
+      float4 dg, du;
+      swiglu_grad(g0.x, u0.x, d0.x, dg.x, du.x);
+      swiglu_grad(g0.y, u0.y, d0.y, dg.y, du.y);
+      swiglu_grad(g1.x, u1.x, d1.x, dg.z, du.z);
+      swiglu_grad(g1.y, u1.y, d1.y, dg.w, du.w);
+      __nv_bfloat16* to = C + row * ldc + col;
+      *reinterpret_cast<uint2*>(to) = make_uint2(pack_bf16(dg.x, dg.y), pack_bf16(dg.z, dg.w));
+      *reinterpret_cast<uint2*>(to + F) = make_uint2(pack_bf16(du.x, du.y), pack_bf16(du.z, du.w));
     }
   }
 }

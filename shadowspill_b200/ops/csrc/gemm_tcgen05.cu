@@ -77,6 +77,7 @@ struct GemmParams {
   int* status;
   float alpha;
   GroupInfo g;
+  EpiArgs e;
 };
 
 struct TileWork {
@@ -122,11 +123,13 @@ __device__ __forceinline__ TileWork decode_tile(const GemmParams& p, int t, int 
   return w;
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const GemmParams p) {
   using Cfg = GemmCfg<BN>;
+  // columns of p.N that a tile takes: with gate and up side by side half of its own
+  constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern repeats every 8 rows = 1024 B.
   uint8_t* smem = align_smem_1024(smem_raw);
@@ -140,7 +143,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_m = (p.M + BM - 1) / BM;
-  const int num_n = (p.N + BN - 1) / BN;
+  const int num_n = (p.N + TILE_N - 1) / TILE_N;
   const int num_tiles = num_m * num_n * (p.g.mode == 2 ? p.g.n_experts : 1);
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -196,7 +199,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           // B is always described by a 3-D map [expert, rows, cols]; plain GEMMs have one expert
           const int bz = p.g.mode == 1 ? w.expert : 0;
-          if (!B_MN) {
+          if (EPI == EPI_SWIGLU) {
+            tma_load_3d(sb, &tmB, &full[stage], kb * BK, nb * TILE_N, bz);
+            tma_load_3d(sb + TILE_N * 128, &tmB, &full[stage], kb * BK, p.N + nb * TILE_N, bz);
+          } else if (!B_MN) {
             tma_load_3d(sb, &tmB, &full[stage], kb * BK, nb * BN, bz);
           } else {
 #pragma unroll
@@ -328,19 +334,30 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       } else
 #pragma unroll 1
-      for (int c = part * (BN / 64); c < (part + 1) * (BN / 64); ++c) {
-        const int col0 = nb * BN + c * 32;
+      for (int c = part * (TILE_N / 64); c < (part + 1) * (TILE_N / 64); ++c) {
+        const int col0 = nb * TILE_N + c * 32, row0 = mb * BM + q * 32;
         if (col0 >= p.N) break;
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-        const int row0 = mb * BM + q * 32;
-        if (p.c_f32)
-          epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C) + w.c_off, p.accumulate, p.alpha, p.ldc,
-                               row0, p.M, col0, p.N);
-        else
-          epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C) + w.c_off, p.accumulate, p.alpha,
-                               p.ldc, row0, p.M, col0, p.N);
+        if constexpr (EPI == EPI_SWIGLU) {
+          uint32_t up[32];
+          tmem_ld_32x32(taddr + TILE_N + c * 32, up);
+          tmem_ld_wait();
+          epilogue_swiglu_32x32(stage_out, r, up, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.e, row0, p.M, col0, p.N);
+        } else if constexpr (EPI == EPI_SWIGLU_BWD) {
+          tmem_ld_wait();
+          epilogue_swiglu_bwd_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.e, row0, p.M, col0, p.N);
+        } else {
+          tmem_ld_wait();
+          if (p.c_f32)
+            epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C) + w.c_off,
+                                 p.accumulate ? reinterpret_cast<const float*>(p.e.src) + w.c_off : nullptr, p.e.ldsrc,
+                                 p.alpha, p.ldc, row0, p.M, col0, p.N);
+          else
+            epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C) + w.c_off,
+                                 p.accumulate ? reinterpret_cast<const __nv_bfloat16*>(p.e.src) + w.c_off : nullptr,
+                                 p.e.ldsrc, p.alpha, p.ldc, row0, p.M, col0, p.N);
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -419,15 +436,16 @@ int make_tmap3_bf16(CUtensorMap* map, const void* base, long long experts, long 
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, int EPI = EPI_PLAIN>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int num_sms,
                   cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
   static SmemOptIn opt_in;
-  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN>;
+  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, EPI>;
+  constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
   if (int e = opt_in.ensure(kern, Cfg::SMEM + Cfg::SCATTER_STAGE)) return e;
   const int smem_bytes = Cfg::SMEM + (p.g.row_dst != nullptr ? Cfg::SCATTER_STAGE : EPI_WARPS * EPI_WARP_STAGE);
-  const long long tiles = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) *
+  const long long tiles = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + TILE_N - 1) / TILE_N) *
                           (p.g.mode == 2 ? p.g.n_experts : 1);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
   // Not the expert banks: chaining them and the kernels around them cost 5 % (64 experts, 8,192 tokens,
@@ -460,6 +478,10 @@ bool gemm_fits_one_wave(int M, int N, int num_sms) {
   return N <= 128 || static_cast<long long>((M + 127) / 128) * ((N + 127) / 128) <= num_sms;
 }
 
+int gemm_from(const void* A, const void* B, const void* src, void* C, long long ldsrc, int M, int N, int K, long long lda,
+              long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn,
+              int num_sms, int* status, void* stream);
+
 static int sm_count() {
   int dev = 0, n = 0;
   cudaGetDevice(&dev);
@@ -477,8 +499,20 @@ extern "C" {
 int ss_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                  long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate,
                  float alpha, int bn, int num_sms, int* status, void* stream) {
-  using namespace ss;
+  return ss::gemm_from(A, B, C, C, ldc, M, N, K, lda, ldb, ldc, a_mn, b_mn, c_f32, accumulate, alpha, bn, num_sms, status,
+                       stream);
+}
+
+}  // extern "C"
+
+namespace ss {
+
+// ss_gemm_bf16 whose `accumulate` adds `src` [M, N] (pitch `ldsrc`, C's type) to the products.
+int gemm_from(const void* A, const void* B, const void* src, void* C, long long ldsrc, int M, int N, int K, long long lda,
+              long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn,
+              int num_sms, int* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (accumulate && ((ldsrc % (c_f32 ? 4 : 8)) || (reinterpret_cast<uintptr_t>(src) & 15))) return -2;
   if ((lda % 8) || (ldb % 8) || (ldc % (c_f32 ? 4 : 8)) || (N % 8) ||
       (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
       (reinterpret_cast<uintptr_t>(C) & 15))
@@ -496,9 +530,14 @@ int ss_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
   GemmParams p{};
   p.C = C; p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.c_f32 = c_f32; p.accumulate = accumulate;
   p.a_mn = a_mn; p.b_mn = b_mn; p.status = status; p.alpha = alpha;
+  p.e.src = src; p.e.ldsrc = ldsrc;
   p.g.mode = 0;
   return dispatch(ta, tb, p, bn, num_sms, reinterpret_cast<cudaStream_t>(stream));
 }
+
+}  // namespace ss
+
+extern "C" {
 
 // Expert-bank GEMMs over token rows sorted by expert into 128-row-aligned segments.
 //   mode 1, b_mn = 0: C[R,N]  = A[R,K] @ bank[e][N,K]^T     (forward through the bank)
@@ -536,6 +575,7 @@ int ss_gemm_grouped_bf16(const void* A, const void* B, void* C, int mode, int ro
     return -2;
   }
   p.C = C; p.ldc = ldc; p.c_f32 = c_f32; p.accumulate = accumulate; p.status = status; p.alpha = 1.f;
+  p.e.src = C; p.e.ldsrc = ldc;
   p.g.mode = mode; p.g.tile_expert = tile_expert; p.g.expert_offset = expert_offset;
   p.g.expert_rows = expert_rows;
   p.g.n_experts = n_experts;
@@ -563,6 +603,76 @@ int ss_gemm_grouped_scatter_bf16(const void* A, const void* B, const long long* 
   p.C = nullptr; p.ldc = 0; p.c_f32 = 0; p.accumulate = 0; p.status = status; p.alpha = 1.f;
   p.g.mode = 1; p.g.tile_expert = tile_expert; p.g.n_experts = n_experts; p.g.row_dst = row_dst;
   return dispatch(ta, tb, p, bn, sm_count(), reinterpret_cast<cudaStream_t>(stream));
+}
+
+// h[M, F] = silu(A gate^T) * (A up^T) for B = [gate; up], [2F, K]; unless gu is null the two products go there, [M, 2F].
+// The single-CTA form; ss_gemm2_swiglu_bf16 hands it the outputs whose 128 x 128 tiles of gate and up fit one wave.
+int ss_gemm_swiglu_bf16(const void* A, const void* B, void* gu, void* h, int M, int F, int K, long long lda,
+                        long long ldb, long long ldgu, long long ldh, int bn, int* status, void* stream) {
+  using namespace ss;
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (ldgu % 8) || (ldh % 8) || (F % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
+      (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(gu) & 15) ||
+      (reinterpret_cast<uintptr_t>(h) & 15))
+    return -2;
+  const int num_sms = sm_count();
+  if (bn != 128 && bn != 256) bn = gemm_fits_one_wave(M, 2 * F, num_sms) ? 128 : 256;
+  CUtensorMap ta, tb;
+  int r;
+  if ((r = make_tmap_bf16(&ta, A, M, K, lda, BM))) return r;
+  if ((r = make_tmap3_bf16(&tb, B, 1, 2LL * F, K, ldb, 2LL * F * ldb, bn / 2))) return r;
+  GemmParams p{};
+  p.C = gu; p.M = M; p.N = F; p.K = K; p.ldc = ldgu; p.status = status; p.alpha = 1.f;
+  p.e.h = reinterpret_cast<__nv_bfloat16*>(h); p.e.ldh = ldh;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (bn == 256) return launch<256, false, false, EPI_SWIGLU>(ta, tb, p, num_sms, s);
+  return launch<128, false, false, EPI_SWIGLU>(ta, tb, p, num_sms, s);
+}
+
+// dgu[M, 2F] = the gradient of [gate, up] in gu [M, 2F] for dh = A[M, K] @ B[K, F], the gradient of silu(gate) * up.
+int ss_gemm_swiglu_bwd_bf16(const void* A, const void* B, const void* gu, void* dgu, int M, int F, int K, long long lda,
+                            long long ldb, long long ldgu, long long lddgu, int bn, int* status, void* stream) {
+  using namespace ss;
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (ldgu % 8) || (lddgu % 8) || (F % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
+      (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(gu) & 15) ||
+      (reinterpret_cast<uintptr_t>(dgu) & 15))
+    return -2;
+  const int num_sms = sm_count();
+  if (bn != 128 && bn != 256) bn = gemm_fits_one_wave(M, F, num_sms) ? 128 : 256;
+  CUtensorMap ta, tb;
+  int r;
+  if ((r = make_tmap_bf16(&ta, A, M, K, lda, BM))) return r;
+  if ((r = make_tmap3_bf16(&tb, B, 1, K, F, ldb, static_cast<long long>(K) * ldb, BK))) return r;
+  GemmParams p{};
+  p.C = dgu; p.M = M; p.N = F; p.K = K; p.ldc = lddgu; p.b_mn = 1; p.status = status; p.alpha = 1.f;
+  p.e.src = gu; p.e.ldsrc = ldgu;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (bn == 256) return launch<256, false, true, EPI_SWIGLU_BWD>(ta, tb, p, num_sms, s);
+  return launch<128, false, true, EPI_SWIGLU_BWD>(ta, tb, p, num_sms, s);
+}
+
+// The forward form over expert-sorted rows (segments as in mode 1 above): bank [E, 2F, K], gu [rows, 2F], h [rows, F].
+int ss_gemm_grouped_swiglu_bf16(const void* A, const void* B, void* gu, void* h, int rows, int F, int K, int n_experts,
+                                long long lda, long long ldb, long long ldgu, long long ldh, const int* tile_expert,
+                                int* status, void* stream) {
+  using namespace ss;
+  if (rows <= 0 || n_experts <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (ldgu % 8) || (ldh % 8) || (F % 8) || (rows % BM) || tile_expert == nullptr ||
+      (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(h) & 15))
+    return -2;
+  const int bn = 2 * F <= 128 ? 128 : 256;
+  CUtensorMap ta, tb;
+  int r;
+  if ((r = make_tmap_bf16(&ta, A, rows, K, lda, BM))) return r;
+  if ((r = make_tmap3_bf16(&tb, B, n_experts, 2LL * F, K, ldb, 2LL * F * ldb, bn / 2))) return r;
+  GemmParams p{};
+  p.C = gu; p.M = rows; p.N = F; p.K = K; p.ldc = ldgu; p.status = status; p.alpha = 1.f;
+  p.e.h = reinterpret_cast<__nv_bfloat16*>(h); p.e.ldh = ldh;
+  p.g.mode = 1; p.g.tile_expert = tile_expert; p.g.n_experts = n_experts;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (bn == 256) return launch<256, false, false, EPI_SWIGLU>(ta, tb, p, sm_count(), s);
+  return launch<128, false, false, EPI_SWIGLU>(ta, tb, p, sm_count(), s);
 }
 
 }  // extern "C"

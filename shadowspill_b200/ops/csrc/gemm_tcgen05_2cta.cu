@@ -45,7 +45,11 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, long long rows, long long
 int make_tmap3_bf16(CUtensorMap* map, const void* base, long long experts, long long rows,
                     long long cols, long long ld, long long expert_pitch_elems, int box_rows);
 
-bool gemm_fits_one_wave(int M, int N, int num_sms);   // gemm_tcgen05.cu
+// gemm_tcgen05.cu
+bool gemm_fits_one_wave(int M, int N, int num_sms);
+int gemm_from(const void* A, const void* B, const void* src, void* C, long long ldsrc, int M, int N, int K, long long lda,
+              long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn,
+              int num_sms, int* status, void* stream);
 
 namespace pair {
 
@@ -68,6 +72,7 @@ struct Params {
   int c_f32, accumulate;
   float alpha;
   int* status;
+  EpiArgs e;
 };
 
 constexpr int GATHER_THREADS = 128;                  // warps 10..13 of the GATHER form
@@ -173,7 +178,7 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& mb
   nb = r / gm;
 }
 
-template <bool A_MN, bool B_MN, bool GATHER>
+template <bool A_MN, bool B_MN, bool GATHER, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_THREADS : THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const Params p, const GatherArgs ga) {
@@ -193,7 +198,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   const int num_m = (p.M + 2 * BM - 1) / (2 * BM);
-  const int num_n = (p.N + BN - 1) / BN;
+  // columns of p.N that a tile takes; with gate and up side by side rank 0 stages the rows of the one, rank 1 the other's
+  constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
+  const int num_n = (p.N + TILE_N - 1) / TILE_N;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -232,7 +239,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         int mb, nb;
         tile_coords<GATHER>(t, num_m, num_n, mb, nb);
         const int m0 = mb * (2 * BM) + static_cast<int>(rank) * BM;
-        const int n0 = nb * BN + static_cast<int>(rank) * (BN / 2);
+        const int n0 = EPI == EPI_SWIGLU ? nb * TILE_N + static_cast<int>(rank) * p.N
+                                         : nb * BN + static_cast<int>(rank) * (BN / 2);
         if (GATHER) {
           // rows [nb*BN, nb*BN + BN) of W are local once every piece of the tile is counted
           const long long tile_bytes = static_cast<long long>(BN) * p.K * 2;
@@ -323,18 +331,30 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
 #pragma unroll 1
-      for (int c = part * (BN / 64); c < (part + 1) * (BN / 64); ++c) {
-        const int col0 = nb * BN + c * 32;
+      for (int c = part * (TILE_N / 64); c < (part + 1) * (TILE_N / 64); ++c) {
+        const int col0 = nb * TILE_N + c * 32;
         if (col0 >= p.N) break;
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-        if (p.c_f32)
-          epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C), p.accumulate, p.alpha, p.ldc, row0, p.M,
-                               col0, p.N);
-        else
-          epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C), p.accumulate, p.alpha, p.ldc, row0,
-                               p.M, col0, p.N);
+        if constexpr (EPI == EPI_SWIGLU) {
+          uint32_t up[32];
+          tmem_ld_32x32(taddr + TILE_N + c * 32, up);
+          tmem_ld_wait();
+          epilogue_swiglu_32x32(stage_out, r, up, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.e, row0, p.M, col0, p.N);
+        } else if constexpr (EPI == EPI_SWIGLU_BWD) {
+          tmem_ld_wait();
+          epilogue_swiglu_bwd_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.e, row0, p.M, col0, p.N);
+        } else {
+          tmem_ld_wait();
+          if (p.c_f32)
+            epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C),
+                                 p.accumulate ? reinterpret_cast<const float*>(p.e.src) : nullptr, p.e.ldsrc, p.alpha,
+                                 p.ldc, row0, p.M, col0, p.N);
+          else
+            epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C),
+                                 p.accumulate ? reinterpret_cast<const __nv_bfloat16*>(p.e.src) : nullptr, p.e.ldsrc,
+                                 p.alpha, p.ldc, row0, p.M, col0, p.N);
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -379,13 +399,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, int EPI = EPI_PLAIN>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int num_sms,
                   cudaStream_t stream) {
   static SmemOptIn opt_in;
-  auto kern = gemm2_bf16_kernel<A_MN, B_MN, false>;
+  auto kern = gemm2_bf16_kernel<A_MN, B_MN, false, EPI>;
+  constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
   if (int e = opt_in.ensure(kern, SMEM)) return e;
-  const long long tiles = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
+  const long long tiles = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + TILE_N - 1) / TILE_N);
   long long pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
   launch_chained(kern, static_cast<int>(2 * pairs), THREADS, SMEM, stream, ta, tb, p, GatherArgs{});
@@ -395,7 +416,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
 static int launch_gather(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const GatherArgs& ga,
                          int num_sms, cudaStream_t stream) {
   static SmemOptIn opt_in;
-  auto kern = gemm2_bf16_kernel<false, false, true>;
+  auto kern = gemm2_bf16_kernel<false, false, true, EPI_PLAIN>;
   if (int e = opt_in.ensure(kern, SMEM)) return e;
   const long long tiles = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   long long pairs = num_sms / 2;
@@ -404,23 +425,11 @@ static int launch_gather(const CUtensorMap& ta, const CUtensorMap& tb, const Par
   return static_cast<int>(cudaGetLastError());
 }
 
-}  // namespace pair
-}  // namespace ss
-
-extern "C" {
-
-int ss_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                 long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn, int num_sms,
-                 int* status, void* stream);
-
-// Same arguments and return codes as ss_gemm_bf16 (without the tile-width hint), which takes the outputs
-// whose 128x128 tiles fit one wave.
-int ss_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
-                  long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate,
-                  float alpha, int num_sms, int* status, void* stream) {
-  using namespace ss;
-  using namespace ss::pair;
+static int gemm2_from(const void* A, const void* B, const void* src, void* C, long long ldsrc, int M, int N, int K,
+                      long long lda, long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate,
+                      float alpha, int num_sms, int* status, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (accumulate && ((ldsrc % (c_f32 ? 4 : 8)) || (reinterpret_cast<uintptr_t>(src) & 15))) return -2;
   if ((lda % 8) || (ldb % 8) || (ldc % (c_f32 ? 4 : 8)) || (N % 8) ||
       (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
       (reinterpret_cast<uintptr_t>(C) & 15))
@@ -431,8 +440,8 @@ int ss_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   if (gemm_fits_one_wave(M, N, num_sms))
-    return ss_gemm_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, c_f32, accumulate, alpha, 128, num_sms, status,
-                        stream);
+    return gemm_from(A, B, src, C, ldsrc, M, N, K, lda, ldb, ldc, a_mn, b_mn, c_f32, accumulate, alpha, 128, num_sms,
+                     status, stream);
   CUtensorMap ta, tb;
   int r;
   if (!a_mn) r = make_tmap_bf16(&ta, A, M, K, lda, BM);
@@ -441,12 +450,86 @@ int ss_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
   if (!b_mn) r = make_tmap3_bf16(&tb, B, 1, N, K, ldb, static_cast<long long>(N) * ldb, BN / 2);
   else       r = make_tmap3_bf16(&tb, B, 1, K, N, ldb, static_cast<long long>(K) * ldb, BK);
   if (r) return r;
-  Params p{C, M, N, K, ldc, c_f32, accumulate, alpha, status};
+  Params p{C, M, N, K, ldc, c_f32, accumulate, alpha, status, {src, ldsrc}};
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (!a_mn && !b_mn) return launch<false, false>(ta, tb, p, num_sms, s);
   if (!a_mn && b_mn) return launch<false, true>(ta, tb, p, num_sms, s);
   if (a_mn && b_mn) return launch<true, true>(ta, tb, p, num_sms, s);
   return launch<true, false>(ta, tb, p, num_sms, s);
+}
+
+}  // namespace pair
+}  // namespace ss
+
+extern "C" {
+
+int ss_gemm_swiglu_bf16(const void* A, const void* B, void* gu, void* h, int M, int F, int K, long long lda,
+                        long long ldb, long long ldgu, long long ldh, int bn, int* status, void* stream);
+int ss_gemm_swiglu_bwd_bf16(const void* A, const void* B, const void* gu, void* dgu, int M, int F, int K, long long lda,
+                            long long ldb, long long ldgu, long long lddgu, int bn, int* status, void* stream);
+
+// Same arguments and return codes as ss_gemm_bf16 (without the tile-width hint), which takes the outputs
+// whose 128x128 tiles fit one wave.
+int ss_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                  long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate,
+                  float alpha, int num_sms, int* status, void* stream) {
+  return ss::pair::gemm2_from(A, B, C, C, ldc, M, N, K, lda, ldb, ldc, a_mn, b_mn, c_f32, accumulate, alpha, num_sms,
+                              status, stream);
+}
+
+// C[M, N] = src[M, N] + A[M, K] @ B[N, K]^T in bf16: a residual added where the products leave, without a copy of it
+// in C first (the copy and the second launch: 23 us at 8,192 x 4,096, 2 us at 768 x 256).
+int ss_gemm2_residual_bf16(const void* A, const void* B, const void* src, void* C, int M, int N, int K, long long lda,
+                           long long ldb, long long ldsrc, long long ldc, int* status, void* stream) {
+  if (M < 256 || N < 128)
+    return ss::gemm_from(A, B, src, C, ldsrc, M, N, K, lda, ldb, ldc, 0, 0, 0, 1, 1.f, 0, 0, status, stream);
+  return ss::pair::gemm2_from(A, B, src, C, ldsrc, M, N, K, lda, ldb, ldc, 0, 0, 0, 1, 1.f, 0, status, stream);
+}
+
+// ss_gemm_swiglu_bf16 and ss_gemm_swiglu_bwd_bf16 on CTA pairs (argument checks as there, which takes M < 256, narrow
+// outputs and those of one wave).
+int ss_gemm2_swiglu_bf16(const void* A, const void* B, void* gu, void* h, int M, int F, int K, long long lda,
+                         long long ldb, long long ldgu, long long ldh, int* status, void* stream) {
+  using namespace ss;
+  using namespace ss::pair;
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  int dev = 0, num_sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  if (M < 2 * BM || gemm_fits_one_wave(M, 2 * F, num_sms))
+    return ss_gemm_swiglu_bf16(A, B, gu, h, M, F, K, lda, ldb, ldgu, ldh, 0, status, stream);
+  if ((lda % 8) || (ldb % 8) || (ldgu % 8) || (ldh % 8) || (F % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
+      (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(gu) & 15) ||
+      (reinterpret_cast<uintptr_t>(h) & 15))
+    return -2;
+  CUtensorMap ta, tb;
+  int r;
+  if ((r = make_tmap_bf16(&ta, A, M, K, lda, BM))) return r;
+  if ((r = make_tmap3_bf16(&tb, B, 1, 2LL * F, K, ldb, 2LL * F * ldb, BN / 2))) return r;
+  Params p{gu, M, F, K, ldgu, 0, 0, 1.f, status, {nullptr, 0, reinterpret_cast<__nv_bfloat16*>(h), ldh}};
+  return launch<false, false, EPI_SWIGLU>(ta, tb, p, num_sms, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int ss_gemm2_swiglu_bwd_bf16(const void* A, const void* B, const void* gu, void* dgu, int M, int F, int K, long long lda,
+                             long long ldb, long long ldgu, long long lddgu, int* status, void* stream) {
+  using namespace ss;
+  using namespace ss::pair;
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  int dev = 0, num_sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  if (M < 2 * BM || gemm_fits_one_wave(M, F, num_sms))
+    return ss_gemm_swiglu_bwd_bf16(A, B, gu, dgu, M, F, K, lda, ldb, ldgu, lddgu, 0, status, stream);
+  if ((lda % 8) || (ldb % 8) || (ldgu % 8) || (lddgu % 8) || (F % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
+      (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(gu) & 15) ||
+      (reinterpret_cast<uintptr_t>(dgu) & 15))
+    return -2;
+  CUtensorMap ta, tb;
+  int r;
+  if ((r = make_tmap_bf16(&ta, A, M, K, lda, BM))) return r;
+  if ((r = make_tmap3_bf16(&tb, B, 1, K, F, ldb, static_cast<long long>(K) * ldb, BK))) return r;
+  Params p{dgu, M, F, K, lddgu, 0, 0, 1.f, status, {gu, ldgu}};
+  return launch<false, true, EPI_SWIGLU_BWD>(ta, tb, p, num_sms, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // C[M, N] (+)= alpha * A[M, K] @ W[N, K]^T where W is gathered into `full` by the same kernel.
@@ -476,7 +559,7 @@ int ss_gemm2_gather_bf16(const void* A, void* full, void* C, int M, int N, int K
   int r;
   if ((r = make_tmap_bf16(&ta, A, M, K, lda, BM))) return r;
   if ((r = make_tmap3_bf16(&tb, full, 1, N, K, K, static_cast<long long>(N) * K, BN / 2))) return r;
-  Params p{C, M, N, K, ldc, c_f32, accumulate, alpha, status};
+  Params p{C, M, N, K, ldc, c_f32, accumulate, alpha, status, {C, ldc}};
   GatherArgs ga{};
   for (int k = 0; k < world; ++k) {
     if (reinterpret_cast<uintptr_t>(shard_ptrs[k]) & 15) return -2;

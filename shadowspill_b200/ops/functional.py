@@ -157,6 +157,63 @@ def _gemm_gather(x: torch.Tensor, info: PendingGather, out, accumulate: bool):
     return out
 
 
+def _plain_rows(*tensors) -> bool:
+    """Are these 2-D bf16 CUDA tensors with rows that TMA and 16-byte stores can take?"""
+    return all(t.is_cuda and t.dtype == _BF16 and t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0
+               and t.shape[1] % 8 == 0 and t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def _fused_gemm(*tensors) -> bool:
+    """Do these operands of a GEMM with more than a store in its epilogue run on the kernels of ``gemm`` as they are?"""
+    return not _LIBRARY and not _pending_gathers and _PAIR_GEMM and _plain_rows(*tensors)
+
+
+def linear_residual(x, w, residual, out=None):
+    """``residual[T,N] + x[T,K] @ w[N,K]^T``; ``residual`` is only read (and may be ``out``)."""
+    if out is None:
+        out = torch.empty_like(residual)
+    M, N, K = x.shape[0], w.shape[0], x.shape[1]
+    if not (_fused_gemm(x, w, residual, out) and w.shape[1] == K and out.shape == residual.shape == (M, N)):
+        if out is not residual:
+            out.copy_(residual)
+        return linear_fwd(x, w, out=out, accumulate=True)
+    _lib.check(_lib.lib().ss_gemm2_residual_bf16(
+        x.data_ptr(), w.data_ptr(), residual.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0),
+        residual.stride(0), out.stride(0), _lib.status_ptr(x), _lib.stream_ptr()), "ss_gemm2_residual_bf16")
+    return out
+
+
+def swiglu_linear(x, w13, gu=None, out=None, keep_gu=True):
+    """``gu = x @ w13^T`` (gate columns, then up columns) and ``h = silu(gate) * up`` by one kernel: ``(gu, h)``.
+    Without ``keep_gu`` the projections are not written and the first is None."""
+    T, F2, K = x.shape[0], w13.shape[0], x.shape[1]
+    keep_gu = keep_gu or gu is not None
+    given = [t for t in (gu, out) if t is not None]
+    if not (_fused_gemm(x, w13, *given) and w13.shape[1] == K and F2 % 16 == 0):
+        gu = linear_fwd(x, w13, out=gu)
+        return (gu if keep_gu else None), swiglu_fwd(gu, out=out)
+    if keep_gu and gu is None:
+        gu = torch.empty((T, F2), dtype=x.dtype, device=x.device)
+    h = torch.empty((T, F2 // 2), dtype=x.dtype, device=x.device) if out is None else out
+    _lib.check(_lib.lib().ss_gemm2_swiglu_bf16(
+        x.data_ptr(), w13.data_ptr(), _ptr(gu), h.data_ptr(), T, F2 // 2, K, x.stride(0), w13.stride(0),
+        0 if gu is None else gu.stride(0), h.stride(0), _lib.status_ptr(x), _lib.stream_ptr()), "ss_gemm2_swiglu_bf16")
+    return gu, h
+
+
+def swiglu_linear_dgrad(dy, w2, gu):
+    """The gradient of ``gu`` for ``y = h @ w2^T`` with ``h = silu(gate) * up``: ``dy @ w2`` goes through SwiGLU's
+    gradient where the products leave, and is never stored."""
+    T, F, K = dy.shape[0], w2.shape[1], dy.shape[1]
+    if not (_fused_gemm(dy, w2, gu) and w2.shape[0] == K and gu.shape == (T, 2 * F)):
+        return swiglu_bwd(gu, linear_dgrad(dy, w2))
+    dgu = torch.empty((T, 2 * F), dtype=gu.dtype, device=gu.device)
+    _lib.check(_lib.lib().ss_gemm2_swiglu_bwd_bf16(
+        dy.data_ptr(), w2.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, F, K, dy.stride(0), w2.stride(0),
+        gu.stride(0), dgu.stride(0), _lib.status_ptr(dy), _lib.stream_ptr()), "ss_gemm2_swiglu_bwd_bf16")
+    return dgu
+
+
 def linear_fwd(x, w, out=None, accumulate=False):
     """``y[T,N] (+)= x[T,K] @ w[N,K]^T``. A weight registered by ``register_gather`` is gathered
     from its shards by this GEMM itself."""

@@ -32,6 +32,8 @@ _lib.register("ss_gemm_grouped_bf16", [_c.c_p, _c.c_p, _c.c_p, _c.c_int, _c.c_in
                                        _c.c_int, _c.c_int, _c.c_int, _c.c_ll, _c.c_ll, _c.c_ll,
                                        _c.c_int, _c.c_int, _c.c_int, _c.c_p, _c.c_p, _c.c_p, _c.c_int,
                                        _c.c_p, _c.c_p])
+_lib.register("ss_gemm_grouped_swiglu_bf16", [_c.c_p, _c.c_p, _c.c_p, _c.c_p, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
+                                              _c.c_ll, _c.c_ll, _c.c_ll, _c.c_ll, _c.c_p, _c.c_p, _c.c_p])
 
 
 def route(logits: torch.Tensor, k: int, renormalize: bool):
@@ -146,6 +148,20 @@ def grouped_linear(x_sorted: torch.Tensor, bank: torch.Tensor, lay: Layout, tran
     return out
 
 
+def grouped_swiglu(x_sorted: torch.Tensor, bank: torch.Tensor, lay: Layout):
+    """``gu[r] = x[r] @ bank[e(r)]^T`` (gate columns, then up columns) and ``h = silu(gate) * up`` by one kernel."""
+    E, F2, K = bank.shape
+    gu = torch.empty((lay.rows, F2), dtype=x_sorted.dtype, device=x_sorted.device)
+    if F2 % 16 or bank.stride(2) != 1 or bank.stride(0) != F2 * bank.stride(1):
+        return grouped_linear(x_sorted, bank, lay, out=gu), lay.swiglu(gu)
+    h = torch.empty((lay.rows, F2 // 2), dtype=x_sorted.dtype, device=x_sorted.device)
+    _lib.check(_lib.lib().ss_gemm_grouped_swiglu_bf16(
+        x_sorted.data_ptr(), bank.data_ptr(), gu.data_ptr(), h.data_ptr(), lay.rows, F2 // 2, K, E, x_sorted.stride(0),
+        bank.stride(1), gu.stride(0), h.stride(0), lay.tile_expert.data_ptr(), _lib.status_ptr(x_sorted),
+        _lib.stream_ptr()), "ss_gemm_grouped_swiglu_bf16")
+    return gu, h
+
+
 def grouped_wgrad(dy_sorted: torch.Tensor, x_sorted: torch.Tensor, lay: Layout, out: torch.Tensor,
                   accumulate: bool) -> None:
     """``out[e] (+)= dy[rows_e]^T @ x[rows_e]`` for every expert of a bank gradient [E, M, N]."""
@@ -170,8 +186,9 @@ class _Experts(torch.autograd.Function):
         ids, wts, counts = route(logits, k, renormalize)
         lay = Layout(ids, counts)
         xs = lay.gather(h)
-        gu = grouped_linear(xs, w13, lay)
-        ys = grouped_linear(lay.swiglu(gu), w2, lay)
+        gu, act = grouped_swiglu(xs, w13, lay)
+        ys = grouped_linear(act, w2, lay)
+        del act
         out = lay.combine(ys, wts)
         ctx.save_for_backward(logits, ids, wts, xs, gu, w13, w2)
         ctx.lay, ctx.sink, ctx.renormalize = lay, sink, renormalize
