@@ -20,6 +20,7 @@ import torch
 from torch.library import custom_op
 
 from ..ops import functional as F
+from ..ops import token_head
 
 Tensor = torch.Tensor
 
@@ -275,18 +276,22 @@ def head_loss_run(h: Tensor, W: Tensor, targets: Tensor, weights: Tensor, block_
     into ``dW`` block by block. Shared by the operator below and its in-place twin."""
     T = h.shape[0]
     loss = torch.zeros(1, dtype=torch.float32, device=h.device)
+    rows = token_head.scored(h, W, targets, weights, dW)
+    h = rows.take(h)
     dh = torch.empty_like(h) if train else None
     acc = accumulate
     for r0 in range(0, T, block_rows):
         r1 = min(T, r0 + block_rows)
-        logits = F.linear_fwd(h[r0:r1], W)
-        F.cross_entropy_(logits, targets[r0:r1], weights[r0:r1], loss, write_grad=train)
+        logits = rows.logits(h, W, r0, r1)
+        rows.cross_entropy_(logits, targets, weights, loss, r0, r1, write_grad=train)
         if train:
             if dW is not None:
-                F.linear_wgrad(logits, h[r0:r1], out=dW, accumulate=acc)
+                rows.wgrad(logits, h, dW, acc, r0, r1)
                 acc = True
-            F.linear_dgrad(logits, W, out=dh[r0:r1])
+            rows.dgrad(logits, W, dh, r0, r1)
         del logits
+    if train:
+        dh = rows.put(dh)
     return loss, dh
 
 

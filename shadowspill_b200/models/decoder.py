@@ -22,6 +22,7 @@ from typing import Callable
 import torch
 
 from ..ops import functional as F
+from ..ops import token_head
 from .config import DecoderConfig
 
 ALIGN = 256  # byte alignment of every tensor inside a flat stage buffer
@@ -492,33 +493,35 @@ class HeadLossStage(Stage):
             Gw = G["head"] if (G and "head" in G) else None
             w_first = first
         h, rstd = F.rmsnorm_fwd(x, P["final_norm"], c.norm_epsilon, c.zero_centered_norm)
+        ob, X = self.objective, meta.extras
+        rows = token_head.scored(h, W, meta.targets, meta.weights, Gw)
+        h = rows.take(h)
         dh = torch.empty_like(h) if train else None
         frozen = not G or "final_norm" not in G
         if train and first and not frozen:
             G["final_norm"].zero_()
         B = self.block_rows
         acc = not w_first
-        ob, X = self.objective, meta.extras
         for r0 in range(0, T, B):
             r1 = min(T, r0 + B)
-            logits = F.linear_fwd(h[r0:r1], W)
+            logits = rows.logits(h, W, r0, r1)
             if ob.kind == "clipped_policy":
-                ref = X["reference_logprobs"][r0:r1] if ob.reference_beta > 0 else None
-                F.clipped_policy_(logits, meta.targets[r0:r1], meta.weights[r0:r1],
-                                  X["old_logprobs"][r0:r1], X["advantages"][r0:r1], loss_sum,
-                                  clip=ob.clip_ratio, ref_logp=ref, ref_beta=ob.reference_beta,
-                                  grad_scale=grad_scale, write_grad=train)
+                ref = X["reference_logprobs"] if ob.reference_beta > 0 else None
+                rows.clipped_policy_(logits, meta.targets, meta.weights, X["old_logprobs"], X["advantages"], loss_sum,
+                                     r0, r1, clip=ob.clip_ratio, ref_logp=ref, ref_beta=ob.reference_beta,
+                                     grad_scale=grad_scale, write_grad=train)
             else:
-                F.cross_entropy_(logits, meta.targets[r0:r1], meta.weights[r0:r1], loss_sum,
-                                 grad_scale=grad_scale, write_grad=train)
+                rows.cross_entropy_(logits, meta.targets, meta.weights, loss_sum, r0, r1, grad_scale=grad_scale,
+                                    write_grad=train)
             if train:
                 if Gw is not None:
-                    F.linear_wgrad(logits, h[r0:r1], out=Gw, accumulate=acc)
-                F.linear_dgrad(logits, W, out=dh[r0:r1])
+                    rows.wgrad(logits, h, Gw, acc, r0, r1)
+                rows.dgrad(logits, W, dh, r0, r1)
                 acc = True
             del logits
         if not train:
             return None
+        dh = rows.put(dh)
         dw = G["final_norm"] if not frozen else torch.zeros(c.d_model, dtype=torch.float32,
                                                             device=x.device)
         return F.rmsnorm_bwd(x, P["final_norm"], dh, rstd, dw, c.zero_centered_norm,

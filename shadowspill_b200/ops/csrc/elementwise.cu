@@ -289,18 +289,44 @@ struct PolicyArgs {
   float clip, ref_beta;
   float* logp_out;          // optional: per-row log-probability of the target
 };
+// A block of logits of listed rows: its row i is token rows[from + i] where from + i < *used. What lies behind them is
+// not a token's, and zeroed up to the next multiple of 64, the depth of the weight gradient's products.
+struct RowList {
+  const int* rows;          // null: row i is token i
+  const int* used;
+  int from;
+};
 constexpr int CE_THREADS = 512;
 __global__ void __launch_bounds__(CE_THREADS)
 cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets,
                      const float* __restrict__ weights, float* __restrict__ loss_sum,
                      float* __restrict__ lse_out, int R, int V, long long ld, float grad_scale,
-                     int write_grad, PolicyArgs pa) {
+                     int write_grad, PolicyArgs pa, RowList list) {
   __shared__ float red[33];
-  const int row = blockIdx.x;
+  int row = blockIdx.x;
   if (row >= R) return;
   bf16* lr = logits + static_cast<long long>(row) * ld;
-  const float wgt = weights ? weights[row] : 1.f;
   const int nv = V >> 3;
+  auto clear = [&] {
+    for (int c = threadIdx.x; c < nv; c += CE_THREADS) reinterpret_cast<uint4*>(lr)[c] = make_uint4(0, 0, 0, 0);
+    for (int c = nv * 8 + threadIdx.x; c < V; c += CE_THREADS) lr[c] = __float2bfloat16_rn(0.f);
+  };
+  if (list.rows != nullptr) {
+    const int at = list.from + row, used = *list.used;
+    if (at >= used) {
+      if (write_grad && at < (used + 63) / 64 * 64) clear();
+      return;
+    }
+    row = list.rows[at];
+  }
+  const float wgt = weights ? weights[row] : 1.f;
+  const long long tgt = targets[row];
+  const bool in_vocab = tgt >= 0 && tgt < V;
+  const bool valid = in_vocab && wgt != 0.f;
+  if (!valid && lse_out == nullptr && pa.logp_out == nullptr) {      // nothing of a masked row is asked for
+    if (write_grad) clear();
+    return;
+  }
   const uint4* lv = reinterpret_cast<const uint4*>(lr);
   float m = -INFINITY, s = 0.f;
   for (int c = threadIdx.x; c < nv; c += CE_THREADS) {
@@ -325,9 +351,6 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
   s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
   const float gs = block_sum(s, red);
   const float lse = gm + __logf(gs);
-  long long tgt = targets[row];
-  const bool in_vocab = tgt >= 0 && tgt < V;
-  const bool valid = in_vocab && wgt != 0.f;
   const float logp = in_vocab ? __bfloat162float(lr[tgt]) - lse : 0.f;
   float row_loss = -logp, dl_dlogp = -1.f;
   if (pa.mode == 1 && valid) {
@@ -368,6 +391,43 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
     float p = __expf(__bfloat162float(lr[c]) - lse);
     if (c == tgt) p -= 1.f;
     lr[c] = __float2bfloat16_rn(p * scale);
+  }
+}
+
+// =============================================================== rows that the loss scores
+__global__ void __launch_bounds__(1024)
+scored_rows_kernel(const long long* __restrict__ targets, const float* __restrict__ weights, int T, int V,
+                   int* __restrict__ rows, int* __restrict__ slot, int* __restrict__ count) {
+  __shared__ int per_warp[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int base = 0;
+  for (int t0 = 0; t0 < T; t0 += 1024) {
+    const int t = t0 + threadIdx.x;
+    const long long tgt = t < T ? targets[t] : -1;
+    const bool scored = tgt >= 0 && tgt < V && (weights == nullptr || weights[t] != 0.f);
+    const unsigned vote = __ballot_sync(0xffffffffu, scored);
+    if (lane == 0) per_warp[warp] = __popc(vote);
+    __syncthreads();
+    const int mine = per_warp[lane];
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? mine : 0);
+    const int at = base + before + __popc(vote & ((1u << lane) - 1));
+    base += __reduce_add_sync(0xffffffffu, mine);
+    if (t < T) slot[t] = scored ? at : -1;
+    if (scored) rows[at] = t;
+    __syncthreads();
+  }
+  for (int i = base + threadIdx.x; i < T; i += 1024) rows[i] = -1;
+  if (threadIdx.x == 0) *count = base;
+}
+__global__ void __launch_bounds__(256)
+take_rows_kernel(const bf16* x, long long ldx, const int* index, bf16* out, long long ldo, int n, int D) {
+  chain_wait();
+  chain_release();
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int from = index[i];
+    const uint4* src = reinterpret_cast<const uint4*>(x + from * ldx);
+    uint4* dst = reinterpret_cast<uint4*>(out + i * ldo);
+    for (int c = threadIdx.x; c < D / 8; c += 256) dst[c] = from < 0 ? make_uint4(0, 0, 0, 0) : src[c];
   }
 }
 
@@ -724,7 +784,7 @@ int ss_cross_entropy(void* logits, const long long* targets, const float* weight
   if (ld % 8) return -2;
   if (R <= 0) return 0;
   cross_entropy_kernel<<<R, CE_THREADS, 0, (cudaStream_t)stream>>>(
-      (bf16*)logits, targets, weights, loss_sum, lse, R, V, ld, grad_scale, write_grad, PolicyArgs{});
+      (bf16*)logits, targets, weights, loss_sum, lse, R, V, ld, grad_scale, write_grad, PolicyArgs{}, RowList{});
   return (int)cudaGetLastError();
 }
 // Token objectives on a logits block: mode 0 cross-entropy, mode 1 clipped policy
@@ -739,7 +799,36 @@ int ss_token_objective(void* logits, const long long* targets, const float* weig
   if (R <= 0) return 0;
   PolicyArgs pa{mode, old_logp, advantage, ref_logp, clip, ref_beta, logp_out};
   cross_entropy_kernel<<<R, CE_THREADS, 0, (cudaStream_t)stream>>>(
-      (bf16*)logits, targets, weights, loss_sum, nullptr, R, V, ld, grad_scale, write_grad, pa);
+      (bf16*)logits, targets, weights, loss_sum, nullptr, R, V, ld, grad_scale, write_grad, pa, RowList{});
+  return (int)cudaGetLastError();
+}
+// The same on a block of listed rows (see RowList): targets, weights and the policy's inputs are indexed by token.
+int ss_token_objective_rows(void* logits, const long long* targets, const float* weights, const int* rows,
+                            const int* used, int from, float* loss_sum, int R, int V, long long ld, float grad_scale,
+                            int write_grad, int mode, const float* old_logp, const float* advantage, float clip,
+                            const float* ref_logp, float ref_beta, void* stream) {
+  if (ld % 8 || mode < 0 || mode > 1 || rows == nullptr || used == nullptr) return -2;
+  if (mode == 1 && (!old_logp || !advantage)) return -2;
+  if (R <= 0) return 0;
+  cross_entropy_kernel<<<R, CE_THREADS, 0, (cudaStream_t)stream>>>(
+      (bf16*)logits, targets, weights, loss_sum, nullptr, R, V, ld, grad_scale, write_grad,
+      PolicyArgs{mode, old_logp, advantage, ref_logp, clip, ref_beta, nullptr}, RowList{rows, used, from});
+  return (int)cudaGetLastError();
+}
+// rows: the tokens whose loss counts (a target in [0, V) and a weight that is not zero), in order, then -1 up to T;
+// slot: each token's place in that list or -1; count: their number.
+int ss_scored_rows(const long long* targets, const float* weights, int T, int V, int* rows, int* slot, int* count,
+                   void* stream) {
+  if (T <= 0) return 0;
+  scored_rows_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(targets, weights, T, V, rows, slot, count);
+  return (int)cudaGetLastError();
+}
+// out[i] = x[index[i]], or a row of zeros where index[i] < 0.
+int ss_take_rows(const void* x, long long ldx, const int* index, void* out, long long ldo, int n, int D, void* stream) {
+  if (D % 8 || ldx % 8 || ldo % 8) return -2;
+  if (n <= 0) return 0;
+  launch_chained(take_rows_kernel, n < 148 * 16 ? n : 148 * 16, 256, 0, (cudaStream_t)stream, (const bf16*)x, ldx, index,
+                 (bf16*)out, ldo, n, D);
   return (int)cudaGetLastError();
 }
 int ss_adamw_sr(void* p, const void* g, void* m, void* v, long long n, int g_f32, float lr,

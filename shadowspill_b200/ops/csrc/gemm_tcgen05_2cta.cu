@@ -73,7 +73,13 @@ struct Params {
   float alpha;
   int* status;
   EpiArgs e;
+  const int* used;                 // optional: rows in use, of which this GEMM has those from `used_from` on
+  int used_from;                   // (rows of A and C, or with A_MN of the contraction, up to M or K)
 };
+
+__device__ __forceinline__ int rows_in_use(const Params& p, int rows) {
+  return p.used == nullptr ? rows : max(0, min(rows, *p.used - p.used_from));
+}
 
 constexpr int GATHER_THREADS = 128;                  // warps 10..13 of the GATHER form
 constexpr int PIECE_BYTES = 32768;
@@ -197,12 +203,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const bool leader = rank == 0;
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
-  const int num_m = (p.M + 2 * BM - 1) / (2 * BM);
   // columns of p.N that a tile takes; with gate and up side by side rank 0 stages the rows of the one, rank 1 the other's
   constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
   const int num_n = (p.N + TILE_N - 1) / TILE_N;
-  const int num_tiles = num_m * num_n;
-  const int num_kb = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -228,6 +231,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   chain_wait();
   if (!GATHER) chain_release();   // a kernel that waits for peers keeps the next one off the GPU
   const uint32_t tmem_base = *tmem_slot;
+  const int rows = A_MN ? p.M : rows_in_use(p, p.M);
+  const int num_m = (rows + 2 * BM - 1) / (2 * BM), num_tiles = num_m * num_n;
+  const int num_kb = ((A_MN ? rows_in_use(p, p.K) : p.K) + BK - 1) / BK;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -290,7 +296,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int t = pair_id; t < num_tiles && ok; t += num_pairs) {
+      for (int t = pair_id; t < num_tiles && ok && num_kb > 0; t += num_pairs) {
         if (!mbar_wait(&tempty[acc], acc_phase ^ 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
@@ -325,7 +331,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     for (int t = pair_id; t < num_tiles; t += num_pairs) {
       int mb, nb;
       tile_coords<GATHER>(t, num_m, num_n, mb, nb);
-      if (!mbar_wait(&tfull[acc], acc_phase, p.status, KS_TIMEOUT_TMEM_FULL)) break;
+      if (A_MN && num_kb == 0) {          // nothing to contract: zero, or what is there already
+        if (p.accumulate) break;
+      } else if (!mbar_wait(&tfull[acc], acc_phase, p.status, KS_TIMEOUT_TMEM_FULL)) {
+        break;
+      }
       tc_fence_after();
       const int row0 = mb * (2 * BM) + static_cast<int>(rank) * BM + q * 32;
       const uint32_t taddr =
@@ -346,6 +356,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           epilogue_swiglu_bwd_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc, p.e, row0, p.M, col0, p.N);
         } else {
           tmem_ld_wait();
+          if (A_MN && num_kb == 0) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) r[e] = 0;
+          }
           if (p.c_f32)
             epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C),
                                  p.accumulate ? reinterpret_cast<const float*>(p.e.src) : nullptr, p.e.ldsrc, p.alpha,
@@ -484,6 +498,36 @@ int ss_gemm2_residual_bf16(const void* A, const void* B, const void* src, void* 
   if (M < 256 || N < 128)
     return ss::gemm_from(A, B, src, C, ldsrc, M, N, K, lda, ldb, ldc, 0, 0, 0, 1, 1.f, 0, 0, status, stream);
   return ss::pair::gemm2_from(A, B, src, C, ldsrc, M, N, K, lda, ldb, ldc, 0, 0, 0, 1, 1.f, 0, status, stream);
+}
+
+// The bf16 GEMM over rows of which the device knows how many are in use: `*used - from` of the M rows of A and C, or with
+// a_mn of the K rows that are contracted (those up to the next multiple of 64 must be zero in one operand and finite in
+// the other). Rows past them are neither computed nor written.
+int ss_gemm2_rows_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                       long long ldc, int a_mn, int b_mn, int accumulate, const int* used, int from, int* status,
+                       void* stream) {
+  using namespace ss;
+  using namespace ss::pair;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (ldc % 8) || (N % 8) || used == nullptr || (a_mn && !b_mn) ||
+      (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) ||
+      (reinterpret_cast<uintptr_t>(C) & 15))
+    return -2;
+  int dev = 0, num_sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  CUtensorMap ta, tb;
+  int r;
+  if (!a_mn) r = make_tmap_bf16(&ta, A, M, K, lda, BM);
+  else       r = make_tmap_bf16(&ta, A, K, M, lda, BK);
+  if (r) return r;
+  if (!b_mn) r = make_tmap3_bf16(&tb, B, 1, N, K, ldb, static_cast<long long>(N) * ldb, BN / 2);
+  else       r = make_tmap3_bf16(&tb, B, 1, K, N, ldb, static_cast<long long>(K) * ldb, BK);
+  if (r) return r;
+  Params p{C, M, N, K, ldc, 0, accumulate, 1.f, status, {C, ldc}, used, from};
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (a_mn) return launch<true, true>(ta, tb, p, num_sms, s);
+  return b_mn ? launch<false, true>(ta, tb, p, num_sms, s) : launch<false, false>(ta, tb, p, num_sms, s);
 }
 
 // ss_gemm_swiglu_bf16 and ss_gemm_swiglu_bwd_bf16 on CTA pairs (argument checks as there, which takes M < 256, narrow
