@@ -39,10 +39,12 @@ struct GemmCfg {
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (BN == 256) ? 4 : 6;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int OFF_EPI = STAGES * STAGE_BYTES;      // epilogue staging, then barriers
+  static constexpr int SMEM = OFF_EPI + EPI_STAGE + 256 /*barriers*/ + 1024 /*align*/;
   // scatter epilogue only: per epilogue warp a 32-row x 128-column bf16 staging tile, so that
   // rows leave the SM as whole 256-byte runs (peer stores want full lines, not 16-byte pieces)
   static constexpr int SCATTER_STAGE = 4 * 32 * 256;
+  static_assert(SCATTER_STAGE <= EPI_STAGE, "it is the epilogue's staging");
   static constexpr int TMEM_COLS = 2 * BN;  // 512 or 256
 };
 
@@ -73,6 +75,7 @@ struct GemmParams {
   long long ldc;
   int c_f32;
   int accumulate;
+  int tma_out;                // the products leave by TMA through tmC
   int a_mn, b_mn;
   int* status;
   float alpha;
@@ -109,8 +112,7 @@ __device__ __forceinline__ TileWork decode_tile(const GemmParams& p, int t, int 
     w.kb0 = lo / BK;
     w.nkb = (hi - lo) / BK;
     // Blocks that are all padding add nothing: a segment of up to 64 rows needs one block of its two
-    // (128 experts, 62 rows each on average, both bank gradients: 410 -> 402 us; the stores of 1.2 GB
-    // at 3.0 TB/s bound them, a kernel that only writes reaches 3.9 TB/s).
+    // (128 experts, 62 rows each on average, both bank gradients: 410 -> 402 us, when their stores bound them).
     if (p.g.expert_rows) w.nkb = min(w.nkb, (p.g.expert_rows[w.expert] + BK - 1) / BK);
     w.c_off = static_cast<long long>(w.expert) * p.g.c_expert_stride;
   } else {
@@ -126,14 +128,14 @@ __device__ __forceinline__ TileWork decode_tile(const GemmParams& p, int t, int 
 template <int BN, bool A_MN, bool B_MN, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
   using Cfg = GemmCfg<BN>;
   // columns of p.N that a tile takes: with gate and up side by side half of its own
   constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: the 128B swizzle pattern repeats every 8 rows = 1024 B.
   uint8_t* smem = align_smem_1024(smem_raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_EPI + EPI_STAGE);
   uint64_t* full = bars;
   uint64_t* empty = bars + Cfg::STAGES;
   uint64_t* tfull = bars + 2 * Cfg::STAGES;
@@ -265,7 +267,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may touch
     const int part = (warp - 2) >> 2;    // the left or the right half of the tile's columns
-    const uint32_t stage_out = smem_u32(smem + Cfg::STAGES * Cfg::STAGE_BYTES + 256) + (warp - 2) * EPI_WARP_STAGE;
+    const uint32_t stage_out = smem_u32(smem + Cfg::OFF_EPI) + (warp - 2) * EPI_WARP_STAGE;
+    const bool issuer = ((warp - 2) & 3) == 0 && lane == 0;
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
@@ -298,7 +301,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // Scatter epilogue. Each thread owns one accumulator row; the rows are transposed
         // through an XOR-swizzled staging tile so that 16 lanes store one row's 256
         // contiguous bytes at its destination address.
-        uint8_t* stg = smem + Cfg::STAGES * Cfg::STAGE_BYTES + 256 + q * (32 * 256);
+        uint8_t* stg = smem + Cfg::OFF_EPI + q * (32 * 256);
         const long long my_dst = (row < p.M) ? p.g.row_dst[row] : 0;
 #pragma unroll 1
         for (int half = 0; half < (part == 0 ? BN / 128 : 0); ++half) {   // one staging tile per lane quarter
@@ -332,6 +335,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           __syncwarp();
         }
+      } else if (EPI == EPI_PLAIN && p.tma_out) {
+        epilogue_tma(smem + Cfg::OFF_EPI + part * EPI_BLOCK, taddr + part * (BN / 2), BN / 128, part, q * 32 + lane, issuer,
+                     &tmC, p.alpha, nb * BN + part * (BN / 2), p.N, mb * BM, p.M,
+                     p.g.mode == 2 ? w.expert : 0, [&] {
+                       tc_fence_before();
+                       __syncwarp();
+                       if (lane == 0) mbar_arrive(&tempty[acc]);
+                     });
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1;
+        }
+        continue;
       } else
 #pragma unroll 1
       for (int c = part * (TILE_N / 64); c < (part + 1) * (TILE_N / 64); ++c) {
@@ -367,6 +383,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         acc_phase ^= 1;
       }
     }
+    if (issuer && p.tma_out) tma_store_wait<0>();
   }
 
   tc_fence_before();
@@ -437,21 +454,30 @@ int make_tmap3_bf16(CUtensorMap* map, const void* base, long long experts, long 
 }
 
 template <int BN, bool A_MN, bool B_MN, int EPI = EPI_PLAIN>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int num_sms,
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& params, int num_sms,
                   cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
+  GemmParams p = params;
+  CUtensorMap tc = ta;                                       // unused unless tma_out
+  p.tma_out = EPI == EPI_PLAIN && !p.c_f32 && !p.accumulate && p.g.row_dst == nullptr;
+  if (p.tma_out) {
+    const long long matrices = p.g.mode == 2 ? p.g.n_experts : 1;
+    if (int r = make_tmap3_bf16(&tc, p.C, matrices, p.M, p.N, p.ldc,
+                                p.g.mode == 2 ? p.g.c_expert_stride : static_cast<long long>(p.M) * p.ldc, BM))
+      return r;
+  }
   static SmemOptIn opt_in;
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, EPI>;
   constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
-  if (int e = opt_in.ensure(kern, Cfg::SMEM + Cfg::SCATTER_STAGE)) return e;
-  const int smem_bytes = Cfg::SMEM + (p.g.row_dst != nullptr ? Cfg::SCATTER_STAGE : EPI_WARPS * EPI_WARP_STAGE);
+  if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
+  const int smem_bytes = Cfg::SMEM;
   const long long tiles = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + TILE_N - 1) / TILE_N) *
                           (p.g.mode == 2 ? p.g.n_experts : 1);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
   // Not the expert banks: chaining them and the kernels around them cost 5 % (64 experts, 8,192 tokens,
   // forward and backward 2883 -> 3034 us) and gave nothing for 128 experts and 1,000 tokens.
-  if (p.g.mode == 0) launch_chained(kern, grid, GEMM_THREADS, smem_bytes, stream, ta, tb, p);
-  else kern<<<grid, GEMM_THREADS, smem_bytes, stream>>>(ta, tb, p);
+  if (p.g.mode == 0) launch_chained(kern, grid, GEMM_THREADS, smem_bytes, stream, ta, tb, tc, p);
+  else kern<<<grid, GEMM_THREADS, smem_bytes, stream>>>(ta, tb, tc, p);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -62,7 +62,9 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int B_BYTES = (BN / 2) * BK * 2;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;       // 32 KB per CTA per stage
 constexpr int STAGES = 6;
-constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256 + EPI_WARPS * EPI_WARP_STAGE;
+constexpr int OFF_EPI = STAGES * STAGE_BYTES;       // epilogue staging, then barriers
+constexpr int SMEM = OFF_EPI + EPI_STAGE + 256 + 1024;
+static_assert(SMEM <= 232448, "shared memory budget");
 constexpr int TMEM_COLS = 2 * BN;
 
 struct Params {
@@ -75,6 +77,7 @@ struct Params {
   EpiArgs e;
   const int* used;                 // optional: rows in use, of which this GEMM has those from `used_from` on
   int used_from;                   // (rows of A and C, or with A_MN of the contraction, up to M or K)
+  int tma_out;                     // the products leave by TMA through tmC
 };
 
 __device__ __forceinline__ int rows_in_use(const Params& p, int rows) {
@@ -187,10 +190,10 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& mb
 template <bool A_MN, bool B_MN, bool GATHER, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_THREADS : THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const Params p, const GatherArgs ga) {
+                  const __grid_constant__ CUtensorMap tmC, const Params p, const GatherArgs ga) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_EPI + EPI_STAGE);
   uint64_t* full = bars;                    // used in the leader only
   uint64_t* empty = bars + STAGES;          // per CTA, signalled by the leader's commit
   uint64_t* tfull = bars + 2 * STAGES;      // per CTA, signalled by the leader's commit
@@ -324,7 +327,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else if (warp < 2 + EPI_WARPS) {
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
-    const uint32_t stage_out = smem_u32(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * EPI_WARP_STAGE;
+    const uint32_t stage_out = smem_u32(smem + OFF_EPI) + (warp - 2) * EPI_WARP_STAGE;
+    const bool issuer = ((warp - 2) & 3) == 0 && lane == 0;
     const int part = (warp - 2) >> 2;    // the left or the right half of the tile's columns
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -340,6 +344,16 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const int row0 = mb * (2 * BM) + static_cast<int>(rank) * BM + q * 32;
       const uint32_t taddr =
           tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN);
+      if (!GATHER && EPI == EPI_PLAIN && p.tma_out && num_kb > 0) {
+        epilogue_tma(smem + OFF_EPI + part * EPI_BLOCK, taddr + part * (BN / 2), BN / 128, part, q * 32 + lane, issuer,
+                     &tmC, p.alpha, nb * BN + part * (BN / 2), p.N, row0 - q * 32, p.M, 0, [&] {
+                       tc_fence_before();
+                       __syncwarp();
+                       if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&tempty[acc]), 0));
+                     });
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        continue;
+      }
 #pragma unroll 1
       for (int c = part * (TILE_N / 64); c < (part + 1) * (TILE_N / 64); ++c) {
         const int col0 = nb * TILE_N + c * 32;
@@ -375,6 +389,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&tempty[acc]), 0));
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
+    if (issuer && p.tma_out) tma_store_wait<0>();
   }
 
   else if (GATHER) {
@@ -414,8 +429,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 }
 
 template <bool A_MN, bool B_MN, int EPI = EPI_PLAIN>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int num_sms,
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& params, int num_sms,
                   cudaStream_t stream) {
+  Params p = params;
+  CUtensorMap tc = ta;                                       // unused unless tma_out
+  p.tma_out = EPI == EPI_PLAIN && !p.c_f32 && !p.accumulate;
+  if (p.tma_out)
+    if (int r = make_tmap3_bf16(&tc, p.C, 1, p.M, p.N, p.ldc, static_cast<long long>(p.M) * p.ldc, BM)) return r;
   static SmemOptIn opt_in;
   auto kern = gemm2_bf16_kernel<A_MN, B_MN, false, EPI>;
   constexpr int TILE_N = EPI == EPI_SWIGLU ? BN / 2 : BN;
@@ -423,7 +443,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p,
   const long long tiles = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + TILE_N - 1) / TILE_N);
   long long pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  launch_chained(kern, static_cast<int>(2 * pairs), THREADS, SMEM, stream, ta, tb, p, GatherArgs{});
+  launch_chained(kern, static_cast<int>(2 * pairs), THREADS, SMEM, stream, ta, tb, tc, p, GatherArgs{});
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -435,7 +455,7 @@ static int launch_gather(const CUtensorMap& ta, const CUtensorMap& tb, const Par
   const long long tiles = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   long long pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  kern<<<static_cast<int>(2 * pairs), THREADS + GATHER_THREADS, SMEM, stream>>>(ta, tb, p, ga);
+  kern<<<static_cast<int>(2 * pairs), THREADS + GATHER_THREADS, SMEM, stream>>>(ta, tb, ta, p, ga);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -502,7 +522,7 @@ int ss_gemm2_residual_bf16(const void* A, const void* B, const void* src, void* 
 
 // The bf16 GEMM over rows of which the device knows how many are in use: `*used - from` of the M rows of A and C, or with
 // a_mn of the K rows that are contracted (those up to the next multiple of 64 must be zero in one operand and finite in
-// the other). Rows past them are neither computed nor written.
+// the other). Tiles past them are neither computed nor written.
 int ss_gemm2_rows_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                        long long ldc, int a_mn, int b_mn, int accumulate, const int* used, int from, int* status,
                        void* stream) {
