@@ -136,7 +136,7 @@ __device__ __forceinline__ void tmem_st_quarter(uint32_t addr, const uint32_t (&
 // Both are issued before dS of this tile is waited for, so two warps may be a tile apart: dS has a barrier
 // for even and one for odd tiles, or a warp a tile ahead would count for one that has yet to write. dP of the
 // next tile waits until all warps have read this one's, so one barrier is enough there.
-template <int DH, int BKV, int KS, int VS>
+template <int DH, int BKV, int KS, int VS, int CTAS>
 struct DqCfg {
   static constexpr int Q_BYTES = 128 * DH * 2;
   static constexpr int KV_BYTES = BKV * DH * 2;
@@ -146,16 +146,17 @@ struct DqCfg {
   static constexpr int OFF_BAR = OFF_V + VS * KV_BYTES;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
   static constexpr int TM_S = 0, TM_DP = 2 * BKV, TM_DQ = 3 * BKV;
-  static_assert(TM_DQ + DH <= 512, "TMEM budget");
-  static_assert(SMEM <= 232448, "shared memory budget");
+  static constexpr int TM_COLS = TM_DQ + DH <= 256 ? 256 : 512;
+  static_assert(TM_DQ + DH <= TM_COLS && CTAS * TM_COLS <= 512, "TMEM budget");
+  static_assert(CTAS * (SMEM + 1024) <= 233472, "shared memory budget");
 };
 
-template <int DH, int BKV, int KS, int VS>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+template <int DH, int BKV, int KS, int VS, int CTAS>
+__global__ void __launch_bounds__(BW_THREADS, CTAS)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const AttnBwdParams p) {
-  using Cfg = DqCfg<DH, BKV, KS, VS>;
+  using Cfg = DqCfg<DH, BKV, KS, VS, CTAS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
@@ -186,7 +187,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(dq_done, 1);
     mbar_fence_init();
   }
-  if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, Cfg::TM_COLS); tmem_relinquish(); }
   chain_wait();
   if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, rank, slot);
   tc_fence_before();
@@ -345,7 +346,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == BW_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  if (warp == BW_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, Cfg::TM_COLS); }
 }
 
 // ============================================================================ dKV kernel
@@ -379,7 +380,7 @@ __device__ __forceinline__ uint32_t sum_offset(int row, int cols, int c4) {
   return row * cols * 4 + (((c4 & ~7) | ((c4 ^ row) & 7)) << 4);
 }
 
-template <int DH, int BQ, int QS, int DOS, int MODE>
+template <int DH, int BQ, int QS, int DOS, int MODE, int CTAS>
 struct DkvCfg {
   static constexpr bool DO_DV = MODE != MODE_DK;
   static constexpr bool DO_DK = MODE != MODE_DV;
@@ -397,17 +398,18 @@ struct DkvCfg {
   static constexpr int TM_DV = 2 * BQ;
   static constexpr int TM_DK = TM_DV + (DO_DV ? DH : 0);
   static constexpr int SUMS = (DO_DV ? DH : 0) + (DO_DK ? DH : 0);
-  static_assert(TM_DK + (DO_DK ? DH : 0) <= 512, "TMEM budget");
+  static constexpr int TM_COLS = TM_DK + (DO_DK ? DH : 0) <= 256 ? 256 : 512;
+  static_assert(TM_DK + (DO_DK ? DH : 0) <= TM_COLS && CTAS * TM_COLS <= 512, "TMEM budget");
   static_assert(128 * SUMS * 4 <= OFF_STAT, "the sums of a tile reuse the operands' space");
-  static_assert(SMEM <= 232448, "shared memory budget");
+  static_assert(CTAS * (SMEM + 1024) <= 233472, "shared memory budget");
 };
 
-template <int DH, int BQ, int QS, int DOS, int MODE>
-__global__ void __launch_bounds__(BW_THREADS, 1)
+template <int DH, int BQ, int QS, int DOS, int MODE, int CTAS>
+__global__ void __launch_bounds__(BW_THREADS, CTAS)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const AttnBwdParams p) {
-  using Cfg = DkvCfg<DH, BQ, QS, DOS, MODE>;
+  using Cfg = DkvCfg<DH, BQ, QS, DOS, MODE, CTAS>;
   constexpr int STS = Cfg::STS, SB = Cfg::SB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
@@ -449,7 +451,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(acc_done, 1);
     mbar_fence_init();
   }
-  if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == BW_MMA_WARP) { tmem_alloc(tmem_slot, Cfg::TM_COLS); tmem_relinquish(); }
   chain_wait();
   if (warp == BW_TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, rank, slot);
   tc_fence_before();
@@ -743,14 +745,14 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == BW_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  if (warp == BW_MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, Cfg::TM_COLS); }
 }
 
-template <int DH, int BKV, int KS, int VS>
+template <int DH, int BKV, int KS, int VS, int CTAS>
 static int launch_dq(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk,
                      const CUtensorMap& tv, const AttnBwdParams& p, int tiles, cudaStream_t s) {
-  using Cfg = DqCfg<DH, BKV, KS, VS>;
-  auto kern = attn_bwd_dq_kernel<DH, BKV, KS, VS>;
+  using Cfg = DqCfg<DH, BKV, KS, VS, CTAS>;
+  auto kern = attn_bwd_dq_kernel<DH, BKV, KS, VS, CTAS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
   const long long grid = static_cast<long long>(p.Hq) * tiles;       // see attention_fwd.cu
@@ -759,11 +761,11 @@ static int launch_dq(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtens
   return static_cast<int>(cudaGetLastError());
 }
 
-template <int DH, int BQ, int QS, int DOS, int MODE>
+template <int DH, int BQ, int QS, int DOS, int MODE, int CTAS>
 static int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tk,
                       const CUtensorMap& tv, const AttnBwdParams& p, int tiles, cudaStream_t s) {
-  using Cfg = DkvCfg<DH, BQ, QS, DOS, MODE>;
-  auto kern = attn_bwd_dkv_kernel<DH, BQ, QS, DOS, MODE>;
+  using Cfg = DkvCfg<DH, BQ, QS, DOS, MODE, CTAS>;
+  auto kern = attn_bwd_dkv_kernel<DH, BQ, QS, DOS, MODE, CTAS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
   cudaLaunchConfig_t cfg = {};
@@ -836,7 +838,7 @@ extern "C" int ss_attn_bwd_g(const void* q, const void* k, const void* v, const 
   const int tiles = (T + 127) / 128 + nseq;
   p.split = key_tile_split(static_cast<long long>((T + 127) / 128) * Hkv, Hq / Hkv);
   const long long qc = static_cast<long long>(Hq) * dh, kc = static_cast<long long>(Hkv) * dh;
-  const int stream_rows = dh == 256 ? 64 : 128;     // rows of the streamed tiles
+  const int stream_rows = dh == 128 ? 128 : 64;     // rows of the streamed tiles
   CUtensorMap tq128, tdo128, tk128, tv128, tqs, tdos, tks, tvs;
   int r;
   if ((r = make_tmap_bf16(&tq128, q, T, qc, ldq, 128))) return r;
@@ -848,17 +850,17 @@ extern "C" int ss_attn_bwd_g(const void* q, const void* k, const void* v, const 
   if ((r = make_tmap_bf16(&tks, k, T, kc, ldk, stream_rows))) return r;
   if ((r = make_tmap_bf16(&tvs, v, T, kc, ldv, stream_rows))) return r;
   if (dh == 128) {
-    if ((r = launch_dq<128, 128, 3, 2>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
-    return launch_dkv<128, 128, 2, 2, MODE_BOTH>(tqs, tdos, tk128, tv128, p, tiles, s);
+    if ((r = launch_dq<128, 128, 3, 2, 1>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
+    return launch_dkv<128, 128, 2, 2, MODE_BOTH, 1>(tqs, tdos, tk128, tv128, p, tiles, s);
   }
   if (dh == 64) {
-    if ((r = launch_dq<64, 128, 3, 2>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
-    return launch_dkv<64, 128, 2, 2, MODE_BOTH>(tqs, tdos, tk128, tv128, p, tiles, s);
+    if ((r = launch_dq<64, 64, 3, 2, 2>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
+    return launch_dkv<64, 64, 2, 2, MODE_BOTH, 2>(tqs, tdos, tk128, tv128, p, tiles, s);
   }
   if (dh == 256) {
-    if ((r = launch_dq<256, 64, 2, 1>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
-    if ((r = launch_dkv<256, 64, 2, 2, MODE_DV>(tqs, tdos, tk128, tv128, p, tiles, s))) return r;
-    return launch_dkv<256, 64, 2, 1, MODE_DK>(tqs, tdos, tk128, tv128, p, tiles, s);
+    if ((r = launch_dq<256, 64, 2, 1, 1>(tq128, tdo128, tks, tvs, p, tiles, s))) return r;
+    if ((r = launch_dkv<256, 64, 2, 2, MODE_DV, 1>(tqs, tdos, tk128, tv128, p, tiles, s))) return r;
+    return launch_dkv<256, 64, 2, 1, MODE_DK, 1>(tqs, tdos, tk128, tv128, p, tiles, s);
   }
   return -2;
 }

@@ -1,22 +1,20 @@
 // Packed variable-length causal GQA attention, forward, for sm_100a.
 //
-// Head widths 64 and 128: one CTA per (two adjacent 128-query tiles of one sequence, query head).
-// Each tile has its own softmax warpgroup, its own two score buffers and its own O accumulator in
-// TMEM (4 x 64 + 2 x DH columns). Head width 256: O takes half of TMEM, so a CTA has one tile.
+// One CTA per (128-query tile of a sequence, query head). Head widths 64 and 128 take half of TMEM (two 64-key score
+// buffers and O) and half of an SM's shared memory, so two CTAs share an SM: one's set-up, waits and epilogue run under
+// the other's steps, and neither waits for the other's probabilities. Two tiles in one CTA shared K and V, but their
+// products were issued by one warp in one order. Head width 256: O takes half of TMEM, one CTA per SM.
 // S = Q K^T of the next 64 keys is always issued before O += P V of these, so the softmax warps never
-// wait for a product; the 64-key score products read shared memory at 1.5 times its rate, but one
-// 128-key buffer per tile instead left each tile waiting for P V and S in turn (1.09 against 1.02 ms
-// in the long case below).
+// wait for a product.
 // P goes back to TMEM over the scores it comes from and is the A operand of P V from there: it never
 // passes through shared memory, whose bandwidth the two products need for K, V and Q.
-// Measured, 16,384 tokens in two sequences, 32/8 heads of 128: 1.41 -> 0.95 ms; 8,192 packed tokens:
-// 0.317 -> 0.209 ms; 6,001 tokens, 16/4 heads of 256: 0.285 -> 0.150 ms, against one tile per CTA and
-// P through shared memory. What is left is the softmax warps' chain (read, maximum, exponentials, write): in
-// the long case 128 x 128 scores take 1804 cycles of an SM, with the exponential unit busy in 58 % of them, the
-// tensor pipe in 58 % and issue slots in 54 %. Replacing a quarter of the exponentials by polynomials of ten
-// instructions made it slower (1.08 against 0.97 ms).
+// Measured (two tiles in a CTA -> two CTAs): 8,192 packed tokens, 32/8 heads of 128: 0.221 -> 0.207 ms; 16,384 tokens in
+// two sequences: 0.970 -> 0.974 ms; 2,048 tokens in five sequences, 32/8 heads of 64, with the backward kernels
+// changed alike: 112 -> 94 us. 6,001 tokens, 16/4 heads of 256: 0.150 ms. What is left is the softmax
+// warps' chain (read, maximum, exponentials, write). Replacing a quarter of the exponentials by polynomials of ten
+// instructions made it slower (1.08 against 0.97 ms), and so did scores two steps ahead (1.04).
 //
-//   warps 0..4*NT-1  softmax, rescaling of O, epilogue: one query row per thread
+//   warps 0..3  softmax, rescaling of O, epilogue: one query row per thread
 //   then one TMA producer warp and one MMA warp
 //
 // The scores of step j + 1 are issued before P of step j is waited for, so two steps are in flight and the
@@ -40,21 +38,22 @@ namespace ss {
 int make_tmap_bf16(CUtensorMap* map, const void* base, long long rows, long long cols,
                    long long ld, int box_rows);  // gemm_tcgen05.cu
 
-// NT query tiles per CTA, BKV keys per step, KS / VS stages of K and V (K is released by its score
-// products, V one step later by P V).
-template <int DH, int NT, int BKV, int KS, int VS>
+// BKV keys per step, KS / VS stages of K and V (K is released by its score products, V one step later by P V), CTAS to
+// an SM.
+template <int DH, int BKV, int KS, int VS, int CTAS>
 struct AttnCfg {
-  static constexpr int THREADS = NT * 128 + 64;
-  static constexpr int TMA_WARP = NT * 4, MMA_WARP = NT * 4 + 1;
+  static constexpr int THREADS = 4 * 32 + 64;
+  static constexpr int TMA_WARP = 4, MMA_WARP = 5;
   static constexpr int QT_BYTES = 128 * DH * 2;
   static constexpr int KV_BYTES = BKV * DH * 2;        // one of K or V
-  static constexpr int OFF_K = NT * QT_BYTES;
+  static constexpr int OFF_K = QT_BYTES;
   static constexpr int OFF_V = OFF_K + KS * KV_BYTES;
   static constexpr int OFF_BAR = OFF_V + VS * KV_BYTES;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
-  static constexpr int TM_O = NT * 2 * BKV;            // behind the two score buffers of each tile
-  static_assert(TM_O + NT * DH <= 512, "TMEM budget");
-  static_assert(SMEM <= 232448, "shared memory budget");
+  static constexpr int TM_O = 2 * BKV;                 // behind the two score buffers
+  static constexpr int TM_COLS = TM_O + DH <= 256 ? 256 : 512;
+  static_assert(TM_O + DH <= TM_COLS && CTAS * TM_COLS <= 512, "TMEM budget");
+  static_assert(CTAS * (SMEM + 1024) <= 233472, "shared memory budget");
 };
 
 struct AttnParams {
@@ -67,11 +66,11 @@ struct AttnParams {
   int* status;
 };
 
-template <int DH, int NT, int BKV, int KS, int VS>
-__global__ void __launch_bounds__(NT * 128 + 64, 1)
+template <int DH, int BKV, int KS, int VS, int CTAS>
+__global__ void __launch_bounds__(192, CTAS)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
-  using Cfg = AttnCfg<DH, NT, BKV, KS, VS>;
+  using Cfg = AttnCfg<DH, BKV, KS, VS, CTAS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
@@ -80,12 +79,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* k_empty = k_full + KS;        // KS
   uint64_t* v_full = k_empty + KS;        // VS
   uint64_t* v_empty = v_full + VS;        // VS
-  uint64_t* s_full = v_empty + VS;        // [tile][buffer]
-  uint64_t* p_full = s_full + 2 * NT;     // [tile][step & 1]
-  uint64_t* o_done = p_full + 2 * NT;     // [tile][step & 1]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2 * NT);
-  TileSlot* slot = reinterpret_cast<TileSlot*>(o_done + 2 * NT + 1);
-  static_assert((1 + 2 * KS + 2 * VS + 6 * NT + 1) * 8 + sizeof(TileSlot) <= 256, "barrier space");
+  uint64_t* s_full = v_empty + VS;        // [buffer]
+  uint64_t* p_full = s_full + 2;          // [step & 1]
+  uint64_t* o_done = p_full + 2;          // [step & 1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+  TileSlot* slot = reinterpret_cast<TileSlot*>(o_done + 3);
+  static_assert((1 + 2 * KS + 2 * VS + 7) * 8 + sizeof(TileSlot) <= 256, "barrier space");
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -96,7 +95,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(q_full, 1);
     for (int i = 0; i < KS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < VS; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-    for (int i = 0; i < 2 * NT; ++i) {
+    for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 4);
       mbar_init(&o_done[i], 1);
@@ -104,40 +103,31 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_fence_init();
   }
   if (warp == Cfg::MMA_WARP) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, Cfg::TM_COLS);
     tmem_relinquish();
   }
   chain_wait();
-  if (warp == Cfg::TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, NT * 128, rank, slot);
+  if (warp == Cfg::TMA_WARP) find_tile_by_work(p.cu_seqlens, p.nseq, 128, rank, slot);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   chain_release();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int seq_start = slot->seq_start, seq_end = slot->seq_end;
-  const int q0 = seq_start + (slot->work - 1) * (NT * 128);
-  // key steps of each tile, up to its diagonal; none for a tile past the end of the sequence
-  int n_kv[NT];
-#pragma unroll
-  for (int i = 0; i < NT; ++i) {
-    const int lo = q0 + i * 128, hi = min(lo + 128, seq_end);
-    n_kv[i] = (slot->work > 0 && hi > lo) ? (hi - seq_start + BKV - 1) / BKV : 0;
-  }
-  const int n_max = max(n_kv[0], n_kv[NT - 1]);
+  const int q0 = seq_start + (slot->work - 1) * 128;
+  // key steps of the tile, up to its diagonal
+  const int n = slot->work > 0 ? (min(q0 + 128, seq_end) - seq_start + BKV - 1) / BKV : 0;
 
   if (warp == Cfg::TMA_WARP) {
     // ---------------------------------------------------------------- producer
-    if (n_max > 0 && elect_one()) {
+    if (n > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
-      mbar_expect_tx(q_full, NT * Cfg::QT_BYTES);
+      mbar_expect_tx(q_full, Cfg::QT_BYTES);
 #pragma unroll
-      for (int i = 0; i < NT; ++i)
-#pragma unroll
-        for (int c = 0; c < DH / 64; ++c)
-          tma_load_2d(smem + i * Cfg::QT_BYTES + c * (128 * 128), &tmQ, q_full, head * DH + c * 64, q0 + i * 128);
-      for (int j = 0; j < n_max; ++j) {
+      for (int c = 0; c < DH / 64; ++c) tma_load_2d(smem + c * (128 * 128), &tmQ, q_full, head * DH + c * 64, q0);
+      for (int j = 0; j < n; ++j) {
         const int ks = j % KS, vs = j % VS;
         const int k0 = seq_start + j * BKV;
         if (j >= KS && !mbar_wait(&k_empty[ks], ((j / KS) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
@@ -156,7 +146,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == Cfg::MMA_WARP) {
     // ---------------------------------------------------------------- MMA issuer
-    if (n_max > 0) {
+    if (n > 0) {
       const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, BKV, false, false);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, DH, false, true);
@@ -164,67 +154,46 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t sk0 = smem_u32(smem + Cfg::OFF_K), sv0 = smem_u32(smem + Cfg::OFF_V);
       // products of one issuing thread run in order: S may be issued over the P that the P V product
       // before it reads
-      auto issue_s = [&](int i, int j) {
-        const int b = 2 * i + (j & 1);
-        const uint32_t a = sq + i * Cfg::QT_BYTES, k = sk0 + (j % KS) * Cfg::KV_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < DH / 16; ++kk)
-          umma_bf16_if(leader, tmem_base + b * BKV, umma_smem_desc(a + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
-                    umma_smem_desc(k + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
-        umma_commit_if(leader, &s_full[b]);
-      };
-      auto wait_k = [&](int j) -> bool {
+      auto issue_s = [&](int j) -> bool {
         if (!mbar_wait(&k_full[j % KS], (j / KS) & 1, p.status, KS_TIMEOUT_FULL)) return false;
         tc_fence_after();
+        const uint32_t k = sk0 + (j % KS) * Cfg::KV_BYTES;
+#pragma unroll
+        for (int kk = 0; kk < DH / 16; ++kk)
+          umma_bf16_if(leader, tmem_base + (j & 1) * BKV, umma_smem_desc(sq + (kk >> 2) * (128 * 128) + (kk & 3) * 32, 16, 1024),
+                    umma_smem_desc(k + (kk >> 2) * (BKV * 128) + (kk & 3) * 32, 16, 1024), idesc_s, kk != 0);
+        umma_commit_if(leader, &s_full[j & 1]);
+        umma_commit_if(leader, &k_empty[j % KS]);
         return true;
       };
-      bool ok = mbar_wait(q_full, 0, p.status, KS_TIMEOUT_FULL) && wait_k(0);
-      if (ok) {
+      bool ok = mbar_wait(q_full, 0, p.status, KS_TIMEOUT_FULL) && issue_s(0);
+      for (int j = 0; j < n && ok; ++j) {
+        if (j + 1 < n) ok = issue_s(j + 1);
+        if (!ok || !mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL) ||
+            !mbar_wait(&p_full[j & 1], (j >> 1) & 1, p.status, KS_TIMEOUT_FULL))
+          break;
+        tc_fence_after();
+        const uint32_t v = sv0 + (j % VS) * Cfg::KV_BYTES, pa = tmem_base + (j & 1) * BKV;
 #pragma unroll
-        for (int i = 0; i < NT; ++i)
-          if (n_kv[i] > 0) issue_s(i, 0);
-        umma_commit_if(leader, &k_empty[0]);
-      }
-      for (int j = 0; j < n_max && ok; ++j) {
-        const bool more = j + 1 < n_max;
-        if (more) ok = wait_k(j + 1);
-        if (ok) ok = mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL);
-        if (!ok) break;
-        const uint32_t v = sv0 + (j % VS) * Cfg::KV_BYTES;
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          if (j + 1 < n_kv[i]) issue_s(i, j + 1);
-          if (more && i == NT - 1) umma_commit_if(leader, &k_empty[(j + 1) % KS]);
-          if (j >= n_kv[i]) continue;
-          ok = mbar_wait(&p_full[2 * i + (j & 1)], (j >> 1) & 1, p.status, KS_TIMEOUT_FULL);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t pa = tmem_base + (2 * i + (j & 1)) * BKV;
-#pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk)
-            umma_bf16_ts_if(leader, tmem_base + Cfg::TM_O + i * DH, pa + kk * 8,
-                         umma_smem_desc(v + kk * (16 * 128), BKV * 128, 1024), idesc_o, (j | kk) != 0);
-          umma_commit_if(leader, &o_done[2 * i + (j & 1)]);
-        }
-        if (!ok) break;
+        for (int kk = 0; kk < BKV / 16; ++kk)
+          umma_bf16_ts_if(leader, tmem_base + Cfg::TM_O, pa + kk * 8, umma_smem_desc(v + kk * (16 * 128), BKV * 128, 1024),
+                       idesc_o, (j | kk) != 0);
+        umma_commit_if(leader, &o_done[j & 1]);
         umma_commit_if(leader, &v_empty[j % VS]);
       }
     }
   } else {
     // ---------------------------------------------------------------- softmax warps
-    const int tile = warp >> 2, quarter = warp & 3;
-    const int n = NT == 2 && tile ? n_kv[NT - 1] : n_kv[0];
-    const int tq0 = q0 + tile * 128;
-    const int gq = tq0 + quarter * 32 + lane;    // global query index; its row is the TMEM lane
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t o_addr = lane_addr + Cfg::TM_O + tile * DH;
+    const int gq = q0 + warp * 32 + lane;        // global query index; its row is the TMEM lane
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    const uint32_t o_addr = lane_addr + Cfg::TM_O;
     const bool negative = p.scale_log2 < 0.f;    // the row maximum is taken before the scale
     const float c = fabsf(p.scale_log2);
     float m_used = -INFINITY;                    // reference max (log2 domain, scaled)
     float l = 0.f;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      const int b = 2 * tile + (j & 1);
+      const int b = j & 1;
       const uint32_t s_addr = lane_addr + b * BKV;
       if (!mbar_wait(&s_full[b], (j >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
@@ -238,7 +207,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int e = 0; e < BKV; ++e) s[e] = -s[e];
       }
       const int k0 = seq_start + j * BKV;
-      const bool diag = k0 + BKV - 1 > tq0;      // some key of this step may exceed some query
+      const bool diag = k0 + BKV - 1 > q0;      // some key of this step may exceed some query
       if (diag) {
 #pragma unroll
         for (int e = 0; e < BKV; ++e)
@@ -301,7 +270,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (lane == 0) mbar_arrive(&p_full[b]);
     }
     // ---------------------------------------------------------------- epilogue
-    if (ok && n > 0 && mbar_wait(&o_done[2 * tile + ((n - 1) & 1)], ((n - 1) >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
+    if (ok && n > 0 && mbar_wait(&o_done[(n - 1) & 1], ((n - 1) >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const bool valid = gq < seq_end;
@@ -334,25 +303,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   if (warp == Cfg::MMA_WARP) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, Cfg::TM_COLS);
   }
 }
 
-template <int DH, int NT, int BKV, int KS, int VS>
+template <int DH, int BKV, int KS, int VS, int CTAS>
 static int launch_fwd(const void* q, const void* k, const void* v, AttnParams p, long long ldq,
                       long long ldk, long long ldv, cudaStream_t stream) {
-  using Cfg = AttnCfg<DH, NT, BKV, KS, VS>;
+  using Cfg = AttnCfg<DH, BKV, KS, VS, CTAS>;
   CUtensorMap tq, tk, tv;
   int r;
   if ((r = make_tmap_bf16(&tq, q, p.T, static_cast<long long>(p.Hq) * DH, ldq, 128))) return r;
   if ((r = make_tmap_bf16(&tk, k, p.T, static_cast<long long>(p.Hkv) * DH, ldk, BKV))) return r;
   if ((r = make_tmap_bf16(&tv, v, p.T, static_cast<long long>(p.Hkv) * DH, ldv, BKV))) return r;
-  auto kern = attn_fwd_kernel<DH, NT, BKV, KS, VS>;
+  auto kern = attn_fwd_kernel<DH, BKV, KS, VS, CTAS>;
   static SmemOptIn opt_in;
   if (int e = opt_in.ensure(kern, Cfg::SMEM)) return e;
   // every sequence adds at most one partial tile; heads and tiles share x, whose limit many short sequences
   // do not reach (y ends at 65,535)
-  const long long grid = ((p.T + NT * 128 - 1) / (NT * 128) + static_cast<long long>(p.nseq)) * p.Hq;
+  const long long grid = ((p.T + 127) / 128 + static_cast<long long>(p.nseq)) * p.Hq;
   if (grid > 0x7fffffffLL) return -2;
   launch_chained(kern, static_cast<unsigned>(grid), Cfg::THREADS, Cfg::SMEM, stream, tq, tk, tv, p);
   return static_cast<int>(cudaGetLastError());
@@ -371,8 +340,8 @@ extern "C" int ss_attn_fwd(const void* q, const void* k, const void* v, void* ou
   p.out = out; p.lse = lse; p.cu_seqlens = cu_seqlens; p.nseq = nseq; p.T = T; p.Hq = Hq;
   p.Hkv = Hkv; p.ldo = ldo; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (dh == 128) return launch_fwd<128, 2, 64, 4, 4>(q, k, v, p, ldq, ldk, ldv, s);
-  if (dh == 64) return launch_fwd<64, 2, 64, 4, 4>(q, k, v, p, ldq, ldk, ldv, s);
-  if (dh == 256) return launch_fwd<256, 1, 64, 3, 2>(q, k, v, p, ldq, ldk, ldv, s);
+  if (dh == 128) return launch_fwd<128, 64, 2, 2, 2>(q, k, v, p, ldq, ldk, ldv, s);
+  if (dh == 64) return launch_fwd<64, 64, 4, 4, 2>(q, k, v, p, ldq, ldk, ldv, s);
+  if (dh == 256) return launch_fwd<256, 64, 3, 2, 1>(q, k, v, p, ldq, ldk, ldv, s);
   return -2;
 }
