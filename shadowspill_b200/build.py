@@ -21,6 +21,7 @@ from pathlib import Path
 ROOT = Path(__file__).resolve().parent
 KERNEL_DIR = ROOT / "ops" / "csrc"
 KERNEL_LIB = ROOT / "ops" / "libss_kernels.so"
+HOST_CALLS = ROOT / "ops" / "_host_calls.so"      # its launchers called with tensors (Python extension, links torch)
 CORE_DIR = ROOT / "csrc"
 CORE_LIB = CORE_DIR / "libss_core.so"
 CUDA_BACKEND_LIB = CORE_DIR / "libss_backend_cuda.so"
@@ -86,6 +87,27 @@ def build_kernels(force: bool = False, verbose: bool = False, ptxas_info: bool =
     return KERNEL_LIB
 
 
+def build_host_calls(force: bool = False, verbose: bool = False) -> Path | None:
+    """Compile the Python extension that calls the kernel library's launchers with tensors."""
+    source, cuda = KERNEL_DIR / "host_calls.cpp", _cuda_home()
+    if cuda is None or not KERNEL_LIB.exists():
+        return None
+    if force or _stale(HOST_CALLS, [source]):
+        import sysconfig
+
+        import torch
+        home = Path(torch.__file__).resolve().parent
+        tmp = HOST_CALLS.with_suffix(".so.tmp")
+        _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+              "-isystem", str(home / "include"), "-isystem", str(home / "include/torch/csrc/api/include"),
+              "-isystem", sysconfig.get_paths()["include"], "-isystem", str(cuda / "include"),
+              "-o", str(tmp), str(source), "-L", str(KERNEL_LIB.parent), "-lss_kernels", "-Wl,-rpath,$ORIGIN",
+              "-L", str(home / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"], verbose)
+        os.replace(tmp, HOST_CALLS)
+    return HOST_CALLS
+
+
 def _cuda_home() -> Path | None:
     for cand in (os.environ.get("CUDA_HOME"), "/usr/local/cuda"):
         if cand and (Path(cand) / "include" / "cuda_runtime.h").exists():
@@ -134,6 +156,7 @@ def build_core(force: bool = False, verbose: bool = False) -> Path:
 
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_kernels(force=force, verbose=verbose)
+    build_host_calls(force=force, verbose=verbose)
     build_core(force=force, verbose=verbose)
 
 
@@ -157,6 +180,7 @@ def verify() -> dict:
     root = Path(CORE_LIB).parent
     report["files"] = {name: (root / name).exists() for name in
                        ("libss_backend_cuda.so", "libss_allocator.so", "ss_memory_daemon")}
+    report["files"][HOST_CALLS.name] = HOST_CALLS.exists()
     import torch
     report["gpu"] = torch.cuda.is_available()
     report["ok"] = not missing and all(report["files"].values())

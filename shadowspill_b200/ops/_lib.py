@@ -1,12 +1,14 @@
 """ctypes binding of ``libss_kernels.so`` (the sm_100a kernel library).
 
 The kernels are exported as plain C launchers that take raw device pointers and
-a stream handle, so this module needs no compiled Python extension. On a machine
-with a GPU a missing library is an error, never a silent fallback.
+a stream handle. The launchers that a training step calls most are also called with tensors, by the extension module
+``_host_calls.so`` (``host()``). On a machine with a GPU a missing library is an error, never a silent fallback.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import threading
 from pathlib import Path
 
@@ -79,6 +81,26 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_HOST_PATH = _LIB_PATH.with_name("_host_calls.so")
+_host = None
+
+
+def host():
+    """Load (once) and return the extension module with the launchers that take tensors."""
+    global _host
+    if _host is None:
+        lib()
+        with _lock:
+            if _host is None:
+                if not _HOST_PATH.exists():
+                    raise KernelLibraryMissing(f"{_HOST_PATH} is not built; run `python -m shadowspill_b200.build`")
+                loader = importlib.machinery.ExtensionFileLoader("_host_calls", str(_HOST_PATH))
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host_calls", loader))
+                loader.exec_module(module)
+                _host = module
+    return _host
+
+
 def register(name: str, argtypes: list) -> None:
     """Declare the signature of another exported launcher (used by sibling modules)."""
     _SIGNATURES[name] = argtypes
@@ -124,6 +146,7 @@ def status_ptr(t: torch.Tensor) -> int:
     ptr = _status_ptrs.get(index)
     if ptr is None:
         ptr = _status_ptrs[index] = status_word(index).data_ptr()
+        host().set_status(index, ptr)
     return ptr
 
 
@@ -139,20 +162,26 @@ def check_status(device: torch.device | int | None = None) -> None:
 # kernels launched by one successful call of each launcher (attention backward:
 # delta + dQ + dKV; sum of squares: partials + final)
 _KERNELS_PER_CALL = {"ss_attn_bwd": 3, "ss_attn_bwd_g": 3, "ss_sumsq": 2}
-launch_count = 0
 _by_entry: dict[str, int] = {}
 
 
 def check(rc: int, what: str) -> None:
     """Raises on a failed launcher; counts the kernels a successful one enqueued."""
-    global launch_count
     if rc != 0:
         raise RuntimeError(f"{what} failed with code {rc}")
     n = _KERNELS_PER_CALL.get(what, 1)
-    launch_count += n
     _by_entry[what] = _by_entry.get(what, 0) + n
 
 
 def launch_counts() -> dict[str, int]:
     """Kernels enqueued so far, by launcher entry point."""
-    return dict(_by_entry)
+    counts = dict(_by_entry)
+    for name, n in (_host.launched() if _host is not None else {}).items():
+        counts[name] = counts.get(name, 0) + n
+    return counts
+
+
+def __getattr__(name: str):
+    if name == "launch_count":           # kernels enqueued so far
+        return sum(launch_counts().values())
+    raise AttributeError(name)

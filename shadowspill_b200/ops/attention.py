@@ -59,6 +59,10 @@ def _row_stride(t: torch.Tensor) -> int:
 
 
 def forward(q, k, v, cu_seqlens, max_seqlen, scale=None, out=None, lse=None):
+    if implementation() == "native":
+        got = _lib.host().attention_fwd(q, k, v, cu_seqlens, scale, out, lse)
+        if got is not NotImplemented:
+            return got
     T, Hq, dh = q.shape
     Hkv = k.shape[1]
     scale = scale if scale is not None else 1.0 / math.sqrt(dh)
@@ -88,6 +92,10 @@ def forward(q, k, v, cu_seqlens, max_seqlen, scale=None, out=None, lse=None):
 
 def backward(q, k, v, out, lse, dout, cu_seqlens, max_seqlen, scale=None, dq=None, dk=None,
              dv=None):
+    if implementation("ss_attn_bwd") == "native":
+        got = _lib.host().attention_bwd(q, k, v, out, lse, dout, cu_seqlens, scale, dq, dk, dv)
+        if got is not NotImplemented:
+            return got
     T, Hq, dh = q.shape
     Hkv = k.shape[1]
     scale = scale if scale is not None else 1.0 / math.sqrt(dh)

@@ -45,6 +45,12 @@ def _gemm_library(a, b, a_mn, b_mn, out, accumulate, alpha, out_dtype):
     return out.add_(res) if accumulate else out.copy_(res)
 
 
+# Calls on the GPU go to the native module first, which takes operands that need nothing done to them and answers
+# NotImplemented for all others (and until a device's status word exists): those go on in Python.
+def _host(t: torch.Tensor):
+    return _lib.host() if t.is_cuda and not _LIBRARY else None
+
+
 def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
@@ -63,6 +69,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     ``a_mn``: A is stored ``[K, M]`` (else ``[M, K]``); ``b_mn``: B is stored
     ``[K, N]`` (else ``[N, K]``). ``accumulate`` adds the existing ``out``.
     """
+    host = _host(a)
+    if host is not None and _PAIR_GEMM and bn == 0 and (out is not None or out_dtype is None or out_dtype == _BF16):
+        got = host.gemm(a, b, bool(a_mn), bool(b_mn), out, bool(accumulate), alpha)
+        if got is not NotImplemented:
+            return got
     M = a.shape[1] if a_mn else a.shape[0]
     K = a.shape[0] if a_mn else a.shape[1]
     N = b.shape[1] if b_mn else b.shape[0]
@@ -170,6 +181,11 @@ def _fused_gemm(*tensors) -> bool:
 
 def linear_residual(x, w, residual, out=None):
     """``residual[T,N] + x[T,K] @ w[N,K]^T``; ``residual`` is only read (and may be ``out``)."""
+    host = _host(x)
+    if host is not None and _PAIR_GEMM and not _pending_gathers:
+        got = host.linear_residual(x, w, residual, out)
+        if got is not NotImplemented:
+            return got
     if out is None:
         out = torch.empty_like(residual)
     M, N, K = x.shape[0], w.shape[0], x.shape[1]
@@ -186,6 +202,11 @@ def linear_residual(x, w, residual, out=None):
 def swiglu_linear(x, w13, gu=None, out=None, keep_gu=True):
     """``gu = x @ w13^T`` (gate columns, then up columns) and ``h = silu(gate) * up`` by one kernel: ``(gu, h)``.
     Without ``keep_gu`` the projections are not written and the first is None."""
+    host = _host(x)
+    if host is not None and _PAIR_GEMM and not _pending_gathers:
+        got = host.swiglu_linear(x, w13, gu, out, bool(keep_gu))
+        if got is not NotImplemented:
+            return got
     T, F2, K = x.shape[0], w13.shape[0], x.shape[1]
     keep_gu = keep_gu or gu is not None
     given = [t for t in (gu, out) if t is not None]
@@ -204,6 +225,11 @@ def swiglu_linear(x, w13, gu=None, out=None, keep_gu=True):
 def swiglu_linear_dgrad(dy, w2, gu):
     """The gradient of ``gu`` for ``y = h @ w2^T`` with ``h = silu(gate) * up``: ``dy @ w2`` goes through SwiGLU's
     gradient where the products leave, and is never stored."""
+    host = _host(dy)
+    if host is not None and _PAIR_GEMM and not _pending_gathers:
+        got = host.swiglu_linear_dgrad(dy, w2, gu)
+        if got is not NotImplemented:
+            return got
     T, F, K = dy.shape[0], w2.shape[1], dy.shape[1]
     if not (_fused_gemm(dy, w2, gu) and w2.shape[0] == K and gu.shape == (T, 2 * F)):
         return swiglu_bwd(gu, linear_dgrad(dy, w2))
@@ -250,6 +276,9 @@ def rmsnorm_fwd(x, w, eps=1e-5, zero_centered=False, delta=None, out=None, rstd=
         if rstd is not None:
             rs = rstd.copy_(rs)
         return y, rs
+    got = _lib.host().rmsnorm_fwd(x, w, eps, bool(zero_centered), delta, out, rstd)
+    if got is not NotImplemented:
+        return got
     T, D = x.shape
     y = torch.empty_like(x) if out is None else out
     rs = torch.empty(T, dtype=torch.float32, device=x.device) if rstd is None else rstd
@@ -271,6 +300,9 @@ def rmsnorm_bwd(x, w, gy, rstd, dw, zero_centered=False, dx=None, accumulate=Fal
             return dxr.to(x.dtype)
         dx.copy_(((dx.float() if accumulate else 0) + dxr).to(dx.dtype))
         return dx
+    got = _lib.host().rmsnorm_bwd(x, w, gy, rstd, dw, bool(zero_centered), dx, bool(accumulate))
+    if got is not NotImplemented:
+        return got
     T, D = x.shape
     if dx is None:
         if accumulate:
@@ -335,6 +367,9 @@ def rope_(buf, positions, *, col0, heads, dh, rot=None, theta=10000.0, inverse=F
     rot = dh if rot is None else rot
     if not _cuda(buf):
         return reference.rope_(buf, positions, col0, heads, dh, rot, theta, inverse)
+    got = _lib.host().rope(buf, positions, col0, heads, dh, rot, theta, bool(inverse))
+    if got is not NotImplemented:
+        return got
     if positions.dtype != torch.int32:
         raise TypeError("positions must be int32")
     rc = _lib.lib().ss_rope(buf.data_ptr(), positions.data_ptr(), buf.shape[0], buf.stride(0),
