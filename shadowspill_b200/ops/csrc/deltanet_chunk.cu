@@ -81,21 +81,12 @@ __device__ __forceinline__ void tmem_row32(uint32_t addr, float* out) {
 #pragma unroll
   for (int e = 0; e < 32; ++e) out[e] = __uint_as_float(r[e]);
 }
-__device__ __forceinline__ void tmem_row64(uint32_t addr, float* out) {
-  tmem_row32(addr, out);
-  tmem_row32(addr + 32, out + 32);
-}
 // Operands written by threads (shared memory, TMEM) become visible to the MMA issuer.
 __device__ __forceinline__ void publish() {
   tc_fence_before();
   fence_async_proxy();
   __syncthreads();
   tc_fence_after();
-}
-// 64 bf16 values -> one 128-byte row of a global array.
-__device__ __forceinline__ void store_row64(__nv_bfloat16* dst, const float* f) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q) reinterpret_cast<uint4*>(dst)[q] = pack8(f + q * 8);
 }
 // Sums of N values per lane over the warp's lanes (each step hands half of the remaining columns to the
 // partner lane; through shared memory it was N stores and a chain of dependent loads per sum), written to
@@ -120,7 +111,6 @@ __device__ __forceinline__ void warp_col_sums(float (&v)[N], float* out) {
   else if constexpr (N == 32) out[lane] = v[0];
   else if ((lane & 1) == 0) out[lane >> 1] = v[0];
 }
-__device__ __forceinline__ void row_threads_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 __device__ __forceinline__ void all_rows_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 // exp(x) where `on`, else 0, without a branch: a choice between an exponential and 0 became one per element, which
 // diverged in every warp that holds a diagonal.
@@ -153,6 +143,7 @@ struct PrepParams {
   Geo geo; float scale; int* status;
 };
 namespace prep {
+constexpr int ROW_THREADS = 256, PTHREADS = ROW_THREADS + 32, PCTRL = ROW_THREADS, MQ_THREAD = 64;
 // A (fp32) and, once the inverse has been formed from it, the two operands share one region: two CTAs
 // fit an SM, and one's substitution runs under the other's loads and stores.
 constexpr int AP = 68;                                  // pitch of A: rows 16-byte aligned for float4 reads
@@ -165,14 +156,14 @@ constexpr int SMEM = OFF_BAR + 64 + 1024;
 static_assert(2 * (SMEM + 1024) <= 233472, "two CTAs per SM");
 }
 
-// (I + A)^-1 over A, 64 x 64 strictly lower triangular (fp32, pitch AP), by the 64 threads of one head (two warps),
-// j = 0..63; what lies above the diagonal 16 x 16 blocks is scratch. The diagonal blocks by forward substitution, a
-// column per thread, then twice [[P, 0], [-Q B P, Q]] from the inverses P and Q of two neighbouring blocks and the block
-// B between them. Substitution in one piece was a chain of 64 steps in 2,000 straight-line multiplications, and
-// fetching those took as long as running them.
-__device__ __forceinline__ void head_sync(int tid) {
-  if (tid < 64) asm volatile("bar.sync 2, 64;" ::: "memory");
-  else asm volatile("bar.sync 3, 64;" ::: "memory");
+// (I + A)^-1 over A, 64 x 64 strictly lower triangular (fp32, pitch AP), by the 128 row threads of one head (four warps:
+// j = 0..63 in two parts); what lies above the diagonal 16 x 16 blocks is scratch. The diagonal blocks by forward
+// substitution, a column per thread of part 0, then twice [[P, 0], [-Q B P, Q]] from the inverses P and Q of two
+// neighbouring blocks and the block B between them. Substitution in one piece was a chain of 64 steps in 2,000
+// straight-line multiplications, and fetching those took as long as running them.
+__device__ __forceinline__ void head_sync(int hh) {
+  if (hh == 0) asm volatile("bar.sync 2, 128;" ::: "memory");
+  else asm volatile("bar.sync 3, 128;" ::: "memory");
 }
 
 __device__ __forceinline__ void fma_row(float (&acc)[4], float a, const float4& b) {
@@ -201,9 +192,9 @@ __device__ __forceinline__ void block_product(float (&acc)[R][4], const float* L
   }
 }
 
-__device__ __forceinline__ void unit_lower_inverse(float* A, int j) {
+__device__ __forceinline__ void unit_lower_inverse(float* A, int hh, int j, int part) {
   using prep::AP;
-  {
+  if (part == 0) {
     float* D = A + (j & ~15) * (AP + 1);
     const int jj = j & 15;
     float x[16];
@@ -223,42 +214,38 @@ __device__ __forceinline__ void unit_lower_inverse(float* A, int j) {
     __syncwarp();                                  // a warp holds both blocks whose columns it has read
 #pragma unroll
     for (int t = 0; t < 16; ++t) D[t * AP + jj] = x[t];
-    __syncwarp();
   }
-  {                                                // 16 -> 32: one pair of blocks per warp, 2 x 4 values per thread
+  head_sync(hh);
+  {                                                // 16 -> 32: two pairs of blocks, 1 x 4 values per thread
     float* B0 = A + (j & 32) * (AP + 1);
-    const int r0 = (j & 31) >> 2 << 1, c0 = (j & 3) * 4;
-    float v[2][4];
-    block_product<2>(v, B0 + (16 + r0) * AP, B0 + c0, 0, 16);                     // B P
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-      *reinterpret_cast<float4*>(B0 + (r0 + r) * AP + 16 + c0) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
-    __syncwarp();
-    block_product<2>(v, B0 + (16 + r0) * AP + 16, B0 + 16 + c0, 0, 16);           // Q (B P)
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-      *reinterpret_cast<float4*>(B0 + (16 + r0 + r) * AP + c0) = make_float4(-v[r][0], -v[r][1], -v[r][2], -v[r][3]);
+    const int r0 = part * 8 + ((j & 31) >> 2), c0 = (j & 3) * 4;
+    float v[1][4];
+    block_product<1>(v, B0 + (16 + r0) * AP, B0 + c0, 0, 16);                     // B P
+    *reinterpret_cast<float4*>(B0 + r0 * AP + 16 + c0) = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+    head_sync(hh);
+    block_product<1>(v, B0 + (16 + r0) * AP + 16, B0 + 16 + c0, 0, 16);           // Q (B P)
+    *reinterpret_cast<float4*>(B0 + (16 + r0) * AP + c0) = make_float4(-v[0][0], -v[0][1], -v[0][2], -v[0][3]);
   }
-  head_sync(threadIdx.x);
-  {                                                // 32 -> 64: 4 x 4 values per thread, zero blocks left out
-    const int r0 = (j >> 3) * 4, c0 = (j & 7) * 4;
-    float v[4][4];
-    block_product<4>(v, A + (32 + r0) * AP, A + c0, c0 & 16, 32);
+  head_sync(hh);
+  {                                                // 32 -> 64: 2 x 4 values per thread, zero blocks left out
+    const int r0 = part * 16 + (j >> 3) * 2, c0 = (j & 7) * 4;
+    float v[2][4];
+    block_product<2>(v, A + (32 + r0) * AP, A + c0, c0 & 16, 32);
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 2; ++r)
       *reinterpret_cast<float4*>(A + (r0 + r) * AP + 32 + c0) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
-    head_sync(threadIdx.x);
-    block_product<4>(v, A + (32 + r0) * AP + 32, A + 32 + c0, 0, (r0 & 16) + 16);
+    head_sync(hh);
+    block_product<2>(v, A + (32 + r0) * AP + 32, A + 32 + c0, 0, (r0 & 16) + 16);
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 2; ++r)
       *reinterpret_cast<float4*>(A + (32 + r0 + r) * AP + c0) = make_float4(-v[r][0], -v[r][1], -v[r][2], -v[r][3]);
   }
 }
 
-// Bound by latency: two CTAs an SM, each with one warp to a scheduler. 8,192 tokens, 16 / 32 heads: 0.199 -> 0.146 ms
-// (436 MB, 0.067 ms at the copy bandwidth) with the inverse in blocks, the scalars' loads ahead of the set-up, no
-// branch around an exponential and Mq through a tile.
-__global__ void __launch_bounds__(THREADS, 2)
+// Bound by latency: two CTAs an SM, each with two row warps to a scheduler (one: 0.146 ms). 8,192 tokens, 16 / 32 heads:
+// 0.199 -> 0.132 ms (436 MB, 0.067 ms at the copy bandwidth) with the inverse in blocks, the scalars' loads ahead of the
+// set-up, no branch around an exponential and Mq through a tile.
+__global__ void __launch_bounds__(prep::PTHREADS, 2)
 dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmWT,
                const __grid_constant__ CUtensorMap tmU0T, const __grid_constant__ CUtensorMap tmQG,
@@ -294,7 +281,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
   if (tid < 64 || (tid == 64 && c > 0)) sid = p.sid[tid < 64 ? t0 + tid : t0 - 1];
 
-  if (tid == CTRL) {
+  if (tid == PCTRL) {
     mbar_init(tma_bar, 1); mbar_init(mma_bar, 1); mbar_fence_init();
     mbar_expect_tx(tma_bar, 32768 + nh * 16384);
 #pragma unroll
@@ -307,7 +294,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       for (int b = 0; b < 2; ++b)
         tma_load_2d(smem + OFF_V + hh * 16384 + b * 8192, &tmV, tma_bar, (h0 + hh) * D + b * 64, t0);
   }
-  if (warp == 4) { __syncwarp(); tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
+  if (warp == 8) { __syncwarp(); tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -338,7 +325,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   __syncthreads();
 
   // ---- [K; Q] K^T
-  if (tid == CTRL) {
+  if (tid == PCTRL) {
     mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
     tc_fence_after();
     constexpr uint32_t idesc = umma_idesc_bf16(128, 64, false, false);
@@ -354,23 +341,23 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   mbar_wait(mma_bar, 0, p.status, KS_TIMEOUT_TMEM_FULL);
   tc_fence_after();
 
-  // ---- A (fp32; only below the diagonal) and Mq, eight columns at a time: a body of more instructions than the
-  // first instruction cache holds ran at a tenth of the issue rate
-  if (tid < 128) {
-    const int t = tid & 63, last = t | 31;               // the warp's last row
+  // ---- A (fp32; only below the diagonal) and Mq, eight columns at a time
+  const int row = tid & 127, part = (tid >> 7) & 1;      // of the row threads: a lane of TMEM and the half of its columns
+  if (tid < ROW_THREADS) {
+    const int t = row & 63, last = t | 31;               // the warp's last row
     const int lo = seq_begin(starts_s, t);
-    const bool is_q = tid >= 64;
+    const bool is_q = row >= 64;
     const int hi = is_q ? t : t - 1;                     // Mq includes the diagonal, A does not
 #pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
       const float gt = gam_s[hh * 64 + t], f = is_q ? p.scale : beta_s[hh * 64 + t];
       float* a = Af + (hh * 64 + t) * AP;
       if (is_q && hh > 0) {                              // the head before has left the tile
-        if (tid == 64) tma_store_wait_read<0>();
-        head_sync(64);
+        if (tid == MQ_THREAD) tma_store_wait_read<0>();
+        head_sync(1);
       }
 #pragma unroll 1
-      for (int i0 = 0; i0 < 64; i0 += 8) {
+      for (int i0 = part * 32; i0 < part * 32 + 32; i0 += 8) {
         float m[8];
         if (i0 > last) {
 #pragma unroll
@@ -397,8 +384,8 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
       if (is_q) {
         fence_async_proxy();
-        head_sync(64);
-        if (tid == 64) {
+        head_sync(1);
+        if (tid == MQ_THREAD) {
           tma_store_2d(&tmMQ, smem + OFF_MQ, 0, (c * G.NP + pr) * 128 + hh * 64);
           tma_store_commit();
         }
@@ -407,41 +394,43 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
   __syncthreads();
 
-  // ---- Tm = (I + A)^-1; thread (hh, j) takes its column j
-  if (tid < 128) {
-    const int hh = tid >> 6, j = tid & 63;
-    float col[64];
-    if (hh < nh) unit_lower_inverse(Af + hh * 64 * AP, j);
-    row_threads_sync();
+  // ---- Tm = (I + A)^-1; thread (hh, j) takes half of its column j
+  if (tid < ROW_THREADS) {
+    const int hh = row >> 6, j = row & 63;
+    float col[32];
     if (hh < nh) {
+      unit_lower_inverse(Af + hh * 64 * AP, hh, j, part);
+      head_sync(hh);
       const float* at = Af + hh * 64 * AP + j;
 #pragma unroll
-      for (int t = 0; t < 64; ++t) col[t] = t >= j ? at[t * AP] : 0.f;
+      for (int e = 0; e < 32; ++e) col[e] = part * 32 + e >= j ? at[(part * 32 + e) * AP] : 0.f;
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");      // A has been read: its region takes the operands
+    all_rows_sync();                                    // A has been read: its region takes the operands
     if (hh < nh) {
-      const float bj = beta_s[tid];
-      const float gtj = (sid_s[j] == sid_s[64]) ? __expf(gam_s[tid]) : 0.f;
-      const int row = hh * 64 + j;
-      const long long grow = ((static_cast<long long>(c) * G.NP + pr) * 128 + row) * 64;
-      float w[64];
+      const float bj = beta_s[row];
+      const float gtj = (sid_s[j] == sid_s[64]) ? __expf(gam_s[row]) : 0.f;
+      float w[32];
 #pragma unroll
-      for (int t = 0; t < 64; ++t) w[t] = col[t] * bj * gtj;
+      for (int e = 0; e < 32; ++e) w[e] = col[e] * bj * gtj;
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<uint4*>(smem + OFF_XW + sw_off(128, row, q)) = pack8(w + q * 8);
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(smem + OFF_XW + sw_off(128, row, part * 4 + q)) = pack8(w + q * 8);
 #pragma unroll
-      for (int t = 0; t < 64; ++t) w[t] = col[t] * bj;
+      for (int e = 0; e < 32; ++e) w[e] = col[e] * bj;
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<uint4*>(smem + OFF_XU + sw_off(128, row, q)) = pack8(w + q * 8);
-      if (p.TMT) store_row64(p.TMT + grow, col);
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(smem + OFF_XU + sw_off(128, row, part * 4 + q)) = pack8(w + q * 8);
+      if (p.TMT) {
+        uint4* dst = reinterpret_cast<uint4*>(p.TMT + ((static_cast<long long>(c) * G.NP + pr) * 128 + row) * 64 + part * 32);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[q] = pack8(col + q * 8);
+      }
     }
   }
   publish();
 
   // ---- W^T = K^T (Tm diag(beta Gt))^T, U0^T = V^T (Tm diag(beta))^T
-  if (tid == CTRL) {
+  if (tid == PCTRL) {
     constexpr uint32_t idesc = umma_idesc_bf16(128, 64, true, true);
     const uint32_t sk = smem_u32(smem + OFF_KQ), sv = smem_u32(smem + OFF_V);
     const uint32_t sxw = smem_u32(smem + OFF_XW), sxu = smem_u32(smem + OFF_XU);
@@ -472,10 +461,10 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   // ---- every result leaves by TMA from a tile laid out like its operands (a row per thread straight to
   // memory is 16 bytes to each of 32 lines per store, half of this kernel's time): W^T over V, U0^T over
   // the operands, then the scaled K and Q rows of the last head in place and those of the first over W^T.
-  uint4 kq[16];
-  const int t = tid & 63;
-  const bool is_q = tid >= 64;
-  auto factor = [&](int hh) {                    // Kd (threads 0..63, K rows) and Qg (threads 64..127, Q rows)
+  uint4 kq[8];
+  const int t = row & 63;
+  const bool is_q = row >= 64;
+  auto factor = [&](int hh) {                    // Kd (rows 0..63, of K) and Qg (rows 64..127, of Q)
     const float gt = gam_s[hh * 64 + t];
     if (is_q) return (sid_s[t] == sid_s[64]) ? p.scale * __expf(gt) : 0.f;
     return (sid_s[t] == sid_s[63]) ? __expf(gam_s[hh * 64 + 63] - gt) : 0.f;
@@ -483,12 +472,12 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   auto write_kq = [&](uint8_t* tile, int hh) {
     const float f = factor(hh);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
+    for (int q = 0; q < 8; ++q) {
       float v[8];
       unpack8(kq[q], v);
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] *= f;
-      *reinterpret_cast<uint4*>(tile + sw_off(128, tid, q)) = pack8(v);
+      *reinterpret_cast<uint4*>(tile + sw_off(128, row, part * 8 + q)) = pack8(v);
     }
   };
   auto store_kq = [&](const uint8_t* tile, int hh) {
@@ -500,24 +489,22 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
     tma_store_commit();
   };
-  if (tid < 128) {
+  if (tid < ROW_THREADS) {
 #pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        float w[32], u[32];
-        tmem_row32(lane_addr + hh * 64 + half * 32, w);
-        tmem_row32(lane_addr + 128 + hh * 64 + half * 32, u);
+      float v[32];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t at = hh * 16384 + sw_off(128, tid, half * 4 + q);
-          *reinterpret_cast<uint4*>(smem + OFF_V + at) = pack8(w + q * 8);
-          *reinterpret_cast<uint4*>(smem + OFF_XW + at) = pack8(u + q * 8);
-        }
+      for (int x = 0; x < 2; ++x) {
+        tmem_row32(lane_addr + x * 128 + hh * 64 + part * 32, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<uint4*>(smem + (x == 0 ? OFF_V : OFF_XW) + hh * 16384 + sw_off(128, row, part * 4 + q)) =
+              pack8(v + q * 8);
       }
     }
 #pragma unroll
-    for (int q = 0; q < 16; ++q) kq[q] = *reinterpret_cast<const uint4*>(smem + OFF_KQ + sw_off(128, tid, q));
+    for (int q = 0; q < 8; ++q)
+      kq[q] = *reinterpret_cast<const uint4*>(smem + OFF_KQ + sw_off(128, row, part * 8 + q));
     write_kq(smem + OFF_KQ, nh - 1);
     if (tid < nh) {
       const float g63 = gam_s[tid * 64 + 63];
@@ -525,7 +512,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
   }
   publish();
-  if (tid == CTRL) {
+  if (tid == PCTRL) {
     for (int hh = 0; hh < nh; ++hh) {
       tma_store_2d(&tmWT, smem + OFF_V + hh * 16384, hh * 64, (c * G.NP + pr) * 128);
       tma_store_2d(&tmU0T, smem + OFF_XW + hh * 16384, hh * 64, (c * G.NP + pr) * 128);
@@ -536,14 +523,14 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
   if (nh == 2) {
     __syncthreads();
-    if (tid < 128) write_kq(smem + OFF_V, 0);
+    if (tid < ROW_THREADS) write_kq(smem + OFF_V, 0);
     publish();
-    if (tid == CTRL) store_kq(smem + OFF_V, 0);
+    if (tid == PCTRL) store_kq(smem + OFF_V, 0);
   }
-  if (tid == CTRL || tid == 64) tma_store_wait<0>();
+  if (tid == PCTRL || tid == MQ_THREAD) tma_store_wait<0>();
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
+  if (warp == 8) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
 
 // ============================================================================ state walks
@@ -1689,7 +1676,7 @@ int ss_dn_prep(const void* q, const void* k, const void* v, const float* beta, c
   p.geo = geo; p.scale = scale; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_prep_kernel, prep::SMEM)) return e;
-  dn_prep_kernel<<<dim3(geo.n, geo.NP), THREADS, prep::SMEM, (cudaStream_t)stream>>>(tq, tk, tv, twt, tu0, tqg, tkd, tmq,
+  dn_prep_kernel<<<dim3(geo.n, geo.NP), prep::PTHREADS, prep::SMEM, (cudaStream_t)stream>>>(tq, tk, tv, twt, tu0, tqg, tkd, tmq,
                                                                                      txw, txu, p);
   return (int)cudaGetLastError();
 }
