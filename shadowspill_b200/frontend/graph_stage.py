@@ -327,7 +327,11 @@ def _head_training_graph(pairs: gp.StagePairs, stage: StageGraph):
         raise NotImplementedError("the head's loss gradient is used in a way the training graph does not fold")
     for t in tangents:
         g.erase_node(t)
-    out_node.args = (tuple(out_node.args[0]),)
+    # vectors' gradients are summed in fp32: the rounding to the parameter's type that autograd appends goes
+    def vector(v):
+        return isinstance(v, fx.Node) and v.meta.get("val") is not None and v.meta["val"].dim() == 1
+    loss, *grads = out_node.args[0]
+    out_node.args = ((loss, *(gp._strip_cast(v) if vector(v) else v for v in grads)),)
     g.eliminate_dead_code()
     g._codegen = fx.graph.CodeGen()          # plain positional inputs instead of (primals, tangents)
     g.lint()

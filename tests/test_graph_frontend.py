@@ -608,3 +608,16 @@ def test_row_chunks_on_the_latent_attention_family():
         return losses
     for a, b in zip(run(whole, desc_w), run(prog, desc)):
         assert abs(a - b) < 5e-4 * max(1.0, abs(a))        # discrete picks: see the eager comparison above
+
+
+def test_the_head_sums_its_norm_gradient_in_fp32():
+    """As every other stage does: no rounding to the parameter's type between the microbatches."""
+    from dataclasses import replace
+    cfg = replace(preset("qwen35-numerical"), n_layers=1)
+    geo = BatchGeometry(microbatch_tokens=64, n_microbatches=1, slots=5, mean_seqlen=32)
+    _, desc = build_step(cfg, geo, StepDataOrdering(), dtype=torch.bfloat16, frontend="graph")
+    head = desc.stages()[-1]
+    head._train_graph()
+    outs = next(n for n in head._train.graph.nodes if n.op == "output").args[0]
+    norm = outs[1 + head._train_grads.index("final_norm")]
+    assert norm.meta["val"].dtype == torch.float32
