@@ -553,19 +553,38 @@ struct WalkParams {
   const float* gc;
   const int* sid;
   int bucket;                               // chunks
-  int save;                                 // forward: keep S and U for the backward pass
   Geo geo; int* status;
 };
 namespace walk {
+// 128 walks at once move 4 to 5 TB/s, and a chunk's operands then take longer than the chunk before: the loads have to
+// be further ahead. A walk without an output leaves Qg and Mq out, and one without saves writes O over the Qg it has
+// used, which makes room for a third stage. Saves leave from a warp of their own, or the next loads would wait for them.
+// 8,192 tokens of four sequences, 32 V heads: 95 us for either walk with two stages, 76 us (0.37 GB) for the one without
+// saves and 81 us (0.40 GB) for the one without an output now; of one sequence 183 us, and now 138 and 172 us.
+// U0 in registers, loaded a chunk ahead for a fourth stage: 117 us, since an mbarrier's arrival waits for the loads.
+template <bool OUT, bool SAVE>
+struct Fwd {
+  static constexpr int OFF_U0 = 16384, OFF_KD = 32768, OFF_QG = 49152, OFF_MQ = 65536;    // of a stage; W^T comes first
+  static constexpr int STAGE = OUT ? 73728 : 49152, STAGES = OUT && SAVE ? 2 : 3;
+  static constexpr int OFF_SOP = STAGES * STAGE;                                  // [128 x 128] saved copy of the state
+  static constexpr int OFF_UOP = OFF_SOP + (SAVE ? 32768 : 0);                    // [128 x 64] saved copy of U
+  static constexpr bool O_IN_STAGE = OUT && !SAVE;
+  static constexpr int OFF_O = OFF_UOP + (SAVE ? 16384 : 0);                      // O of a chunk
+  static constexpr int OFF_BAR = OFF_O + (OUT && !O_IN_STAGE ? 16384 : 0);
+  static constexpr int SMEM = OFF_BAR + 256 + 1024;
+  static constexpr int MMA_WARP = 8 + (OUT ? 4 : 0), LOAD_WARP = MMA_WARP + 1, SAVE_WARP = MMA_WARP + 2;
+  static constexpr int THREADS = (MMA_WARP + (SAVE ? 3 : 2)) * 32;
+  static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
+};
+// backward
 constexpr int STAGE = 73728;
 constexpr int OFF_SOP = 2 * STAGE;          // [128 x 128] saved copy of the state
-constexpr int OFF_UOP = OFF_SOP + 32768;    // [128 x 64] saved copy of U or dU
-constexpr int OFF_O = OFF_UOP + 16384;      // forward: O of a chunk
-constexpr int OFF_BAR = OFF_O + 16384;
+constexpr int OFF_UOP = OFF_SOP + 32768;    // [128 x 64] saved copy of dU
+constexpr int OFF_BAR = OFF_UOP + 16384;
 constexpr int SMEM = OFF_BAR + 256 + 1024;
 constexpr int STATE_WARPS = 8, STATE_COLS = 512 / STATE_WARPS, TOKEN_COLS = STATE_COLS / 2;
 constexpr int TM_DS = 0, TM_WS = 128, TM_O = 192, TM_SOP = 320, TM_UOP = 384;   // TMEM columns: 128, 64, 2 x 64, 64, 32
-constexpr int FWD_THREADS = (STATE_WARPS + 4 + 2) * 32, BWD_THREADS = (STATE_WARPS + 2) * 32;
+constexpr int BWD_THREADS = (STATE_WARPS + 3) * 32;
 static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
 }
 
@@ -645,29 +664,32 @@ __device__ __forceinline__ void warp_publish_copy(uint64_t* bar) {
   if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 
-// Stage layout (forward): WT @0, U0T @16384, QG @32768, KD @49152, MQ @65536.
-__global__ void __launch_bounds__(walk::FWD_THREADS, 1)
+// OUT: the rule's output; SAVE: S and U are kept for a backward pass.
+template <bool OUT, bool SAVE>
+__global__ void __launch_bounds__(walk::Fwd<OUT, SAVE>::THREADS, 1)
 dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ CUtensorMap tmU0T,
               const __grid_constant__ CUtensorMap tmQG, const __grid_constant__ CUtensorMap tmKD,
               const __grid_constant__ CUtensorMap tmMQ, const __grid_constant__ CUtensorMap tmST,
               const __grid_constant__ CUtensorMap tmUT, const __grid_constant__ CUtensorMap tmO, const WalkParams p) {
   using namespace walk;
+  using W = Fwd<OUT, SAVE>;
+  constexpr int NST = W::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  uint64_t* full = bars;               // [2] a stage has arrived
-  uint64_t* stage_free = bars + 2;     // [2] its products are done
-  uint64_t* sop_ready = bars + 4;      // S^T operand written
-  uint64_t* ws_done = bars + 5;
-  uint64_t* u_ready = bars + 6;        // U^T operand written
-  uint64_t* s_done = bars + 7;
-  uint64_t* o_full = bars + 8;         // [2]
-  uint64_t* o_free = bars + 10;        // [2]
-  uint64_t* s_copied = bars + 12;      // the copies to be saved have been written
-  uint64_t* u_copied = bars + 13;
-  uint64_t* saved = bars + 14;         // both have been read by their stores
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
-  int* run = reinterpret_cast<int*>(bars + 16);          // first chunk, one behind the last, warm
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + W::OFF_BAR);
+  uint64_t* full = bars;               // [STAGES] a stage has arrived
+  uint64_t* stage_free = bars + 4;     // [STAGES] its products are done, and O has left it
+  uint64_t* sop_ready = bars + 8;      // S^T operand written
+  uint64_t* ws_done = bars + 9;
+  uint64_t* u_ready = bars + 10;       // U^T operand written
+  uint64_t* s_done = bars + 11;
+  uint64_t* o_full = bars + 12;        // [2]
+  uint64_t* o_free = bars + 14;        // [2]
+  uint64_t* s_copied = bars + 16;      // the copies to be saved have been written
+  uint64_t* u_copied = bars + 17;
+  uint64_t* saved = bars + 18;         // both have been read by their stores
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  int* run = reinterpret_cast<int*>(bars + 20);          // first chunk, one behind the last, warm
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const Geo G = p.geo;
@@ -681,10 +703,8 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
     if (lane == 0) { run[0] = first; run[1] = end; run[2] = run_warm(p.sid, G.n, first); }
   }
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&full[i], 1); mbar_init(&stage_free[i], 1);
-      mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4);
-    }
+    for (int i = 0; i < NST; ++i) { mbar_init(&full[i], 1); mbar_init(&stage_free[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4); }
     mbar_init(sop_ready, STATE_WARPS); mbar_init(ws_done, 1);
     mbar_init(u_ready, STATE_WARPS); mbar_init(s_done, 1);
     mbar_init(s_copied, STATE_WARPS); mbar_init(u_copied, STATE_WARPS); mbar_init(saved, 1);
@@ -693,7 +713,7 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
   __syncthreads();
   if (run[0] >= run[1]) return;
   const int skip = run[2], c0 = run[0] - skip, steps = run[1] - c0;    // the first `skip` steps leave no results
-  if (warp == STATE_WARPS + 4) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == W::MMA_WARP) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -708,8 +728,8 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
     for (int e = 0; e < STATE_COLS; ++e) S[e] = 0.f;
     float gc = 0.f;
     for (int it = 0; it < steps; ++it) {
-      const int st = it & 1;
-      const bool keep = p.save && it >= skip;
+      const int st = it % NST;
+      const bool keep = SAVE && it >= skip;
       const float gc_next = p.gc[static_cast<long long>(c0 + it) * G.H + h];
       if (it > 0) {
         if (!mbar_wait(s_done, (it - 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
@@ -722,37 +742,42 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
       gc = gc_next;
       if (keep) {
         if (it > skip && !mbar_wait(saved, (it - skip - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
-        smem_put_bf16<STATE_COLS>(smem + OFF_SOP, row, part, sk);
+        smem_put_bf16<STATE_COLS>(smem + W::OFF_SOP, row, part, sk);
         warp_publish_copy(s_copied);
       }
-      if (!mbar_wait(&full[st], (it >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
-      float u[TOKEN_COLS];
+      if (!mbar_wait(&full[st], (it / NST) & 1, p.status, KS_TIMEOUT_FULL)) break;
+      uint4 u0[TOKEN_COLS / 8];
 #pragma unroll
       for (int q = 0; q < TOKEN_COLS / 8; ++q)
-        unpack8(*reinterpret_cast<const uint4*>(smem + st * STAGE + 16384 +
-                                                sw_off(128, row, part * (TOKEN_COLS / 8) + q)), u + q * 8);
+        u0[q] = *reinterpret_cast<const uint4*>(smem + st * W::STAGE + W::OFF_U0 +
+                                                sw_off(128, row, part * (TOKEN_COLS / 8) + q));
       if (!mbar_wait(ws_done, it & 1, p.status, KS_TIMEOUT_TMEM_FULL)) break;
       tc_fence_after();
-      float ws[TOKEN_COLS];
-      tmem_cols(lane_addr + TM_WS + part * TOKEN_COLS, ws);
+      float u[TOKEN_COLS];
+      tmem_cols(lane_addr + TM_WS + part * TOKEN_COLS, u);
 #pragma unroll
-      for (int e = 0; e < TOKEN_COLS; ++e) u[e] -= ws[e];
+      for (int q = 0; q < TOKEN_COLS / 8; ++q) {
+        float f[8];
+        unpack8(u0[q], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) u[q * 8 + e] = f[e] - u[q * 8 + e];
+      }
       uint32_t uk[TOKEN_COLS / 2];
       tmem_put_bf16(lane_addr + TM_UOP + part * (TOKEN_COLS / 2), u, uk);
       warp_publish(u_ready);
       if (keep) {
-        smem_put_bf16<TOKEN_COLS>(smem + OFF_UOP, row, part, uk);
+        smem_put_bf16<TOKEN_COLS>(smem + W::OFF_UOP, row, part, uk);
         warp_publish_copy(u_copied);
       }
     }
-  } else if (warp < STATE_WARPS + 4) {
+  } else if (OUT && warp < STATE_WARPS + 4) {
     // O^T is transposed through shared memory and leaves by TMA, which also clips the last chunk's
     // rows: 64 two-byte stores per thread straight to memory took longer than the rest of the chunk
-    uint8_t* so = smem + OFF_O + (row >> 6) * 8192;
     const int col = (row & 63) * 2;
     const bool issuer = tid == STATE_WARPS * 32;
     for (int it = 0; it < steps; ++it) {
-      const int b = it & 1;
+      const int b = it & 1, st = it % NST;
+      uint8_t* o_tile = smem + (W::O_IN_STAGE ? st * W::STAGE + W::OFF_QG : W::OFF_O);
       const bool ok = mbar_wait(&o_full[b], (it >> 1) & 1, p.status, KS_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       float o[64];
@@ -760,36 +785,42 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&o_free[b]);
-      if (issuer) tma_store_wait_read<0>();
+      if (!W::O_IN_STAGE && issuer) tma_store_wait_read<0>();
       // the chunk before has left the tile; the four warps also agree on whether to go on, so that none
       // waits at a barrier for one that gave up
       uint32_t all_ok;
       asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\t"
                    "selp.u32 %0, 1, 0, q;\n\t}" : "=r"(all_ok) : "r"(static_cast<uint32_t>(ok)) : "memory");
       if (!all_ok) break;
-      if (it < skip) continue;
+      if (it >= skip) {
+        uint8_t* so = o_tile + (row >> 6) * 8192;
 #pragma unroll
-      for (int t = 0; t < 64; ++t)
-        *reinterpret_cast<__nv_bfloat16*>(so + t * 128 + (col ^ ((t & 7) << 4))) = __float2bfloat16_rn(o[t]);
-      fence_async_proxy();
-      asm volatile("bar.sync 2, 128;" ::: "memory");
-      if (issuer) {
+        for (int t = 0; t < 64; ++t)
+          *reinterpret_cast<__nv_bfloat16*>(so + t * 128 + (col ^ ((t & 7) << 4))) = __float2bfloat16_rn(o[t]);
+        fence_async_proxy();
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+        if (issuer) {
 #pragma unroll
-        for (int x = 0; x < 2; ++x) tma_store_2d(&tmO, smem + OFF_O + x * 8192, h * D + x * 64, (c0 + it) * CH);
-        tma_store_commit();
+          for (int x = 0; x < 2; ++x) tma_store_2d(&tmO, o_tile + x * 8192, h * D + x * 64, (c0 + it) * CH);
+          tma_store_commit();
+        }
+      }
+      if (W::O_IN_STAGE && issuer) {
+        tma_store_wait_read<0>();
+        mbar_arrive(&stage_free[st]);
       }
     }
     if (issuer) tma_store_wait<0>();
-  } else if (warp == STATE_WARPS + 4) {
+  } else if (warp == W::MMA_WARP) {
     const uint32_t leader = elect_one();
     const uint32_t sop = tmem_base + TM_SOP, uop = tmem_base + TM_UOP;
     constexpr uint32_t idesc_w = umma_idesc_bf16(128, 64, false, true);
     constexpr uint32_t idesc_o = umma_idesc_bf16(128, 64, false, false);
     constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, true);
     for (int it = 0; it < steps; ++it) {
-      const int st = it & 1;
-      const uint32_t sst = smem_u32(smem + st * STAGE), to = tmem_base + TM_O + st * 64;
-      if (!mbar_wait(&full[st], (it >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
+      const int st = it % NST, ob = it & 1;
+      const uint32_t sst = smem_u32(smem + st * W::STAGE), to = tmem_base + TM_O + ob * 64;
+      if (!mbar_wait(&full[st], (it / NST) & 1, p.status, KS_TIMEOUT_FULL)) break;
       if (!mbar_wait(sop_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
       tc_fence_after();
       // (W S)^T = S^T W^T
@@ -798,68 +829,68 @@ dn_fwd_kernel(const __grid_constant__ CUtensorMap tmWT, const __grid_constant__ 
         umma_bf16_ts_if(leader, tmem_base + TM_WS, sop + kk * 8, umma_smem_desc(sst + kk * 2048, 16384, 1024), idesc_w,
                         kk != 0);
       umma_commit_if(leader, ws_done);
-      // O^T = S^T Qg^T, while the state warps form U
-      if (it >= 2 && !mbar_wait(&o_free[st], ((it >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
-      tc_fence_after();
+      if constexpr (OUT) {
+        // O^T = S^T Qg^T, while the state warps form U
+        if (it >= 2 && !mbar_wait(&o_free[ob], ((it >> 1) - 1) & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+        tc_fence_after();
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk)
-        umma_bf16_ts_if(leader, to, sop + kk * 8,
-                        umma_smem_desc(sst + 32768 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), idesc_o, kk != 0);
+        for (int kk = 0; kk < 8; ++kk)
+          umma_bf16_ts_if(leader, to, sop + kk * 8,
+                          umma_smem_desc(sst + W::OFF_QG + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), idesc_o, kk != 0);
+      }
       if (!mbar_wait(u_ready, it & 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
       tc_fence_after();
       // dS^T = U^T Kd, then O^T += U^T Mq^T behind it
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16_ts_if(leader, tmem_base + TM_DS, uop + kk * 8, umma_smem_desc(sst + 49152 + kk * 2048, 8192, 1024),
+        umma_bf16_ts_if(leader, tmem_base + TM_DS, uop + kk * 8, umma_smem_desc(sst + W::OFF_KD + kk * 2048, 8192, 1024),
                         idesc_s, kk != 0);
       umma_commit_if(leader, s_done);
+      if constexpr (OUT) {
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-        umma_bf16_ts_if(leader, to, uop + kk * 8, umma_smem_desc(sst + 65536 + kk * 32, 16, 1024), idesc_o, 1);
-      umma_commit_if(leader, &o_full[st]);
-      umma_commit_if(leader, &stage_free[st]);
+        for (int kk = 0; kk < 4; ++kk)
+          umma_bf16_ts_if(leader, to, uop + kk * 8, umma_smem_desc(sst + W::OFF_MQ + kk * 32, 16, 1024), idesc_o, 1);
+        umma_commit_if(leader, &o_full[ob]);
+      }
+      if (!W::O_IN_STAGE) umma_commit_if(leader, &stage_free[st]);
     }
-  } else if (elect_one()) {
-    auto load_stage = [&](int it) {
-      const int c = c0 + it, st = it & 1;
-      uint8_t* s = smem + st * STAGE;
-      const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 64;
-      mbar_expect_tx(&full[st], STAGE);
-      tma_load_2d(s, &tmWT, &full[st], hh * 64, prow);
-      tma_load_2d(s + 16384, &tmU0T, &full[st], hh * 64, prow);
+  } else if (warp == W::LOAD_WARP) {
+    if (elect_one()) {
+      for (int it = 0; it < steps; ++it) {
+        const int c = c0 + it, st = it % NST;
+        if (it >= NST && !mbar_wait(&stage_free[st], (it / NST - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* s = smem + st * W::STAGE;
+        const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 64;
+        mbar_expect_tx(&full[st], W::STAGE);
+        tma_load_2d(s, &tmWT, &full[st], hh * 64, prow);
+        tma_load_2d(s + W::OFF_U0, &tmU0T, &full[st], hh * 64, prow);
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        tma_load_2d(s + 32768 + b * 8192, &tmQG, &full[st], b * 64, hrow);
-        tma_load_2d(s + 49152 + b * 8192, &tmKD, &full[st], b * 64, hrow);
+        for (int b = 0; b < 2; ++b) {
+          tma_load_2d(s + W::OFF_KD + b * 8192, &tmKD, &full[st], b * 64, hrow);
+          if (OUT) tma_load_2d(s + W::OFF_QG + b * 8192, &tmQG, &full[st], b * 64, hrow);
+        }
+        if (OUT) tma_load_2d(s + W::OFF_MQ, &tmMQ, &full[st], 0, prow + hh * 64);
       }
-      tma_load_2d(s + 65536, &tmMQ, &full[st], 0, prow + hh * 64);
-    };
-    load_stage(0);
-    if (steps > 1) load_stage(1);
-    for (int it = 0; it < steps; ++it) {
-      if (p.save && it >= skip) {
-        const int c = c0 + it;
-        if (!mbar_wait(s_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
+    }
+  } else if (SAVE && elect_one()) {
+    for (int it = skip; it < steps; ++it) {
+      const int c = c0 + it;
+      if (!mbar_wait(s_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
-          tma_store_2d(&tmST, smem + OFF_SOP + b * 16384, b * 64, (c * G.H + h) * 128);
-        tma_store_commit();
-        if (!mbar_wait(u_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
-        tma_store_2d(&tmUT, smem + OFF_UOP, hh * 64, (c * G.NP + pr) * 128);
-        tma_store_commit();
-        tma_store_wait_read<0>();
-        mbar_arrive(saved);
-      }
-      if (it + 2 < steps) {
-        if (!mbar_wait(&stage_free[it & 1], (it >> 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
-        load_stage(it + 2);
-      }
+      for (int b = 0; b < 2; ++b)
+        tma_store_2d(&tmST, smem + W::OFF_SOP + b * 16384, b * 64, (c * G.H + h) * 128);
+      tma_store_commit();
+      if (!mbar_wait(u_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
+      tma_store_2d(&tmUT, smem + W::OFF_UOP, hh * 64, (c * G.NP + pr) * 128);
+      tma_store_commit();
+      tma_store_wait_read<0>();
+      mbar_arrive(saved);
     }
     tma_store_wait<0>();
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == STATE_WARPS + 4) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  if (warp == W::MMA_WARP) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
 // ============================================================================ backward state walk
@@ -992,41 +1023,37 @@ dn_bwd_state_kernel(const __grid_constant__ CUtensorMap tmDO, const __grid_const
       umma_commit_if(leader, s_done);
       umma_commit_if(leader, &stage_free[st]);
     }
+  } else if (warp == STATE_WARPS + 1) {
+    if (elect_one()) {
+      for (int it = 0; it < steps; ++it) {
+        const int c = c_top - it, st = it & 1;
+        if (it >= 2 && !mbar_wait(&stage_free[st], ((it >> 1) - 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
+        uint8_t* s = smem + st * STAGE;
+        const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 64;
+        mbar_expect_tx(&full[st], STAGE);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          tma_load_2d(s + b * 8192, &tmDO, &full[st], h * D + b * 64, c * CH);
+          tma_load_2d(s + 24576 + b * 8192, &tmKD, &full[st], b * 64, hrow);
+          tma_load_2d(s + 40960 + b * 8192, &tmQG, &full[st], b * 64, hrow);
+        }
+        tma_load_2d(s + 16384, &tmMQ, &full[st], 0, prow + hh * 64);
+        tma_load_2d(s + 57344, &tmWT, &full[st], hh * 64, prow);
+      }
+    }
   } else if (elect_one()) {
-    auto load_stage = [&](int it) {
-      const int c = c_top - it, st = it & 1;
-      uint8_t* s = smem + st * STAGE;
-      const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 64;
-      mbar_expect_tx(&full[st], STAGE);
+    for (int it = skip; it < steps; ++it) {
+      const int c = c_top - it;
+      if (!mbar_wait(s_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        tma_load_2d(s + b * 8192, &tmDO, &full[st], h * D + b * 64, c * CH);
-        tma_load_2d(s + 24576 + b * 8192, &tmKD, &full[st], b * 64, hrow);
-        tma_load_2d(s + 40960 + b * 8192, &tmQG, &full[st], b * 64, hrow);
-      }
-      tma_load_2d(s + 16384, &tmMQ, &full[st], 0, prow + hh * 64);
-      tma_load_2d(s + 57344, &tmWT, &full[st], hh * 64, prow);
-    };
-    load_stage(0);
-    if (steps > 1) load_stage(1);
-    for (int it = 0; it < steps; ++it) {
-      if (it >= skip) {
-        const int c = c_top - it;
-        if (!mbar_wait(s_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-          tma_store_2d(&tmDSP, smem + OFF_SOP + b * 16384, b * 64, (c * G.H + h) * 128);
-        tma_store_commit();
-        if (!mbar_wait(u_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
-        tma_store_2d(&tmDUT, smem + OFF_UOP, hh * 64, (c * G.NP + pr) * 128);
-        tma_store_commit();
-        tma_store_wait_read<0>();
-        mbar_arrive(saved);
-      }
-      if (it + 2 < steps) {
-        if (!mbar_wait(&stage_free[it & 1], (it >> 1) & 1, p.status, KS_TIMEOUT_EMPTY)) break;
-        load_stage(it + 2);
-      }
+      for (int b = 0; b < 2; ++b)
+        tma_store_2d(&tmDSP, smem + OFF_SOP + b * 16384, b * 64, (c * G.H + h) * 128);
+      tma_store_commit();
+      if (!mbar_wait(u_copied, (it - skip) & 1, p.status, KS_TIMEOUT_FULL)) break;
+      tma_store_2d(&tmDUT, smem + OFF_UOP, hh * 64, (c * G.NP + pr) * 128);
+      tma_store_commit();
+      tma_store_wait_read<0>();
+      mbar_arrive(saved);
     }
     tma_store_wait<0>();
   }
@@ -1633,6 +1660,7 @@ static int walk_bucket(const Geo& g) {
 }  // namespace ss_dnc
 
 // ---------------------------------------------------------------------------- launchers
+// ss_dn_fwd: `out` may be null where ST and UTp are given, which may be null where `out` is.
 // Shapes: q, k [T, Hk, 128] bf16; v, out, dout, dv [T, H, 128] bf16; beta, g, dbeta, dg [T, H] fp32;
 // sid int32 [n*64]; n = ceil(T/64); P = ceil((H/Hk)/2); NP = Hk*P.
 // Pair arrays [n, NP, 128, 128] bf16: WTp U0Tp UTp dUTp dWTp dKdTp dQgTp (columns = (head of pair, token)).
@@ -1688,26 +1716,34 @@ int ss_dn_fwd(const void* WTp, const void* U0Tp, const void* QG, const void* KD,
   if (H <= 0 || Hk <= 0 || H % Hk) return -2;
   const Geo geo = make_geo(T, H, Hk);
   const long long prow = (long long)geo.n * geo.NP * 128, hrow = (long long)geo.n * H * 64;
+  const bool save = ST != nullptr;
+  if (save != (UTp != nullptr) || (out == nullptr && !save)) return -2;
   CUtensorMap twt, tu0, tqg, tkd, tmq, tst, tut, to;
-  const bool save = ST != nullptr && UTp != nullptr;
   int r;
   if ((r = ss::make_tmap_bf16(&twt, WTp, prow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tu0, U0Tp, prow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tqg, QG, hrow, 128, 128, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tkd, KD, hrow, 128, 128, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tmq, MQ, prow, 64, 64, 64))) return r;
-  if ((ST != nullptr) != (UTp != nullptr)) return -2;
-  if ((r = ss::make_tmap_bf16(&tst, save ? ST : WTp, save ? (long long)geo.n * H * 128 : prow, 128, 128, 128))) return r;
-  if ((r = ss::make_tmap_bf16(&to, out, T, (long long)H * D, (long long)H * D, 64))) return r;
-  if ((r = ss::make_tmap_bf16(&tut, save ? UTp : WTp, prow, 128, 128, 128))) return r;
+  tst = tut = to = twt;                            // maps of what this walk does not write are not used
+  if (save) {
+    if ((r = ss::make_tmap_bf16(&tst, ST, (long long)geo.n * H * 128, 128, 128, 128))) return r;
+    if ((r = ss::make_tmap_bf16(&tut, UTp, prow, 128, 128, 128))) return r;
+  }
+  if (out != nullptr && (r = ss::make_tmap_bf16(&to, out, T, (long long)H * D, (long long)H * D, 64))) return r;
   WalkParams p;
-  p.gc = gc; p.sid = sid; p.bucket = walk_bucket(geo); p.save = save;
-  p.geo = geo; p.status = status;
-  static ss::SmemOptIn opt_in;
-  if (int e = opt_in.ensure(dn_fwd_kernel, walk::SMEM)) return e;
-  dn_fwd_kernel<<<dim3(H, (geo.n + p.bucket - 1) / p.bucket), walk::FWD_THREADS, walk::SMEM, (cudaStream_t)stream>>>(
-      twt, tu0, tqg, tkd, tmq, tst, tut, to, p);
-  return (int)cudaGetLastError();
+  p.gc = gc; p.sid = sid; p.bucket = walk_bucket(geo); p.geo = geo; p.status = status;
+  auto go = [&](auto kern, auto w, ss::SmemOptIn& opt_in) -> int {
+    using W = decltype(w);
+    if (int e = opt_in.ensure(kern, W::SMEM)) return e;
+    kern<<<dim3(H, (geo.n + p.bucket - 1) / p.bucket), W::THREADS, W::SMEM, (cudaStream_t)stream>>>(twt, tu0, tqg, tkd,
+                                                                                                    tmq, tst, tut, to, p);
+    return (int)cudaGetLastError();
+  };
+  static ss::SmemOptIn o1, o2, o3;
+  if (!save) return go(dn_fwd_kernel<true, false>, walk::Fwd<true, false>{}, o1);
+  return out != nullptr ? go(dn_fwd_kernel<true, true>, walk::Fwd<true, true>{}, o2)
+                        : go(dn_fwd_kernel<false, true>, walk::Fwd<false, true>{}, o3);
 }
 
 int ss_dn_bwd_state(const void* dout, const void* MQ, const void* KD, const void* QG, const void* WTp,
@@ -1727,7 +1763,7 @@ int ss_dn_bwd_state(const void* dout, const void* MQ, const void* KD, const void
   if ((r = ss::make_tmap_bf16(&tdsp, dSpT, (long long)geo.n * H * 128, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tdut, dUTp, prow, 128, 128, 128))) return r;
   WalkParams p;
-  p.gc = gc; p.sid = sid; p.bucket = walk_bucket(geo); p.save = 1; p.geo = geo; p.status = status;
+  p.gc = gc; p.sid = sid; p.bucket = walk_bucket(geo); p.geo = geo; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_bwd_state_kernel, walk::SMEM)) return e;
   dn_bwd_state_kernel<<<dim3(H, (geo.n + p.bucket - 1) / p.bucket), walk::BWD_THREADS, walk::SMEM,

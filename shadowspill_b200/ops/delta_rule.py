@@ -92,7 +92,7 @@ def _operand_key(q, k, v, beta, g, cu_seqlens):
     return tuple((t.data_ptr(), t._version, tuple(t.shape)) for t in (q, k, v, beta, g, cu_seqlens))
 
 
-def _forward(q, k, v, beta, g, cu_seqlens, backward: bool):
+def _forward(q, k, v, beta, g, cu_seqlens, backward: bool, output: bool = True):
     T, Hk, _ = q.shape
     H = v.shape[1]
     geo = _Geometry(T, H, Hk)
@@ -105,9 +105,9 @@ def _forward(q, k, v, beta, g, cu_seqlens, backward: bool):
                             B.sid.data_ptr(), B.WTp.data_ptr(), B.U0Tp.data_ptr(), B.QG.data_ptr(),
                             B.KD.data_ptr(), B.MQ.data_ptr(), _ptr(B.TMT), _ptr(B.XW), _ptr(B.XU),
                             B.gam.data_ptr(), B.gc.data_ptr(), T, H, Hk, scale, status, st), "ss_dn_prep")
-    out = torch.empty((T, H, WIDTH), dtype=torch.bfloat16, device=q.device)
+    out = torch.empty((T, H, WIDTH), dtype=torch.bfloat16, device=q.device) if output else None
     _lib.check(L.ss_dn_fwd(B.WTp.data_ptr(), B.U0Tp.data_ptr(), B.QG.data_ptr(), B.KD.data_ptr(),
-                           B.MQ.data_ptr(), B.gc.data_ptr(), B.sid.data_ptr(), out.data_ptr(), _ptr(B.ST), _ptr(B.UTp),
+                           B.MQ.data_ptr(), B.gc.data_ptr(), B.sid.data_ptr(), _ptr(out), _ptr(B.ST), _ptr(B.UTp),
                            T, H, Hk, status, st), "ss_dn_fwd")
     return out, B, geo
 
@@ -189,7 +189,7 @@ def _backward_all(q, k, v, beta, g, cu_seqlens, dout):
         _scope["key"] = _scope["value"] = None
     else:
         q, k, v, beta, g = _operands(q, k, v, beta, g)
-        _, B, geo = _forward(q, k, v, beta, g, cu_seqlens, backward=True)
+        _, B, geo = _forward(q, k, v, beta, g, cu_seqlens, backward=True, output=False)
     T, H, Hk = geo.T, geo.H, geo.Hk
     L, st, status = _lib.lib(), _lib.stream_ptr(), _lib.status_ptr(q)
     _lib.check(L.ss_dn_bwd_state(dout.data_ptr(), B.MQ.data_ptr(), B.KD.data_ptr(), B.QG.data_ptr(),

@@ -190,6 +190,32 @@ def test_walks_split_into_runs_give_the_whole_rule(T, Hk, Hv, bounds):
         assert _rel(x.grad, y.grad) < 3e-2, name
 
 
+@pytest.mark.parametrize("chunks", [1, 2, 3, 4, 5, 8, 9])
+def test_walks_with_and_without_output_and_saves_agree(chunks):
+    """One sequence of fewer and more chunks than any walk has stages: the walk that keeps nothing, the one that leaves
+    the output out and the one that does both run the same products in the same order, so they agree bit for bit; and
+    the result is the rule's (bf16 operands, as above)."""
+    from shadowspill_b200.ops import _lib, delta_rule
+    T = 64 * chunks - 1
+    q, k, v, beta, gl, dout, cu = _delta_case(T, 1, 3, [0, T], seed=chunks)
+    a, b = ([t.clone().cuda().requires_grad_(True) for t in (q, k, v, beta, gl)] for _ in range(2))
+    c = [t.clone().cuda().float().requires_grad_(True) for t in (q, k, v, beta, gl)]
+    got = seq.gated_delta_rule_chunked(*a, None, 64, cu_seqlens=cu.cuda())
+    got.backward(dout.cuda())
+    with delta_rule.keeping_intermediates():
+        both = seq.gated_delta_rule_chunked(*b, None, 64, cu_seqlens=cu.cuda())
+        both.backward(dout.cuda())
+    want = seq._gated_delta_rule_torch(*c, None, 64, cu_seqlens=cu.cuda())
+    want.backward(dout.cuda().float())
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(got, both)
+    assert _rel(got, want) < 1.5e-2
+    for name, x, y, z in zip("q k v beta g".split(), a, b, c):
+        assert torch.equal(x.grad, y.grad), name
+        assert _rel(x.grad, z.grad) < 3e-2, name
+
+
 @pytest.mark.gpu
 def test_head_groups_compute_the_same_rule_in_pieces():
     """Running the rule in groups of key heads (less intermediate memory) gives the same output
