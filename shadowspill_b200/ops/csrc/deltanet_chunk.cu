@@ -1219,10 +1219,11 @@ constexpr int OFF_KKF = 49152, OFF_QKF = OFF_KKF + 16640;          // fp32 [64][
 constexpr int OFF_DTM = 82944, OFF_XOP = OFF_DTM + 16384;          // operands
 constexpr int OFF_SYM = OFF_XOP + 16384, OFF_DQK = OFF_SYM + 8192;
 constexpr int OFF_KKA = OFF_DQK + 8192, OFF_QKA = OFF_KKA + 16640;  // fp32 accumulators over heads
-constexpr int OFF_OUT = OFF_KKF;                                   // 16 KiB tile of the output transposes
+constexpr int OFF_OUT = OFF_KKF;                                   // two 16 KiB tiles of the output transposes
 constexpr int OFF_DKD = OFF_XU + 16384, OFF_DQG = OFF_DTM;         // dKd^T and dQg^T of both heads, 32 KiB each
 constexpr int OFF_MISC = OFF_DKD + 32768;
 constexpr int OFF_BAR = OFF_MISC + 10240;
+static_assert(OFF_OUT + 32768 <= OFF_DTM, "output tiles overlap dQg");
 static_assert(OFF_QKA + 16640 <= OFF_MISC, "scratch overlaps the per-token values");
 constexpr int SMEM = OFF_BAR + 64 + 1024;
 static_assert(OFF_KKF >= OFF_TMT + 16384, "scratch overlaps a tile that stays live");
@@ -1259,9 +1260,10 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   int* sid_s = reinterpret_cast<int*>(misc + 2432);     // [65]
   unsigned* starts_s = reinterpret_cast<unsigned*>(misc + 2500);   // [2]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
-  uint64_t* dkd_bar = bars + 2; uint64_t* dqg_bar = bars + 3;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+  uint64_t* kq_bar = bars; uint64_t* u_bar = bars + 1; uint64_t* w_bar = bars + 2;   // groups of operands, as loaded
+  uint64_t* dkd_bar = bars + 3; uint64_t* dqg_bar = bars + 4;
+  uint64_t* mma_bar = bars + 5;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Geo G = p.geo;
@@ -1272,33 +1274,41 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const long long prow0 = (static_cast<long long>(c) * G.NP + pr) * 128;
 
   // the chunk's scalars, asked for ahead of all else: a memory latency that the set-up runs under
-  float gam = 0.f, beta = 0.f;
+  float gam = 0.f, beta = 0.f, dgc = 0.f;
   int sid = -1;
   if (tid < 128 && (tid >> 6) < nh) {
     const int hh = tid >> 6, j = tid & 63;
+    const long long hi = static_cast<long long>(c) * G.H + h0 + hh;
+    dgc = p.dgc[hi] * p.gc[hi];
     gam = p.gam[(static_cast<long long>(c) * G.H + h0 + hh) * 64 + j];
     if (t0 + j < G.T) beta = p.beta[static_cast<long long>(t0 + j) * G.H + h0 + hh];
   }
   if (tid < 64 || (tid == 64 && c > 0)) sid = p.sid[tid < 64 ? t0 + tid : t0 - 1];
 
   if (tid == BCTRL) {
-    mbar_init(tma_bar, 1); mbar_init(mma_bar, 1); mbar_init(dkd_bar, 1); mbar_init(dqg_bar, 1);
+    for (int i = 0; i < 6; ++i) mbar_init(&bars[i], 1);
     mbar_fence_init();
-    mbar_expect_tx(tma_bar, 32768 + nh * 16384 + 32768 + 32768 + 3 * 16384);
+    mbar_expect_tx(kq_bar, 32768);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      tma_load_2d(smem + OFF_KQ + b * 16384, &tmK, tma_bar, kh * D + b * 64, t0);
-      tma_load_2d(smem + OFF_KQ + b * 16384 + 64 * 128, &tmQ, tma_bar, kh * D + b * 64, t0);
-      tma_load_2d(smem + OFF_DWT + b * 16384, &tmDWT, tma_bar, b * 64, static_cast<int>(prow0));
-      tma_load_2d(smem + OFF_DUT + b * 16384, &tmDUT, tma_bar, b * 64, static_cast<int>(prow0));
+      tma_load_2d(smem + OFF_KQ + b * 16384, &tmK, kq_bar, kh * D + b * 64, t0);
+      tma_load_2d(smem + OFF_KQ + b * 16384 + 64 * 128, &tmQ, kq_bar, kh * D + b * 64, t0);
     }
+    mbar_expect_tx(u_bar, 32768 + nh * 16384 + 16384);
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      tma_load_2d(smem + OFF_DUT + b * 16384, &tmDUT, u_bar, b * 64, static_cast<int>(prow0));
     for (int hh = 0; hh < nh; ++hh)
 #pragma unroll
       for (int b = 0; b < 2; ++b)
-        tma_load_2d(smem + OFF_V + hh * 16384 + b * 8192, &tmV, tma_bar, (h0 + hh) * D + b * 64, t0);
-    tma_load_2d(smem + OFF_TMT, &tmTMT, tma_bar, 0, static_cast<int>(prow0));
-    tma_load_2d(smem + OFF_XW, &tmXW, tma_bar, 0, static_cast<int>(prow0));
-    tma_load_2d(smem + OFF_XU, &tmXU, tma_bar, 0, static_cast<int>(prow0));
+        tma_load_2d(smem + OFF_V + hh * 16384 + b * 8192, &tmV, u_bar, (h0 + hh) * D + b * 64, t0);
+    tma_load_2d(smem + OFF_XU, &tmXU, u_bar, 0, static_cast<int>(prow0));
+    mbar_expect_tx(w_bar, 32768 + 2 * 16384);
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      tma_load_2d(smem + OFF_DWT + b * 16384, &tmDWT, w_bar, b * 64, static_cast<int>(prow0));
+    tma_load_2d(smem + OFF_XW, &tmXW, w_bar, 0, static_cast<int>(prow0));
+    tma_load_2d(smem + OFF_TMT, &tmTMT, w_bar, 0, static_cast<int>(prow0));
     mbar_expect_tx(dkd_bar, nh * 16384);
     for (int hh = 0; hh < nh; ++hh)
       tma_load_2d(smem + OFF_DKD + hh * 16384, &tmDKD, dkd_bar, hh * 64, static_cast<int>(prow0));
@@ -1324,37 +1334,43 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     d_s[tid] = (sid_s[j] == sid_s[63]) ? __expf(gam_s[hh * 64 + 63] - gam_s[tid]) : 0.f;
   }
 
-  // ---- first group of products
+  // ---- first group of products, each as soon as its operands are there: the loads take longer than the products
   if (tid == BCTRL) {
-    mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
-    tc_fence_after();
     const uint32_t skq = smem_u32(smem + OFF_KQ), sv = smem_u32(smem + OFF_V);
     const uint32_t sdw = smem_u32(smem + OFF_DWT), sdu = smem_u32(smem + OFF_DUT);
     const uint32_t sxw = smem_u32(smem + OFF_XW), sxu = smem_u32(smem + OFF_XU);
     constexpr uint32_t i_kk = umma_idesc_bf16(128, 64, false, false);
     constexpr uint32_t i_mk = umma_idesc_bf16(128, 64, true, false);
+    auto kq = [&](int kk) { return umma_smem_desc(skq + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024); };
+    mbar_wait(kq_bar, 0, p.status, KS_TIMEOUT_FULL);
+    tc_fence_after();
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      const uint64_t kq = umma_smem_desc(skq + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-      umma_bf16(tmem_base, kq, kq, i_kk, kk != 0);                                   // [K;Q] K^T
-      umma_bf16(tmem_base + 64, umma_smem_desc(sdw + kk * 2048, 16384, 1024), kq, i_mk, kk != 0);   // P1 = dW K^T
-      for (int h2 = 0; h2 < nh; ++h2)                                                // P2 = dU V^T
-        umma_bf16(tmem_base + 128 + h2 * 64, umma_smem_desc(sdu + kk * 2048, 16384, 1024),
-                  umma_smem_desc(sv + h2 * 16384 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), i_mk,
-                  kk != 0);
-    }
+    for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem_base, kq(kk), kq(kk), i_kk, kk != 0);       // [K;Q] K^T
+    mbar_wait(u_bar, 0, p.status, KS_TIMEOUT_FULL);
+    tc_fence_after();
     for (int hh = 0; hh < nh; ++hh) {
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        umma_bf16(tmem_base + 256, umma_smem_desc(sdw + hh * 16384 + kk * 32, 16, 1024),       // dK^T
-                  umma_smem_desc(sxw + hh * 8192 + kk * 32, 16, 1024), i_kk, (hh | kk) != 0);
-        umma_bf16(tmem_base + 320 + hh * 64, umma_smem_desc(sdu + hh * 16384 + kk * 32, 16, 1024),  // dV^T
+      for (int kk = 0; kk < 8; ++kk)                                                   // P2 = dU V^T
+        umma_bf16(tmem_base + 128 + hh * 64, umma_smem_desc(sdu + kk * 2048, 16384, 1024),
+                  umma_smem_desc(sv + hh * 16384 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), i_mk, kk != 0);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)                                                   // dV^T
+        umma_bf16(tmem_base + 320 + hh * 64, umma_smem_desc(sdu + hh * 16384 + kk * 32, 16, 1024),
                   umma_smem_desc(sxu + hh * 8192 + kk * 32, 16, 1024), i_kk, kk != 0);
-      }
     }
+    mbar_wait(w_bar, 0, p.status, KS_TIMEOUT_FULL);
+    tc_fence_after();
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk)                                                     // P1 = dW K^T
+      umma_bf16(tmem_base + 64, umma_smem_desc(sdw + kk * 2048, 16384, 1024), kq(kk), i_mk, kk != 0);
+    for (int hh = 0; hh < nh; ++hh)
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)                                                   // dK^T
+        umma_bf16(tmem_base + 256, umma_smem_desc(sdw + hh * 16384 + kk * 32, 16, 1024),
+                  umma_smem_desc(sxw + hh * 8192 + kk * 32, 16, 1024), i_kk, (hh | kk) != 0);
     umma_commit(mma_bar);
   }
-  mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
+  mbar_wait(w_bar, 0, p.status, KS_TIMEOUT_FULL);
   mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
   mma_phase ^= 1;
   tc_fence_after();
@@ -1532,29 +1548,32 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     umma_commit(mma_bar);
   }
-  mbar_wait(dkd_bar, 0, p.status, KS_TIMEOUT_FULL);
-  mbar_wait(dqg_bar, 0, p.status, KS_TIMEOUT_FULL);
-  mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
-  mma_phase ^= 1;
-  tc_fence_after();
 
-  // ---- the diagonals (K rows on the first two warps' lanes, Q rows on the other two's), then the feature rows:
-  // dk, dq and dv, 16 tokens at a time, through the tile that turns them into token rows
+  // ---- the feature rows, 16 tokens at a time, through tiles that turn them into token rows: dv of the heads while
+  // those products run, then dk and dq
   const int lim = min(CH, G.T - t0);
   if (tid < ROW_THREADS) {
-    if (part < nh) {                                    // the left halves' threads take head 0, the right's head 1
-      uint32_t r[32];
-      tmem_ld_32x32(lane_addr + (row < 64 ? 0 : 128) + part * 64 + (warp & 1) * 32, r);
-      tmem_ld_wait();
-      float v = 0.f;
-#pragma unroll
-      for (int e = 0; e < 32; ++e) v = lane == e ? __uint_as_float(r[e]) : v;
-      (row < 64 ? dotk : dotq)[part * 64 + t_me] = v;
-    }
 #pragma unroll 1
-    for (int x = 0; x < 2 + nh; ++x) {                 // dk (with Kd), dq (with Qg), dv of the heads
+    for (int y = 0; y < nh + 2; ++y) {
+      const int x = y < nh ? 2 + y : y - nh;           // dk (with Kd), dq (with Qg), dv of the heads
       const uint32_t col = x == 0 ? 256 : x == 1 ? 448 : 320 + (x - 2) * 64;
-      if (x > 0) all_rows_sync();                    // the tile's last reader is done
+      uint8_t* out = smem + OFF_OUT + (y & 1) * 16384; // read two steps ago, and all have been at a barrier since
+      if (y == nh) {
+        mbar_wait(dkd_bar, 0, p.status, KS_TIMEOUT_FULL);
+        mbar_wait(dqg_bar, 0, p.status, KS_TIMEOUT_FULL);
+        mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
+        tc_fence_after();
+        // the diagonals: K rows on the first two warps' lanes, Q rows on the other two's
+        if (part < nh) {                               // the left halves' threads take head 0, the right's head 1
+          uint32_t r[32];
+          tmem_ld_32x32(lane_addr + (row < 64 ? 0 : 128) + part * 64 + (warp & 1) * 32, r);
+          tmem_ld_wait();
+          float v = 0.f;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v = lane == e ? __uint_as_float(r[e]) : v;
+          (row < 64 ? dotk : dotq)[part * 64 + t_me] = v;
+        }
+      }
 #pragma unroll 1
       for (int i0 = part * 32; i0 < part * 32 + 32; i0 += 16) {
         uint32_t r[16];
@@ -1584,7 +1603,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
 #pragma unroll
         for (int e = 0; e < 16; ++e)
-          *reinterpret_cast<__nv_bfloat16*>(smem + OFF_OUT + (i0 + e) * 256 + row * 2) = __float2bfloat16_rn(acc[e]);
+          *reinterpret_cast<__nv_bfloat16*>(out + (i0 + e) * 256 + row * 2) = __float2bfloat16_rn(acc[e]);
       }
       all_rows_sync();
       __nv_bfloat16* dst;
@@ -1601,7 +1620,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int t = q * 16 + (tid >> 4), ch = tid & 15;
         if (t < lim)
           *reinterpret_cast<uint4*>(dst + t * ld + ch * 8) =
-              *reinterpret_cast<const uint4*>(smem + OFF_OUT + t * 256 + ch * 16);
+              *reinterpret_cast<const uint4*>(out + t * 256 + ch * 16);
       }
     }
   }
@@ -1630,8 +1649,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   __syncthreads();
   if (live && tid < 128 && t_me < lim) {
-    const long long hi = static_cast<long long>(c) * G.H + h0 + hh_me;
-    s += (sums_s[hh_me * 2] + sums_s[hh_me * 2 + 1]) + p.dgc[hi] * p.gc[hi];
+    s += (sums_s[hh_me * 2] + sums_s[hh_me * 2 + 1]) + dgc;
     if (t_me < 32) s += sums_s[4 + hh_me * 2 + 1];
     const long long o = static_cast<long long>(t0 + t_me) * G.H + h0 + hh_me;
     p.dg[o] = s;
