@@ -94,6 +94,7 @@ __device__ __forceinline__ void publish() {
 template <int N>
 __device__ __forceinline__ void warp_col_sums(float (&v)[N], float* out) {
   const int lane = threadIdx.x & 31;
+  __syncwarp();                                 // lanes that a branch has left apart take each shuffle one by one
 #pragma unroll
   for (int o = 16, n = N / 2; o > 0; o >>= 1, n >>= 1) {
     if (n == 0) {                               // one column left, in both partners
@@ -264,7 +265,8 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const Geo G = p.geo;
   const int c = blockIdx.x, pr = blockIdx.y;
   const int kh = pr / G.P, z = pr % G.P, h0 = kh * G.rep + 2 * z;
@@ -298,7 +300,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 
   if (tid < 128) beta_s[tid] = beta;
@@ -325,7 +327,8 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   __syncthreads();
 
   // ---- [K; Q] K^T
-  if (tid == PCTRL) {
+  if (warp == 8) {
+    const uint32_t leader = elect_one();
     mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
     tc_fence_after();
     constexpr uint32_t idesc = umma_idesc_bf16(128, 64, false, false);
@@ -333,9 +336,9 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
       const uint64_t d = umma_smem_desc(s + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-      umma_bf16(tmem_base, d, d, idesc, kk != 0);
+      umma_bf16_if(leader, tmem_base, d, d, idesc, kk != 0);
     }
-    umma_commit(mma_bar);
+    umma_commit_if(leader, mma_bar);
   }
   mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
   mbar_wait(mma_bar, 0, p.status, KS_TIMEOUT_TMEM_FULL);
@@ -430,22 +433,23 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   publish();
 
   // ---- W^T = K^T (Tm diag(beta Gt))^T, U0^T = V^T (Tm diag(beta))^T
-  if (tid == PCTRL) {
+  if (warp == 8) {
+    const uint32_t leader = elect_one();
     constexpr uint32_t idesc = umma_idesc_bf16(128, 64, true, true);
     const uint32_t sk = smem_u32(smem + OFF_KQ), sv = smem_u32(smem + OFF_V);
     const uint32_t sxw = smem_u32(smem + OFF_XW), sxu = smem_u32(smem + OFF_XU);
     for (int hh = 0; hh < nh; ++hh) {
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem_base + hh * 64, umma_smem_desc(sk + kk * 2048, 16384, 1024),
+        umma_bf16_if(leader, tmem_base + hh * 64, umma_smem_desc(sk + kk * 2048, 16384, 1024),
                   umma_smem_desc(sxw + hh * 8192 + kk * 2048, 8192, 1024), idesc, kk != 0);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem_base + 128 + hh * 64, umma_smem_desc(sv + hh * 16384 + kk * 2048, 8192, 1024),
+        umma_bf16_if(leader, tmem_base + 128 + hh * 64, umma_smem_desc(sv + hh * 16384 + kk * 2048, 8192, 1024),
                   umma_smem_desc(sxu + hh * 8192 + kk * 2048, 8192, 1024), idesc, kk != 0);
     }
-    umma_commit(mma_bar);
-    if (p.save) {                                // the operands are saved from the tiles the products read
+    umma_commit_if(leader, mma_bar);
+    if (p.save && tid == PCTRL) {                // the operands are saved from the tiles the products read
       for (int hh = 0; hh < nh; ++hh) {
         tma_store_2d(&tmXW, smem + OFF_XW + hh * 8192, 0, (c * G.NP + pr) * 128 + hh * 64);
         tma_store_2d(&tmXU, smem + OFF_XU + hh * 8192, 0, (c * G.NP + pr) * 128 + hh * 64);
@@ -1095,7 +1099,8 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* tma_bar = bars; uint64_t* mma_bar = bars + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const Geo G = p.geo;
   const int c = blockIdx.x, h = blockIdx.y;
   int pr, hh;
@@ -1106,20 +1111,23 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 
-  if (tid == CTRL) {
-    const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 128;
-    mbar_expect_tx(tma_bar, 114688);
+  if (warp == 4) {
+    const uint32_t leader = elect_one();
+    if (leader) {
+      const int prow = (c * G.NP + pr) * 128, hrow = (c * G.H + h) * 128;
+      mbar_expect_tx(tma_bar, 114688);
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      tma_load_2d(smem + OFF_DSP + b * 16384, &tmDSP, tma_bar, b * 64, hrow);
-      tma_load_2d(smem + OFF_ST + b * 16384, &tmST, tma_bar, b * 64, hrow);
-      tma_load_2d(smem + OFF_DO + b * 8192, &tmDO, tma_bar, h * D + b * 64, c * CH);
+      for (int b = 0; b < 2; ++b) {
+        tma_load_2d(smem + OFF_DSP + b * 16384, &tmDSP, tma_bar, b * 64, hrow);
+        tma_load_2d(smem + OFF_ST + b * 16384, &tmST, tma_bar, b * 64, hrow);
+        tma_load_2d(smem + OFF_DO + b * 8192, &tmDO, tma_bar, h * D + b * 64, c * CH);
+      }
+      tma_load_2d(smem + OFF_UT, &tmUT, tma_bar, hh * 64, prow);
+      tma_load_2d(smem + OFF_DUT, &tmDUT, tma_bar, hh * 64, prow);
     }
-    tma_load_2d(smem + OFF_UT, &tmUT, tma_bar, hh * 64, prow);
-    tma_load_2d(smem + OFF_DUT, &tmDUT, tma_bar, hh * 64, prow);
     mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
     tc_fence_after();
     const uint32_t sdsp = smem_u32(smem + OFF_DSP), sst = smem_u32(smem + OFF_ST);
@@ -1135,12 +1143,12 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
       const uint64_t b_ut = umma_smem_desc(sut + kk * 2048, 16384, 1024);
       const uint64_t b_dut = umma_smem_desc(sdut + kk * 2048, 16384, 1024);
       const uint64_t k_do = umma_smem_desc(sdo + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024);
-      umma_bf16(tmem_base, a_dsp, b_ut, i_mm, kk != 0);          // dKd^T = dS' U^T
-      umma_bf16(tmem_base + 64, a_st, k_do, i_mk, kk != 0);      // dQg^T = S dO^T
-      umma_bf16(tmem_base + 128, a_st, b_dut, i_mm, kk != 0);    // (S dU^T), negated below
-      umma_bf16(tmem_base + 192, k_do, b_ut, i_km, kk != 0);     // dMq = dO U^T (rows 0..63; the tile has no others)
+      umma_bf16_if(leader, tmem_base, a_dsp, b_ut, i_mm, kk != 0);          // dKd^T = dS' U^T
+      umma_bf16_if(leader, tmem_base + 64, a_st, k_do, i_mk, kk != 0);      // dQg^T = S dO^T
+      umma_bf16_if(leader, tmem_base + 128, a_st, b_dut, i_mm, kk != 0);    // (S dU^T), negated below
+      umma_bf16_if(leader, tmem_base + 192, k_do, b_ut, i_km, kk != 0);     // dMq = dO U^T (rows 0..63; the tile has no others)
     }
-    umma_commit(mma_bar);
+    umma_commit_if(leader, mma_bar);
   }
   mbar_wait(tma_bar, 0, p.status, KS_TIMEOUT_FULL);
   // dGc = <S, dS'> while the MMAs run (both tiles share one layout, so no unswizzling)
@@ -1203,13 +1211,13 @@ dn_bwd_chunk_kernel(const __grid_constant__ CUtensorMap tmDSP, const __grid_cons
 struct BwdPrepParams {
   const float* beta; const int* sid; const float* gam; const float* gc; const float* dgc;
   const __nv_bfloat16* dMQ;
-  __nv_bfloat16 *dq, *dk, *dv;     // dq, dk: [T, NP, D] (summed over pairs by the caller); dv [T, H, D]
   float *dbeta, *dg;               // [T, H]
   Geo geo; float scale; int* status;
 };
 // Eight row warps, two to each quarter of the TMEM lanes: a thread has half the columns of its row. One CTA an SM, so its
-// chain of loads, products and row work is all there is: 44,000 -> 34,000 cycles, 0.373 -> 0.264 ms at 8,192 tokens
-// and 16 / 32 heads, with the tokens' dot products on the tensor cores, dKd and dQg by TMA and twice the warps.
+// chain of loads, products and row work is all there is: 44,000 -> 26,000 cycles, 0.373 -> 0.209 ms at 8,192 tokens
+// and 16 / 32 heads, with the tokens' dot products on the tensor cores, all operands and results by TMA, twice the warps,
+// products as their operands arrive (0.026 ms) and a warp in step that issues them from uniform registers (0.021 ms).
 namespace bprep {
 constexpr int ROW_THREADS = 256, BTHREADS = ROW_THREADS + 32, BCTRL = ROW_THREADS;
 constexpr int OFF_KQ = 0, OFF_TMT = 32768, OFF_V = 49152, OFF_DWT = 81920, OFF_DUT = 114688;
@@ -1236,7 +1244,8 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmDUT, const __grid_constant__ CUtensorMap tmTMT,
                    const __grid_constant__ CUtensorMap tmXW, const __grid_constant__ CUtensorMap tmXU,
                    const __grid_constant__ CUtensorMap tmDKD, const __grid_constant__ CUtensorMap tmDQG,
-                   const BwdPrepParams p) {
+                   const __grid_constant__ CUtensorMap tmOK, const __grid_constant__ CUtensorMap tmOQ,
+                   const __grid_constant__ CUtensorMap tmOV, const BwdPrepParams p) {
   using namespace bprep;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_smem_1024(smem_raw);
@@ -1265,7 +1274,8 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* mma_bar = bars + 5;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = static_cast<int>(warp_uniform(tid >> 5));
   const Geo G = p.geo;
   const int c = blockIdx.x, pr = blockIdx.y;
   const int kh = pr / G.P, z = pr % G.P, h0 = kh * G.rep + 2 * z;
@@ -1317,7 +1327,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   uint32_t mma_phase = 0;
 
@@ -1335,7 +1345,8 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
 
   // ---- first group of products, each as soon as its operands are there: the loads take longer than the products
-  if (tid == BCTRL) {
+  if (warp == 8) {
+    const uint32_t leader = elect_one();
     const uint32_t skq = smem_u32(smem + OFF_KQ), sv = smem_u32(smem + OFF_V);
     const uint32_t sdw = smem_u32(smem + OFF_DWT), sdu = smem_u32(smem + OFF_DUT);
     const uint32_t sxw = smem_u32(smem + OFF_XW), sxu = smem_u32(smem + OFF_XU);
@@ -1345,30 +1356,39 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_wait(kq_bar, 0, p.status, KS_TIMEOUT_FULL);
     tc_fence_after();
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) umma_bf16(tmem_base, kq(kk), kq(kk), i_kk, kk != 0);       // [K;Q] K^T
+    for (int kk = 0; kk < 8; ++kk) umma_bf16_if(leader, tmem_base, kq(kk), kq(kk), i_kk, kk != 0);       // [K;Q] K^T
     mbar_wait(u_bar, 0, p.status, KS_TIMEOUT_FULL);
     tc_fence_after();
     for (int hh = 0; hh < nh; ++hh) {
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)                                                   // P2 = dU V^T
-        umma_bf16(tmem_base + 128 + hh * 64, umma_smem_desc(sdu + kk * 2048, 16384, 1024),
+        umma_bf16_if(leader, tmem_base + 128 + hh * 64, umma_smem_desc(sdu + kk * 2048, 16384, 1024),
                   umma_smem_desc(sv + hh * 16384 + (kk >> 2) * 8192 + (kk & 3) * 32, 16, 1024), i_mk, kk != 0);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)                                                   // dV^T
-        umma_bf16(tmem_base + 320 + hh * 64, umma_smem_desc(sdu + hh * 16384 + kk * 32, 16, 1024),
+        umma_bf16_if(leader, tmem_base + 320 + hh * 64, umma_smem_desc(sdu + hh * 16384 + kk * 32, 16, 1024),
                   umma_smem_desc(sxu + hh * 8192 + kk * 32, 16, 1024), i_kk, kk != 0);
     }
     mbar_wait(w_bar, 0, p.status, KS_TIMEOUT_FULL);
     tc_fence_after();
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk)                                                     // P1 = dW K^T
-      umma_bf16(tmem_base + 64, umma_smem_desc(sdw + kk * 2048, 16384, 1024), kq(kk), i_mk, kk != 0);
+      umma_bf16_if(leader, tmem_base + 64, umma_smem_desc(sdw + kk * 2048, 16384, 1024), kq(kk), i_mk, kk != 0);
     for (int hh = 0; hh < nh; ++hh)
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)                                                   // dK^T
-        umma_bf16(tmem_base + 256, umma_smem_desc(sdw + hh * 16384 + kk * 32, 16, 1024),
+        umma_bf16_if(leader, tmem_base + 256, umma_smem_desc(sdw + hh * 16384 + kk * 32, 16, 1024),
                   umma_smem_desc(sxw + hh * 8192 + kk * 32, 16, 1024), i_kk, (hh | kk) != 0);
-    umma_commit(mma_bar);
+    umma_commit_if(leader, mma_bar);
+  }
+  const int row = tid & 127, part = (tid >> 7) & 1;      // of the row threads: a lane of TMEM and the half of its columns
+  const int hh_me = row >> 6, t_me = row & 63;
+  const bool live = tid < ROW_THREADS && hh_me < nh;
+  uint4 m[4] = {};                                       // dMq, ahead of the wait for the products
+  if (live) {
+    const uint4* mq = reinterpret_cast<const uint4*>(p.dMQ + (prow0 + row) * 64 + part * 32);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) m[x] = mq[x];
   }
   mbar_wait(w_bar, 0, p.status, KS_TIMEOUT_FULL);
   mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
@@ -1376,7 +1396,6 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_after();
 
   // ---- K K^T and Q K^T to shared memory (both heads need both)
-  const int row = tid & 127, part = (tid >> 7) & 1;      // of the row threads: a lane of TMEM and the half of its columns
   if (tid < ROW_THREADS) {
     float v[32];
     tmem_row32(lane_addr + part * 32, v);
@@ -1386,8 +1405,6 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   __syncthreads();
 
-  const int hh_me = row >> 6, t_me = row & 63;
-  const bool live = tid < ROW_THREADS && hh_me < nh;
   // ---- dTm = (P1, P2) scaled per column; column sums of Tm o P1 and Tm o P2
   if (tid < ROW_THREADS) {
     float p1[32], p2[32], dtm[32];
@@ -1411,15 +1428,16 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   publish();
 
   // ---- X = dTm Tm^T
-  if (tid == BCTRL) {
+  if (warp == 8) {
+    const uint32_t leader = elect_one();
     constexpr uint32_t i_km = umma_idesc_bf16(128, 64, false, true);
     const uint32_t sd = smem_u32(smem + OFF_DTM), st = smem_u32(smem + OFF_TMT);
     for (int h2 = 0; h2 < nh; ++h2)
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem_base + 64 + h2 * 64, umma_smem_desc(sd + kk * 32, 16, 1024),
+        umma_bf16_if(leader, tmem_base + 64 + h2 * 64, umma_smem_desc(sd + kk * 32, 16, 1024),
                   umma_smem_desc(st + h2 * 8192 + kk * 2048, 8192, 1024), i_km, kk != 0);
-    umma_commit(mma_bar);
+    umma_commit_if(leader, mma_bar);
   }
   mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
   mma_phase ^= 1;
@@ -1434,15 +1452,16 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   publish();
 
   // ---- dA = -Tm^T X
-  if (tid == BCTRL) {
+  if (warp == 8) {
+    const uint32_t leader = elect_one();
     constexpr uint32_t i_km = umma_idesc_bf16(128, 64, false, true);
     const uint32_t st = smem_u32(smem + OFF_TMT), sx = smem_u32(smem + OFF_XOP);
     for (int h2 = 0; h2 < nh; ++h2)
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
-        umma_bf16(tmem_base + (h2 == 0 ? 192 : 0), umma_smem_desc(st + kk * 32, 16, 1024),
+        umma_bf16_if(leader, tmem_base + (h2 == 0 ? 192 : 0), umma_smem_desc(st + kk * 32, 16, 1024),
                   umma_smem_desc(sx + h2 * 8192 + kk * 2048, 8192, 1024), i_km, kk != 0);
-    umma_commit(mma_bar);
+    umma_commit_if(leader, mma_bar);
   }
   mbar_wait(mma_bar, mma_phase, p.status, KS_TIMEOUT_TMEM_FULL);
   mma_phase ^= 1;
@@ -1459,10 +1478,6 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   // warps per scheduler, and fetching straight-line code was its largest stall.
   float rowG = 0.f, rowdb = 0.f;
   if (tid < ROW_THREADS) {
-    const uint4* mq = reinterpret_cast<const uint4*>(p.dMQ + (prow0 + row) * 64 + part * 32);
-    uint4 m[4];
-#pragma unroll
-    for (int x = 0; x < 4; ++x) m[x] = live ? mq[x] : make_uint4(0, 0, 0, 0);
     const int lo = seq_begin(starts_s, t_me);
     const float gt = gam_s[row], bt = beta_s[row];
 #pragma unroll 1
@@ -1520,7 +1535,8 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   // ---- dK^T += K^T (dKK + dKK^T) + Q^T dQK;  dQ^T = K^T dQK^T;  and [K; Q] dKd^T, [K; Q] dQg^T, whose diagonals are
   // the tokens' <dKd, K> and <dQg, Q> (as sums over the row threads they were 260 shuffles and two-byte loads each)
-  if (tid == BCTRL) {
+  if (warp == 8) {
+    const uint32_t leader = elect_one();
     constexpr uint32_t i_mm = umma_idesc_bf16(128, 64, true, true);
     constexpr uint32_t i_mk = umma_idesc_bf16(128, 64, true, false);
     constexpr uint32_t i_km = umma_idesc_bf16(128, 64, false, true);
@@ -1530,9 +1546,9 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     for (int kk = 0; kk < 4; ++kk) {
       const uint64_t ak = umma_smem_desc(skq + kk * 2048, 16384, 1024);
       const uint64_t aq = umma_smem_desc(skq + 8192 + kk * 2048, 16384, 1024);
-      umma_bf16(tmem_base + 256, ak, umma_smem_desc(ssym + kk * 2048, 8192, 1024), i_mm, 1);
-      umma_bf16(tmem_base + 256, aq, umma_smem_desc(sdqk + kk * 2048, 8192, 1024), i_mm, 1);
-      umma_bf16(tmem_base + 448, ak, umma_smem_desc(sdqk + kk * 32, 16, 1024), i_mk, kk != 0);
+      umma_bf16_if(leader, tmem_base + 256, ak, umma_smem_desc(ssym + kk * 2048, 8192, 1024), i_mm, 1);
+      umma_bf16_if(leader, tmem_base + 256, aq, umma_smem_desc(sdqk + kk * 2048, 8192, 1024), i_mm, 1);
+      umma_bf16_if(leader, tmem_base + 448, ak, umma_smem_desc(sdqk + kk * 32, 16, 1024), i_mk, kk != 0);
     }
     mbar_wait(dkd_bar, 0, p.status, KS_TIMEOUT_FULL);
     mbar_wait(dqg_bar, 0, p.status, KS_TIMEOUT_FULL);
@@ -1543,21 +1559,21 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint32_t sb = smem_u32(smem + (x < 2 ? OFF_DKD : OFF_DQG) + (x & 1) * 16384);
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
-        umma_bf16(tmem_base + x * 64, umma_smem_desc(skq + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
+        umma_bf16_if(leader, tmem_base + x * 64, umma_smem_desc(skq + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024),
                   umma_smem_desc(sb + kk * 2048, 16384, 1024), i_km, kk != 0);
     }
-    umma_commit(mma_bar);
+    umma_commit_if(leader, mma_bar);
   }
 
-  // ---- the feature rows, 16 tokens at a time, through tiles that turn them into token rows: dv of the heads while
-  // those products run, then dk and dq
+  // ---- the feature rows, 16 tokens at a time, through tiles that turn them into token rows, which leave by TMA (the last
+  // chunk's rows clipped): dv of the heads while those products run, then dk and dq
   const int lim = min(CH, G.T - t0);
   if (tid < ROW_THREADS) {
 #pragma unroll 1
     for (int y = 0; y < nh + 2; ++y) {
       const int x = y < nh ? 2 + y : y - nh;           // dk (with Kd), dq (with Qg), dv of the heads
       const uint32_t col = x == 0 ? 256 : x == 1 ? 448 : 320 + (x - 2) * 64;
-      uint8_t* out = smem + OFF_OUT + (y & 1) * 16384; // read two steps ago, and all have been at a barrier since
+      uint8_t* out = smem + OFF_OUT + (y & 1) * 16384; // has left: see below
       if (y == nh) {
         mbar_wait(dkd_bar, 0, p.status, KS_TIMEOUT_FULL);
         mbar_wait(dqg_bar, 0, p.status, KS_TIMEOUT_FULL);
@@ -1603,24 +1619,19 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
 #pragma unroll
         for (int e = 0; e < 16; ++e)
-          *reinterpret_cast<__nv_bfloat16*>(out + (i0 + e) * 256 + row * 2) = __float2bfloat16_rn(acc[e]);
+          *reinterpret_cast<__nv_bfloat16*>(out + (row >> 6) * 8192 + (i0 + e) * 128 + (((row & 63) * 2) ^ ((e & 7) << 4))) =
+              __float2bfloat16_rn(acc[e]);
       }
+      fence_async_proxy();
+      if (tid == 0) tma_store_wait_read<0>();          // the tile before has left when all have passed the barrier
       all_rows_sync();
-      __nv_bfloat16* dst;
-      long long ld;
-      if (x < 2) {
-        ld = static_cast<long long>(G.NP) * D;
-        dst = (x == 0 ? p.dk : p.dq) + (static_cast<long long>(t0) * G.NP + pr) * D;
-      } else {
-        ld = static_cast<long long>(G.H) * D;
-        dst = p.dv + (static_cast<long long>(t0) * G.H + h0 + x - 2) * D;
-      }
+      if (tid == 0) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int t = q * 16 + (tid >> 4), ch = tid & 15;
-        if (t < lim)
-          *reinterpret_cast<uint4*>(dst + t * ld + ch * 8) =
-              *reinterpret_cast<const uint4*>(out + t * 256 + ch * 16);
+        for (int b = 0; b < 2; ++b) {
+          if (x >= 2) tma_store_2d(&tmOV, out + b * 8192, (h0 + x - 2) * D + b * 64, t0);
+          else tma_store_2d(x == 0 ? &tmOK : &tmOQ, out + b * 8192, pr * D + b * 64, t0);
+        }
+        tma_store_commit();
       }
     }
   }
@@ -1638,6 +1649,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tail = d_s[tid] * dotk[tid];
       s = rowG - two(colG, t_me) + beta_s[tid] * gt_s[tid] * two(cs1, t_me) + p.scale * gt_s[tid] * dotq[tid] - tail;
     }
+    __syncwarp();                                       // see warp_col_sums: here 3,100 -> 900 cycles
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tail += __shfl_xor_sync(0xffffffffu, tail, o);
 #pragma unroll
@@ -1658,6 +1670,7 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before();
   __syncthreads();
   if (warp == 8) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+  if (tid == 0) tma_store_wait<0>();
 }
 
 static Geo make_geo(int T, int H, int Hk) {
@@ -1825,7 +1838,7 @@ int ss_dn_bwd_prep(const void* q, const void* k, const void* v, const float* bet
   if (H <= 0 || Hk <= 0 || H % Hk) return -2;
   const Geo geo = make_geo(T, H, Hk);
   const long long prow = (long long)geo.n * geo.NP * 128;
-  CUtensorMap tq, tk, tv, tdw, tdu, ttm, txw, txu, tkd, tqg;
+  CUtensorMap tq, tk, tv, tdw, tdu, ttm, txw, txu, tkd, tqg, tok, toq, tov;
   int r;
   if ((r = ss::make_tmap_bf16(&tq, q, T, (long long)Hk * D, (long long)Hk * D, 64))) return r;
   if ((r = ss::make_tmap_bf16(&tk, k, T, (long long)Hk * D, (long long)Hk * D, 64))) return r;
@@ -1837,14 +1850,17 @@ int ss_dn_bwd_prep(const void* q, const void* k, const void* v, const float* bet
   if ((r = ss::make_tmap_bf16(&txu, XU, prow, 64, 64, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tkd, dKdTp, prow, 128, 128, 128))) return r;
   if ((r = ss::make_tmap_bf16(&tqg, dQgTp, prow, 128, 128, 128))) return r;
+  const long long owidth = (long long)geo.NP * D;        // dq, dk: [T, NP, D], summed over pairs by the caller
+  if ((r = ss::make_tmap_bf16(&tok, dk, T, owidth, owidth, 64))) return r;
+  if ((r = ss::make_tmap_bf16(&toq, dq, T, owidth, owidth, 64))) return r;
+  if ((r = ss::make_tmap_bf16(&tov, dv, T, (long long)H * D, (long long)H * D, 64))) return r;
   BwdPrepParams p;
   p.beta = beta; p.sid = sid; p.gam = gam; p.gc = gc; p.dgc = dgc;
-  p.dMQ = (const __nv_bfloat16*)dMQ; p.dq = (__nv_bfloat16*)dq; p.dk = (__nv_bfloat16*)dk;
-  p.dv = (__nv_bfloat16*)dv; p.dbeta = dbeta; p.dg = dg; p.geo = geo; p.scale = scale; p.status = status;
+  p.dMQ = (const __nv_bfloat16*)dMQ; p.dbeta = dbeta; p.dg = dg; p.geo = geo; p.scale = scale; p.status = status;
   static ss::SmemOptIn opt_in;
   if (int e = opt_in.ensure(dn_bwd_prep_kernel, bprep::SMEM)) return e;
   dn_bwd_prep_kernel<<<dim3(geo.n, geo.NP), bprep::BTHREADS, bprep::SMEM, (cudaStream_t)stream>>>(
-      tq, tk, tv, tdw, tdu, ttm, txw, txu, tkd, tqg, p);
+      tq, tk, tv, tdw, tdu, ttm, txw, txu, tkd, tqg, tok, toq, tov, p);
   return (int)cudaGetLastError();
 }
 }  // extern "C"
