@@ -121,6 +121,11 @@ __device__ __forceinline__ int seq_begin(const unsigned* starts, int t) {
   const unsigned long long m = (static_cast<unsigned long long>(starts[1]) << 32) | starts[0];
   return 63 - __clzll(static_cast<long long>(m & (~0ull >> (63 - t))));
 }
+// Bits lo..hi of the 32 columns from c0 on: what a thread's tests of 32 columns come to.
+__device__ __forceinline__ uint32_t span_bits(int lo, int hi, int c0) {
+  const int b0 = max(lo - c0, 0), b1 = min(hi - c0, 31);
+  return b0 <= b1 ? (0xffffffffu >> (31 - b1)) & (0xffffffffu << b0) : 0u;
+}
 // ============================================================================ sequence ids
 __global__ void dn_seq_ids_kernel(const int* __restrict__ cu, int nseq, int T, int Tp,
                                   int* __restrict__ sid) {
@@ -350,7 +355,7 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const int t = row & 63, last = t | 31;               // the warp's last row
     const int lo = seq_begin(starts_s, t);
     const bool is_q = row >= 64;
-    const int hi = is_q ? t : t - 1;                     // Mq includes the diagonal, A does not
+    const uint32_t span = span_bits(lo, is_q ? t : t - 1, part * 32);    // Mq includes the diagonal, A does not
 #pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
       const float gt = gam_s[hh * 64 + t], f = is_q ? p.scale : beta_s[hh * 64 + t];
@@ -360,29 +365,34 @@ dn_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         head_sync(1);
       }
 #pragma unroll 1
-      for (int i0 = part * 32; i0 < part * 32 + 32; i0 += 8) {
-        float m[8];
+      for (int i0 = part * 32; i0 < part * 32 + 32; i0 += 16) {
+        float m[16];
         if (i0 > last) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) m[e] = 0.f;
+          for (int e = 0; e < 16; ++e) m[e] = 0.f;
         } else {
-          uint32_t r[8];
-          tmem_ld_32x8(lane_addr + i0, r);
-          *reinterpret_cast<float4*>(m) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0);
-          *reinterpret_cast<float4*>(m + 4) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0 + 4);
+          uint32_t r[16];
+          tmem_ld_32x16(lane_addr + i0, r);
+#pragma unroll
+          for (int e = 0; e < 16; e += 4)
+            *reinterpret_cast<float4*>(m + e) = *reinterpret_cast<const float4*>(gam_s + hh * 64 + i0 + e);
+          const uint32_t seen = span >> (i0 & 31);
           tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const bool seen = i0 + e >= lo && i0 + e <= hi;
-            const float v = f * decay_if(seen, gt - m[e]) * __uint_as_float(r[e]);
-            m[e] = seen ? v : 0.f;
+          for (int e = 0; e < 16; ++e) {
+            const bool on = seen & (1u << e);
+            const float v = f * decay_if(on, gt - m[e]) * __uint_as_float(r[e]);
+            m[e] = on ? v : 0.f;
           }
         }
         if (is_q) {
-          *reinterpret_cast<uint4*>(smem + OFF_MQ + sw_off(64, t, i0 >> 3)) = pack8(m);
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            *reinterpret_cast<uint4*>(smem + OFF_MQ + sw_off(64, t, (i0 >> 3) + q)) = pack8(m + q * 8);
         } else {
-          *reinterpret_cast<float4*>(a + i0) = *reinterpret_cast<const float4*>(m);
-          *reinterpret_cast<float4*>(a + i0 + 4) = *reinterpret_cast<const float4*>(m + 4);
+#pragma unroll
+          for (int e = 0; e < 16; e += 4)
+            *reinterpret_cast<float4*>(a + i0 + e) = *reinterpret_cast<const float4*>(m + e);
         }
       }
       if (is_q) {
@@ -1478,7 +1488,8 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   // warps per scheduler, and fetching straight-line code was its largest stall.
   float rowG = 0.f, rowdb = 0.f;
   if (tid < ROW_THREADS) {
-    const int lo = seq_begin(starts_s, t_me);
+    const uint32_t span = live ? span_bits(seq_begin(starts_s, t_me), t_me, part * 32) : 0u;
+    const uint32_t below = t_me >> 5 == part ? span & ~(1u << (t_me & 31)) : span;       // without the diagonal
     const float gt = gam_s[row], bt = beta_s[row];
 #pragma unroll 1
     for (int i0 = part * 32; i0 < part * 32 + 32; i0 += 16) {
@@ -1494,16 +1505,16 @@ dn_bwd_prep_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       unpack8(m[0], dmq);
       unpack8(m[1], dmq + 8);
       m[0] = m[2]; m[1] = m[3];
+      const uint32_t on = span >> (i0 & 31), under = below >> (i0 & 31);
       tmem_ld_wait();
       all_rows_sync();
       float* ko = (hh_me == 0 ? KKa : KKf) + t_me * 65 + i0;
       float* qo = (hh_me == 0 ? QKa : QKf) + t_me * 65 + i0;
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        const int i = i0 + e;
-        const bool seen = live && i >= lo && i <= t_me;
+        const bool seen = on & (1u << e);
         const float R = decay_if(seen, gt - gi[e]);
-        const float da = seen && i < t_me ? -__uint_as_float(acc[e]) : 0.f;
+        const float da = under & (1u << e) ? -__uint_as_float(acc[e]) : 0.f;
         rowdb += da * R * kk[e];
         const float dkk = da * bt * R, dqk = dmq[e] * p.scale * R;
         w[e] = seen ? dkk * kk[e] + dqk * qk[e] : 0.f;           // dR o R
