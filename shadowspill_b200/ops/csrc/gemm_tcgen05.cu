@@ -142,7 +142,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const int num_m = (p.M + BM - 1) / BM;
   const int num_n = (p.N + TILE_N - 1) / TILE_N;
@@ -171,7 +171,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after();
   chain_wait();
   chain_release();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -220,47 +220,46 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const TileWork w = decode_tile(p, t, num_m, num_n, num_kb);
-        if (w.skip || w.nkb == 0) continue;
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+    const uint32_t leader = elect_one();
+    constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const TileWork w = decode_tile(p, t, num_m, num_n, num_kb);
+      if (w.skip || w.nkb == 0) continue;
+      if (!mbar_wait(&tempty[acc], acc_phase ^ 1, p.status, KS_TIMEOUT_TMEM_EMPTY)) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+      for (int kb = 0; kb < w.nkb; ++kb) {
+        if (!mbar_wait(&full[stage], phase, p.status, KS_TIMEOUT_FULL)) {
+          ok = false;
+          break;
+        }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int kb = 0; kb < w.nkb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, p.status, KS_TIMEOUT_FULL)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
-          const uint32_t sb = sa + Cfg::A_BYTES;
+        const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
+        const uint32_t sb = sa + Cfg::A_BYTES;
 #pragma unroll
-          for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            const uint64_t adesc = A_MN ? umma_smem_desc(sa + kk * (UMMA_K * 128), BK * 128, 1024)
-                                        : umma_smem_desc(sa + kk * (UMMA_K * 2), 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_smem_desc(sb + kk * (UMMA_K * 128), BK * 128, 1024)
-                                        : umma_smem_desc(sb + kk * (UMMA_K * 2), 16, 1024);
-            umma_bf16(d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
-          }
-          umma_commit(&empty[stage]);  // stage reusable once these MMAs retire
-          if (++stage == Cfg::STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
+        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+          const uint64_t adesc = A_MN ? umma_smem_desc(sa + kk * (UMMA_K * 128), BK * 128, 1024)
+                                      : umma_smem_desc(sa + kk * (UMMA_K * 2), 16, 1024);
+          const uint64_t bdesc = B_MN ? umma_smem_desc(sb + kk * (UMMA_K * 128), BK * 128, 1024)
+                                      : umma_smem_desc(sb + kk * (UMMA_K * 2), 16, 1024);
+          umma_bf16_if(leader, d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
         }
-        if (!ok) break;
-        umma_commit(&tfull[acc]);
-        if (++acc == 2) {
-          acc = 0;
-          acc_phase ^= 1;
+        umma_commit_if(leader, &empty[stage]);  // stage reusable once these MMAs retire
+        if (++stage == Cfg::STAGES) {
+          stage = 0;
+          phase ^= 1;
         }
+      }
+      if (!ok) break;
+      umma_commit_if(leader, &tfull[acc]);
+      if (++acc == 2) {
+        acc = 0;
+        acc_phase ^= 1;
       }
     }
   } else {

@@ -149,24 +149,30 @@ __device__ __forceinline__ void tma2_load_3d(void* smem_dst, const CUtensorMap* 
       "r"(y), "r"(z)
       : "memory");
 }
-__device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                           uint32_t idesc, uint32_t accumulate) {
+// For a whole warp in step, of which the lane with `one` set issues (see umma_bf16_if).
+__device__ __forceinline__ void umma2_bf16_if(uint32_t one, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
+      ".reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(one)
       : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in BOTH CTAs of the pair once every
 // MMA issued so far by this thread has retired.
-__device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
+__device__ __forceinline__ void umma2_commit_both_if(uint32_t one, uint64_t* bar) {
   const uint16_t mask = 3;
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(smem_u32(bar)), "h"(mask)
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
+      "}\n"
+      ::"r"(smem_u32(bar)), "h"(mask), "r"(one)
       : "memory");
 }
 
@@ -200,7 +206,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* tempty = tfull + 2;             // leader only: the epilogue warps of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
@@ -233,7 +239,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_after();
   chain_wait();
   if (!GATHER) chain_release();   // a kernel that waits for peers keeps the next one off the GPU
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const int rows = A_MN ? p.M : rows_in_use(p, p.M);
   const int num_m = (rows + 2 * BM - 1) / (2 * BM), num_tiles = num_m * num_n;
   const int num_kb = ((A_MN ? rows_in_use(p, p.K) : p.K) + BK - 1) / BK;
@@ -292,7 +298,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
-    if (leader && elect_one()) {
+    if (leader) {
+      const uint32_t one = elect_one();
       constexpr uint32_t idesc = umma_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
@@ -314,13 +321,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                                         : umma_smem_desc(sa + kk * (UMMA_K * 2), 16, 1024);
             const uint64_t bdesc = B_MN ? umma_smem_desc(sb + kk * (UMMA_K * 128), BK * 128, 1024)
                                         : umma_smem_desc(sb + kk * (UMMA_K * 2), 16, 1024);
-            umma2_bf16(d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma2_bf16_if(one, d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
           }
-          umma2_commit_both(&empty[stage]);
+          umma2_commit_both_if(one, &empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma2_commit_both(&tfull[acc]);
+        umma2_commit_both_if(one, &tfull[acc]);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
