@@ -19,7 +19,8 @@
 // Kernels (dk = dv = 128; QK heads are shared by `rep` V heads, handled two V heads at a time):
 //   dn_prep_kernel   per (chunk, pair of V heads): K K^T and Q K^T on the tensor cores, the
 //                    64x64 triangular inverse in blocks, then W^T and U0^T as MMAs; writes every per-chunk operand.
-//   dn_fwd_kernel    per V head, sequential over chunks: the state S^T lives in registers (fp32);
+//   dn_fwd_kernel    per V head and run of chunks between two that hold a sequence's start, sequential over its chunks:
+//                    the state S^T lives in registers (fp32);
 //                    U^T = U0^T - S^T W^T, O^T = S^T Qg^T + U^T Mq^T, S'^T = Gc S^T + U^T Kd.
 //   dn_bwd_state_kernel   the same walk in reverse for dS and dU.
 //   dn_bwd_chunk_kernel   per (chunk, V head): the products that need S or dS' of one chunk.

@@ -1,10 +1,10 @@
 """Gated DeltaNet chunked rule on the tcgen05 kernels of ``ops/csrc/deltanet_chunk.cu``.
 
 Forward is two launches after a tiny sequence-id kernel: ``ss_dn_prep`` (per chunk and pair of
-V heads: K K^T, Q K^T, the 64x64 triangular inverse, W^T, U0^T) and ``ss_dn_fwd`` (per V head, the
-state walk over chunks with the state in the registers of eight warps). Backward recomputes both with their saves
-switched on, then runs the reverse state walk, the per-chunk products and the gradient of the
-chunk-local algebra. Nothing but the inputs is kept between forward and backward.
+V heads: K K^T, Q K^T, the 64x64 triangular inverse in blocks, W^T, U0^T) and ``ss_dn_fwd`` (per V head and
+run of sequences, the state walk over chunks with the state in the registers of eight warps). Backward recomputes both
+with their saves switched on and without the output, then runs the reverse state walk, the per-chunk products and the
+gradient of the chunk-local algebra. Nothing but the inputs is kept between forward and backward.
 
 Reference math: packages/workloads/src/shadowspill_workloads/models/qwen35/implementations/
 pytorch/delta_rule/reference.py:8-41 (forward) and :43-132 (backward).
