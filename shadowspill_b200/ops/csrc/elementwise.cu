@@ -290,7 +290,8 @@ struct PolicyArgs {
   float* logp_out;          // optional: per-row log-probability of the target
 };
 // A block of logits of listed rows: its row i is token rows[from + i] where from + i < *used. What lies behind them is
-// not a token's, and zeroed up to the next multiple of 64, the depth of the weight gradient's products.
+// not a token's, and zeroed up to the next multiple of 64 rows of the block, the depth to which the weight gradient's
+// products read it.
 struct RowList {
   const int* rows;          // null: row i is token i
   const int* used;
@@ -314,7 +315,7 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
   if (list.rows != nullptr) {
     const int at = list.from + row, used = *list.used;
     if (at >= used) {
-      if (write_grad && at < (used + 63) / 64 * 64) clear();
+      if (write_grad && row < (used - list.from + 63) / 64 * 64) clear();
       return;
     }
     row = list.rows[at];

@@ -71,3 +71,23 @@ def test_a_masked_row_of_a_logits_block_is_cleared():
     F.cross_entropy_(logits, targets, weights, loss)
     assert float(logits[1:4].abs().max()) == 0.0
     assert _rel(logits, want) < 1e-2 and abs(float(loss) - float(total)) < 2e-3 * abs(float(total))
+
+
+@pytest.mark.parametrize("r0,used,R", [(1000, 1010, 300), (500, 505, 100), (500, 512, 500), (100, 192, 64), (64, 70, 80), (500, 400, 70),
+                                       (500, 500, 70)])
+def test_rows_behind_the_scored_ones_are_cleared_as_deep_as_the_products_read(r0, used, R):
+    """The products contract whole steps of 64 rows counted from the block, wherever the block starts in the list; what
+    the block's memory held there must not reach them."""
+    V, T = 4104, 2048
+    slot = object.__new__(token_head.ScoredRows)
+    slot.T, slot.V = T, V
+    slot.rows = torch.arange(T, dtype=torch.int32, device=DEV)
+    slot.count = torch.tensor([used], dtype=torch.int32, device=DEV)
+    scored = max(0, min(R, used - r0))
+    logits = torch.full((R, V), float("nan"), dtype=torch.bfloat16, device=DEV)
+    logits[:scored] = _rand(scored, V)
+    targets, weights = torch.zeros(T, dtype=torch.int64, device=DEV), torch.ones(T, device=DEV)
+    slot.cross_entropy_(logits, targets, weights, torch.zeros(1, device=DEV), r0, r0 + R)
+    depth = min(R, -(-scored // 64) * 64)
+    assert not torch.isnan(logits[:depth]).any() and float(logits[scored:depth].abs().sum()) == 0.0
+    assert torch.isnan(logits[depth:]).all()                               # nothing past them is touched
