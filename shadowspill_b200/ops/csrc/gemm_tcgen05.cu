@@ -76,6 +76,8 @@ struct GemmParams {
   int c_f32;
   int accumulate;
   int tma_out;                // the products leave by TMA through tmC
+  const int* used;            // optional: of the M rows those up to *used - used_from are in use
+  int used_from;
   int a_mn, b_mn;
   int* status;
   float alpha;
@@ -144,9 +146,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
-  const int num_m = (p.M + BM - 1) / BM;
   const int num_n = (p.N + TILE_N - 1) / TILE_N;
-  const int num_tiles = num_m * num_n * (p.g.mode == 2 ? p.g.n_experts : 1);
   const int num_kb = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -172,6 +172,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   chain_wait();
   chain_release();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int rows = p.used == nullptr ? p.M : max(0, min(p.M, *p.used - p.used_from));
+  const int num_m = (rows + BM - 1) / BM;
+  const int num_tiles = num_m * num_n * (p.g.mode == 2 ? p.g.n_experts : 1);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -505,7 +508,7 @@ bool gemm_fits_one_wave(int M, int N, int num_sms) {
 
 int gemm_from(const void* A, const void* B, const void* src, void* C, long long ldsrc, int M, int N, int K, long long lda,
               long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn,
-              int num_sms, int* status, void* stream);
+              int num_sms, int* status, void* stream, const int* used = nullptr, int used_from = 0);
 
 static int sm_count() {
   int dev = 0, n = 0;
@@ -532,10 +535,11 @@ int ss_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
 
 namespace ss {
 
-// ss_gemm_bf16 whose `accumulate` adds `src` [M, N] (pitch `ldsrc`, C's type) to the products.
+// ss_gemm_bf16 whose `accumulate` adds `src` [M, N] (pitch `ldsrc`, C's type) to the products; with `used` (not for a_mn)
+// of the first `*used - used_from` rows only, in whole tiles.
 int gemm_from(const void* A, const void* B, const void* src, void* C, long long ldsrc, int M, int N, int K, long long lda,
               long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn,
-              int num_sms, int* status, void* stream) {
+              int num_sms, int* status, void* stream, const int* used, int used_from) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (accumulate && ((ldsrc % (c_f32 ? 4 : 8)) || (reinterpret_cast<uintptr_t>(src) & 15))) return -2;
   if ((lda % 8) || (ldb % 8) || (ldc % (c_f32 ? 4 : 8)) || (N % 8) ||
@@ -555,7 +559,7 @@ int gemm_from(const void* A, const void* B, const void* src, void* C, long long 
   GemmParams p{};
   p.C = C; p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.c_f32 = c_f32; p.accumulate = accumulate;
   p.a_mn = a_mn; p.b_mn = b_mn; p.status = status; p.alpha = alpha;
-  p.e.src = src; p.e.ldsrc = ldsrc;
+  p.e.src = src; p.e.ldsrc = ldsrc; p.used = used; p.used_from = used_from;
   p.g.mode = 0;
   return dispatch(ta, tb, p, bn, num_sms, reinterpret_cast<cudaStream_t>(stream));
 }

@@ -49,7 +49,7 @@ int make_tmap3_bf16(CUtensorMap* map, const void* base, long long experts, long 
 bool gemm_fits_one_wave(int M, int N, int num_sms);
 int gemm_from(const void* A, const void* B, const void* src, void* C, long long ldsrc, int M, int N, int K, long long lda,
               long long ldb, long long ldc, int a_mn, int b_mn, int c_f32, int accumulate, float alpha, int bn,
-              int num_sms, int* status, void* stream);
+              int num_sms, int* status, void* stream, const int* used = nullptr, int used_from = 0);
 
 namespace pair {
 
@@ -529,7 +529,10 @@ int ss_gemm2_residual_bf16(const void* A, const void* B, const void* src, void* 
 
 // The bf16 GEMM over rows of which the device knows how many are in use: `*used - from` of the M rows of A and C, or with
 // a_mn of the K rows that are contracted (those up to the next multiple of 64 must be zero in one operand and finite in
-// the other). Tiles past them are neither computed nor written.
+// the other). Tiles past them are neither computed nor written. Outputs whose 128 x 128 tiles fit one wave are the
+// single-CTA kernel's here too: a pair's tile takes as long as two of its, and half the SMs would have none (gradient of
+// 1,000 rows of 2,048 channels from a vocabulary of 151,936: 674 us on CTA pairs, 496 there; of 852 rows and 50,304: 238
+// and 185).
 int ss_gemm2_rows_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                        long long ldc, int a_mn, int b_mn, int accumulate, const int* used, int from, int* status,
                        void* stream) {
@@ -543,6 +546,9 @@ int ss_gemm2_rows_bf16(const void* A, const void* B, void* C, int M, int N, int 
   int dev = 0, num_sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!a_mn && gemm_fits_one_wave(M, N, num_sms))
+    return gemm_from(A, B, C, C, ldc, M, N, K, lda, ldb, ldc, 0, b_mn, 0, accumulate, 1.f, 128, num_sms, status, stream,
+                     used, from);
   CUtensorMap ta, tb;
   int r;
   if (!a_mn) r = make_tmap_bf16(&ta, A, M, K, lda, BM);

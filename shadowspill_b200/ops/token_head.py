@@ -19,8 +19,14 @@ _lib.register("ss_take_rows", [_P, _L, _P, _P, _L, _I, _I, _P])
 _lib.register("ss_gemm2_rows_bf16", [_P, _P, _P, _I, _I, _I, _L, _L, _L, _I, _I, _I, _P, _I, _P, _P])
 _lib.register("ss_token_objective_rows", [_P, _P, _P, _P, _P, _I, _P, _I, _I, _L, _F, _I, _I, _P, _P, _F, _P, _F, _P])
 
-# Multiply-adds of one product over all rows from which the rows are worth finding. The three small kernels take 22 us
-# at 4,096 rows of 4,096 channels, the head's products 8.1 ms where every row is scored.
+# Multiply-adds of one product over all rows from which the rows are worth finding: a head whose rows are all scored
+# pays for the three small kernels and gains nothing, so the line lies where that is 2 % at most. All rows -> scored rows,
+# us, both in turn, for all / nine in ten / half of them scored:
+#   512 rows, 50,304 x 2,048 (5e10): 348 -> 376, 347 -> 375, 341 -> 323;  1,000 rows (1e11): 488 -> 503, 491 -> 502, 551 -> 435
+#   1,000 rows, 128,256 x 2,048 (2.6e11): 1408 -> 1436, 1453 -> 1454, 1461 -> 1058
+#   1,000 rows, 151,936 x 2,048 (3.1e11): 1508 -> 1532, 1805 -> 1790, 1762 -> 1276
+#   1,000 rows, 128,256 x 4,096 (5.3e11): 2405 -> 2427, 2792 -> 2741, 2499 -> 1801;  8,192 rows: 21190 -> 21260, .., 19860 -> 10300
+# Below the line half-masked heads go without what they could gain.
 MIN_WORK = 3e11
 
 

@@ -91,3 +91,20 @@ def test_rows_behind_the_scored_ones_are_cleared_as_deep_as_the_products_read(r0
     depth = min(R, -(-scored // 64) * 64)
     assert not torch.isnan(logits[:depth]).any() and float(logits[scored:depth].abs().sum()) == 0.0
     assert torch.isnan(logits[depth:]).all()                               # nothing past them is touched
+
+
+@pytest.mark.parametrize("R,D,used", [(700, 512, 130), (1000, 2048, 1000), (1100, 2176, 700), (2048, 2048, 1), (2049, 2056, 1031), (2048, 2048, 0)])
+def test_gradients_of_the_scored_rows_have_the_bits_of_all_rows(R, D, used):
+    """Outputs of one wave of 128 x 128 tiles and larger ones, which CTA pairs take: the same sums in either."""
+    V = 1032
+    slot = object.__new__(token_head.ScoredRows)
+    slot.T, slot.V = R, V
+    slot.count = torch.tensor([300 + used], dtype=torch.int32, device=DEV)
+    dlogits, W = _rand(R, V, seed=1), _rand(V, D, seed=2)
+    dh = torch.empty(R, D, dtype=torch.bfloat16, device=DEV)
+    whole = dh.new_zeros(300 + R, D)
+    dlogits[used:] = float("nan")
+    slot.dgrad(dlogits, W, whole, 300, 300 + R)
+    F.linear_dgrad(dlogits[:max(used, 1)], W, out=dh[:max(used, 1)])
+    assert torch.equal(whole[300:300 + used], dh[:used]) and float(whole[:300].abs().sum()) == 0.0
+    _lib.check_status()
