@@ -120,6 +120,19 @@ __device__ __forceinline__ void epilogue_part_sync(int part) {
   if (part == 0) asm volatile("bar.sync 3, 128;" ::: "memory");
   else asm volatile("bar.sync 4, 128;" ::: "memory");
 }
+// Have all four warps of a part what they waited for? A wait gives up in each warp by itself (once the status word is
+// set it may do so in one warp and succeed in the next), and none may be left alone at the barriers of epilogue_tma:
+// they enter it, or leave their loop, together.
+__device__ __forceinline__ bool epilogue_part_agree(int part, bool ok) {
+  uint32_t all;
+  if (part == 0)
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 3, 128, p;\n\t"
+                 "selp.u32 %0, 1, 0, q;\n\t}" : "=r"(all) : "r"(static_cast<uint32_t>(ok)) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 4, 128, p;\n\t"
+                 "selp.u32 %0, 1, 0, q;\n\t}" : "=r"(all) : "r"(static_cast<uint32_t>(ok)) : "memory");
+  return all != 0;
+}
 template <class F>
 __device__ __forceinline__ void epilogue_tma(uint8_t* block, uint32_t taddr, int blocks, int part, int row, bool issuer,
                                              const CUtensorMap* out, float alpha, int col0, int N, int row0, int M, int z,

@@ -294,7 +294,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         continue;
       }
-      if (!mbar_wait(&tfull[acc], acc_phase, p.status, KS_TIMEOUT_TMEM_FULL)) break;
+      bool ok = mbar_wait(&tfull[acc], acc_phase, p.status, KS_TIMEOUT_TMEM_FULL);
+      if (EPI == EPI_PLAIN && p.tma_out) ok = epilogue_part_agree(part, ok);
+      if (!ok) break;
       tc_fence_after();
       const int row = mb * BM + q * 32 + lane;
       const uint32_t taddr =

@@ -344,8 +344,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tile_coords<GATHER>(t, num_m, num_n, mb, nb);
       if (A_MN && num_kb == 0) {          // nothing to contract: zero, or what is there already
         if (p.accumulate) break;
-      } else if (!mbar_wait(&tfull[acc], acc_phase, p.status, KS_TIMEOUT_TMEM_FULL)) {
-        break;
+      } else {
+        bool ok = mbar_wait(&tfull[acc], acc_phase, p.status, KS_TIMEOUT_TMEM_FULL);
+        if (!GATHER && EPI == EPI_PLAIN && p.tma_out) ok = epilogue_part_agree(part, ok);
+        if (!ok) break;
       }
       tc_fence_after();
       const int row0 = mb * (2 * BM) + static_cast<int>(rank) * BM + q * 32;
