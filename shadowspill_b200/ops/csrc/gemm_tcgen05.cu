@@ -287,8 +287,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               *reinterpret_cast<float4*>(d) = make_float4(0, 0, 0, 0);
               *reinterpret_cast<float4*>(d + 4) = make_float4(0, 0, 0, 0);
             } else {
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C) + w.c_off +
-                                        static_cast<long long>(zr) * p.ldc + c) = make_uint4(0, 0, 0, 0);
+              uint2* d = reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.C) + w.c_off +
+                                                  static_cast<long long>(zr) * p.ldc + c);
+              d[0] = d[1] = make_uint2(0, 0);
             }
           }
         }
@@ -463,7 +464,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
   using Cfg = GemmCfg<BN>;
   GemmParams p = params;
   CUtensorMap tc = ta;                                       // unused unless tma_out
-  p.tma_out = EPI == EPI_PLAIN && !p.c_f32 && !p.accumulate && p.g.row_dst == nullptr;
+  // TMA stores from 16-byte boundaries on, the staged stores from 8-byte ones
+  p.tma_out = EPI == EPI_PLAIN && !p.c_f32 && !p.accumulate && p.g.row_dst == nullptr &&
+              (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
   if (p.tma_out) {
     const long long matrices = p.g.mode == 2 ? p.g.n_experts : 1;
     if (int r = make_tmap3_bf16(&tc, p.C, matrices, p.M, p.N, p.ldc,
@@ -583,7 +586,9 @@ int ss_gemm_grouped_bf16(const void* A, const void* B, void* C, int mode, int ro
                          void* stream) {
   using namespace ss;
   if (rows <= 0 || n_experts <= 0) return 0;
-  if ((lda % 8) || (ldb % 8) || (ldc % (c_f32 ? 4 : 8)) || (N % 8) || (rows % BM)) return -2;
+  if ((lda % 8) || (ldb % 8) || (ldc % (c_f32 ? 4 : 8)) || (N % 8) || (rows % BM) ||
+      (reinterpret_cast<uintptr_t>(C) & (c_f32 ? 15 : 7)))
+    return -2;
   if (bn != 128 && bn != 256) bn = (N <= 128) ? 128 : 256;
   CUtensorMap ta, tb;
   GemmParams p{};

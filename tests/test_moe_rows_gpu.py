@@ -114,3 +114,40 @@ def test_fewer_comparable_scores_than_picks(E, k, finite, renorm):
     assert bool(torch.isfinite(got).all())
     # fp32 products and sums of up to 32 terms of order one
     assert float((got.double() - leaf.grad).abs().max()) < 1e-5
+
+
+def _off_by_8_bytes(*shape):
+    n = 1
+    for d in shape:
+        n *= d
+    return torch.zeros(n + 4, dtype=torch.bfloat16, device=DEV)[4:].view(*shape)
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_grouped_outputs_on_8_byte_boundaries(accumulate):
+    """The staged stores take them (TMA would not); experts without rows among them. On 2 bytes they are refused."""
+    E, T, D, N, k = 8, 300, 136, 200, 2
+    g = torch.Generator(device=DEV).manual_seed(3)
+    logits = torch.randn(T, E, generator=g, device=DEV)
+    logits[:, 5] = -1e4
+    ids, _, counts = moe.route(logits, k, True)
+    assert int(counts[5]) == 0
+    lay = moe.Layout(ids, counts)
+    used = int(lay.used)
+    x = torch.randn(T, D, generator=g, device=DEV).bfloat16()
+    bank = (torch.randn(E, N, D, generator=g, device=DEV) * 0.1).bfloat16()
+    xs = lay.gather(x)
+    want = moe.grouped_linear(xs, bank, lay)
+    got = moe.grouped_linear(xs, bank, lay, out=_off_by_8_bytes(lay.rows, N))
+    assert got.data_ptr() % 16 == 8 and torch.equal(got[:used], want[:used])
+    start = torch.randn(E, N, D, generator=g, device=DEV).bfloat16()
+    a, b = start.clone(), _off_by_8_bytes(E, N, D).copy_(start)
+    moe.grouped_wgrad(want, xs, lay, a, accumulate)
+    moe.grouped_wgrad(want, xs, lay, b, accumulate)
+    assert b.data_ptr() % 16 == 8 and torch.equal(a, b)
+    assert accumulate or not bool(b[5].any())
+    flat = torch.zeros(lay.rows * N + 1, dtype=torch.bfloat16, device=DEV)[1:].view(lay.rows, N)
+    with pytest.raises(RuntimeError):
+        moe.grouped_linear(xs, bank, lay, out=flat)
+    torch.cuda.synchronize()
+    _lib.check_status()
