@@ -174,7 +174,7 @@ PyObject* linear_residual(PyObject*, PyObject* const* v, Py_ssize_t n) {
     plain_rows(x); plain_rows(w); plain_rows(res);
     const Call c(x);
     const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
-    want(w.size(1) == K && res.size(0) == M && res.size(1) == N);
+    want(K > 0 && w.size(1) == K && res.size(0) == M && res.size(1) == N);    // no launch without a product: no sum either
     at::Tensor made;
     const at::Tensor* out = &made;
     if (none(v[3])) made = empty({M, N}, c.bf16);

@@ -189,7 +189,7 @@ def linear_residual(x, w, residual, out=None):
     if out is None:
         out = torch.empty_like(residual)
     M, N, K = x.shape[0], w.shape[0], x.shape[1]
-    if not (_fused_gemm(x, w, residual, out) and w.shape[1] == K and out.shape == residual.shape == (M, N)):
+    if not (_fused_gemm(x, w, residual, out) and w.shape[1] == K > 0 and out.shape == residual.shape == (M, N)):
         if out is not residual:
             out.copy_(residual)
         return linear_fwd(x, w, out=out, accumulate=True)

@@ -64,3 +64,10 @@ def test_the_expert_form_has_the_bits_of_the_separate_kernels():
     gu = moe.grouped_linear(xs, bank, lay)
     got_gu, got_h = moe.grouped_swiglu(xs, bank, lay)
     assert torch.equal(got_gu[:used], gu[:used]) and torch.equal(got_h[:used], lay.swiglu(gu)[:used])
+
+
+def test_a_residual_with_nothing_to_add_is_the_residual():
+    x, w, res = _rand(300, 8)[:, :0], _rand(256, 8)[:, :0], _rand(300, 256, seed=1)
+    out = torch.full_like(res, float("nan"))
+    assert F.linear_residual(x, w, res, out=out) is out and torch.equal(out, res)
+    assert torch.equal(F.linear_residual(x, w, res), res)
