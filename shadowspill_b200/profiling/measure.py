@@ -51,6 +51,18 @@ class Profiles:
         return Profiles({k: TaskProfile(**v) for k, v in d["tasks"].items()}, d.get("device", ""))
 
 
+# what of a batch decides how long a task takes, besides its sizes: part of a stored profile's identity
+SCORED = "every row"
+
+
+def profiling_batch(runner: TaskRunner, vocab: int, fixed_len: int = 0) -> list:
+    """The packed sequences tasks are timed on, every row of them scored by the loss: the output head works on the
+    scored rows only (``ops/token_head.py``), and a plan has to hold for data that scores them all."""
+    return make_batch(0, vocab=vocab, tokens_per_step=runner.T * runner.n_mb, microbatch_tokens=runner.T,
+                      slots=runner.slots, max_len=min(8192, runner.T), fixed_len=min(fixed_len, runner.T) or None,
+                      median=min(1200.0, runner.T / 4), min_len=min(32, runner.T // 4), masked_fraction=0.0)
+
+
 def _fill_inputs(runner: TaskRunner, task: int, flats: list[torch.Tensor], host_batch) -> None:
     prog = runner.program
     t = prog.tasks[task]
@@ -96,10 +108,7 @@ def measure_program(program: Program, desc: TrainingDescription, device: str = "
     runner = TaskRunner(program, desc, Hyperparameters(lr=0.0, rule=rule), seed=0, stochastic_rounding=True)
     meta = program.metadata
     cfg = desc.cfg
-    host_batch = make_batch(0, vocab=cfg.vocab_size, tokens_per_step=runner.T * runner.n_mb,
-                            microbatch_tokens=runner.T, slots=runner.slots,
-                            max_len=min(8192, runner.T), fixed_len=min(fixed_len, runner.T) or None,
-                            median=min(1200.0, runner.T / 4), min_len=min(32, runner.T // 4))
+    host_batch = profiling_batch(runner, cfg.vocab_size, fixed_len)
     profiles = Profiles(device=torch.cuda.get_device_name(dev) if cuda else "cpu")
     seen: dict[str, int] = {}
     for ti, t in enumerate(program.tasks):

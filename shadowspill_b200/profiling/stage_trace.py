@@ -22,11 +22,10 @@ import sys
 
 import torch
 
-from ..data.synthetic import make_batch
 from ..execution.executor import Hyperparameters, TaskRunner
 from ..frontend.capture import BatchGeometry, StepDataOrdering, build_step
 from ..models.config import preset
-from .measure import _fill_inputs
+from .measure import _fill_inputs, profiling_batch
 
 
 def parse_selection(text: str) -> dict[int, str]:
@@ -54,9 +53,7 @@ def trace_task(model: str, task: str, microbatch_tokens: int = 2048, microbatche
     dev = torch.device(device)
     cuda = dev.type == "cuda"
     runner = TaskRunner(program, desc, Hyperparameters(lr=0.0), seed=0, stochastic_rounding=True)
-    host = make_batch(0, vocab=cfg.vocab_size, tokens_per_step=runner.T * runner.n_mb, microbatch_tokens=runner.T,
-                      slots=runner.slots, max_len=min(8192, runner.T), median=min(1200.0, runner.T / 4),
-                      min_len=min(32, runner.T // 4))
+    host = profiling_batch(runner, cfg.vocab_size)
     flats = [torch.empty(program.objects[u.object].bytes, dtype=torch.uint8, device=dev) for u in runner.uses[ti]]
     _fill_inputs(runner, ti, flats, host)
     bound = runner.bind(ti, flats)

@@ -30,7 +30,7 @@ from ..frontend.capture import (BatchGeometry, StepDataOrdering, build_forward,
 from ..models.config import DecoderConfig, preset
 from ..planning.plan import (MemoryBudgets, PlanningError, SearchOptions, StateLayout,
                              plan_program, sweep_programs)
-from ..profiling.measure import Profiles, apply_profiles, measure_program
+from ..profiling.measure import SCORED, Profiles, apply_profiles, measure_program
 from ..runtime.core import Runtime
 
 GIB = 1 << 30
@@ -397,7 +397,7 @@ class TrainingSession:
                     store = ContentStore(setup.store, setup.store_mode)
                     ident = {"device": torch.cuda.get_device_name(setup.device_index) if cuda else "cpu",
                              "kernels": kernel_library_digest(), "dtype": setup.dtype,
-                             "sequence_tokens": setup.profile_sequence_tokens}
+                             "sequence_tokens": setup.profile_sequence_tokens, "scored": SCORED}
                 for prog, desc in candidates + list(extras.values()):
                     missing = {t.profile_key for t in prog.tasks} - set(self.profiles.tasks)
                     if store is not None:

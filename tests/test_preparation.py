@@ -127,3 +127,22 @@ def test_preparation_as_four_fresh_processes(tmp_path):
     again = prepare_job(setup, directory)               # nothing to do: every result is there
     assert again == bundle
     assert all(p.get("skipped") for p in json.loads((directory / "job.json").read_text())["phases"])
+
+
+def test_tasks_are_profiled_on_batches_whose_every_row_is_scored(monkeypatch):
+    """The output head leaves out rows that the loss does not score; a plan has to hold for data that scores all."""
+    from shadowspill_b200.frontend.capture import BatchGeometry, StepDataOrdering, build_step
+    from shadowspill_b200.models.config import preset
+    from shadowspill_b200.profiling import measure
+    seen = []
+    fill = measure._fill_inputs
+    monkeypatch.setattr(measure, "_fill_inputs", lambda runner, task, flats, batch: (seen.extend(batch), fill(runner, task, flats, batch)))
+    import torch
+    prog, desc = build_step(preset("llama3-tiny"), BatchGeometry(256, 2, slots=16, mean_seqlen=64), StepDataOrdering(),
+                            dtype=torch.float32)
+    keys = {t.profile_key for t in prog.tasks if ":head:" in (t.profile_key or "")}
+    assert keys and set(measure.measure_program(prog, desc, "cpu", keys=keys).tasks) == keys
+    for mb in seen:
+        ends = len(set(mb.cu_seqlens.tolist())) - 1                # the last token of a sequence has no target
+        assert int((mb.weights > 0).sum()) == int((mb.targets >= 0).sum()) >= 256 - ends
+    assert seen
