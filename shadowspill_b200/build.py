@@ -89,22 +89,28 @@ def build_kernels(force: bool = False, verbose: bool = False, ptxas_info: bool =
 
 def build_host_calls(force: bool = False, verbose: bool = False) -> Path | None:
     """Compile the Python extension that calls the kernel library's launchers with tensors."""
-    source, cuda = KERNEL_DIR / "host_calls.cpp", _cuda_home()
+    sources, cuda = [KERNEL_DIR / "host_calls.cpp", KERNEL_DIR / "launchers.h"], _cuda_home()
     if cuda is None or not KERNEL_LIB.exists():
         return None
-    if force or _stale(HOST_CALLS, [source]):
-        import sysconfig
+    import sysconfig
 
-        import torch
+    import torch
+    # what it is linked against: it calls torch's C++ interface, which changes with the version
+    built_for = f"torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}\n"
+    stamp = KERNEL_DIR / "build" / "host_calls.txt"
+    known = stamp.read_text() if stamp.exists() else ""
+    if force or known != built_for or _stale(HOST_CALLS, sources):
         home = Path(torch.__file__).resolve().parent
         tmp = HOST_CALLS.with_suffix(".so.tmp")
         _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
               "-isystem", str(home / "include"), "-isystem", str(home / "include/torch/csrc/api/include"),
               "-isystem", sysconfig.get_paths()["include"], "-isystem", str(cuda / "include"),
-              "-o", str(tmp), str(source), "-L", str(KERNEL_LIB.parent), "-lss_kernels", "-Wl,-rpath,$ORIGIN",
+              "-o", str(tmp), str(sources[0]), "-L", str(KERNEL_LIB.parent), "-lss_kernels", "-Wl,-rpath,$ORIGIN",
               "-L", str(home / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"], verbose)
         os.replace(tmp, HOST_CALLS)
+        stamp.parent.mkdir(exist_ok=True)
+        stamp.write_text(built_for)
     return HOST_CALLS
 
 

@@ -880,6 +880,7 @@ extern "C" int ss_attn_bwd(const void* q, const void* k, const void* v, const vo
 // (delta, fp32 [Hq, T]) lives here in a fixed device array instead, so the call
 // performs no allocation of any kind.
 #include "attention_noalloc.h"
+#include "launchers.h"
 
 #include <mutex>
 

@@ -29,6 +29,7 @@
 // each [cu_seqlens[i], cu_seqlens[i+1]) is an independent causal sequence.
 #include "sm100_ptx.cuh"
 #include "attention_tiles.cuh"
+#include "launchers.h"
 
 #include <cudaTypedefs.h>
 #include <math.h>

@@ -11,6 +11,7 @@
 
 #include "chained_launch.cuh"
 #include "swiglu_math.cuh"
+#include "launchers.h"
 
 namespace ss {
 

@@ -22,6 +22,7 @@
 // i overlap the main loop of tile i+1.
 #include "sm100_ptx.cuh"
 #include "gemm_epilogue.cuh"
+#include "launchers.h"
 
 #include <cudaTypedefs.h>
 #include <stdio.h>

@@ -35,6 +35,7 @@
 // (packages/engine/src/shadowspill/pytorch/operations.py:15).
 #include "sm100_ptx.cuh"
 #include "gemm_epilogue.cuh"
+#include "launchers.h"
 
 #include <cudaTypedefs.h>
 
@@ -505,11 +506,6 @@ static int gemm2_from(const void* A, const void* B, const void* src, void* C, lo
 }  // namespace ss
 
 extern "C" {
-
-int ss_gemm_swiglu_bf16(const void* A, const void* B, void* gu, void* h, int M, int F, int K, long long lda,
-                        long long ldb, long long ldgu, long long ldh, int bn, int* status, void* stream);
-int ss_gemm_swiglu_bwd_bf16(const void* A, const void* B, const void* gu, void* dgu, int M, int F, int K, long long lda,
-                            long long ldb, long long ldgu, long long lddgu, int bn, int* status, void* stream);
 
 // Same arguments and return codes as ss_gemm_bf16 (without the tile-width hint), which takes the outputs
 // whose 128x128 tiles fit one wave.

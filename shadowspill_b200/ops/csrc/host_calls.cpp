@@ -15,26 +15,7 @@
 
 #include <cmath>
 
-extern "C" {
-int ss_gemm_bf16(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, int,
-                 float, int, int, int*, void*);
-int ss_gemm2_bf16(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, int,
-                  float, int, int*, void*);
-int ss_gemm2_residual_bf16(const void*, const void*, const void*, void*, int, int, int, long long, long long, long long,
-                           long long, int*, void*);
-int ss_gemm2_swiglu_bf16(const void*, const void*, void*, void*, int, int, int, long long, long long, long long,
-                         long long, int*, void*);
-int ss_gemm2_swiglu_bwd_bf16(const void*, const void*, const void*, void*, int, int, int, long long, long long,
-                             long long, long long, int*, void*);
-int ss_rmsnorm_fwd(void*, const void*, const void*, void*, float*, int, int, float, int, int*, void*);
-int ss_rmsnorm_bwd(const void*, const void*, const void*, const float*, void*, float*, int, int, int, int, int*, void*);
-int ss_rope(void*, const int*, int, long long, int, int, int, int, float, int, void*);
-int ss_attn_fwd(const void*, const void*, const void*, void*, float*, const int*, int, int, int, int, int, long long,
-                long long, long long, long long, float, int*, void*);
-int ss_attn_bwd_g(const void*, const void*, const void*, const void*, const float*, const void*, void*, void*, void*,
-                  const int*, float*, int, int, int, int, int, long long, long long, long long, long long, long long,
-                  long long, long long, float, int*, void*);
-}
+#include "launchers.h"
 
 namespace {
 

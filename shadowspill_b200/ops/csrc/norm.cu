@@ -23,6 +23,7 @@
 // The math follows the reference's pure-PyTorch definition
 // (packages/workloads/src/shadowspill_workloads/models/shared/decoder.py:18).
 #include "sm100_ptx.cuh"
+#include "launchers.h"
 
 #include <stdint.h>
 

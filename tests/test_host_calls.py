@@ -1,9 +1,67 @@
 """The native module that calls the launchers with tensors: what it takes gives the bits of the Python path, and what
 it does not take is answered NotImplemented, so that the Python path decides as before."""
+import re
+from pathlib import Path
+
 import pytest
 import torch
 
+from shadowspill_b200 import build
+
 from shadowspill_b200.ops import _lib, attention, functional as F
+
+
+CSRC = Path(build.KERNEL_DIR)
+
+
+def test_the_launchers_are_declared_once():
+    """One header gives the parameters to the sources that define the launchers and to the module that calls them; the
+    ctypes table has the same."""
+    kinds = {"int": _lib.c_int, "long long": _lib.c_ll, "float": _lib.c_f}
+    text = re.sub(r"//.*", "", (CSRC / "launchers.h").read_text())
+    found = {}
+    for name, params in re.findall(r"\bint (ss_\w+)\(([^)]*)\);", text):
+        found[name] = [_lib.c_p if "*" in p else kinds[" ".join(p.split()[:-1])] for p in params.split(",")]
+    called = set(re.findall(r"\bss_[a-z]\w+(?=,)", (CSRC / "host_calls.cpp").read_text().split("namespace {")[1]))
+    assert called and called <= set(found)
+    for name, types in found.items():
+        if name in _lib._SIGNATURES:
+            assert _lib._SIGNATURES[name] == types, name
+        defining = [f for f in CSRC.glob("*.cu") if re.search(rf"\bint {name}\([^;{{]*\{{", f.read_text())]
+        assert len(defining) == 1 and '#include "launchers.h"' in defining[0].read_text(), name
+    assert called <= set(_lib._SIGNATURES)
+    assert not re.search(r"\bint ss_\w+\(", (CSRC / "host_calls.cpp").read_text())
+
+
+def test_the_module_is_built_again_for_another_torch(monkeypatch, tmp_path):
+    csrc = tmp_path / "csrc"
+    csrc.mkdir()
+    for name in ("host_calls.cpp", "launchers.h"):
+        (csrc / name).write_text("")
+    for name in ("libss_kernels.so", "_host_calls.so"):
+        (tmp_path / name).write_text("")
+    runs = []
+
+    def run(cmd, verbose):
+        runs.append(cmd)
+        Path(cmd[cmd.index("-o") + 1]).write_text("")
+    monkeypatch.setattr(build, "KERNEL_DIR", csrc)
+    monkeypatch.setattr(build, "KERNEL_LIB", tmp_path / "libss_kernels.so")
+    monkeypatch.setattr(build, "HOST_CALLS", tmp_path / "_host_calls.so")
+    monkeypatch.setattr(build, "_run", run)
+    if build._cuda_home() is None:
+        pytest.skip("no CUDA headers here")
+    import os
+    build.build_host_calls()
+    build.build_host_calls()
+    assert len(runs) == 1                                  # a module of unknown origin is built once
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    build.build_host_calls()
+    assert len(runs) == 2
+    later = (tmp_path / "_host_calls.so").stat().st_mtime + 10
+    os.utime(csrc / "launchers.h", (later, later))
+    build.build_host_calls()
+    assert len(runs) == 3
 
 
 def _operands(device, rows=72, dh=64):
