@@ -242,3 +242,49 @@ def test_head_groups_compute_the_same_rule_in_pieces():
     assert torch.equal(whole, pieces)
     for a, b in zip(grads, grads2):
         assert torch.equal(a, b)
+
+
+def _random_bounds(r, chunks):
+    """Packed lengths that begin on and off chunk edges, short and long, and leave a ragged end."""
+    at, end, bounds = 0, 64 * chunks - r.choice([0, 1, 37]), [0]
+    while at < end:
+        longest = r.choice([3, 60, 300, 64 * chunks])
+        at = min(end, (at // 64 + r.randint(1, 9)) * 64 if r.random() < 0.4 else at + r.randint(1, longest))
+        bounds.append(at)
+    return end, bounds
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_every_chunk_of_random_packed_batches(seed):
+    """The walks are cut where a chunk passes no state on. A sequence that begins on a chunk edge has the bits of itself
+    alone, and every single chunk of the batch is the rule's: a norm over all tokens would not show one that is not.
+    (bf16 operands as above; a chunk's error is measured against its own norm.)"""
+    import random
+    from shadowspill_b200.ops import _lib
+    r = random.Random(seed)
+    Hk, Hv = r.choice([(1, 1), (2, 6), (4, 4), (16, 32)])
+    T, bounds = _random_bounds(r, r.choice([2, 9, 33, 70]))
+    q, k, v, beta, gl, dout, _ = _delta_case(T, Hk, Hv, bounds, seed=seed + 100)
+    names = "out q k v beta g".split()
+
+    def run(rule, rows, edges, cast):
+        leaves = [t[rows].cuda().to(cast(t)).requires_grad_(True) for t in (q, k, v, beta, gl)]
+        got = rule(*leaves, None, 64, cu_seqlens=torch.tensor(edges, dtype=torch.int32, device="cuda"))
+        got.backward(dout[rows].cuda().to(got.dtype))
+        return [got.detach(), *(t.grad for t in leaves)]
+    packed = run(seq.gated_delta_rule_chunked, slice(0, T), bounds, lambda t: t.dtype)
+    exact = run(seq._gated_delta_rule_torch, slice(0, T), bounds, lambda t: torch.float64)
+    for a, b in zip(bounds[:-1], bounds[1:]):
+        if a % 64 == 0 and b > a:
+            alone = run(seq.gated_delta_rule_chunked, slice(a, b), [0, b - a], lambda t: t.dtype)
+            for name, x, y in zip(names, packed, alone):
+                if name == "g":      # a sum over the rest of the chunk, in which the other sequences' terms cancel in fp32
+                    near = x[a:-(-b // 64) * 64].norm()
+                    assert float((x[a:b] - y).norm()) <= 1e-5 * float(near) + 1e-6, (a, b)
+                else:
+                    assert torch.equal(x[a:b], y), (name, a, b)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for name, x, y in zip(names, packed, exact):
+        worst = max(_rel(x[c:c + 64], y[c:c + 64]) for c in range(0, T, 64))
+        assert worst < 1.5e-2, (name, worst)
