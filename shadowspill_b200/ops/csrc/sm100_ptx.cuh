@@ -224,11 +224,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -288,23 +283,11 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, bool a_mn, 
          (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same for a whole warp in step (`_ts`: A from TMEM), of which only the lane with `leader` set issues. With no branch
-// around them the addresses and descriptors are computed once per warp in uniform registers, where the
-// instruction takes them from; inside a one-lane branch each has to be moved there first (attention on 16,384
-// tokens: forward 1020 -> 968 us, dQ 1260 -> 1205, dK/dV 1710 -> 1632; GEMMs on 2,000 rows 1,145 -> 1,115 us, on 8,192 the
-// same to 1 %).
+// D[tmem] (+)= A[smem] * B[smem] (`_ts`: A from TMEM) for a whole warp in step, of which only the lane with `leader` set
+// issues. With no branch around them the addresses and descriptors are computed once per warp in uniform registers, where
+// the instruction takes them from; inside a one-lane branch each has to be moved there first (attention on 16,384
+// tokens: forward 1020 -> 968 us, dQ 1260 -> 1205, dK/dV 1710 -> 1632; a layer on 2,000 rows, forward and backward, by its
+// GEMMs 961 -> 955).
 __device__ __forceinline__ void umma_bf16_if(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -329,6 +312,7 @@ __device__ __forceinline__ void umma_bf16_ts_if(uint32_t leader, uint32_t tmem_d
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// Arrive on an mbarrier once every tcgen05.mma that the lane with `leader` set has issued so far is done.
 __device__ __forceinline__ void umma_commit_if(uint32_t leader, uint64_t* bar) {
   asm volatile(
       "{\n\t"
@@ -341,13 +325,6 @@ __device__ __forceinline__ void umma_commit_if(uint32_t leader, uint64_t* bar) {
 }
 // A value that every lane holds, as one the compiler knows to be the same in all of them.
 __device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_or_sync(0xffffffffu, v); }
-
-// Arrive on an mbarrier once every tcgen05.mma issued so far by this thread is done.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
 
 // ------------------------------------------------------------------ packing
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
