@@ -8,10 +8,10 @@
 // wait for a product.
 // P goes back to TMEM over the scores it comes from and is the A operand of P V from there: it never
 // passes through shared memory, whose bandwidth the two products need for K, V and Q.
-// Measured (two tiles in a CTA -> two CTAs): 8,192 packed tokens, 32/8 heads of 128: 0.221 -> 0.207 ms; 16,384 tokens in
-// two sequences: 0.970 -> 0.974 ms; 2,048 tokens in five sequences, 32/8 heads of 64, with the backward kernels
-// changed alike: 112 -> 94 us. 6,001 tokens, 16/4 heads of 256: 0.150 ms. What is left is the softmax
-// warps' chain (read, maximum, exponentials, write). Replacing a quarter of the exponentials by polynomials of ten
+// Measured (two tiles in a CTA -> two CTAs, both kernels in turn, the forward kernel alone): 8,192 packed tokens, 32/8 heads
+// of 128: 208 -> 192.5 us; 16,384 tokens in two sequences: 1,013 -> 968; 2,048 tokens in five sequences: 47 -> 39; heads of
+// 64, 2,048 tokens: 39 -> 32.7, 16,384: 810 -> 784. 6,001 tokens, 16/4 heads of 256 (one CTA): 158 us. What is left is the
+// softmax warps' chain (read, maximum, exponentials, write). Replacing a quarter of the exponentials by polynomials of ten
 // instructions made it slower (1.08 against 0.97 ms), and so did scores two steps ahead (1.04).
 //
 //   warps 0..3  softmax, rescaling of O, epilogue: one query row per thread
@@ -169,10 +169,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       };
       bool ok = mbar_wait(q_full, 0, p.status, KS_TIMEOUT_FULL) && issue_s(0);
       for (int j = 0; j < n && ok; ++j) {
-        if (j + 1 < n) ok = issue_s(j + 1);
-        if (!ok || !mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL) ||
-            !mbar_wait(&p_full[j & 1], (j >> 1) & 1, p.status, KS_TIMEOUT_FULL))
-          break;
+        // V ahead of the next scores where a CTA has the SM to itself: 160.4 -> 157.9 us at 6,001 tokens of width 256 (two
+        // to an SM: 192.5 -> 193.3 for the packed case above)
+        if constexpr (CTAS == 1) {
+          if (!mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL)) break;
+          if (j + 1 < n) ok = issue_s(j + 1);
+        } else {
+          if (j + 1 < n) ok = issue_s(j + 1);
+          if (ok) ok = mbar_wait(&v_full[j % VS], (j / VS) & 1, p.status, KS_TIMEOUT_FULL);
+        }
+        if (!ok || !mbar_wait(&p_full[j & 1], (j >> 1) & 1, p.status, KS_TIMEOUT_FULL)) break;
         tc_fence_after();
         const uint32_t v = sv0 + (j % VS) * Cfg::KV_BYTES, pa = tmem_base + (j & 1) * BKV;
 #pragma unroll
