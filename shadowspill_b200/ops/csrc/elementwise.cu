@@ -321,13 +321,15 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
     }
     row = list.rows[at];
   }
-  const float wgt = weights ? weights[row] : 1.f;
-  const long long tgt = targets[row];
-  const bool in_vocab = tgt >= 0 && tgt < V;
-  const bool valid = in_vocab && wgt != 0.f;
-  if (!valid && lse_out == nullptr && pa.logp_out == nullptr) {      // nothing of a masked row is asked for
-    if (write_grad) clear();
-    return;
+  // Nothing is asked of a masked row but its gradient, so a row longer than one load per thread is looked at first; its
+  // start is on its way meanwhile. Shorter ones would only wait for their target (300 rows of 1,000: 4.7 -> 5.5 us).
+  if (V > 8 * CE_THREADS && lse_out == nullptr && pa.logp_out == nullptr) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4*>(lr) + threadIdx.x));
+    const long long t = targets[row];
+    if (t < 0 || t >= V || (weights != nullptr && weights[row] == 0.f)) {
+      if (write_grad) clear();
+      return;
+    }
   }
   const uint4* lv = reinterpret_cast<const uint4*>(lr);
   float m = -INFINITY, s = 0.f;
@@ -349,6 +351,12 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
     if (f > m) { s *= __expf(m - f); m = f; }
     s += __expf(f - m);
   }
+  // read again rather than kept: with two registers less for the pass above, 2,048 rows of 128,256 took 271 us, not 255
+  asm volatile("" : "+r"(row));
+  const float wgt = weights ? weights[row] : 1.f;
+  const long long tgt = targets[row];
+  const bool in_vocab = tgt >= 0 && tgt < V;
+  const bool valid = in_vocab && wgt != 0.f;
   const float gm = block_max(m, red);
   s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
   const float gs = block_sum(s, red);
@@ -375,7 +383,11 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
   }
   if (!write_grad) return;
   __syncthreads();
-  const float scale = valid ? -wgt * grad_scale * dl_dlogp : 0.f;
+  if (!valid) {
+    clear();
+    return;
+  }
+  const float scale = -wgt * grad_scale * dl_dlogp;
   uint4* gv = reinterpret_cast<uint4*>(lr);
   for (int c = threadIdx.x; c < nv; c += CE_THREADS) {
     float f[8];

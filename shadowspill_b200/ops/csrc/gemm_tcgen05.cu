@@ -147,6 +147,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int warp = static_cast<int>(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
+  int num_m = (p.M + BM - 1) / BM;
   const int num_n = (p.N + TILE_N - 1) / TILE_N;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -173,8 +174,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   chain_wait();
   chain_release();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  const int rows = p.used == nullptr ? p.M : max(0, min(p.M, *p.used - p.used_from));
-  const int num_m = (rows + BM - 1) / BM;
+  if (p.used != nullptr) num_m = (max(0, min(p.M, *p.used - p.used_from)) + BM - 1) / BM;
   const int num_tiles = num_m * num_n * (p.g.mode == 2 ? p.g.n_experts : 1);
 
   if (warp == 0) {
@@ -373,11 +373,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tmem_ld_wait();
           if (p.c_f32)
             epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C) + w.c_off,
-                                 p.accumulate ? reinterpret_cast<const float*>(p.e.src) + w.c_off : nullptr, p.e.ldsrc,
+                                 p.accumulate, reinterpret_cast<const float*>(p.e.src) + w.c_off, p.e.ldsrc,
                                  p.alpha, p.ldc, row0, p.M, col0, p.N);
           else
             epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C) + w.c_off,
-                                 p.accumulate ? reinterpret_cast<const __nv_bfloat16*>(p.e.src) + w.c_off : nullptr,
+                                 p.accumulate, reinterpret_cast<const __nv_bfloat16*>(p.e.src) + w.c_off,
                                  p.e.ldsrc, p.alpha, p.ldc, row0, p.M, col0, p.N);
         }
       }

@@ -386,11 +386,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           }
           if (p.c_f32)
             epilogue_store_32x32(stage_out, r, reinterpret_cast<float*>(p.C),
-                                 p.accumulate ? reinterpret_cast<const float*>(p.e.src) : nullptr, p.e.ldsrc, p.alpha,
+                                 p.accumulate, reinterpret_cast<const float*>(p.e.src), p.e.ldsrc, p.alpha,
                                  p.ldc, row0, p.M, col0, p.N);
           else
             epilogue_store_32x32(stage_out, r, reinterpret_cast<__nv_bfloat16*>(p.C),
-                                 p.accumulate ? reinterpret_cast<const __nv_bfloat16*>(p.e.src) : nullptr, p.e.ldsrc,
+                                 p.accumulate, reinterpret_cast<const __nv_bfloat16*>(p.e.src), p.e.ldsrc,
                                  p.alpha, p.ldc, row0, p.M, col0, p.N);
         }
       }
